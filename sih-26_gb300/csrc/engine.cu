@@ -105,6 +105,9 @@ template struct DeviceArray<ChunkSeg>;
 template struct DeviceArray<QpChunk>;
 template struct DeviceArray<QpCtl>;
 template struct DeviceArray<QpHist>;
+template struct DeviceArray<SliceItem>;
+template struct DeviceArray<SliceSeg>;
+template struct DeviceArray<unsigned short>;
 
 namespace {
 
@@ -277,9 +280,13 @@ size_t estimate_memory(long long rows, long long cols, long long nnz, int precis
   size_t bytes = 0;
   bytes += (m + 1 + n + 1) * sizeof(int) + 2 * z * sizeof(int);  // CSR + CSC pattern
   bytes += (m + n) * sizeof(int2);                                // tiles (upper bound)
-  bytes += 4 * z * sizeof(double);      // unscaled + scaled values, both layouts
-  bytes += 18 * n * sizeof(double);     // column vectors (see Engine members)
-  bytes += 14 * m * sizeof(double);     // row vectors
+  // The sliced layouts: indices, unscaled and scaled values (an eighth for the slices' padding;
+  // a padded slice has at most 31 empty places per entry of its longest row, and the rows are
+  // dealt by length), and the scaled values in the compressed order.
+  bytes += 2 * (z + z / 8) * (sizeof(int) + 2 * sizeof(double)) + 2 * z * sizeof(double);
+  bytes += 4 * (m + n);  // slice records
+  bytes += 20 * n * sizeof(double);     // column vectors (see Engine members)
+  bytes += 16 * m * sizeof(double);     // row vectors
   if (precision == SANKHYA_GB300_MIXED) {
     bytes += 2 * z * sizeof(float) + (10 * n + 8 * m) * sizeof(float);
   }
@@ -290,6 +297,9 @@ size_t estimate_memory(long long rows, long long cols, long long nnz, int precis
   bytes += static_cast<size_t>(kStepFactorTable) * sizeof(double2);
   return bytes;
 }
+
+// Power steps of the spectral-norm estimate (src/la/scaling.cpp:161).
+constexpr int kPowerSteps = 30;
 
 Engine::Engine(int device) : device_(device) {
   int count = 0;
@@ -314,7 +324,7 @@ Engine::Engine(int device) : device_(device) {
   SGB_CUDA(cudaMemset(ctl_.ptr, 0, sizeof(Ctl)));
   ctl_mixed_.allocate(1);
   SGB_CUDA(cudaMemset(ctl_mixed_.ptr, 0, sizeof(Ctl)));
-  if (!configure_tile_kernels() || !configure_mixed_kernels()) {
+  if (!configure_fp64_kernels() || !configure_mixed_kernels()) {
     throw EngineError{SANKHYA_GB300_ERROR_DEVICE,
                       format("device %d refused the kernels' shared-memory limits", device)};
   }
@@ -543,38 +553,21 @@ void Engine::load(const sankhya_gb300_lp& lp) {
       rval[slot] = lp.values[k];
     }
   }
-  // Two tile layouts per pattern. FP64 kernels run one row per thread: GB300's FP64 pipe
-  // charges per warp instruction, so lanes that sit out an epilogue or add up a row that is
-  // split across lanes cost as much as working ones. The FP32 kernels are bound by memory
-  // latency instead and split rows over `lanes` threads so every thread issues gathers.
-  // The chunking of long rows does not depend on the lanes, so both layouts share it.
-  std::vector<Tile> ctiles, rtiles, ctiles_f, rtiles_f;
+  // The FP32 evaluation kernels' tiles: bound by memory latency, they split rows over `lanes`
+  // threads so every thread issues gathers.
+  std::vector<Tile> ctiles_f, rtiles_f;
   std::vector<LongRow> clongs, rlongs;
-  int unused_chunks = 0;
-  lanes_csc_ = 1;
-  lanes_csr_ = 1;
   lanes_csc_f_ = wide_lanes(n > 0 ? static_cast<double>(nnz) / n : 1.0, kWideThreads);
   lanes_csr_f_ = wide_lanes(m > 0 ? static_cast<double>(nnz) / m : 1.0, kWideThreads);
-  build_tiles(cptr, n, lanes_csc_, kTileThreads, &ctiles, &clongs, &nchunks_csc_);
-  build_tiles(rptr, m, lanes_csr_, kTileThreads, &rtiles, &rlongs, &nchunks_csr_);
-  {
-    std::vector<LongRow> same;
-    build_tiles(cptr, n, lanes_csc_f_, kWideThreads, &ctiles_f, &same, &unused_chunks);
-    build_tiles(rptr, m, lanes_csr_f_, kWideThreads, &rtiles_f, &same, &unused_chunks);
-  }
-  ntiles_csc_ = static_cast<int>(ctiles.size());
-  ntiles_csr_ = static_cast<int>(rtiles.size());
+  build_tiles(cptr, n, lanes_csc_f_, kWideThreads, &ctiles_f, &clongs, &nchunks_csc_);
+  build_tiles(rptr, m, lanes_csr_f_, kWideThreads, &rtiles_f, &rlongs, &nchunks_csr_);
   ntiles_csc_f_ = static_cast<int>(ctiles_f.size());
   ntiles_csr_f_ = static_cast<int>(rtiles_f.size());
   nlong_csc_ = static_cast<int>(clongs.size());
   nlong_csr_ = static_cast<int>(rlongs.size());
-  const int resident = tile_blocks_per_sm() * num_sms_;
-  grid_csc_ = std::max(1, std::min(ntiles_csc_, resident));
-  grid_csr_ = std::max(1, std::min(ntiles_csr_, resident));
   const int resident_f = mixed_blocks_per_sm() * num_sms_;
   grid_csc_f_ = std::max(1, std::min(ntiles_csc_f_, resident_f));
   grid_csr_f_ = std::max(1, std::min(ntiles_csr_f_, resident_f));
-  int grid_c = std::max(grid_csc_, grid_csc_f_), grid_r = std::max(grid_csr_, grid_csr_f_);
 
   // Minimise-space cost and the norms of src/pdhg/pdhg.cpp:95-111, summed in the
   // reference's order on the host (they are computed once).
@@ -604,43 +597,12 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   // windows hold any entry, so tests run the split form.
   int cap = -1;
   if (const char* env = std::getenv("SANKHYA_GB300_WINDOW_CAP")) cap = std::max(0, std::atoi(env)) & ~3;
-  const auto make_layout = [&](StepLayout& L, const std::vector<Tile>& tiles, const int* idx,
-                               int extent, int pass) {
-    int wmax = fp64_window_capacity(pass);
-    if (cap >= 0) wmax = std::min(wmax, cap);
-    std::vector<int> tile_win;
-    std::vector<int2> windows;
-    long long covered = build_windows(tiles, idx, extent, wmax, &tile_win, &windows);
-    // A window leaves room for one block per SM, whose few warps cannot hide the latency of
-    // the gathers that miss it; below kMinStagedShare the unstaged form (several blocks per
-    // SM, every gather from L2) is faster, so the layout keeps no window. A fixed rule, not a
-    // timing: the grid decides the order of the block partial sums, so it must not vary from
-    // run to run.
-    // (A capacity set through SANKHYA_GB300_WINDOW_CAP keeps its windows whatever their
-    // share, so tests can run the partly staged form.)
-    constexpr double kMinStagedShare = 0.95;
-    if (cap < 0 && nnz > 0 &&
-        static_cast<double>(covered) < kMinStagedShare * static_cast<double>(nnz)) {
-      tile_win.assign(tile_win.size(), -1);
-      windows.clear();
-      covered = 0;
-    }
-    L.staged = nnz > 0 ? static_cast<double>(covered) / static_cast<double>(nnz) : 0.0;
-    L.nwindows = static_cast<int>(windows.size());
-    L.wmax = 0;
-    for (const int2& w : windows) L.wmax = std::max(L.wmax, w.y);
-    L.smem = fp64_step_smem(pass, L.wmax);
-    const int per_sm = fp64_step_blocks_per_sm(pass, L.smem);
-    L.grid = std::max(1, std::min(static_cast<int>(tiles.size()), per_sm * num_sms_));
-    L.tile_win.upload(tile_win.data(), tile_win.size(), s);
-    L.windows.upload(windows.data(), windows.size(), s);
-  };
-  make_layout(step_csc_, ctiles, lp.row_index, m, 0);
-  make_layout(step_csr_, rtiles, ridx.data(), n, 1);
+  plan_sliced(sl_csc_, cptr, lp.row_index, n, m, 0, cap);
+  plan_sliced(sl_csr_, rptr, ridx.data(), m, n, 1, cap);
   plan_layout(ck_csc_f_, cptr, lp.row_index, n, m, 0, cap);
   plan_layout(ck_csr_f_, rptr, ridx.data(), m, n, 1, cap);
-  grid_c = std::max({grid_c, step_csc_.grid, ck_csc_f_.grid});
-  grid_r = std::max({grid_r, step_csr_.grid, ck_csr_f_.grid});
+  const int grid_c = std::max({sl_csc_.view.grid, grid_csc_f_, ck_csc_f_.grid});
+  const int grid_r = std::max({sl_csr_.view.grid, grid_csr_f_, ck_csr_f_.grid});
 
   // Row pointers are staged per tile in 16-byte units too: kPad entries of padding.
   csc_ptr_.upload_padded(cptr.data(), cptr.size(), kPad, s);
@@ -648,13 +610,15 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   // Index and value arrays carry kPad zero entries: a tile copy widened to 16-byte
   // boundaries may read up to 3 entries past the last nonzero.
   csc_idx_.upload_padded(lp.row_index, z, kPad, s);
-  csc_raw_.upload_padded(lp.values, z, kPad, s);
   csr_idx_.upload_padded(ridx.data(), z, kPad, s);
-  csr_raw_.upload_padded(rval.data(), z, kPad, s);
-  csc_s_.allocate_padded(z, kPad, s);
-  csr_s_.allocate_padded(z, kPad, s);
-  csc_tiles_.upload(ctiles.data(), ctiles.size(), s);
-  csr_tiles_.upload(rtiles.data(), rtiles.size(), s);
+  // The compressed values are only the source of the sliced copies: the array that later holds
+  // the scaled values in this order carries them.
+  csc_s_.upload_padded(lp.values, z, kPad, s);
+  csr_s_.upload_padded(rval.data(), z, kPad, s);
+  launch_slice_fill(sl_csc_.view, csc_ptr_.ptr, csc_idx_.ptr, csc_s_.ptr, sl_csc_.idx.ptr,
+                    sl_csc_.raw.ptr, s);
+  launch_slice_fill(sl_csr_.view, csr_ptr_.ptr, csr_idx_.ptr, csr_s_.ptr, sl_csr_.idx.ptr,
+                    sl_csr_.raw.ptr, s);
   csc_tiles_f_.upload(ctiles_f.data(), ctiles_f.size(), s);
   csr_tiles_f_.upload(rtiles_f.data(), rtiles_f.size(), s);
   csc_longs_.upload(clongs.data(), clongs.size(), s);
@@ -668,12 +632,12 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   // Every per-row and per-column vector carries kPad elements of padding: the step passes
   // stage a tile's operand slices widened to 4-element bounds, and their windows of the
   // gathered vector may end up to 3 elements past the last one.
-  for (DeviceArray<double>* a : {&cs_, &ls_, &us_, &dc_, &col_acc_, &x0_, &x1_, &x_sum_, &x_rst_,
+  for (DeviceArray<double>* a : {&cs_, &ls_, &us_, &dc_, &col_factor_[0], &col_factor_[1], &x0_, &x1_, &x_sum_, &x_rst_,
                                  &xu0_, &xu1_, &reduced_, &best_x_, &power_v_}) {
     a->allocate(static_cast<size_t>(n) + kPad);
   }
   xd_.allocate(static_cast<size_t>(n) + kPad);
-  for (DeviceArray<double>* a : {&rls_, &rus_, &dr_, &row_acc_, &y0_, &y1_, &y_sum_, &y_rst_,
+  for (DeviceArray<double>* a : {&rls_, &rus_, &dr_, &row_factor_[0], &row_factor_[1], &y0_, &y1_, &y_sum_, &y_rst_,
                                  &yu0_, &yu1_, &best_y_, &power_av_}) {
     a->allocate(static_cast<size_t>(m) + kPad);
   }
@@ -683,13 +647,16 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   part_rows0_.allocate(static_cast<size_t>(grid_r) * kEvalRowSlots);
   part_cols_.allocate(static_cast<size_t>(grid_c + 1) * kEvalColSlots);
   part_rows1_.allocate(static_cast<size_t>(grid_r) * kEvalRowSlots);
+  // Piece partials of long rows (the sliced layouts and the FP32 tiles cut them alike).
   chunk_primal_.allocate(static_cast<size_t>(nchunks_csc_) + 1);
   chunk_dual_.allocate(2 * static_cast<size_t>(nchunks_csr_) + 2);
   chunk_cols_.allocate(2 * static_cast<size_t>(nchunks_csc_) + 2);
   chunk_rows_.allocate(2 * static_cast<size_t>(nchunks_csr_) + 2);
-  chunk_spmv_.allocate(static_cast<size_t>(std::max(nchunks_csc_, nchunks_csr_)) + 1);
+  chunk_spmv_.allocate(
+      static_cast<size_t>(std::max(sl_csc_.view.nchunks, sl_csr_.view.nchunks)) + 1);
   scalars_.allocate(static_cast<size_t>(pgrid) * 2 + 16);
-  power_norms_.allocate(64);
+  power_norms_.allocate(2 * (kPowerSteps + 1));
+  minmax_.allocate(2 * static_cast<size_t>(scale_blocks(sl_csc_.view)) + 2);
   if (step_factors_.ptr == nullptr) {
     step_factors_.allocate(static_cast<size_t>(kStepFactorTable));
     launch_step_factors(step_factors_.ptr, kStepFactorTable, s);
@@ -699,6 +666,53 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   SGB_CUDA(cudaStreamSynchronize(s));
   fill_buffers();
   loaded_ = true;
+}
+
+// One FP64 sliced layout: planned on the host (plan_slices) and uploaded; its indices and values
+// are filled on the device from the compressed layout. Windows are kept where they hold at
+// least 95% of the entries: a gather that misses stalls its warp on L2, and a block without a
+// window leaves its shared memory to L1, which then serves the gathers better. A capacity set
+// through SANKHYA_GB300_WINDOW_CAP (window_cap >= 0) keeps its windows whatever their share.
+// A fixed rule, not a timing: the blocks decide the order of the partial sums, so they must not
+// vary from run to run.
+void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* lidx, int lines,
+                         int extent, int pass, int window_cap) {
+  cudaStream_t s = stream_;
+  int wmax = fp64_window_capacity(pass);
+  if (window_cap >= 0) wmax = std::min(wmax, window_cap);
+  const SlicePlan P = plan_slices(lptr, lidx, lines, extent, wmax, window_cap >= 0 ? 0.0 : 0.95,
+                                  num_sms_, pass == 0 ? 1 : 2);
+  D.meta.upload(P.meta.data(), P.meta.size(), s);
+  D.base.upload(P.base.data(), P.base.size(), s);
+  D.items.upload(P.items.data(), P.items.size(), s);
+  D.longs.upload(P.longs.data(), P.longs.size(), s);
+  D.segs.upload(P.segs.data(), P.segs.size(), s);
+  D.seg_start.upload(P.seg_start.data(), P.seg_start.size(), s);
+  const size_t e = static_cast<size_t>(P.entries);
+  D.idx.allocate(e);
+  D.raw.allocate(e);
+  D.scaled.allocate(e);
+  SGB_CUDA(cudaStreamSynchronize(s));  // the plan's arrays end here
+  D.staged = P.staged;
+  SliceSet& S = D.view;
+  S = SliceSet{};
+  S.meta = D.meta.ptr;
+  S.base = D.base.ptr;
+  S.idx = D.idx.ptr;
+  S.val = D.scaled.ptr;
+  S.items = D.items.ptr;
+  S.longs = D.longs.ptr;
+  S.segs = D.segs.ptr;
+  S.seg_start = D.seg_start.ptr;
+  S.long_base = P.long_base;
+  S.nslices = P.nslices;
+  S.nitems = static_cast<int>(P.items.size());
+  S.nlong = static_cast<int>(P.longs.size());
+  S.nchunks = P.nchunks;
+  S.nrows = lines;
+  S.wmax = P.wmax;
+  S.grid = P.grid;
+  S.threads = P.threads;
 }
 
 // One FP32 step pass's chunk layout: planned on the host (plan_chunks), uploaded, and its
@@ -783,16 +797,10 @@ ChunkSet<float> Engine::chunk_set(const ChunkDev& D, const int* full_ptr, const 
 }
 
 void Engine::fill_buffers() {
-  const TileSet<double> csc{csc_ptr_.ptr,   csc_idx_.ptr, csc_s_.ptr,   csc_tiles_.ptr,
-                            csc_longs_.ptr, ntiles_csc_,  nlong_csc_,   nchunks_csc_,
-                            n_,             lanes_csc_};
-  const TileSet<double> csr{csr_ptr_.ptr,   csr_idx_.ptr, csr_s_.ptr,   csr_tiles_.ptr,
-                            csr_longs_.ptr, ntiles_csr_,  nlong_csr_,   nchunks_csr_,
-                            m_,             lanes_csr_};
   StepBuffers& b = step_;
   b.ctl = ctl_.ptr;
-  b.csc = csc;
-  b.csr = csr;
+  b.csc = sl_csc_.view;
+  b.csr = sl_csr_.view;
   b.x[0] = x0_.ptr;
   b.x[1] = x1_.ptr;
   b.y[0] = y0_.ptr;
@@ -811,23 +819,14 @@ void Engine::fill_buffers() {
   b.part_dual = part_dual_.ptr;
   b.chunk_primal = chunk_primal_.ptr;
   b.chunk_dual = chunk_dual_.ptr;
-  b.csc.tile_win = step_csc_.tile_win.ptr;
-  b.csc.windows = step_csc_.windows.ptr;
-  b.csc.wmax = step_csc_.wmax;
-  b.csr.tile_win = step_csr_.tile_win.ptr;
-  b.csr.windows = step_csr_.windows.ptr;
-  b.csr.wmax = step_csr_.wmax;
-  b.grid_primal = step_csc_.grid;
-  b.grid_dual = step_csr_.grid;
-  b.smem_primal = step_csc_.smem;
-  b.smem_dual = step_csr_.smem;
+  b.grid_primal = b.csc.grid;
 
   EvalBuffers& e = eval_;
   e.ctl = ctl_.ptr;
-  e.csc = csc;
-  e.csc.val = csc_raw_.ptr;
-  e.csr = csr;
-  e.csr.val = csr_raw_.ptr;
+  e.csc = sl_csc_.view;
+  e.csc.val = sl_csc_.raw.ptr;
+  e.csr = sl_csr_.view;
+  e.csr.val = sl_csr_.raw.ptr;
   e.x[0] = x0_.ptr;
   e.x[1] = x1_.ptr;
   e.y[0] = y0_.ptr;
@@ -859,8 +858,8 @@ void Engine::fill_buffers() {
   e.part_rows0 = part_rows0_.ptr;
   e.part_cols = part_cols_.ptr;
   e.part_rows1 = part_rows1_.ptr;
-  e.grid_rows = grid_csr_;
-  e.grid_cols = grid_csc_;
+  e.grid_rows = e.csr.grid;
+  e.grid_cols = e.csc.grid;
   e.m = m_;
   e.n = n_;
 }
@@ -868,21 +867,36 @@ void Engine::fill_buffers() {
 void Engine::precondition(long long seed) {
   (void)seed;
   cudaStream_t s = stream_;
-  const size_t nb = static_cast<size_t>(nnz_) * sizeof(double);
-  if (nnz_ > 0) {
-    SGB_CUDA(cudaMemcpyAsync(csc_s_.ptr, csc_raw_.ptr, nb, cudaMemcpyDeviceToDevice, s));
-    SGB_CUDA(cudaMemcpyAsync(csr_s_.ptr, csr_raw_.ptr, nb, cudaMemcpyDeviceToDevice, s));
-  }
   launch_fill(dr_.ptr, m_, 1.0, s);
   launch_fill(dc_.ptr, n_, 1.0, s);
-  for (int pass = 0; pass < 11; ++pass) {  // 10 Ruiz rounds, then Pock-Chambolle
-    launch_scaling_round(m_, n_, step_.csr, step_.csc, csr_s_.ptr, csc_s_.ptr, row_acc_.ptr,
-                         col_acc_.ptr, dr_.ptr, dc_.ptr, pass == 10 ? 1 : 0, s);
+  ScalingBuffers b{};
+  b.csr = sl_csr_.view;
+  b.csc = sl_csc_.view;
+  b.csr_raw = sl_csr_.raw.ptr;
+  b.csc_raw = sl_csc_.raw.ptr;
+  b.csr_val = sl_csr_.scaled.ptr;
+  b.csc_val = sl_csc_.scaled.ptr;
+  for (int k = 0; k < 2; ++k) {
+    b.row_factor[k] = row_factor_[k].ptr;
+    b.col_factor[k] = col_factor_[k].ptr;
   }
+  b.dr = dr_.ptr;
+  b.dc = dc_.ptr;
+  b.minmax = minmax_.ptr;
+  b.minmax_out = minmax_.ptr + 2 * scale_blocks(b.csc);
+  b.nnz = nnz_;
+  launch_scaling(b, s);
   launch_scale_vectors(m_, n_, cost_.ptr, l_.ptr, u_.ptr, rl_.ptr, ru_.ptr, dr_.ptr, dc_.ptr,
                        cs_.ptr, ls_.ptr, us_.ptr, rls_.ptr, rus_.ptr, s);
   SGB_CUDA(cudaGetLastError());
   scaled_ = true;
+}
+
+// The scaled values in the compressed layouts' order, for scaling() and the FP32 copies.
+void Engine::unslice_scaled() {
+  launch_slice_unfill(sl_csc_.view, csc_ptr_.ptr, sl_csc_.scaled.ptr, csc_s_.ptr, stream_);
+  launch_slice_unfill(sl_csr_.view, csr_ptr_.ptr, sl_csr_.scaled.ptr, csr_s_.ptr, stream_);
+  SGB_CUDA(cudaGetLastError());
 }
 
 // The FP32 scaled values of the split chunk layouts' main and outer parts, gathered from the
@@ -910,27 +924,26 @@ double Engine::power_iteration(long long seed) {
   for (double& value : v) value = spread(rng);
   SGB_CUDA(cudaMemcpyAsync(power_v_.ptr, v.data(), v.size() * sizeof(double),
                            cudaMemcpyHostToDevice, s));
-  const int iterations = 30;
   const int grid = std::min(num_sms_ * 4, std::max(1, (n_ + 255) / 256));
-  double* norms = power_norms_.ptr;  // [2*step] = length^2, [2*step+1] = next
-  for (int step = 0; step < iterations; ++step) {
-    launch_sumsq(power_v_.ptr, n_, scalars_.ptr, norms + 2 * step, tickets_.ptr, s, grid);
-    launch_scale_div(power_v_.ptr, n_, norms + 2 * step, s);
-    launch_spmv(step_.csr, power_v_.ptr, power_av_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1,
-                product_error(), s, grid_csr_);
-    launch_spmv(step_.csc, power_av_.ptr, power_v_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1,
-                product_error(), s, grid_csc_);
-    launch_sumsq(power_v_.ptr, n_, scalars_.ptr, norms + 2 * step + 1, tickets_.ptr, s, grid);
+  // norms[2 k] = |v_k|^2 and norms[2 k + 1] = 1 / |v_k|, where v_{k+1} = A' (A v_k / |v_k|): the
+  // start is normalised where its product is formed, one multiplication per row.
+  double* norms = power_norms_.ptr;
+  launch_sumsq(power_v_.ptr, n_, scalars_.ptr, norms, tickets_.ptr, s, grid);
+  for (int step = 0; step < kPowerSteps; ++step) {
+    launch_spmv_scaled(step_.csr, power_v_.ptr, power_av_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1,
+                       norms + 2 * step + 1, s);
+    launch_spmv_norm(step_.csc, power_av_.ptr, power_v_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1,
+                     scalars_.ptr, norms + 2 * step + 2, s);
   }
   SGB_CUDA(cudaGetLastError());
-  std::vector<double> host(2 * iterations);
+  std::vector<double> host(2 * (kPowerSteps + 1));
   SGB_CUDA(cudaMemcpyAsync(host.data(), norms, host.size() * sizeof(double),
                            cudaMemcpyDeviceToHost, s));
-  check_product_error();
+  SGB_CUDA(cudaStreamSynchronize(s));
   double norm = 0.0;
-  for (int step = 0; step < iterations; ++step) {
+  for (int step = 0; step < kPowerSteps; ++step) {
     if (std::sqrt(host[2 * step]) == 0.0) return 1.0;
-    norm = std::sqrt(std::sqrt(host[2 * step + 1]));
+    norm = std::sqrt(std::sqrt(host[2 * step + 2]));
   }
   return norm > 0.0 ? norm * 1.01 : 1.0;
 }
@@ -942,6 +955,7 @@ void Engine::scaling(long long seed, double* row_scale, double* col_scale, doubl
   precondition(seed);
   const double norm = power_iteration(seed);
   cudaStream_t s = stream_;
+  if (scaled_values) unslice_scaled();
   if (row_scale) SGB_CUDA(cudaMemcpyAsync(row_scale, dr_.ptr, m_ * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (col_scale) SGB_CUDA(cudaMemcpyAsync(col_scale, dc_.ptr, n_ * sizeof(double), cudaMemcpyDeviceToHost, s));
   if (scaled_values && nnz_ > 0) {
@@ -964,35 +978,14 @@ void Engine::spmv(int op, int scaled, const double* in, double* out) {
   DeviceArray<double> din, dout;
   din.upload(in, static_cast<size_t>(in_len), s);
   dout.allocate(static_cast<size_t>(out_len));
-  TileSet<double> a = op == 0 ? step_.csr : step_.csc;
-  if (!scaled) a.val = op == 0 ? csr_raw_.ptr : csc_raw_.ptr;
-  launch_spmv(a, din.ptr, dout.ptr, chunk_spmv_.ptr, tickets_.ptr + 1, product_error(), s,
-              op == 0 ? grid_csr_ : grid_csc_);
+  SliceSet a = op == 0 ? step_.csr : step_.csc;
+  if (!scaled) a.val = op == 0 ? sl_csr_.raw.ptr : sl_csc_.raw.ptr;
+  launch_spmv(a, din.ptr, dout.ptr, chunk_spmv_.ptr, tickets_.ptr + 1, s);
   SGB_CUDA(cudaGetLastError());
   if (out_len > 0) {
     SGB_CUDA(cudaMemcpyAsync(out, dout.ptr, out_len * sizeof(double), cudaMemcpyDeviceToHost, s));
   }
-  check_product_error();
-}
-
-// The error word of the tile products (k_spmv), read at a synchronising point: it waits for
-// the stream, and a product whose bounded wait gave up since the last check makes the call
-// fail with a device error (the word is cleared for the next one).
-void Engine::check_product_error() {
-  unsigned int word = 0;
-  SGB_CUDA(cudaMemcpyAsync(&word, product_error(), sizeof(word), cudaMemcpyDeviceToHost,
-                           stream_));
-  SGB_CUDA(cudaStreamSynchronize(stream_));
-  if (product_error_status(word) != SANKHYA_GB300_OK) {
-    SGB_CUDA(cudaMemsetAsync(product_error(), 0, sizeof(word), stream_));
-    SGB_CUDA(cudaStreamSynchronize(stream_));
-    throw EngineError{product_error_status(word), "a sparse product's tile copy did not complete "
-                                                  "in time; its result was not used"};
-  }
-}
-
-int product_error_status(unsigned int word) {
-  return word == 0 ? SANKHYA_GB300_OK : SANKHYA_GB300_ERROR_DEVICE;
+  SGB_CUDA(cudaStreamSynchronize(s));
 }
 
 static_assert(kNoAllocMaxChunks == SANKHYA_GB300_NOALLOC_MAX_CHUNKS,
@@ -1012,7 +1005,7 @@ void Engine::spmv_noalloc(int op, int scaled, const double* in, double* out,
   if ((in_len > 0 && in == nullptr) || (out_len > 0 && out == nullptr)) {
     throw EngineError{SANKHYA_GB300_ERROR_ARGUMENT, "null device buffer"};
   }
-  TileSet<double> a = op == 0 ? step_.csr : step_.csc;
+  SliceSet a = op == 0 ? step_.csr : step_.csc;
   if (a.nchunks > kNoAllocMaxChunks) {
     throw EngineError{
         SANKHYA_GB300_ERROR_ARGUMENT,
@@ -1024,10 +1017,9 @@ void Engine::spmv_noalloc(int op, int scaled, const double* in, double* out,
   cudaStream_t s = stream != nullptr ? stream : stream_;
   double* chunks = nullptr;
   unsigned int* ticket = nullptr;
-  unsigned int* error = nullptr;
-  SGB_CUDA(noalloc_scratch(device_, s, &chunks, &ticket, &error));
-  if (!scaled) a.val = op == 0 ? csr_raw_.ptr : csc_raw_.ptr;
-  launch_spmv(a, in, out, chunks, ticket, error, s, op == 0 ? grid_csr_ : grid_csc_);
+  SGB_CUDA(noalloc_scratch(device_, s, &chunks, &ticket));
+  if (!scaled) a.val = op == 0 ? sl_csr_.raw.ptr : sl_csc_.raw.ptr;
+  launch_spmv(a, in, out, chunks, ticket, s);
   SGB_CUDA(cudaGetLastError());
 }
 
@@ -1132,11 +1124,8 @@ void Engine::setup(const sankhya_gb300_params& p, sankhya_gb300_result* r, doubl
   cudaStream_t s = stream_;
   precondition(p.random_seed);
   *norm = power_iteration(p.random_seed);
-  const int grid = std::min(num_sms_ * 4, std::max(1, static_cast<int>((nnz_ + 255) / 256)));
-  launch_abs_minmax(csc_s_.ptr, static_cast<int>(nnz_), scalars_.ptr,
-                    scalars_.ptr + 2 * grid + 2, tickets_.ptr, s, grid);
   double mm[2] = {0.0, 0.0};
-  SGB_CUDA(cudaMemcpyAsync(mm, scalars_.ptr + 2 * grid + 2, 2 * sizeof(double),
+  SGB_CUDA(cudaMemcpyAsync(mm, minmax_.ptr + 2 * scale_blocks(sl_csc_.view), 2 * sizeof(double),
                            cudaMemcpyDeviceToHost, s));
   SGB_CUDA(cudaStreamSynchronize(s));
   r->scaled_max_abs = mm[0];
@@ -1252,8 +1241,8 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   launches_ = launches_setup + (kernel_launch_count() - count_after_capture) +
               graphs_launched_ * graph_kernel_launches(graph_steps_);
   r->kernel_launches = launches_;
-  r->staged_fraction[0] = step_csc_.staged;
-  r->staged_fraction[1] = step_csr_.staged;
+  r->staged_fraction[0] = sl_csc_.staged;
+  r->staged_fraction[1] = sl_csr_.staged;
   if (c.error) {
     throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "a tile copy did not complete in time"};
   }
@@ -1273,6 +1262,7 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
   double norm = 1.0;
   setup(p, r, &norm);
   // FP32 copies of the scaled values; the FP64 anchor starts at proj(0), y = 0.
+  unslice_scaled();
   launch_to_float(csc_s_.ptr, csc_f_.ptr, nnz_, s);
   launch_to_float(csr_s_.ptr, csr_f_.ptr, nnz_, s);
   launch_to_float(cs_.ptr, csf_.ptr, n_, s);
@@ -1381,15 +1371,13 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
   };
   for (;; ++rounds) {
     // Anchor residuals in FP64, then the scales of this round's correction problem.
-    launch_spmv(step_.csr, anchor_x_.ptr, ax64_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1,
-                product_error(), s, grid_csr_);
-    launch_spmv(step_.csc, anchor_y_.ptr, aty64_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1,
-                product_error(), s, grid_csc_);
+    launch_spmv(step_.csr, anchor_x_.ptr, ax64_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1, s);
+    launch_spmv(step_.csc, anchor_y_.ptr, aty64_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1, s);
     launch_round_measure(rb, s);
     extra_launches_ += 3;
     double out[3];
     SGB_CUDA(cudaMemcpyAsync(out, rb.out, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    check_product_error();
+    SGB_CUDA(cudaStreamSynchronize(s));
     // 1 / residual, never below 1, at most 1e3 times the previous scale and 1e15 overall: an
     // anchor whose residual is exactly zero must not push the FP32 data out of range.
     const auto scale = [&](double residual, double prev) {

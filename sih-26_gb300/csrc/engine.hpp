@@ -86,9 +86,6 @@ class Engine {
   void run_graphs(const sankhya_gb300_params& p, double t0, cudaGraphExec_t* graphs,
                   Ctl* snapshot, bool forward_log, long long iteration_offset, int* stop_status);
   void final_evaluation();
-  // The tile products' error word (tickets_ slot 3, zero after load) and its check.
-  unsigned int* product_error() const { return tickets_.ptr + 3; }
-  void check_product_error();
   void setup(const sankhya_gb300_params& p, sankhya_gb300_result* r, double* norm);
   void solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, double t0);
   void solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r, double t0);
@@ -107,30 +104,29 @@ class Engine {
   long long nnz_ = 0;
   double sense_ = 1.0, offset_ = 0.0;
   double bound_norm_ = 0.0, cost_norm_ = 0.0;
-  int ntiles_csr_ = 0, ntiles_csc_ = 0;
   int nlong_csr_ = 0, nlong_csc_ = 0;
   int nchunks_csr_ = 0, nchunks_csc_ = 0;
-  int lanes_csr_ = 1, lanes_csc_ = 1;
-  int grid_csr_ = 1, grid_csc_ = 1;
-  // The FP32 evaluation kernels' tile layout (same chunks of long rows, `lanes` threads per
-  // row).
+  // The FP32 evaluation kernels' tile layout (`lanes` threads per row).
   int ntiles_csr_f_ = 0, ntiles_csc_f_ = 0;
   int lanes_csr_f_ = 1, lanes_csc_f_ = 1;
   int grid_csr_f_ = 1, grid_csc_f_ = 1;
   DeviceArray<Tile> csc_tiles_f_, csr_tiles_f_;
-  // The FP64 step passes' gathered-vector windows per layout (CSC / CSR): tile -> window
-  // id, the {lo, len} list, the capacity, and the grid and dynamic shared memory of the step
-  // kernel that stages them.
-  struct StepLayout {
-    DeviceArray<int> tile_win;
-    DeviceArray<int2> windows;
-    int wmax = 0;
-    int nwindows = 0;
-    int grid = 1;
-    int smem = 0;
+  // The FP64 passes' sliced layouts (slices.cuh) of A by columns and by rows, with the values
+  // unscaled (evaluation) and scaled (iterations).
+  struct SliceDev {
+    DeviceArray<unsigned short> meta;
+    DeviceArray<unsigned int> base;
+    DeviceArray<int> idx, seg_start;
+    DeviceArray<double> raw, scaled;
+    DeviceArray<SliceItem> items;
+    DeviceArray<LongRow> longs;
+    DeviceArray<SliceSeg> segs;
+    SliceSet view{};      // val = the scaled values
     double staged = 0.0;  // share of the nonzeros gathered from a staged window
   };
-  StepLayout step_csc_, step_csr_;
+  SliceDev sl_csc_, sl_csr_;
+  void plan_sliced(SliceDev& D, const std::vector<int>& ptr, const int* idx, int lines,
+                   int extent, int pass, int window_cap);
   // The FP32 step passes' chunk layouts (chunks.cuh): CSC (column pass) and CSR (row pass).
   // A split layout owns its main and outer index arrays (and the maps from their entries to
   // the full layout's, through which each solve fills their values); otherwise it reads the
@@ -159,16 +155,18 @@ class Engine {
 
   // Pattern (shared by scaled and unscaled values).
   DeviceArray<int> csc_ptr_, csc_idx_, csr_ptr_, csr_idx_;
-  DeviceArray<Tile> csc_tiles_, csr_tiles_;
   DeviceArray<LongRow> csc_longs_, csr_longs_;
-  // Values: unscaled (evaluation) and scaled (iterations), both layouts.
-  DeviceArray<double> csc_raw_, csr_raw_, csc_s_, csr_s_;
+  // Scaled values in the compressed layouts' order (scaling() and the mixed method's FP32
+  // copies), allocated and filled when they are asked for.
+  DeviceArray<double> csc_s_, csr_s_;
+  void unslice_scaled();
   // Unscaled vectors.
   DeviceArray<double> cost_, col_cost_, l_, u_, rl_, ru_;
   // The step-size factors for iteration counts below kStepFactorTable (filled once).
   DeviceArray<double2> step_factors_;
   // Scaled vectors and scaling.
-  DeviceArray<double> cs_, ls_, us_, rls_, rus_, dr_, dc_, row_acc_, col_acc_;
+  DeviceArray<double> cs_, ls_, us_, rls_, rus_, dr_, dc_;
+  DeviceArray<double> row_factor_[2], col_factor_[2], minmax_;
   // Iterates.
   DeviceArray<double> x0_, x1_, y0_, y1_, x_sum_, y_sum_, x_rst_, y_rst_;
   DeviceArray<double> xu0_, xu1_, yu0_, yu1_, reduced_, best_x_, best_y_;
@@ -210,6 +208,22 @@ class Engine {
   long long extra_launches_ = 0;
 };
 
+// The sliced layout of one matrix layout (layout.cu): windows of at most `wmax` elements are
+// kept where they hold at least `window_min` of the entries; at most `sms` blocks.
+struct SlicePlan {
+  int nslices = 0, nchunks = 0, wmax = 0, grid = 1, threads = 128;
+  long long long_base = 0, entries = 0;  // first entry of the long region; entries stored
+  double staged = 0.0;
+  std::vector<unsigned short> meta;
+  std::vector<unsigned int> base;
+  std::vector<SliceItem> items;
+  std::vector<LongRow> longs;
+  std::vector<SliceSeg> segs;
+  std::vector<int> seg_start;
+};
+SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, int extent, int wmax,
+                      double window_min, int sms, int np);
+
 size_t estimate_memory(long long rows, long long cols, long long nnz, int precision);
 
 // The step passes' chunk layout of one matrix layout (layout.cu): `ptr` / `idx` its lines
@@ -232,9 +246,6 @@ struct ChunkPlan {
 ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, int extent, int cap,
                       int wmax, int grid, int elem_bytes, double split_min, double full_min,
                       int outer_round_cap);
-
-// The status a tile product's error word maps to: 0 = ok, otherwise a device error.
-int product_error_status(unsigned int word);
 
 // Throws EngineError (ARGUMENT / MODEL) when an LP is malformed.
 void validate_lp(const sankhya_gb300_lp& lp);

@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "chunks.cuh"
+#include "slices.cuh"
 #include "tiles.cuh"
 
 namespace sgb {
@@ -95,7 +96,7 @@ constexpr int kEvalRowSlots = 8;
 
 struct StepBuffers {
   Ctl* ctl;
-  TileSet<double> csc, csr;  // scaled
+  SliceSet csc, csr;  // scaled
   double* x[2];
   double* y[2];
   double* x_sum;
@@ -108,8 +109,7 @@ struct StepBuffers {
   double* part_dual;     // [grid_dual * 2]
   double* chunk_primal;  // [csc.nchunks]
   double* chunk_dual;    // [csr.nchunks * 2]
-  int grid_primal, grid_dual;
-  int smem_primal, smem_dual;  // dynamic shared memory: pipeline + staged window
+  int grid_primal;
   // The step-size factors by iteration count (decisions.cuh, step_factors).
   const double2* step_factors;
   long long step_factors_n;
@@ -117,7 +117,7 @@ struct StepBuffers {
 
 struct EvalBuffers {
   Ctl* ctl;
-  TileSet<double> csc, csr;  // UNSCALED values
+  SliceSet csc, csr;  // UNSCALED values
   const double* x[2];
   const double* y[2];
   double* x_sum;
@@ -163,49 +163,60 @@ long long kernel_launch_count();
 void launch_evaluation(const EvalBuffers& e, cudaStream_t s);
 
 // Setup kernels.
-void launch_scaling_round(int m, int n, TileSet<double> csr, TileSet<double> csc, double* csr_val,
-                          double* csc_val, double* row_acc, double* col_acc, double* dr,
-                          double* dc, int sum_mode, cudaStream_t s);
+// The preconditioner (src/la/scaling.cpp:111-159) on both sliced layouts: raw values in, scaled
+// values, Dr and Dc (ones on entry) out, and the scaled values' magnitude range.
+struct ScalingBuffers {
+  SliceSet csr, csc;
+  const double *csr_raw, *csc_raw;
+  double *csr_val, *csc_val;
+  double *row_factor[2], *col_factor[2];  // the rounds' factors, alternating
+  double *dr, *dc;
+  double* minmax;      // 2 * scale_blocks(csc)
+  double* minmax_out;  // {max, min}
+  long long nnz;
+};
+int scale_blocks(const SliceSet& S);
+void launch_scaling(const ScalingBuffers& b, cudaStream_t s);
+// The sliced copy of a compressed layout's indices and values, and the values back.
+void launch_slice_fill(const SliceSet& S, const int* ptr, const int* idx, const double* val,
+                       int* sidx, double* sval, cudaStream_t s);
+void launch_slice_unfill(const SliceSet& S, const int* ptr, const double* sval, double* val,
+                         cudaStream_t s);
 void launch_scale_vectors(int m, int n, const double* cost, const double* l, const double* u,
                           const double* rl, const double* ru, const double* dr, const double* dc,
                           double* cs, double* ls, double* us, double* rls, double* rus,
                           cudaStream_t s);
 // Fixed device scratch of the allocation-free product: chunk partials for at most
-// kNoAllocMaxChunks chunk tiles, its completion counter and its error word. Set up once per
-// device (the symbol addresses, and the counter and error word cleared to zero) under a
-// lock; later calls only read the cached addresses.
+// kNoAllocMaxChunks pieces of long rows and its completion counter. Set up once per device
+// (the symbol addresses, and the counter cleared to zero) under a lock; later calls only read
+// the cached addresses.
 constexpr int kNoAllocMaxChunks = 16384;
-cudaError_t noalloc_scratch(int device, cudaStream_t s, double** chunks, unsigned int** ticket,
-                            unsigned int** error);
+cudaError_t noalloc_scratch(int device, cudaStream_t s, double** chunks, unsigned int** ticket);
 
-// y = A x with the tile kernel (CSR gives A x; CSC gives A^T x). chunk holds a.nchunks
-// doubles; ticket is one device counter that is zero on entry and on exit. A bounded wait
-// that gives up sets *error (which the caller clears and reads) and leaves NaN in the rows
-// the product could not finish.
 // table[e] = step_factors(e) for e < n (decisions.cuh).
 void launch_step_factors(double2* table, long long n, cudaStream_t s);
-void launch_spmv(TileSet<double> a, const double* x, double* y, double* chunk,
-                 unsigned int* ticket, unsigned int* error, cudaStream_t s, int grid);
-// out[0] = sum v^2, deterministic; part holds grid doubles.
+// y = A x (CSR gives A x; CSC gives A^T x). chunk holds a.nchunks doubles; ticket is one device
+// counter that is zero on entry and on exit.
+void launch_spmv(const SliceSet& a, const double* x, double* y, double* chunk,
+                 unsigned int* ticket, cudaStream_t s);
+// y = (A x) * *by.
+void launch_spmv_scaled(const SliceSet& a, const double* x, double* y, double* chunk,
+                        unsigned int* ticket, const double* by, cudaStream_t s);
+// y = A x, norm[0] = sum y^2, norm[1] = 1 / its root; part holds a.grid doubles.
+void launch_spmv_norm(const SliceSet& a, const double* x, double* y, double* chunk,
+                      unsigned int* ticket, double* part, double* norm, cudaStream_t s);
+// out[0] = sum v^2, out[1] = 1 / its root, deterministic; part holds grid doubles.
 void launch_sumsq(const double* v, int count, double* part, double* out, unsigned int* ticket,
                   cudaStream_t s, int grid);
-void launch_scale_div(double* v, int count, const double* by_sqrt_of, cudaStream_t s);
-void launch_abs_minmax(const double* v, int count, double* part, double* out,
-                       unsigned int* ticket, cudaStream_t s, int grid);
 void launch_project_start(int n, const double* l, const double* u, double* x, cudaStream_t s);
 void launch_fill(double* v, int count, double value, cudaStream_t s);
 
-// Resident tile blocks per SM of the step kernels (occupancy query).
-int tile_blocks_per_sm();
-// The FP64 step passes (pass 0 = column pass, 1 = row pass): the gathered-vector window
-// that fits beside their pipeline, their dynamic shared memory for a window of `wmax`
-// elements, and how many of their blocks fit one SM with it.
+// The FP64 step passes (pass 0 = column pass, 1 = row pass): the elements of the gathered
+// vector's window that fit a block.
 int fp64_window_capacity(int pass);
-int fp64_step_smem(int pass, int wmax);
-int fp64_step_blocks_per_sm(int pass, int smem);
 // Sets the dynamic shared-memory limits of the FP64 kernels on the current device (once per
 // device); false if the device refused.
-bool configure_tile_kernels();
+bool configure_fp64_kernels();
 // Fills dst[k] = src[map[k]] in FP32 (the values of a split layout's part), k < count.
 void launch_gather_values(const double* src, const int* map, float* dst, long long count,
                           cudaStream_t s);

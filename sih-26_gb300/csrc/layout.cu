@@ -9,8 +9,9 @@
 //     from windows only and an outer part gathered from L2;
 //   * which chunks each block of the grid owns (a cost model: entries plus a fixed cost per
 //     window staged), the block's segments, and for a split layout the block's outer chunks.
+// plan_slices() plans the FP64 passes' sliced layouts (slices.cuh) the same way.
 // Everything here is plain host code: the engine uploads the result, and
-// tests/host/layout_check.cu checks it on the CPU.
+// tests/host/layout_check.cu checks the chunk layouts on the CPU.
 #include "engine.hpp"
 
 #include <algorithm>
@@ -335,6 +336,114 @@ ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, in
                  p.chunks.size(), windows.size(), p.segs.size(), p.oidx.size(),
                  p.orounds.size(), p.npieces);
   }
+  return p;
+}
+
+// The sliced layout of one matrix layout (slices.cuh): rows dealt to slices by length inside
+// each group, the long rows' items, the windows over the groups and the blocks' segments.
+// `np` products are accumulated per entry by the kernel that runs on it (the cost model: a
+// slice costs its longest row's entries times np FP64 instructions, plus its epilogue).
+SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, int extent, int wmax,
+                      double window_min, int sms, int np) {
+  SlicePlan p;
+  const int ngroups = (lines + kGroupRows - 1) / kGroupRows;
+  const long long nnz = lines > 0 ? ptr[lines] : 0;
+  p.nslices = ngroups * kGroupSlices;
+  p.meta.assign(static_cast<size_t>(p.nslices) * 32, kNoRow);
+  p.base.assign(static_cast<size_t>(p.nslices), 0);
+  std::vector<double> cost(static_cast<size_t>(ngroups) + 1, 0.0);
+  std::vector<Tile> groups(static_cast<size_t>(ngroups));
+  long long rows32 = 0;  // entries stored so far, / 32
+  long long lentries = 0;
+  for (int g = 0; g < ngroups; ++g) {
+    const int r0 = g * kGroupRows, r1 = std::min(lines, r0 + kGroupRows);
+    groups[static_cast<size_t>(g)] = Tile{r0, r1, ptr[r0], ptr[r1]};
+    // A counting sort by length, longest first, rows of equal length in row order.
+    int start[kSliceLong + 2] = {0};
+    for (int r = r0; r < r1; ++r) {
+      const int len = ptr[r + 1] - ptr[r];
+      if (len <= kSliceLong) ++start[kSliceLong - len + 1];
+    }
+    for (int k = 0; k <= kSliceLong; ++k) start[k + 1] += start[k];
+    unsigned short* meta = p.meta.data() + static_cast<size_t>(g) * kGroupRows;
+    for (int r = r0; r < r1; ++r) {
+      const int len = ptr[r + 1] - ptr[r];
+      if (len > kSliceLong) {
+        const int pieces = (len + kSlicePiece - 1) / kSlicePiece;
+        if (pieces > 1) p.longs.push_back(LongRow{r, p.nchunks, pieces});
+        for (int c = 0; c < pieces; ++c) {
+          const int b = c * kSlicePiece, e = std::min(len, b + kSlicePiece);
+          p.items.push_back(SliceItem{r, pieces > 1 ? p.nchunks++ : -1,
+                                      static_cast<int>(lentries) + b, e - b});
+        }
+        lentries += len;
+        continue;
+      }
+      meta[start[kSliceLong - len]++] =
+          static_cast<unsigned short>((r - r0) | (static_cast<unsigned>(len) << 8));
+    }
+    double c = 0.0;
+    for (int q = 0; q < kGroupSlices; ++q) {
+      const unsigned short head = meta[q * 32];
+      const int width = head == kNoRow ? 0 : head >> 8;
+      p.base[static_cast<size_t>(g) * kGroupSlices + q] = static_cast<unsigned>(rows32);
+      rows32 += width;
+      c += static_cast<double>(width) * np + 12.0;
+    }
+    cost[static_cast<size_t>(g) + 1] = cost[static_cast<size_t>(g)] + c;
+  }
+  p.long_base = rows32 * 32;
+  p.entries = p.long_base + lentries;
+
+  // Windows, over the groups; kept where they hold at least window_min of the entries.
+  std::vector<int> group_win;
+  std::vector<int2> windows;
+  long long covered = build_windows(groups, idx, extent, wmax, &group_win, &windows);
+  if (nnz > 0 && static_cast<double>(covered) < window_min * static_cast<double>(nnz)) {
+    group_win.assign(group_win.size(), -1);
+    windows.clear();
+    covered = 0;
+  }
+  p.staged = nnz > 0 ? static_cast<double>(covered) / static_cast<double>(nnz) : 0.0;
+  for (const int2& w : windows) p.wmax = std::max(p.wmax, w.y);
+
+  // Blocks: one per SM, cut where the running cost passes the next share; a block has as many
+  // warps as its slices or items keep busy, at most kSliceThreads threads.
+  const int G = std::max(1, std::min(std::max(ngroups, static_cast<int>(p.items.size())), sms));
+  p.grid = G;
+  p.seg_start.assign(static_cast<size_t>(G) + 1, 0);
+  int g0 = 0, most = 1;
+  for (int b = 0; b < G; ++b) {
+    p.seg_start[static_cast<size_t>(b)] = static_cast<int>(p.segs.size());
+    const double upto = cost[static_cast<size_t>(ngroups)] * (b + 1) / G;
+    int g1 = g0;
+    while (g1 < ngroups && (b + 1 == G || cost[static_cast<size_t>(g1) + 1] <= upto * (1 + 1e-12) ||
+                            (cost[static_cast<size_t>(g1)] + cost[static_cast<size_t>(g1) + 1]) < 2.0 * upto)) {
+      ++g1;
+    }
+    most = std::max(most, (g1 - g0) * kGroupSlices);
+    for (int g = g0; g < g1;) {
+      int e = g + 1;
+      while (e < g1 && group_win[static_cast<size_t>(e)] == group_win[static_cast<size_t>(g)]) ++e;
+      SliceSeg sg{g * kGroupSlices, e * kGroupSlices, 0, 0};
+      if (group_win[static_cast<size_t>(g)] >= 0) {
+        sg.lo = windows[static_cast<size_t>(group_win[static_cast<size_t>(g)])].x;
+        sg.len = windows[static_cast<size_t>(group_win[static_cast<size_t>(g)])].y;
+      }
+      p.segs.push_back(sg);
+      g = e;
+    }
+    // A block of items only still visits them: they belong to its first segment.
+    if (static_cast<int>(p.segs.size()) == p.seg_start[static_cast<size_t>(b)]) {
+      p.segs.push_back(SliceSeg{0, 0, 0, 0});
+    }
+    g0 = g1;
+  }
+  p.seg_start[static_cast<size_t>(G)] = static_cast<int>(p.segs.size());
+  most = std::max(most, (static_cast<int>(p.items.size()) + G - 1) / G);
+  int warps = 4;
+  while (warps * 32 < kSliceThreads && warps < most) warps *= 2;
+  p.threads = warps * 32;
   return p;
 }
 

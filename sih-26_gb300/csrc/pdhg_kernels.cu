@@ -1,8 +1,8 @@
 // pdhg_kernels.cu -- the FP64 hot path of the GB300 PDHG engine.
 //
-// Per attempted step (src/pdhg/pdhg.cpp:220-335) there are TWO kernels, both on the tile
-// engine of tiles.cuh (the FP32 method's step kernels run on the warp chunks of chunks.cuh
-// instead; on GB300's FP64 pipe these tile kernels measured faster than chunk versions):
+// Per attempted step (src/pdhg/pdhg.cpp:220-335) there are TWO kernels, both on the sliced
+// rows of slices.cuh (the FP32 method's step kernels run on the warp chunks of chunks.cuh
+// instead):
 //   k_primal  one pass over the CSC copy of Ahat: A^T y gathered per column, fused with the
 //             projected primal update x' = proj(x - tau (c + A^T y)), xbar = 2x' - x and
 //             dx = x' - x (written once per column so the row pass needs one FMA per entry
@@ -22,7 +22,7 @@
 #include "common.cuh"
 #include "decisions.cuh"
 #include "kernels.cuh"
-#include "tiles.cuh"
+#include "slices.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -34,20 +34,13 @@ namespace {
 
 long long g_launches = 0;
 
-constexpr int kScratch = 16 * (kBlockThreads / 32);
-// The step passes keep one tile in flight beside the staged window (a larger window pays
-// more in FP64 than a deeper pipeline); each tile brings its
-// rows' operands: x, c, l, u, x_sum (column pass) and y, rl, ru, y_sum (row pass).
-constexpr int kStepStages = 2;
-using PrimalPipe = TilePipe<double, kStepStages, 5>;
-using DualPipe = TilePipe<double, kStepStages, 4>;
+constexpr int kScratch = 16 * (kSliceThreads / 32);
 
 // Per-device state: whether the kernels' shared-memory limits are set on the device, and
 // its occupancy and SM count (an engine on device 1 needs its own opt-in).
 constexpr int kMaxDevices = 64;
 struct DeviceConfig {
   bool configured;
-  int tile_blocks_per_sm;
   int sms;
 };
 std::mutex g_config_mutex;
@@ -90,51 +83,53 @@ __device__ bool fp64_stop_test(const Ctl* c, const Residuals& r) {
 }
 
 // ---- k_primal ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlockThreads) k_primal(StepBuffers b) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
+__global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
+  extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
+  grid_dependency_wait();  // the previous kernel's results (launch_after)
   Ctl* ctl = b.ctl;
-  if (ctl->done != kRunning || ctl->eval_now != 0) return;
-  if (ctl->iteration >= ctl->iteration_limit) {  // src/pdhg/pdhg.cpp:206
+  // Every control field the pass reads, loaded together before the first test.
+  const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
+  const bool add = ctl->pending_add != 0;
+  const long long iteration = ctl->iteration, limit = ctl->iteration_limit;
+  const double omega = ctl->omega, eta = ctl->eta;
+  if (done != kRunning || eval_now != 0) return;
+  if (iteration >= limit) {  // src/pdhg/pdhg.cpp:206
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->done = kIterationLimit;
     return;
   }
-  const int cur = ctl->cur;
-  const double* x = b.x[cur];
+  const double* __restrict__ x = b.x[cur];
   double* __restrict__ xn = b.x[cur ^ 1];
   const double* __restrict__ y = b.y[cur];
-  const double omega = ctl->omega;
   // Formed once per block: an FP64 division per thread would hold GB300's slow FP64 pipe.
   __shared__ double s_tau;
-  if (threadIdx.x == 0) s_tau = ctl->eta / omega;
+  if (threadIdx.x == 0) s_tau = eta / omega;
   __syncthreads();
   const double tau = s_tau;
-  const bool add = ctl->pending_add != 0;
   double mv[1] = {0.0};  // sum of dx^2
-  PrimalPipe pipe;
-  pipe.setup(dsmem);
-  pipe.rsrc[0] = x;
-  pipe.rsrc[1] = b.c;
-  pipe.rsrc[2] = b.l;
-  pipe.rsrc[3] = b.u;
-  pipe.rsrc[4] = b.x_sum;
-  Window<double> win;
-  win.setup(y, pipe, dsmem);
-  auto gather = [&](int row, double v, double* acc) { acc[0] = fma(v, win.get(row), acc[0]); };
-  auto epi = [&](int j, const double* s) {
-    const double xj = pipe.row(0, j);
-    if (add) b.x_sum[j] = pipe.row(4, j) + xj;
-    const double gradient = pipe.row(1, j) + s[0];
+  auto fetch = [&](int i) { return __ldg(y + i); };
+  auto mac = [](double v, double g, double* acc) { acc[0] = fma(v, g, acc[0]); };
+  // Operands of column j: x, c, l, u and (when the last step is still to be added) x_sum.
+  auto load = [&](int j, double* o) {
+    o[0] = x[j];
+    o[1] = b.c[j];
+    o[2] = b.l[j];
+    o[3] = b.u[j];
+    o[4] = add ? b.x_sum[j] : 0.0;
+  };
+  auto epi = [&](int j, const double* s, const double* o) {
+    const double xj = o[0];
+    if (add) b.x_sum[j] = o[4] + xj;
+    const double gradient = o[1] + s[0];
     // Unfused, as src/pdhg/pdhg.cpp:232-233 rounds it.
-    const double xnj =
-        clamp_box(__dsub_rn(xj, __dmul_rn(tau, gradient)), pipe.row(2, j), pipe.row(3, j));
+    const double xnj = clamp_box(__dsub_rn(xj, __dmul_rn(tau, gradient)), o[2], o[3]);
     xn[j] = xnj;
     const double d = xnj - xj;
     // 2 x' is exact, so the FMA rounds once, as the reference's 2.0 * x' - x does.
     b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
     mv[0] = fma(d, d, mv[0]);
   };
-  if (!run_tiles<1, double>(pipe, b.csc, win, b.chunk_primal, gather, epi) &&
+  if (!run_slices<true, 1, 5>(b.csc, y, fetch, dsmem, b.chunk_primal, mac, load, epi) &&
       threadIdx.x == 0) {
     raise_error(ctl);
   }
@@ -148,7 +143,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_primal(StepBuffers b) {
   }
   if (!arrive_last<1>(mv, scratch, b.part_primal, &ctl->ticket[kTicketPrimal])) return;
   mv[0] = 0.0;
-  run_long_rows<1>(b.csc, b.chunk_primal, epi);
+  run_slice_long_rows<1, 5>(b.csc, b.chunk_primal, load, epi);
   double longs[1], total[1];
   block_sum<1>(mv, scratch, longs);
   sum_partials<1>(b.part_primal, gridDim.x, scratch, total);
@@ -159,12 +154,15 @@ __global__ void __launch_bounds__(kBlockThreads) k_primal(StepBuffers b) {
 }
 
 // ---- k_dual ------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlockThreads) k_dual(StepBuffers b) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
+__global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
+  extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
+  grid_dependency_wait();  // the previous kernel's results (launch_after)
   Ctl* ctl = b.ctl;
-  if (ctl->done != kRunning || ctl->eval_now != 0) return;
-  const int cur = ctl->cur;
+  const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
+  const bool add = ctl->pending_add != 0;
+  const double omega = ctl->omega, eta = ctl->eta;
+  if (done != kRunning || eval_now != 0) return;
   // The step-size factors of this step, loaded now for the decision the last block takes.
   const double2 factors = threadIdx.x == 0
                               ? step_factors(ctl->iteration, b.step_factors, b.step_factors_n)
@@ -172,27 +170,24 @@ __global__ void __launch_bounds__(kBlockThreads) k_dual(StepBuffers b) {
   const double* __restrict__ y = b.y[cur];
   double* __restrict__ yn = b.y[cur ^ 1];
   const double2* __restrict__ xd = b.xd;
-  const double omega = ctl->omega;
-  const double sigma = ctl->eta * omega;
-  const bool add = ctl->pending_add != 0;
+  const double sigma = eta * omega;
   double acc2[2] = {0.0, 0.0};  // sum dy^2, sum dy (A dx)
-  DualPipe pipe;
-  pipe.setup(dsmem);
-  pipe.rsrc[0] = y;
-  pipe.rsrc[1] = b.rl;
-  pipe.rsrc[2] = b.ru;
-  pipe.rsrc[3] = b.y_sum;
-  Window<double2> win;
-  win.setup(xd, pipe, dsmem);
-  auto gather = [&](int col, double v, double* acc) {
-    const double2 p = win.get(col);
+  auto fetch = [&](int j) { return __ldg(xd + j); };
+  auto mac = [](double v, double2 p, double* acc) {
     acc[0] = fma(v, p.x, acc[0]);
     acc[1] = fma(v, p.y, acc[1]);
   };
-  auto epi = [&](int i, const double* s) {
-    const double yi = pipe.row(0, i);
-    if (add) b.y_sum[i] = pipe.row(3, i) + yi;
-    const double rl = pipe.row(1, i), ru = pipe.row(2, i);
+  // Operands of row i: y, rl, ru and (when the last step is still to be added) y_sum.
+  auto load = [&](int i, double* o) {
+    o[0] = y[i];
+    o[1] = b.rl[i];
+    o[2] = b.ru[i];
+    o[3] = add ? b.y_sum[i] : 0.0;
+  };
+  auto epi = [&](int i, const double* s, const double* o) {
+    const double yi = o[0];
+    if (add) b.y_sum[i] = o[3] + yi;
+    const double rl = o[1], ru = o[2];
     // Unfused, as the reference rounds it (src/pdhg/pdhg.cpp:244-245): a fused
     // v - sigma * (v / sigma) would leave the division's rounding error on a free row. On
     // an equality row the projection is the bound whatever v is, so no division is needed.
@@ -204,13 +199,13 @@ __global__ void __launch_bounds__(kBlockThreads) k_dual(StepBuffers b) {
     acc2[0] = fma(d, d, acc2[0]);
     acc2[1] = fma(d, s[1], acc2[1]);
   };
-  if (!run_tiles<2, double>(pipe, b.csr, win, b.chunk_dual, gather, epi) &&
+  if (!run_slices<true, 2, 4>(b.csr, xd, fetch, dsmem, b.chunk_dual, mac, load, epi) &&
       threadIdx.x == 0) {
     raise_error(ctl);
   }
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
   acc2[0] = acc2[1] = 0.0;
-  run_long_rows<2>(b.csr, b.chunk_dual, epi);
+  run_slice_long_rows<2, 4>(b.csr, b.chunk_dual, load, epi);
   double longs[2], total[2];
   block_sum<2>(acc2, scratch, longs);
   sum_partials<2>(b.part_dual, gridDim.x, scratch, total);
@@ -279,8 +274,7 @@ __global__ void __launch_bounds__(kTileThreads) k_eval_rows0(EvalBuffers e) {
 // E1: columns over the unscaled CSC. Reduced costs d = c + A^T y of both candidates, the
 // column half of the dual violation / dual objective / complementarity, the primal objective
 // (src/pdhg/pdhg_evaluate.cpp:54-78,111-139) and |x - x_restart|^2.
-__global__ void __launch_bounds__(kBlockThreads) k_eval_cols(EvalBuffers e) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
+__global__ void __launch_bounds__(kSliceThreads, 1) k_eval_cols(EvalBuffers e) {
   __shared__ double scratch[kScratch];
   Ctl* c = e.ctl;
   if (!eval_active(c)) return;
@@ -294,11 +288,13 @@ __global__ void __launch_bounds__(kBlockThreads) k_eval_cols(EvalBuffers e) {
   // sums: viol0, bc0, pobj0, viol1, bc1, pobj1, dx^2, model objective; maxes: comp0, comp1
   double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   double cmax[2] = {0.0, 0.0};
-  auto gather = [&](int row, double v, double* a) {
-    a[0] = fma(v, yu0[row], a[0]);
-    if (avg) a[1] = fma(v, yu1[row], a[1]);
+  auto fetch = [&](int i) { return make_double2(yu0[i], avg ? yu1[i] : 0.0); };
+  auto mac = [&](double v, double2 g, double* a) {
+    a[0] = fma(v, g.x, a[0]);
+    if (avg) a[1] = fma(v, g.y, a[1]);
   };
-  auto epi = [&](int j, const double* s) {
+  auto load = [](int, double*) {};
+  auto epi = [&](int j, const double* s, const double*) {
     const double cj = e.cost[j], lj = e.l[j], uj = e.u[j];
     double xc[2];
     const int nc = avg ? 2 : 1;
@@ -332,12 +328,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_eval_cols(EvalBuffers e) {
       acc[3 * q + 2] += cj * xc[q];
     }
   };
-  TilePipe<double> pipe;
-  pipe.setup(dsmem);
-  if (!run_tiles<2, double>(pipe, e.csc, e.chunk_cols, gather, epi) &&
-      threadIdx.x == 0) {
-    raise_error(c);
-  }
+  run_slices<false, 2, 0, double2>(e.csc, nullptr, fetch, nullptr, e.chunk_cols, mac, load, epi);
   double out[8], mout[2];
   block_sum<8>(acc, scratch, out);
   block_max<2>(cmax, scratch, mout);
@@ -356,7 +347,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_eval_cols(EvalBuffers e) {
   // Last block: long columns into the extra slot e.part_cols[grid_cols].
   for (int q = 0; q < 8; ++q) acc[q] = 0.0;
   cmax[0] = cmax[1] = 0.0;
-  run_long_rows<2>(e.csc, e.chunk_cols, epi);
+  run_slice_long_rows<2, 0>(e.csc, e.chunk_cols, load, epi);
   block_sum<8>(acc, scratch, out);
   block_max<2>(cmax, scratch, mout);
   if (threadIdx.x == 0) {
@@ -387,8 +378,7 @@ __device__ Residuals assemble(double pviol, double cviol, double rviol, double b
 // E2: rows over the unscaled CSR. Activities of both candidates, primal violation and the
 // row complementarity (src/pdhg/pdhg_evaluate.cpp:29-45,99-110). The last block assembles
 // the Residuals and takes the best / stop / restart decisions (src/pdhg/pdhg.cpp:349-483).
-__global__ void __launch_bounds__(kBlockThreads) k_eval_rows1(EvalBuffers e) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
+__global__ void __launch_bounds__(kSliceThreads, 1) k_eval_rows1(EvalBuffers e) {
   __shared__ double scratch[kScratch];
   Ctl* c = e.ctl;
   if (!eval_active(c)) return;
@@ -398,11 +388,13 @@ __global__ void __launch_bounds__(kBlockThreads) k_eval_rows1(EvalBuffers e) {
   const double* __restrict__ xu1 = e.xu[1];
   double acc[2] = {0.0, 0.0};
   double cmax[2] = {0.0, 0.0};
-  auto gather = [&](int col, double v, double* a) {
-    a[0] = fma(v, xu0[col], a[0]);
-    if (avg) a[1] = fma(v, xu1[col], a[1]);
+  auto fetch = [&](int j) { return make_double2(xu0[j], avg ? xu1[j] : 0.0); };
+  auto mac = [&](double v, double2 g, double* a) {
+    a[0] = fma(v, g.x, a[0]);
+    if (avg) a[1] = fma(v, g.y, a[1]);
   };
-  auto epi = [&](int i, const double* s) {
+  auto load = [](int, double*) {};
+  auto epi = [&](int i, const double* s, const double*) {
     const double rl = e.rl[i], ru = e.ru[i];
     const int nc = avg ? 2 : 1;
     for (int q = 0; q < nc; ++q) {
@@ -418,12 +410,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_eval_rows1(EvalBuffers e) {
       }
     }
   };
-  TilePipe<double> pipe;
-  pipe.setup(dsmem);
-  if (!run_tiles<2, double>(pipe, e.csr, e.chunk_rows, gather, epi) &&
-      threadIdx.x == 0) {
-    raise_error(c);
-  }
+  run_slices<false, 2, 0, double2>(e.csr, nullptr, fetch, nullptr, e.chunk_rows, mac, load, epi);
   double mout[2], sums[2];
   block_max<2>(cmax, scratch, mout);
   block_sum<2>(acc, scratch, sums);
@@ -444,7 +431,7 @@ __global__ void __launch_bounds__(kBlockThreads) k_eval_rows1(EvalBuffers e) {
   // ---- Last block: long rows, then every partial in a fixed order. ----
   acc[0] = acc[1] = 0.0;
   cmax[0] = cmax[1] = 0.0;
-  run_long_rows<2>(e.csr, e.chunk_rows, epi);
+  run_slice_long_rows<2, 0>(e.csr, e.chunk_rows, load, epi);
   double s[15];
 #pragma unroll
   for (int q = 0; q < 15; ++q) s[q] = 0.0;
@@ -516,36 +503,196 @@ __global__ void k_eval_apply(EvalBuffers e) {
 
 // ---- Setup kernels (src/la/scaling.cpp) ----------------------------------------------------
 
-// One thread per row (CSR) or column (CSC): the maximum (Ruiz) or the sum (Pock-Chambolle)
-// of |a| in ascending index order -- the reference's accumulation order -- then the pass
-// factor 1/sqrt(.) (1 for an empty line).
-__global__ void k_line_factor(const int* ptr, const double* val, int lines, int sum_mode,
-                              double* factor) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < lines; r += gridDim.x * blockDim.x) {
+// The scaling rounds run on the sliced layouts: one lane per line, every load and store of the
+// values coalesced, a line's magnitudes taken in ascending index order, the reference's
+// accumulation order. (One thread per line on the compressed layouts read 32 scattered
+// entries per load: 101 us for the factors of one layout and 123 us to apply them on the
+// 500,000 x 1M block-angular LP, and 1.35 and 2.5 ms where a Zipf row of 6,674 entries held one
+// thread.) One kernel per layout and round applies the round's factors, takes the next round's
+// from the values it has in registers and folds its own into the accumulated scale, so a
+// round reads and writes each layout's values once.
+enum ScaleMode { kScaleMax = 0, kScaleSum = 1, kScaleNone = 2 };
+
+struct ScaleArgs {
+  SliceSet S;            // the layout; S.val is not used
+  const double* in;      // the values before the round
+  double* out;           // and after it (may be `in`)
+  const double* line;    // the round's factors of the layout's lines (nullptr: first, no apply)
+  const double* other;   // and of the other side
+  double* next;          // the next round's line factors (not for kScaleNone)
+  double* scale;         // accumulated line scale, multiplied by `line`
+  int line_is_row;
+  // kScaleNone: per-block {max, -min} magnitudes of the final values, or nullptr.
+  double* minmax;
+};
+
+// value <- (value * row factor) * column factor (src/la/scaling.cpp:21-28).
+__device__ __forceinline__ double scaled_value(double v, double lp, double op, int line_is_row) {
+  return line_is_row ? (v * lp) * op : (v * op) * lp;
+}
+
+// The pass factor of a line: 1 / sqrt of its maximum (Ruiz) or sum (Pock-Chambolle) of
+// magnitudes, 1 for an empty line.
+__device__ __forceinline__ double pass_factor(double acc) {
+  return acc > 0.0 ? 1.0 / sqrt(acc) : 1.0;
+}
+
+constexpr int kScaleThreads = 256;
+
+template <int MODE, bool APPLY>
+__global__ void __launch_bounds__(kScaleThreads) k_scale_round(ScaleArgs a) {
+  __shared__ double scratch[2 * (kScaleThreads / 32)];
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int warp = static_cast<int>(threadIdx.x) >> 5;
+  const int slice_blocks = (a.S.nslices + kScaleThreads / 32 - 1) / (kScaleThreads / 32);
+  double mm[2] = {0.0, -HUGE_VAL};  // kScaleNone: max, max of -magnitude
+  const auto take = [&](double mag, double& acc) {
+    if (MODE == kScaleMax) acc = dmax(acc, mag);
+    if (MODE == kScaleSum) acc = acc + mag;
+    if (MODE == kScaleNone) {
+      mm[0] = dmax(mm[0], mag);
+      mm[1] = dmax(mm[1], -mag);
+    }
+  };
+  if (static_cast<int>(blockIdx.x) < slice_blocks) {
+    const int s = static_cast<int>(blockIdx.x) * (kScaleThreads / 32) + warp;
+    if (s < a.S.nslices) {
+      const unsigned m = __ldg(a.S.meta + static_cast<size_t>(s) * 32 + lane);
+      if (m != kNoRow) {
+        const int len = static_cast<int>(m >> 8), row = slice_row(s, m);
+        const size_t at = static_cast<size_t>(__ldg(a.S.base + s)) * 32 + lane;
+        const double lp = APPLY ? a.line[row] : 1.0;
+        double acc = 0.0;
+#pragma unroll 4
+        for (int k = 0; k < len; ++k) {
+          double v = ld_stream(a.in + at + static_cast<size_t>(k) * 32);
+          if (APPLY) {
+            const int o = ld_stream(a.S.idx + at + static_cast<size_t>(k) * 32);
+            v = scaled_value(v, lp, __ldg(a.other + o), a.line_is_row);
+            a.out[at + static_cast<size_t>(k) * 32] = v;
+          }
+          take(fabs(v), acc);
+        }
+        if (APPLY) a.scale[row] *= lp;
+        if (MODE != kScaleNone) a.next[row] = pass_factor(acc);
+      }
+    }
+  } else {
+    // A block per long row: its warps take 32-entry runs in turn; the sum is taken by one warp
+    // in index order.
+    const int r = static_cast<int>(blockIdx.x) - slice_blocks;
+    const SliceItem first = a.S.items[r];
+    // Items of one row follow one another: only the row's first runs, over all its entries.
+    if (r > 0 && a.S.items[r - 1].row == first.row) {
+      if (MODE == kScaleNone && a.minmax != nullptr && threadIdx.x == 0) {
+        a.minmax[2 * blockIdx.x] = 0.0;
+        a.minmax[2 * blockIdx.x + 1] = -HUGE_VAL;
+      }
+      return;
+    }
+    int count = 0;
+    for (int q = r; q < a.S.nitems && a.S.items[q].row == first.row; ++q) count += a.S.items[q].count;
+    const size_t at = static_cast<size_t>(a.S.long_base) + static_cast<size_t>(first.begin);
+    const double lp = APPLY ? a.line[first.row] : 1.0;
     double acc = 0.0;
-    for (int k = ptr[r]; k < ptr[r + 1]; ++k) {
-      const double mag = fabs(val[k]);
-      acc = sum_mode ? acc + mag : dmax(acc, mag);
+    for (int k = static_cast<int>(threadIdx.x); k < count; k += kScaleThreads) {
+      double v = ld_stream(a.in + at + k);
+      if (APPLY) {
+        v = scaled_value(v, lp, __ldg(a.other + ld_stream(a.S.idx + at + k)), a.line_is_row);
+        a.out[at + k] = v;
+      }
+      if (MODE != kScaleSum) take(fabs(v), acc);
     }
-    factor[r] = acc > 0.0 ? 1.0 / sqrt(acc) : 1.0;
+    if (MODE == kScaleMax) {
+      double v[1] = {acc}, total[1];
+      block_max<1>(v, scratch, total);
+      acc = total[0];
+    }
+    if (MODE == kScaleSum) {
+      __syncthreads();  // the block's stores to `out` before warp 0 reads them
+      const double* src = APPLY ? a.out : a.in;
+      if (warp == 0) {
+        double v = lane < count ? fabs(__ldcg(src + at + lane)) : 0.0;
+        for (int k = 0; k < count; k += 32) {
+          const int kn = k + 32 + lane;
+          const double ahead = kn < count ? fabs(__ldcg(src + at + kn)) : 0.0;
+          const int n = count - k < 32 ? count - k : 32;
+          for (int q = 0; q < n; ++q) acc = acc + __shfl_sync(0xffffffffu, v, q);
+          v = ahead;
+        }
+      }
+    }
+    if (threadIdx.x == 0) {
+      if (APPLY) a.scale[first.row] *= lp;
+      if (MODE != kScaleNone) a.next[first.row] = pass_factor(acc);
+    }
+  }
+  if (MODE == kScaleNone && a.minmax != nullptr) {
+    double out[2];
+    block_max<2>(mm, scratch, out);
+    if (threadIdx.x == 0) {
+      a.minmax[2 * blockIdx.x] = out[0];
+      a.minmax[2 * blockIdx.x + 1] = out[1];
+    }
   }
 }
 
-// value <- (value * row_pass[i]) * col_pass[j], in both layouts (src/la/scaling.cpp:21-28).
-__global__ void k_apply_pass(const int* ptr, const int* idx, double* val, int lines,
-                             const double* line_pass, const double* other_pass, int line_is_row) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < lines; r += gridDim.x * blockDim.x) {
-    const double lp = line_pass[r];
-    for (int k = ptr[r]; k < ptr[r + 1]; ++k) {
-      const double op = other_pass[idx[k]];
-      val[k] = line_is_row ? (val[k] * lp) * op : (val[k] * op) * lp;
-    }
+// out[0] = max, out[1] = min of the magnitudes from the blocks' {max, -min} pairs (0 when there
+// are none). One block.
+__global__ void __launch_bounds__(kScaleThreads) k_minmax_final(const double* part, int count,
+                                                               long long entries, double* out) {
+  __shared__ double scratch[2 * (kScaleThreads / 32)];
+  double a[2] = {0.0, -HUGE_VAL};
+  for (int b = static_cast<int>(threadIdx.x); b < count; b += kScaleThreads) {
+    a[0] = dmax(a[0], part[2 * b]);
+    a[1] = dmax(a[1], part[2 * b + 1]);
+  }
+  double o[2];
+  block_max<2>(a, scratch, o);
+  if (threadIdx.x == 0) {
+    out[0] = o[0];
+    out[1] = entries > 0 ? -o[1] : 0.0;
   }
 }
 
-__global__ void k_mul_into(double* acc, const double* factor, int count) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < count; r += gridDim.x * blockDim.x) {
-    acc[r] *= factor[r];
+// The sliced copy of a compressed layout (load), one warp per slice or item; and back, the
+// values only (the scaled values in the caller's or the FP32 layouts' order).
+template <bool BACK>
+__global__ void __launch_bounds__(256) k_slice_copy(SliceSet S, const int* __restrict__ ptr,
+                                                    int* idx, double* val, int* sidx,
+                                                    double* sval) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int w = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (w < S.nslices) {
+    const unsigned m = S.meta[static_cast<size_t>(w) * 32 + lane];
+    if (m == kNoRow) return;
+    const int len = static_cast<int>(m >> 8), a = ptr[slice_row(w, m)];
+    const size_t at = static_cast<size_t>(S.base[w]) * 32 + lane;
+    for (int k = 0; k < len; ++k) {
+      const size_t q = at + static_cast<size_t>(k) * 32;
+      if (BACK) {
+        val[a + k] = sval[q];
+      } else {
+        sidx[q] = idx[a + k];
+        sval[q] = val[a + k];
+      }
+    }
+    return;
+  }
+  if (w - S.nslices >= S.nitems) return;
+  const SliceItem it = S.items[w - S.nslices];
+  // An item's place in its row: the entries of the row's items before it.
+  int before = 0;
+  for (int q = w - S.nslices - 1; q >= 0 && S.items[q].row == it.row; --q) before += S.items[q].count;
+  const int a = ptr[it.row] + before;
+  const size_t at = static_cast<size_t>(S.long_base) + static_cast<size_t>(it.begin);
+  for (int k = lane; k < it.count; k += 32) {
+    if (BACK) {
+      val[a + k] = sval[at + k];
+    } else {
+      sidx[at + k] = idx[a + k];
+      sval[at + k] = val[a + k];
+    }
   }
 }
 
@@ -573,46 +720,56 @@ __global__ void k_scale_vectors(int m, int n, const double* cost, const double* 
   }
 }
 
-// y = A x with products summed in ascending index order per row. A block whose bounded wait
-// gives up (a tile copy that never lands) sets *error and writes NaN to every row of its tile
-// range and to the partials of its chunk tiles (so a long row it took part in sums to NaN):
-// a product that could not be finished is never left looking like a result.
-__global__ void __launch_bounds__(kBlockThreads) k_spmv(TileSet<double> a, const double* x,
-                                                       double* y, double* chunk,
-                                                       unsigned int* ticket,
-                                                       unsigned int* error) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
-  auto gather = [&](int col, double v, double* acc) { acc[0] = fma(v, __ldg(x + col), acc[0]); };
-  auto epi = [&](int r, const double* s) { y[r] = 0.0 + s[0]; };
-  TilePipe<double> pipe;
-  pipe.setup(dsmem);
-  if (!run_tiles<1, double>(pipe, a, chunk, gather, epi)) {
-    int first, last;
-    block_tile_range(a.ntiles, first, last);
-    const double nan = __longlong_as_double(0x7ff8000000000000LL);
-    for (int t = first; t < last; ++t) {
-      const Tile tl = a.tiles[t];
-      if (tl.r1 < 0) {
-        if (threadIdx.x == 0) chunk[-tl.r1 - 1] = nan;
-      } else {
-        for (int r = tl.r0 + static_cast<int>(threadIdx.x); r < tl.r1; r += blockDim.x) y[r] = nan;
-      }
+// y = A x, a short row summed in ascending index order. SCALE multiplies every row's sum by
+// *by; NORM leaves the sum of y^2 in norm[0] and the reciprocal of its root in norm[1]
+// (part holds a double per block). The vector is gathered from L1 and L2 (x may lie at any
+// 8-byte boundary, so no window is staged from it).
+template <bool SCALE, bool NORM>
+__global__ void __launch_bounds__(kSliceThreads, 1) k_spmv(SliceSet a, const double* x, double* y,
+                                                           double* chunk, unsigned int* ticket,
+                                                           const double* by, double* part,
+                                                           double* norm) {
+  __shared__ double scratch[kSliceThreads / 32];
+  const double scale = SCALE ? *by : 1.0;
+  double sq[1] = {0.0};
+  auto fetch = [&](int c) { return __ldg(x + c); };
+  auto mac = [](double v, double g, double* acc) { acc[0] = fma(v, g, acc[0]); };
+  auto load = [](int, double*) {};
+  auto epi = [&](int r, const double* s, const double*) {
+    const double v = SCALE ? s[0] * scale : 0.0 + s[0];
+    y[r] = v;
+    if (NORM) sq[0] = fma(v, v, sq[0]);
+  };
+  run_slices<false, 1, 0, double>(a, nullptr, fetch, nullptr, chunk, mac, load, epi);
+  if (NORM) {
+    if (!arrive_last<1>(sq, scratch, part, ticket)) return;
+    sq[0] = 0.0;
+    run_slice_long_rows<1, 0>(a, chunk, load, epi);
+    double longs[1], total[1];
+    block_sum<1>(sq, scratch, longs);
+    sum_partials<1>(part, gridDim.x, scratch, total);
+    if (threadIdx.x == 0) {
+      *ticket = 0;
+      norm[0] = total[0] + longs[0];
+      norm[1] = 1.0 / sqrt(norm[0]);
     }
-    if (threadIdx.x == 0) atomicExch(error, 1u);
+    return;
   }
   if (a.nlong == 0) return;
   __shared__ int s_last;
+  __syncthreads();  // the block's piece partials before thread 0's fence
   if (threadIdx.x == 0) {
-    __threadfence();  // this block's chunk partials (written by thread 0) before the ticket
+    __threadfence();
     s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  run_long_rows<1>(a, chunk, epi);
+  run_slice_long_rows<1, 0>(a, chunk, load, epi);
   if (threadIdx.x == 0) *ticket = 0;
 }
 
+// norm[0] = sum v^2, norm[1] = 1 / its root.
 __global__ void k_sumsq(const double* v, int count, double* part, double* out,
                         unsigned int* ticket) {
   __shared__ double scratch[kTileThreads / 32];
@@ -635,48 +792,8 @@ __global__ void k_sumsq(const double* v, int count, double* part, double* out,
   for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) a[0] += __ldcg(part + b);
   block_sum<1>(a, scratch, o);
   if (threadIdx.x == 0) {
-    *out = o[0];
-    *ticket = 0;
-  }
-}
-
-__global__ void k_div_by_sqrt(double* v, int count, const double* sq) {
-  const double length = sqrt(*sq);
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-    v[k] /= length;
-  }
-}
-
-__global__ void k_abs_minmax(const double* v, int count, double* part, double* out,
-                             unsigned int* ticket) {
-  __shared__ double scratch[2 * (kTileThreads / 32)];
-  double mx[2] = {0.0, -HUGE_VAL};  // max |v|, max -|v| (= -min |v|)
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-    const double a = fabs(v[k]);
-    mx[0] = dmax(mx[0], a);
-    mx[1] = dmax(mx[1], -a);
-  }
-  double o[2];
-  block_max<2>(mx, scratch, o);
-  __shared__ bool is_last;
-  if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = o[0];
-    part[2 * blockIdx.x + 1] = o[1];
-    __threadfence();
-    is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  double a[2] = {0.0, -HUGE_VAL};
-  for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-    a[0] = dmax(a[0], __ldcg(part + 2 * b));
-    a[1] = dmax(a[1], __ldcg(part + 2 * b + 1));
-  }
-  block_max<2>(a, scratch, o);
-  if (threadIdx.x == 0) {
     out[0] = o[0];
-    out[1] = count > 0 ? -o[1] : 0.0;
+    out[1] = 1.0 / sqrt(o[0]);
     *ticket = 0;
   }
 }
@@ -700,8 +817,6 @@ int elementwise_grid(int count) {
   return blocks < 1 ? 1 : blocks;
 }
 
-constexpr int kTileSmem = TilePipe<double>::bytes();
-
 __global__ void k_gather_values(const double* __restrict__ src, const int* __restrict__ map,
                                 float* __restrict__ dst, long long count) {
   for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < count;
@@ -712,7 +827,7 @@ __global__ void k_gather_values(const double* __restrict__ src, const int* __res
 
 }  // namespace
 
-bool configure_tile_kernels() {
+bool configure_fp64_kernels() {
   const int dev = current_device();
   if (dev < 0) return false;
   std::lock_guard<std::mutex> lock(g_config_mutex);
@@ -722,68 +837,34 @@ bool configure_tile_kernels() {
       cudaFuncSetAttribute(k_primal, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_primal))),
       cudaFuncSetAttribute(k_dual, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           max_dynamic_smem(reinterpret_cast<const void*>(k_dual))),
-      cudaFuncSetAttribute(k_eval_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem),
-      cudaFuncSetAttribute(k_eval_rows1, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem),
-      cudaFuncSetAttribute(k_spmv, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem)};
+                           max_dynamic_smem(reinterpret_cast<const void*>(k_dual)))};
   for (cudaError_t e : errs) {
     if (e != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
   }
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eval_rows1, kBlockThreads,
-                                                    kTileSmem) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  c.tile_blocks_per_sm = per_sm > 0 ? per_sm : 1;
   c.configured = true;
   return true;
-}
-
-int tile_blocks_per_sm() {
-  if (!configure_tile_kernels()) return 1;
-  const int dev = current_device();
-  std::lock_guard<std::mutex> lock(g_config_mutex);
-  return dev >= 0 ? g_config[dev].tile_blocks_per_sm : 1;
 }
 
 long long kernel_launch_count() { return g_launches; }
 
 int fp64_window_capacity(int pass) {
-  configure_tile_kernels();
-  return pass == 0 ? window_capacity(reinterpret_cast<const void*>(k_primal),
-                                     PrimalPipe::bytes(), sizeof(double))
-                   : window_capacity(reinterpret_cast<const void*>(k_dual), DualPipe::bytes(),
+  configure_fp64_kernels();
+  return pass == 0 ? window_capacity(reinterpret_cast<const void*>(k_primal), kSliceBarBytes,
+                                     sizeof(double))
+                   : window_capacity(reinterpret_cast<const void*>(k_dual), kSliceBarBytes,
                                      sizeof(double2));
 }
 
-int fp64_step_smem(int pass, int wmax) {
-  return pass == 0 ? PrimalPipe::bytes() + window_bytes(wmax, sizeof(double))
-                   : DualPipe::bytes() + window_bytes(wmax, sizeof(double2));
-}
-
-int fp64_step_blocks_per_sm(int pass, int smem) {
-  configure_tile_kernels();
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, pass == 0 ? k_primal : k_dual, kBlockThreads, static_cast<size_t>(smem)) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
-  return per_sm > 0 ? per_sm : 1;
-}
-
 void launch_primal_pass(const StepBuffers& b, cudaStream_t s) {
-  k_primal<<<b.grid_primal, kBlockThreads, b.smem_primal, s>>>(b);
+  launch_after(k_primal, b.csc.grid, b.csc.threads, slice_smem<double>(b.csc.wmax), s, b);
   ++g_launches;
 }
 
 void launch_dual_pass(const StepBuffers& b, cudaStream_t s) {
-  k_dual<<<b.grid_dual, kBlockThreads, b.smem_dual, s>>>(b);
+  launch_after(k_dual, b.csr.grid, b.csr.threads, slice_smem<double2>(b.csr.wmax), s, b);
   ++g_launches;
 }
 
@@ -803,24 +884,81 @@ void launch_gather_values(const double* src, const int* map, float* dst, long lo
 void launch_evaluation(const EvalBuffers& e, cudaStream_t s) {
   g_launches += 4;
   k_eval_rows0<<<e.grid_rows, kTileThreads, 0, s>>>(e);
-  k_eval_cols<<<e.grid_cols, kBlockThreads, kTileSmem, s>>>(e);
-  k_eval_rows1<<<e.grid_rows, kBlockThreads, kTileSmem, s>>>(e);
+  k_eval_cols<<<e.grid_cols, e.csc.threads, 0, s>>>(e);
+  k_eval_rows1<<<e.grid_rows, e.csr.threads, 0, s>>>(e);
   const int total = e.m > e.n ? e.m : e.n;
   k_eval_apply<<<elementwise_grid(total), 256, 0, s>>>(e);
 }
 
-void launch_scaling_round(int m, int n, TileSet<double> csr, TileSet<double> csc, double* csr_val,
-                          double* csc_val, double* row_acc, double* col_acc, double* dr,
-                          double* dc, int sum_mode, cudaStream_t s) {
-  g_launches += 6;
-  k_line_factor<<<elementwise_grid(m), 256, 0, s>>>(csr.ptr, csr_val, m, sum_mode, row_acc);
-  k_line_factor<<<elementwise_grid(n), 256, 0, s>>>(csc.ptr, csc_val, n, sum_mode, col_acc);
-  k_apply_pass<<<elementwise_grid(m), 256, 0, s>>>(csr.ptr, csr.idx, csr_val, m, row_acc, col_acc,
-                                                   1);
-  k_apply_pass<<<elementwise_grid(n), 256, 0, s>>>(csc.ptr, csc.idx, csc_val, n, col_acc, row_acc,
-                                                   0);
-  k_mul_into<<<elementwise_grid(m), 256, 0, s>>>(dr, row_acc, m);
-  k_mul_into<<<elementwise_grid(n), 256, 0, s>>>(dc, col_acc, n);
+int scale_blocks(const SliceSet& S) {
+  return (S.nslices + kScaleThreads / 32 - 1) / (kScaleThreads / 32) + S.nitems;
+}
+
+namespace {
+
+template <int MODE, bool APPLY>
+void scale_round(const ScaleArgs& a, cudaStream_t s) {
+  const int grid = scale_blocks(a.S);
+  if (grid == 0) return;
+  ++g_launches;
+  k_scale_round<MODE, APPLY><<<grid, kScaleThreads, 0, s>>>(a);
+}
+
+}  // namespace
+
+void launch_scaling(const ScalingBuffers& b, cudaStream_t s) {
+  // Factors of the raw values, then 11 rounds: ten Ruiz rounds and the Pock-Chambolle round
+  // apply factors; each takes the next round's, the last none.
+  const auto args = [&](int side, int round) {
+    ScaleArgs a{};
+    a.S = side ? b.csc : b.csr;
+    a.in = round <= 0 ? (side ? b.csc_raw : b.csr_raw) : (side ? b.csc_val : b.csr_val);
+    a.out = side ? b.csc_val : b.csr_val;
+    const int now = round & 1, then = now ^ 1;
+    a.line = side ? b.col_factor[now] : b.row_factor[now];
+    a.other = side ? b.row_factor[now] : b.col_factor[now];
+    a.next = side ? b.col_factor[then] : b.row_factor[then];
+    a.scale = side ? b.dc : b.dr;
+    a.line_is_row = side ? 0 : 1;
+    return a;
+  };
+  for (int side = 0; side < 2; ++side) {
+    ScaleArgs a = args(side, -1);  // next = the factors of round 0
+    scale_round<kScaleMax, false>(a, s);
+  }
+  for (int round = 0; round < 11; ++round) {
+    for (int side = 0; side < 2; ++side) {
+      ScaleArgs a = args(side, round);
+      if (round < 9) {
+        scale_round<kScaleMax, true>(a, s);
+      } else if (round == 9) {
+        scale_round<kScaleSum, true>(a, s);
+      } else {
+        a.minmax = side ? b.minmax : nullptr;
+        scale_round<kScaleNone, true>(a, s);
+      }
+    }
+  }
+  ++g_launches;
+  k_minmax_final<<<1, kScaleThreads, 0, s>>>(b.minmax, scale_blocks(b.csc), b.nnz, b.minmax_out);
+}
+
+void launch_slice_fill(const SliceSet& S, const int* ptr, const int* idx, const double* val,
+                       int* sidx, double* sval, cudaStream_t s) {
+  const int warps = S.nslices + S.nitems;
+  if (warps == 0) return;
+  ++g_launches;
+  k_slice_copy<false><<<(warps + 7) / 8, 256, 0, s>>>(S, ptr, const_cast<int*>(idx),
+                                                      const_cast<double*>(val), sidx, sval);
+}
+
+void launch_slice_unfill(const SliceSet& S, const int* ptr, const double* sval, double* val,
+                         cudaStream_t s) {
+  const int warps = S.nslices + S.nitems;
+  if (warps == 0) return;
+  ++g_launches;
+  k_slice_copy<true><<<(warps + 7) / 8, 256, 0, s>>>(S, ptr, nullptr, val, nullptr,
+                                                     const_cast<double*>(sval));
 }
 
 void launch_scale_vectors(int m, int n, const double* cost, const double* l, const double* u,
@@ -845,17 +983,30 @@ void launch_step_factors(double2* table, long long n, cudaStream_t s) {
   k_step_factors<<<std::max(1, device_sms()) * 8, 256, 0, s>>>(table, n);
 }
 
-void launch_spmv(TileSet<double> a, const double* x, double* y, double* chunk,
-                 unsigned int* ticket, unsigned int* error, cudaStream_t s, int grid) {
+void launch_spmv(const SliceSet& a, const double* x, double* y, double* chunk,
+                 unsigned int* ticket, cudaStream_t s) {
   if (a.nrows == 0) return;
   ++g_launches;
-  k_spmv<<<grid, kBlockThreads, kTileSmem, s>>>(a, x, y, chunk, ticket, error);
+  k_spmv<false, false><<<a.grid, a.threads, 0, s>>>(a, x, y, chunk, ticket, nullptr, nullptr,
+                                                    nullptr);
+}
+
+void launch_spmv_scaled(const SliceSet& a, const double* x, double* y, double* chunk,
+                        unsigned int* ticket, const double* by, cudaStream_t s) {
+  ++g_launches;
+  k_spmv<true, false><<<a.grid, a.threads, 0, s>>>(a, x, y, chunk, ticket, by, nullptr, nullptr);
+}
+
+void launch_spmv_norm(const SliceSet& a, const double* x, double* y, double* chunk,
+                      unsigned int* ticket, double* part, double* norm, cudaStream_t s) {
+  ++g_launches;
+  k_spmv<false, true><<<a.grid, a.threads, 0, s>>>(a, x, y, chunk, ticket, nullptr, part, norm);
 }
 
 namespace {
 
 // The allocation-free product's scratch: file-scope device arrays, never cudaMalloc'd.
-// g_noalloc_ticket[0] is the product's completion counter, [1] its error word.
+// g_noalloc_ticket[0] is the product's completion counter.
 static __device__ __align__(256) double g_noalloc_chunks[kNoAllocMaxChunks];
 static __device__ __align__(256) unsigned int g_noalloc_ticket[4];
 
@@ -870,8 +1021,7 @@ NoAllocSlot g_noalloc_slots[kNoAllocMaxDevices];
 
 }  // namespace
 
-cudaError_t noalloc_scratch(int device, cudaStream_t s, double** chunks, unsigned int** ticket,
-                            unsigned int** error) {
+cudaError_t noalloc_scratch(int device, cudaStream_t s, double** chunks, unsigned int** ticket) {
   if (device < 0 || device >= kNoAllocMaxDevices) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(g_noalloc_mutex);
   NoAllocSlot& slot = g_noalloc_slots[device];
@@ -885,8 +1035,7 @@ cudaError_t noalloc_scratch(int device, cudaStream_t s, double** chunks, unsigne
     err = cudaGetSymbolAddress(&t, g_noalloc_ticket);
     if (err != cudaSuccess) return err;
     // The completion counter must start at zero; k_spmv's last block puts it back to zero.
-    // The error word starts at zero too. The chunk partials need no clearing: each is
-    // written before it is read.
+    // The chunk partials need no clearing: each is written before it is read.
     err = cudaMemsetAsync(t, 0, sizeof(g_noalloc_ticket), s);
     if (err != cudaSuccess) return err;
     err = cudaStreamSynchronize(s);
@@ -897,7 +1046,6 @@ cudaError_t noalloc_scratch(int device, cudaStream_t s, double** chunks, unsigne
   }
   *chunks = slot.chunks;
   *ticket = slot.ticket;
-  *error = slot.ticket + 1;
   return cudaSuccess;
 }
 
@@ -905,17 +1053,6 @@ void launch_sumsq(const double* v, int count, double* part, double* out, unsigne
                   cudaStream_t s, int grid) {
   ++g_launches;
   k_sumsq<<<grid, kTileThreads, 0, s>>>(v, count, part, out, ticket);
-}
-
-void launch_scale_div(double* v, int count, const double* by_sqrt_of, cudaStream_t s) {
-  ++g_launches;
-  k_div_by_sqrt<<<elementwise_grid(count), 256, 0, s>>>(v, count, by_sqrt_of);
-}
-
-void launch_abs_minmax(const double* v, int count, double* part, double* out,
-                       unsigned int* ticket, cudaStream_t s, int grid) {
-  ++g_launches;
-  k_abs_minmax<<<grid, kTileThreads, 0, s>>>(v, count, part, out, ticket);
 }
 
 void launch_project_start(int n, const double* l, const double* u, double* x, cudaStream_t s) {

@@ -1,0 +1,285 @@
+// slices.cuh -- sliced rows: the FP64 sparse-product engine.
+//
+// A SLICE is 32 rows (of the CSR copy, or columns of the CSC copy) that one warp sums, one row
+// per lane, with the entries stored so that lane l's k-th entry is at base + 32 k + l: every
+// matrix load of a warp is one contiguous 256-byte (values) or 128-byte (indices) run. A lane
+// walks its own row in ascending index order with FMA, so every short row is summed in the
+// reference's order.
+//
+// Rows are dealt to slices inside GROUPS of kGroupRows consecutive rows, longest first, so the
+// rows of a slice have nearly the same length: GB300 retires two FP64 lane operations per clock
+// per SM and charges a warp instruction in full whatever its active lanes, so a slice costs its
+// longest row. (Rows of 9 to 31 entries, the 1M x 2M block-angular LP: in row order the 32
+// lanes of a warp wait for about 30 entries where the mean is 20; dealt by length inside 128
+// rows, for about 21.) A group spans 128 rows only, so the rows of a slice stay close together:
+// the per-row operands of the epilogue are read from the same few cache lines by the group's
+// four slices, and the group's gathers share a window.
+//
+// A row of more than kSliceLong entries is LONG: a whole warp sums it (lane l takes entries l,
+// l + 32, ...; a fixed tree adds the lanes) from a region of its own behind the slices, in
+// pieces of kSlicePiece entries when it is longer than that; the pieces of a row are combined in
+// order by the kernel's last block.
+//
+// WINDOWS. A random 8-byte gather from L1 or L2 costs a tag lookup and a sector each, 32 per
+// warp-wide gather at about one per clock per SM; from shared memory a warp-wide gather of
+// doubles costs about 7 clocks of bank conflicts. So a block keeps a window [lo, lo + len) of
+// the gathered vector in shared memory where the layout's windows hold at least 95% of its
+// entries (build_windows over the groups), copied in by one bulk copy per segment of groups.
+//
+// Block b owns a contiguous run of groups, cut by cost, and its warps take the run's slices in
+// turn: every sum and every block partial is taken in a fixed order, so runs are
+// bit-reproducible. Warps do not wait for one another except where the window changes. Every
+// wait is bounded: a wait that gives up raises the block's abort flag, the block's remaining
+// slices are skipped, a copy still in flight is given a bounded time to land, and the caller
+// records the error.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "chunks.cuh"
+#include "common.cuh"
+#include "tiles.cuh"
+
+namespace sgb {
+
+constexpr int kGroupRows = 128;
+constexpr int kGroupSlices = kGroupRows / 32;
+constexpr int kSliceLong = 64;     // entries past which a row is long
+constexpr int kSlicePiece = kCap;  // entries per piece of a long row
+constexpr int kSliceThreads = 1024;  // the largest block of a slice kernel
+constexpr unsigned short kNoRow = 0xffff;
+
+// A piece of a long row (or all of it): entries [begin, begin + count) of the layout's long
+// region. slot < 0: the whole row, whose epilogue the warp runs; otherwise the partial slot.
+struct SliceItem {
+  int row;
+  int slot;
+  int begin;
+  int count;
+};
+
+// Consecutive slices of one block that gather from the same window (len = 0: none).
+struct SliceSeg {
+  int s0, s1;
+  int lo, len;
+};
+
+struct SliceSet {
+  // Per slice and lane: the row's place in its group (7 bits) and its length (from bit 8), or
+  // kNoRow (no row, or a long one).
+  const unsigned short* meta;
+  const unsigned int* base;  // per slice: first entry / 32
+  const int* idx;
+  const double* val;
+  const SliceItem* items;
+  const LongRow* longs;      // rows of several pieces
+  const SliceSeg* segs;
+  const int* seg_start;      // per block: its segments [seg_start[b], seg_start[b + 1])
+  long long long_base;       // first entry of the long region
+  int nslices, nitems, nlong, nchunks, nrows;
+  int wmax;                  // window capacity in gathered elements (0: none)
+  int grid, threads;
+};
+
+// Shared memory of a slice kernel's window: the mbarrier, then the window.
+constexpr int kSliceBarBytes = 128;
+template <typename G>
+__host__ __device__ constexpr int slice_smem(int wmax) {
+  return wmax > 0 ? kSliceBarBytes + ((wmax * static_cast<int>(sizeof(G)) + 127) & ~127) : 0;
+}
+
+// The row a meta word of slice s names.
+__device__ __forceinline__ int slice_row(int s, unsigned m) {
+  return (s / kGroupSlices) * kGroupRows + static_cast<int>(m & 127u);
+}
+
+// One slice. `m` is the lane's meta word and `base` the slice's first entry / 32. A lane loads
+// the indices and values of kBatch entries, then gathers them, then accumulates: two memory
+// latencies per kBatch entries.
+constexpr int kSliceBatch = 4;
+
+template <int NP, int NR, typename G, typename Get, typename Mac, typename Load, typename Epi>
+__device__ __forceinline__ void slice_step(const SliceSet& S, int s, unsigned m, unsigned base,
+                                           Get get, Mac mac, Load load, Epi epi) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const bool has = m != kNoRow;
+  const int len = has ? static_cast<int>(m >> 8) : 0;
+  const int row = slice_row(s, m);
+  double ops[NR > 0 ? NR : 1];
+  if (has) load(row, ops);
+  const int width = __shfl_sync(0xffffffffu, len, 0);  // lane 0 holds the longest row
+  const size_t at = static_cast<size_t>(base) * 32 + static_cast<size_t>(lane);
+  const int* __restrict__ ip = S.idx + at;
+  const double* __restrict__ vp = S.val + at;
+  double acc[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) acc[q] = 0.0;
+  for (int k = 0; k < width; k += kSliceBatch) {
+    int c[kSliceBatch];
+    double v[kSliceBatch];
+#pragma unroll
+    for (int u = 0; u < kSliceBatch; ++u) {
+      const bool in = k + u < len;
+      c[u] = in ? ld_stream(ip + (k + u) * 32) : -1;
+      v[u] = in ? ld_stream(vp + (k + u) * 32) : 0.0;
+    }
+    G g[kSliceBatch];
+#pragma unroll
+    for (int u = 0; u < kSliceBatch; ++u) g[u] = c[u] >= 0 ? get(c[u]) : G{};
+#pragma unroll
+    for (int u = 0; u < kSliceBatch; ++u) {
+      if (k + u < width) mac(v[u], g[u], acc);
+    }
+  }
+  if (has) epi(row, acc, ops);
+}
+
+// One long item, by the whole warp.
+template <int NP, int NR, typename G, typename Get, typename Mac, typename Load, typename Epi>
+__device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& it,
+                                           double* chunk_part, Get get, Mac mac, Load load,
+                                           Epi epi) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int* __restrict__ ip = S.idx + S.long_base + it.begin;
+  const double* __restrict__ vp = S.val + S.long_base + it.begin;
+  double ops[NR > 0 ? NR : 1];
+  if (it.slot < 0 && lane == 0) load(it.row, ops);
+  double acc[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) acc[q] = 0.0;
+  for (int k = lane; k < it.count; k += 32 * kSliceBatch) {
+    int c[kSliceBatch];
+    double v[kSliceBatch];
+#pragma unroll
+    for (int u = 0; u < kSliceBatch; ++u) {
+      const bool in = k + 32 * u < it.count;
+      c[u] = in ? ld_stream(ip + k + 32 * u) : -1;
+      v[u] = in ? ld_stream(vp + k + 32 * u) : 0.0;
+    }
+    G g[kSliceBatch];
+#pragma unroll
+    for (int u = 0; u < kSliceBatch; ++u) g[u] = c[u] >= 0 ? get(c[u]) : G{};
+#pragma unroll
+    for (int u = 0; u < kSliceBatch; ++u) mac(v[u], g[u], acc);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < NP; ++q) acc[q] = warp_sum(acc[q]);
+  if (lane != 0) return;
+  if (it.slot < 0) {
+    epi(it.row, acc, ops);
+  } else {
+#pragma unroll
+    for (int q = 0; q < NP; ++q) chunk_part[it.slot * NP + q] = acc[q];
+  }
+}
+
+// Visit this block's rows (a multiple of 32 threads; every thread calls it):
+//   fetch(c) reads element c of the gathered vector from global memory; where the layout has
+//   windows they are staged from `vec`, the same vector
+//   mac(v, g, acc) adds the entry's products
+//   load(row, ops), epi(row, acc, ops) the row's NR operands and its epilogue
+// WIN is false in kernels that stage no window whatever the layout has. Returns false -- in
+// every thread -- if a wait gave up (only a staged window waits).
+template <bool WIN, int NP, int NR, typename G, typename Fetch, typename Mac, typename Load,
+          typename Epi>
+__device__ __forceinline__ bool run_slices(const SliceSet& S, const G* vec, Fetch fetch,
+                                           unsigned char* dsmem, double* chunk_part, Mac mac,
+                                           Load load, Epi epi) {
+  __shared__ volatile int s_abort;
+  const int W = static_cast<int>(blockDim.x) >> 5;
+  const int warp = static_cast<int>(threadIdx.x) >> 5;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(dsmem);
+  G* win = reinterpret_cast<G*>(dsmem + kSliceBarBytes);
+  const bool windowed = WIN && S.wmax > 0;
+  if (windowed) {
+    if (threadIdx.x == 0) {
+      s_abort = 0;
+      mbar_init(bar, 1);
+      fence_mbar_init();
+    }
+    __syncthreads();
+  }
+  bool pending = false;  // thread 0: a copy issued and not yet seen complete
+  uint32_t phase = 0;
+  const int g0 = S.seg_start[blockIdx.x], g1 = S.seg_start[blockIdx.x + 1];
+  bool ok = true;
+  for (int g = g0; g < g1; ++g) {
+    const SliceSeg sg = S.segs[g];
+    if (WIN && sg.len > 0) {
+      if (g != g0) __syncthreads();  // every warp is done with the window held
+      if (threadIdx.x == 0) {
+        const uint32_t bytes = static_cast<uint32_t>(sg.len) * static_cast<uint32_t>(sizeof(G));
+        fence_proxy_async_smem();
+        mbar_arrive_expect_tx(bar, bytes);
+        bulk_copy_g2s(win, vec + sg.lo, bytes, bar);
+        pending = true;
+      }
+      if (mbar_wait_or_abort(bar, phase, &s_abort)) {
+        pending = false;
+      } else {
+        s_abort = 1;
+      }
+      phase ^= 1u;
+      __syncthreads();
+      ok = s_abort == 0;
+    }
+    if (!ok) break;
+    const int lo = sg.lo;
+    const unsigned len = static_cast<unsigned>(sg.len);
+    auto get = [&](int c) {
+      const unsigned o = static_cast<unsigned>(c - lo);
+      return WIN && o < len ? win[o] : fetch(c);
+    };
+    if (g == g0) {
+      for (int i = static_cast<int>(blockIdx.x) + warp * static_cast<int>(gridDim.x);
+           i < S.nitems; i += W * static_cast<int>(gridDim.x)) {
+        slice_item<NP, NR, G>(S, S.items[i], chunk_part, get, mac, load, epi);
+      }
+    }
+    // The next slice's meta word and base are loaded while this one is worked on.
+    int s = sg.s0 + warp;
+    unsigned m = kNoRow, base = 0;
+    if (s < sg.s1) {
+      m = __ldg(S.meta + static_cast<size_t>(s) * 32 + lane);
+      base = __ldg(S.base + s);
+    }
+    for (; s < sg.s1; s += W) {
+      const unsigned cm = m, cb = base;
+      const int sn = s + W;
+      if (sn < sg.s1) {
+        m = __ldg(S.meta + static_cast<size_t>(sn) * 32 + lane);
+        base = __ldg(S.base + sn);
+      }
+      slice_step<NP, NR, G>(S, s, cm, cb, get, mac, load, epi);
+    }
+  }
+  if (!windowed || ok) return true;
+  // A copy still in flight must land before the block exits (bounded).
+  if (threadIdx.x == 0 && pending) mbar_wait_bounded(bar, phase ^ 1u);
+  __syncthreads();
+  return false;
+}
+
+// Last block only: the rows of several pieces, each combined from its partials in order.
+template <int NP, int NR, typename Load, typename Epi>
+__device__ __forceinline__ void run_slice_long_rows(const SliceSet& S, const double* chunk_part,
+                                                    Load load, Epi epi) {
+  for (int l = threadIdx.x; l < S.nlong; l += blockDim.x) {
+    const LongRow lr = S.longs[l];
+    double acc[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) acc[q] = 0.0;
+    for (int c = 0; c < lr.nchunks; ++c) {
+#pragma unroll
+      for (int q = 0; q < NP; ++q) acc[q] += __ldcg(chunk_part + (lr.chunk0 + c) * NP + q);
+    }
+    double ops[NR > 0 ? NR : 1];
+    load(lr.row, ops);
+    epi(lr.row, acc, ops);
+  }
+}
+
+}  // namespace sgb

@@ -1,0 +1,100 @@
+"""The FP64 passes' sliced layouts (csrc/slices.cuh).
+
+* On the CPU, `tests/host/slices_check.cu` checks plan_slices on every row count around a slice
+  and a group, and on row lengths around the long-row limit (64) and a piece (2,048).
+* On the GPU, the preconditioner, the products and a short FP64 solve over the same lengths
+  against the oracle: the scaling bit for bit; products within (2 + n_i) u sum |a_ij| |x_j| of the
+  oracle's, u = 2^-53 and n_i the row's entries (each side rounds once or twice per entry); the
+  solve's point after 40 accepted steps within 1e-9 (its rounding differences, measured at 1e-13
+  on LPs of these sizes, grow with the iterations).
+"""
+import os
+import shutil
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from sankhya_gb300 import capi
+from sankhya_gb300.model import LP
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def test_sliced_layouts(tmp_path):
+    nvcc = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc is not available")
+    from sankhya_gb300 import _paths, build
+
+    build.build_engine()
+    objdir = os.path.join(os.path.dirname(_paths.ENGINE_LIB), "obj")
+    objs = [os.path.join(objdir, s.replace(".cu", ".o")) for s in build.CUDA_SOURCES]
+    exe = str(tmp_path / "slices_check")
+    cmd = ([nvcc] + build.ARCH + ["-O2", "-std=c++17", "--expt-relaxed-constexpr", "-I",
+                                  _paths.INCLUDE_DIR, "-I", _paths.CSRC_DIR,
+                                  os.path.join(ROOT, "tests", "host", "slices_check.cu")] + objs +
+           ["-lcudart", "-o", exe])
+    proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    assert proc.returncode == 0, proc.stdout
+    run = subprocess.run([exe], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True,
+                         timeout=300)
+    assert run.returncode == 0 and run.stdout.startswith("OK"), run.stdout
+
+
+def lp_with_rows(lengths, n, seed):
+    """An LP whose row i has lengths[i] entries (at distinct random columns), with feasible
+    equality and range rows around a point of the box."""
+    rng = np.random.default_rng(seed)
+    m = len(lengths)
+    rows = [np.sort(rng.choice(n, size=k, replace=False)) for k in lengths]
+    r = np.repeat(np.arange(m), [len(c) for c in rows])
+    c = np.concatenate(rows) if m else np.zeros(0, int)
+    order = np.lexsort((r, c))
+    r, c = r[order], c[order]
+    v = rng.normal(size=len(r))
+    starts = np.zeros(n + 1, np.int32)
+    np.cumsum(np.bincount(c, minlength=n), out=starts[1:])
+    x = rng.uniform(0, 10, n)
+    ax = np.bincount(r, v * x[c], m)
+    slack = np.where(rng.random(m) < 0.5, 0.0, 1.0)
+    return LP(m, n, starts, r.astype(np.int32), v, rng.normal(size=n), np.zeros(n),
+              np.full(n, 10.0), ax - slack, ax + slack)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,longest", [(1, 1, 1), (31, 40, 12), (129, 257, 30), (130, 70, 66),
+                                         (40, 2060, 2050), (300, 6200, 6150)])
+def test_slices_match_the_oracle(oracle, m, n, longest):
+    rng = np.random.default_rng(m + n)
+    lengths = rng.integers(0, min(n, 21), size=m)
+    for k, want in enumerate((longest, 0, 64, 65, 2048, 2049)):
+        if k < m and want <= min(n, longest):
+            lengths[(k * 37) % m] = want
+    lp = lp_with_rows(lengths, n, seed=m)
+    a = LP(lp.rows, lp.cols, lp.col_starts, lp.row_index, np.abs(lp.values), lp.col_cost,
+           lp.col_lower, lp.col_upper, lp.row_lower, lp.row_upper)
+    u = 2.0 ** -53
+    with capi.PdhgEngine(0) as eng:
+        eng.load(lp)
+        x, y = rng.normal(size=n), rng.normal(size=m)
+        for op, v, f, entries in ((0, x, "multiply", lengths),
+                                  (1, y, "transpose_multiply", np.diff(lp.col_starts))):
+            bound = (2 + entries) * u * getattr(oracle, f)(a, np.abs(v))
+            assert np.all(np.abs(eng.spmv(op, v) - getattr(oracle, f)(lp, v)) <= bound)
+        dr, dc, values, norm = eng.scaling()
+        ref = oracle.build_scaling(lp)
+        assert np.array_equal(dr, ref["row"]) and np.array_equal(dc, ref["col"])
+        assert np.array_equal(values, ref["values"])
+        got = eng.solve(tolerance=1e-13, iteration_limit=40)
+        px, _, py = eng.solution()
+    ref = oracle.solve(lp, tolerance=1e-13, iteration_limit=40)
+    if ref.status_name != "iteration_limit" or got.status_name != "iteration_limit":
+        # The smallest LPs are solved before the limit: the points are then both optimal.
+        assert got.status_name == ref.status_name
+        assert abs(got.objective - ref.objective) <= 1e-6 * max(1.0, abs(ref.objective))
+        return
+    scale = max(1.0, np.abs(ref.col_value).max())
+    assert np.abs(px - ref.col_value).max() <= 1e-9 * scale
+    assert np.abs(py - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
