@@ -114,6 +114,18 @@ void BatchEngine::load(int count, const sankhya_gb300_lp* lps) {
         rval[base + slot] = lp.values[k];
       }
     }
+    // Slice padding of a compact basis matrix in either orientation (ensure_adjoint_buffers).
+    const auto padding = [](const int* p, int lines) {
+      long long longest = 0, past = 0;
+      for (int q = 0; q < lines; ++q) {
+        const long long len = p[q + 1] - p[q];
+        longest = std::max(longest, len);
+        past += len > kSortLength;
+      }
+      return 32 * longest * (2 + (past + 31) / 32);
+    };
+    mats_.back().line_padding =
+        std::max(padding(r.data(), m), padding(lp.col_starts, n));
     rptr.insert(rptr.end(), r.begin(), r.end());
     nz += nnz;
     cp += n + 1;
@@ -589,8 +601,8 @@ void BatchEngine::adjoint(const double* const* dl_dx, const double* const* dl_dy
                            cudaMemcpyHostToDevice, s));
   AdjointBuffers a = adjoint_buffers();
   SGB_CUDA(cudaMemsetAsync(d_queue_.ptr + 2, 0, sizeof(unsigned int), s));
-  const int grid =
-      std::max(1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a.smem_vec)));
+  const int grid = std::max(
+      1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a.threads, a.smem_bytes)));
   launch_batch_adjoint(buffers_, a, grid, s);
   SGB_CUDA(cudaGetLastError());
   finish_adjoint(dl_dc, dl_drl, dl_dru, dl_dl, dl_du, info);
@@ -607,18 +619,34 @@ void BatchEngine::ensure_adjoint_buffers() {
   a_cpos_.allocate(N);
   a_rrow_.allocate(M);
   a_rpos_.allocate(M);
-  a_kcp_.allocate(N + static_cast<size_t>(count_));
-  a_krp_.allocate(M + static_cast<size_t>(count_));
-  // Each LP's compact basis matrix holds at most its matrix's entries.
+  a_tmp_.allocate(M);
+  a_kcl_.allocate(M);
+  a_krl_.allocate(M);
+  a_kcb_.allocate(M + static_cast<size_t>(count_));
+  a_krb_.allocate(M + static_cast<size_t>(count_));
+  // Each LP's compact basis matrix holds at most its matrix's entries, and its slices' padding:
+  // lines come longest first, so a slice is no wider than the lines of the slice before it, which
+  // leaves the first slice (and those of lines past the sort's range) to be covered.
   std::vector<long long> knz(static_cast<size_t>(count_));
   long long nz = 0;
-  int dim = 1;
+  const size_t room = static_cast<size_t>(adjoint_max_smem());
+  size_t need = 0, likely = 0;
   for (int k = 0; k < count_; ++k) {
     const BatchInstance& I = inst_[static_cast<size_t>(k)];
+    const BatchMatrix& M = mats_[static_cast<size_t>(I.matrix)];
     knz[static_cast<size_t>(k)] = nz;
-    nz += mats_[static_cast<size_t>(I.matrix)].nnz;
-    dim = std::max(dim, std::min(I.m, I.n));
+    nz += M.nnz + M.line_padding;
+    // Shared memory that holds the LP's solves whatever its basis, and with a basis of half
+    // its entries (solve_basis: six vectors, both matrices, the slices' records).
+    const size_t d = static_cast<size_t>(std::min(I.m, I.n));
+    const size_t z = static_cast<size_t>(M.nnz);
+    need = std::max(need, 64 * d + 20 * (z + 64 * 16) + 256);
+    likely = std::max(likely, 64 * d + 11 * z);
   }
+  // One block of 256 threads holds the FP64 pipe busy from shared memory; gathers from global
+  // memory want more warps in flight.
+  a_smem_ = static_cast<int>(std::min(room, need)) & ~15;
+  a_threads_ = likely <= room ? 256 : kAdjThreads;
   const size_t Z = static_cast<size_t>(std::max(nz, 1LL));
   a_kci_.allocate(Z);
   a_kri_.allocate(Z);
@@ -627,7 +655,6 @@ void BatchEngine::ensure_adjoint_buffers() {
   a_knz_.allocate(knz.size());
   SGB_CUDA(cudaMemcpy(a_knz_.ptr, knz.data(), knz.size() * sizeof(long long),
                       cudaMemcpyHostToDevice));
-  a_smem_vec_ = std::min(dim, kAdjSmemVec);
   a_gf_.allocate(static_cast<size_t>(count_));
   a_cs_.allocate(N);
   a_rs_.allocate(M);
@@ -650,8 +677,11 @@ AdjointBuffers BatchEngine::adjoint_buffers() {
   a.cpos = a_cpos_.ptr;
   a.rrow = a_rrow_.ptr;
   a.rpos = a_rpos_.ptr;
-  a.kcp = a_kcp_.ptr;
-  a.krp = a_krp_.ptr;
+  a.kcl = a_kcl_.ptr;
+  a.krl = a_krl_.ptr;
+  a.kcb = a_kcb_.ptr;
+  a.krb = a_krb_.ptr;
+  a.tmp = a_tmp_.ptr;
   a.kci = a_kci_.ptr;
   a.kri = a_kri_.ptr;
   a.kcv = a_kcv_.ptr;
@@ -662,7 +692,8 @@ AdjointBuffers BatchEngine::adjoint_buffers() {
   a.outcome = a_out_.ptr;
   a.max_iterations = 20000;
   a.cg_tolerance = 1e-13;
-  a.smem_vec = a_smem_vec_;
+  a.threads = a_threads_;
+  a.smem_bytes = a_smem_;
   return a;
 }
 
@@ -722,8 +753,8 @@ void BatchEngine::polish(sankhya_gb300_batch_item* items, sankhya_gb300_adjoint_
   ensure_adjoint_buffers();
   AdjointBuffers a = adjoint_buffers();
   SGB_CUDA(cudaMemsetAsync(d_queue_.ptr + 3, 0, sizeof(unsigned int), s));
-  const int grid =
-      std::max(1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a.smem_vec)));
+  const int grid = std::max(
+      1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a.threads, a.smem_bytes)));
   launch_batch_polish(buffers_, a, grid, s);
   SGB_CUDA(cudaGetLastError());
   std::vector<BatchOutcome> out(static_cast<size_t>(count_));

@@ -28,11 +28,11 @@ namespace sgb {
 
 constexpr int kBatchThreads = 256;     // scaling launches
 constexpr int kBatchMaxThreads = 512;  // the largest block a batched solve runs with
-constexpr int kAdjThreads = 512;       // adjoint and polish launches
-constexpr int kAdjVectors = 9;         // compact per-LP vectors of the square solves
-// The square solves gather from two vectors of |B| entries; they sit in shared memory for
-// |B| up to this many (2 x 96 KB), else in global memory.
-constexpr int kAdjSmemVec = 12288;
+constexpr int kAdjThreads = 512;       // adjoint and polish launches, at most
+constexpr int kAdjVectors = 8;         // compact per-LP vectors of the square solves
+
+// Lines of a basis matrix longer than this are ordered among the longest in index order.
+constexpr int kSortLength = 1023;
 
 // A distinct constraint matrix. Offsets index the packed arrays of BatchBuffers.
 struct BatchMatrix {
@@ -45,6 +45,7 @@ struct BatchMatrix {
   long long nnz;
   double spectral_norm;  // written by the scaling launch
   double scaled_min_abs, scaled_max_abs;
+  long long line_padding;  // most padding the slices of a compact basis matrix can need
 };
 
 // One LP of the batch.
@@ -120,25 +121,29 @@ struct AdjointBuffers {
   double* kw[kAdjVectors];                         // m-sized compact vectors per LP
   int *bcol, *cpos;                                // basic columns; a column's number in B
   int *rrow, *rpos;                                // active rows; a row's number in R
-  int *kcp, *krp;                                  // A_RB's CSC / CSR starts (n+1, m+1 per LP)
-  int *kci, *kri;                                  // their entries' positions
+  int *kcl, *krl;                                  // A_RB's sliced lines: lengths (m per LP),
+  unsigned *kcb, *krb;                             // slice bases (m + 1 per LP),
+  int *kci, *kri;                                  // entries' positions
   double *kcv, *krv;                               // and values
   const long long* knz;                            // per LP: offset of its entries
   signed char *col_state, *row_state;              // active sets
   AdjointOutcome* outcome;
   int max_iterations;                              // per conjugate-gradient run
   double cg_tolerance;
-  int smem_vec;                                    // |B| up to which the gathers use smem
+  int* tmp;                                        // m per LP
+  int threads, smem_bytes;                         // of the launches
 };
 
 void launch_batch_scaling(const BatchBuffers& b, int grid, cudaStream_t s);
-// The adjoint and polish launches run kAdjThreads-thread blocks with 2 * a.smem_vec
-// doubles of dynamic shared memory; adjoint_blocks_per_sm is their occupancy.
+// The adjoint and polish launches run blocks of a.threads threads with a.smem_bytes of dynamic
+// shared memory; adjoint_max_smem is the most they can have, adjoint_blocks_per_sm their
+// occupancy.
 void launch_batch_adjoint(const BatchBuffers& b, const AdjointBuffers& a, int grid,
                           cudaStream_t s);
 void launch_batch_polish(const BatchBuffers& b, const AdjointBuffers& a, int grid,
                          cudaStream_t s);
-int adjoint_blocks_per_sm(int smem_vec);
+int adjoint_max_smem();
+int adjoint_blocks_per_sm(int threads, int smem_bytes);
 // The solve launches run blocks of `threads` threads (a multiple of 32, at most
 // kBatchMaxThreads); the occupancy queries are for that block size.
 void launch_batch_solve(const BatchBuffers& b, int grid, int threads, cudaStream_t s);

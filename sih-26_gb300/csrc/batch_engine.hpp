@@ -89,10 +89,11 @@ class BatchEngine {
   bool adjoint_ready_ = false;
   DeviceArray<double> a_gx_, a_gy_, a_gf_, a_dc_, a_dl_, a_du_, a_drl_, a_dru_;
   DeviceArray<double> a_kw_[kAdjVectors];
-  DeviceArray<int> a_bcol_, a_cpos_, a_rrow_, a_rpos_, a_kcp_, a_krp_, a_kci_, a_kri_;
+  DeviceArray<int> a_bcol_, a_cpos_, a_rrow_, a_rpos_, a_kcl_, a_krl_, a_kci_, a_kri_, a_tmp_;
+  DeviceArray<unsigned int> a_kcb_, a_krb_;
   DeviceArray<double> a_kcv_, a_krv_;
   DeviceArray<long long> a_knz_;
-  int a_smem_vec_ = 0;
+  int a_smem_ = 0, a_threads_ = 256;
   DeviceArray<signed char> a_cs_, a_rs_;
   DeviceArray<AdjointOutcome> a_out_;
   long long total_n_ = 0, total_m_ = 0, mat_n_ = 0, mat_m_ = 0;

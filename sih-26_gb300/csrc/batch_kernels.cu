@@ -1229,10 +1229,15 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 2) k_batch_solve_mixed(Batch
 // minimise space (cost sense * c, as src/pdhg/pdhg.cpp:95-111 folds it); the host folds the
 // sense into g_y, g_f and dL/dc, so a maximisation LP is differentiated the same way.
 //
-// The basis matrix is built once per LP in compact form: B and R numbered 0..|B|-1 in index
-// order, A_RB stored as a CSR (lines: active rows; entries: basic-column numbers) and as a
-// CSC (lines: basic columns; entries: active-row numbers). The solves' products then read no
-// masks and gather from vectors of length |B| kept in shared memory. A square solve
+// The basis matrix is built once per LP in compact form: R and B numbered 0..|B|-1 longest line
+// first (lines of equal length in index order), A_RB stored twice as sliced lines (slices.cuh:
+// 32 lines a slice, entry e of lane l at base + 32 e + l), by active rows with basic-column
+// numbers and by basic columns with active-row numbers. Products read no masks and no scattered
+// matrix entries, and the lines a warp sums have nearly the same length (GB300's FP64 pipe
+// charges a warp for its longest). Where both copies and the solve's six vectors fit the
+// block's shared memory they are kept there for the LP's two solves (an iteration then touches
+// no global memory); else the vectors alone are, else the two gathered ones, else none. A square
+// solve
 // S u = h (S = A_RB or A_RB') runs as iterative refinement around the normal equations of
 // the second kind: u += F z with (S F) z = h - S u and F = S', by conjugate gradients with
 // the diagonal of S F (the squared lengths of S's lines) as preconditioner. Each pass starts
@@ -1245,8 +1250,10 @@ struct AdjView {
   double *dc, *dl, *du, *drl, *dru;
   double* kw[kAdjVectors];  // compact vectors (|B| entries used)
   int *bcol, *cpos, *rrow, *rpos;
-  int *kcp, *kci, *krp, *kri;
-  double *kcv, *krv;
+  int *kcl, *kci, *krl, *kri;   // sliced lines: lengths and entries' positions,
+  unsigned *kcb, *krb;          // slice bases,
+  double *kcv, *krv;            // and values
+  int* tmp;                     // m entries
   signed char *cs, *rs;
 };
 
@@ -1266,8 +1273,11 @@ __device__ AdjView make_adj_view(const AdjointBuffers& a, const BatchInstance& I
   w.cpos = a.cpos + c;
   w.rrow = a.rrow + r;
   w.rpos = a.rpos + r;
-  w.kcp = a.kcp + c + li;
-  w.krp = a.krp + r + li;
+  w.kcl = a.kcl + r;
+  w.krl = a.krl + r;
+  w.kcb = a.kcb + r + li;
+  w.krb = a.krb + r + li;
+  w.tmp = a.tmp + r;
   w.kci = a.kci + z;
   w.kri = a.kri + z;
   w.kcv = a.kcv + z;
@@ -1275,20 +1285,6 @@ __device__ AdjView make_adj_view(const AdjointBuffers& a, const BatchInstance& I
   w.cs = a.col_state + c;
   w.rs = a.row_state + r;
   return w;
-}
-
-// block_sum with the totals handed to every thread.
-template <int NV>
-__device__ __forceinline__ void all_sum(double (&v)[NV], double* scratch, double (&out)[NV]) {
-  __shared__ double s_all[NV];
-  block_sum<NV>(v, scratch, out);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) s_all[q] = out[q];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < NV; ++q) out[q] = s_all[q];
 }
 
 // Exclusive prefix sum of one int per thread over the block (blockDim a multiple of 32);
@@ -1336,21 +1332,6 @@ __device__ int compact_set(int count, On on, int* list, int* pos) {
   }
   __syncthreads();
   return base;
-}
-
-// ptr[k] (k < count) holds line k's length on entry and its first entry on exit; ptr[count]
-// receives the total.
-__device__ void starts_from_lengths(int* ptr, int count) {
-  int base = 0;
-  for (int start = 0; start < count; start += blockDim.x) {
-    const int k = start + threadIdx.x;
-    int total = 0;
-    const int e = block_scan(k < count ? ptr[k] : 0, &total);
-    if (k < count) ptr[k] = base + e;
-    base += total;
-  }
-  if (threadIdx.x == 0) ptr[count] = base;
-  __syncthreads();
 }
 
 // The active sets of a reported point (best_x, reduced costs, best_y): column states 0 basic,
@@ -1407,6 +1388,82 @@ __device__ void b_active_sets(const LpView& v, const AdjView& w, double* scratch
   __syncthreads();
 }
 
+// Reorders list (count entries, in index order) by len(list[k]), longest first and stable, through
+// tmp; pos[list[k]] becomes k and out_len[k] the length.
+template <typename Len>
+__device__ void order_by_length(int count, Len len, int* list, int* pos, int* tmp, int* out_len) {
+  __shared__ int s_bin[kSortLength + 1];
+  const int T = blockDim.x, t = threadIdx.x, lane = t & 31;
+  for (int q = t; q <= kSortLength; q += T) s_bin[q] = 0;
+  __syncthreads();
+  for (int k = t; k < count; k += T) {
+    const int l = len(list[k]);
+    atomicAdd(&s_bin[kSortLength - (l < kSortLength ? l : kSortLength)], 1);
+  }
+  __syncthreads();
+  if (t < 32) {
+    // Exclusive prefix sum of the bins, 32 of them at a time.
+    int base = 0;
+    for (int q = 0; q <= kSortLength; q += 32) {
+      const int v = s_bin[q + lane];
+      int x = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      s_bin[q + lane] = base + x - v;
+      base += __shfl_sync(0xffffffffu, x, 31);
+    }
+    __syncwarp();
+    // One warp places the lines in index order, 32 at a time: stable, so reproducible.
+    for (int k0 = 0; k0 < count; k0 += 32) {
+      const int k = k0 + lane;
+      const bool in = k < count;
+      const int l = in ? len(list[k]) : 0;
+      const int bin = in ? kSortLength - (l < kSortLength ? l : kSortLength) : -1;
+      const unsigned same = __match_any_sync(0xffffffffu, bin);
+      const int rank = __popc(same & ((1u << lane) - 1u));
+      int at = 0;
+      if (in) at = s_bin[bin] + rank;
+      __syncwarp();
+      if (in) {
+        tmp[at] = list[k];
+        if (rank == 0) s_bin[bin] += __popc(same);
+      }
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int k = t; k < count; k += T) {
+    const int item = tmp[k];
+    list[k] = item;
+    pos[item] = k;
+    out_len[k] = len(item);
+  }
+  __syncthreads();
+}
+
+// Slices of `count` lines of the given lengths: base[s] receives slice s's first entry / 32 and
+// base[slices] the total. A slice is as wide as its longest line.
+__device__ void slice_bases(const int* len, int count, unsigned* base) {
+  const int T = blockDim.x, t = threadIdx.x;
+  const int slices = (count + 31) / 32;
+  int sum = 0;
+  for (int start = 0; start < slices; start += T) {
+    const int s = start + t;
+    int width = 0;
+    if (s < slices) {
+      for (int k = s * 32; k < count && k < s * 32 + 32; ++k) width = len[k] > width ? len[k] : width;
+    }
+    int total = 0;
+    const int e = block_scan(width, &total);
+    if (s < slices) base[s] = static_cast<unsigned>(sum + e);
+    sum += total;
+  }
+  if (t == 0) base[slices] = static_cast<unsigned>(sum);
+  __syncthreads();
+}
+
 // The compact basis matrix of the active sets in w.cs / w.rs (see above). Returns |B|, with
 // |R| in *nr; the matrix is built only when they are equal.
 __device__ int build_basis(const LpView& v, const AdjView& w, int* nr) {
@@ -1415,38 +1472,43 @@ __device__ int build_basis(const LpView& v, const AdjView& w, int* nr) {
   const int na = compact_set(v.m, [&](int i) { return w.rs[i] != 0; }, w.rrow, w.rpos);
   *nr = na;
   if (nb != na) return nb;
+  order_by_length(
+      nb,
+      [&](int i) {
+        int len = 0;
+        for (int k = v.rp[i]; k < v.rp[i + 1]; ++k) len += w.cs[v.ri[k]] == 0 ? 1 : 0;
+        return len;
+      },
+      w.rrow, w.rpos, w.tmp, w.krl);
+  order_by_length(
+      nb,
+      [&](int j) {
+        int len = 0;
+        for (int k = v.cp[j]; k < v.cp[j + 1]; ++k) len += w.rs[v.ci[k]] != 0 ? 1 : 0;
+        return len;
+      },
+      w.bcol, w.cpos, w.tmp, w.kcl);
+  slice_bases(w.krl, nb, w.krb);
+  slice_bases(w.kcl, nb, w.kcb);
   for (int p = t; p < nb; p += T) {
     const int i = w.rrow[p];
-    int len = 0;
-    for (int k = v.rp[i]; k < v.rp[i + 1]; ++k) len += w.cpos[v.ri[k]] >= 0 ? 1 : 0;
-    w.krp[p] = len;
-    const int j = w.bcol[p];
-    len = 0;
-    for (int k = v.cp[j]; k < v.cp[j + 1]; ++k) len += w.rpos[v.ci[k]] >= 0 ? 1 : 0;
-    w.kcp[p] = len;
-  }
-  __syncthreads();
-  starts_from_lengths(w.krp, nb);
-  starts_from_lengths(w.kcp, nb);
-  for (int p = t; p < nb; p += T) {
-    const int i = w.rrow[p];
-    int o = w.krp[p];
+    size_t o = static_cast<size_t>(w.krb[p >> 5]) * 32 + (p & 31);
     for (int k = v.rp[i]; k < v.rp[i + 1]; ++k) {
-      const int c = w.cpos[v.ri[k]];
-      if (c >= 0) {
-        w.kri[o] = c;
+      const int c = v.ri[k];
+      if (w.cs[c] == 0) {
+        w.kri[o] = w.cpos[c];
         w.krv[o] = v.rraw[k];
-        ++o;
+        o += 32;
       }
     }
     const int j = w.bcol[p];
-    o = w.kcp[p];
+    o = static_cast<size_t>(w.kcb[p >> 5]) * 32 + (p & 31);
     for (int k = v.cp[j]; k < v.cp[j + 1]; ++k) {
-      const int r = w.rpos[v.ci[k]];
-      if (r >= 0) {
-        w.kci[o] = r;
+      const int r = v.ci[k];
+      if (w.rs[r] != 0) {
+        w.kci[o] = w.rpos[r];
         w.kcv[o] = v.craw[k];
-        ++o;
+        o += 32;
       }
     }
   }
@@ -1454,67 +1516,104 @@ __device__ int build_basis(const LpView& v, const AdjView& w, int* nr) {
   return nb;
 }
 
-// A compact line matrix: line k holds entries ptr[k] .. ptr[k+1]-1 (positions, values).
+// Sliced lines; I is int in global memory and unsigned short in shared memory.
+template <typename I>
 struct Lines {
-  const int *ptr, *idx;
+  const int* len;
+  const unsigned* base;
+  const I* idx;
   const double* val;
 };
 
-__device__ __forceinline__ double line_dot(const Lines& L, int k, const double* x) {
+template <typename I>
+__device__ __forceinline__ double line_dot(const Lines<I>& L, int k, const double* x) {
+  const int n = L.len[k];
+  size_t e = static_cast<size_t>(L.base[k >> 5]) * 32 + (k & 31);
   double s = 0.0;
-  for (int e = L.ptr[k]; e < L.ptr[k + 1]; ++e) s = fma(L.val[e], x[L.idx[e]], s);
+#pragma unroll 4
+  for (int q = 0; q < n; ++q, e += 32) s = fma(L.val[e], x[L.idx[e]], s);
   return s;
 }
 
-// Conjugate gradients on (S F) z = h from z = 0, preconditioned by diag. p and t are the
-// two gathered vectors (shared memory when |B| fits). Stops when ||h - S F z|| (the
-// recurrence's residual) is at most tol ||h||. Returns the iterations.
-__device__ int pcg_sf(const Lines& S, const Lines& F, int nb, const double* h, double* z,
-                      double* r, double* wv, const double* diag, double* p, double* t,
-                      double* scratch, int max_it, double tol) {
+// Block-wide sums handed to every thread, in one barrier: each warp's total goes to `scratch`
+// (NV * 32 doubles, not in use by the reduction before this one), and every warp adds the
+// totals in the same order. The barrier also publishes what the threads wrote before it.
+template <int NV>
+__device__ __forceinline__ void quick_sum(double (&v)[NV], double* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    const double s = warp_sum(v[q]);
+    if (lane == 0) scratch[q * 32 + warp] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    double s = lane < nw ? scratch[q * 32 + lane] : 0.0;
+    for (int o = nw >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    v[q] = __shfl_sync(0xffffffffu, s, 0);
+  }
+}
+
+// The vectors of a solve: p and t are gathered, dinv holds the reciprocal preconditioner.
+struct SqVectors {
+  double *p, *t, *r, *z, *q, *dinv;
+};
+constexpr int kSqVectors = 6;
+
+// Conjugate gradients on (S F) z = r from z = 0 (x.r holds the right-hand side), preconditioned
+// by x.dinv. Stops when the recurrence's residual is at most tol ||h||. Returns the iterations.
+// Bound by the FP64 pipe: per line and iteration the two products' entries and eight vector
+// operations. So no thread repeats a division: the reciprocals of the preconditioner are formed
+// once, and the two step scalars by one thread each while the other warps are in the products
+// (512 threads each forming the three scalars took as long as the products).
+template <typename I>
+__device__ __forceinline__ int pcg_sf(const Lines<I>& S, const Lines<I>& F, int nb,
+                                      const SqVectors& x, double* scratch, int max_it,
+                                      double tol) {
+  __shared__ double s_alpha, s_inv;
   const int T = blockDim.x, th = threadIdx.x;
+  double* const scr2 = scratch + 64;
   double a0[2] = {0.0, 0.0};
   for (int k = th; k < nb; k += T) {
-    const double rk = h[k], wk = rk / diag[k];
-    z[k] = 0.0;
-    r[k] = rk;
-    wv[k] = wk;
-    p[k] = wk;
+    const double rk = x.r[k], wk = rk * x.dinv[k];
+    x.z[k] = 0.0;
+    x.p[k] = wk;
     a0[0] = fma(rk, rk, a0[0]);
     a0[1] = fma(rk, wk, a0[1]);
   }
-  double s0[2];
-  all_sum<2>(a0, scratch, s0);
-  const double hnorm = sqrt(s0[0]);
-  double rw = s0[1], rnorm = hnorm;
+  quick_sum<2>(a0, scratch);
+  double rr = a0[0], rw = a0[1];
+  const double goal = tol * tol * rr;
   int it = 0;
-  while (hnorm > 0.0 && rnorm > tol * hnorm && it < max_it) {
+  while (rr > goal && it < max_it) {
     double a1[1] = {0.0};
     for (int k = th; k < nb; k += T) {
-      const double s = line_dot(F, k, p);
-      t[k] = s;
+      const double s = line_dot(F, k, x.p);
+      x.t[k] = s;
       a1[0] = fma(s, s, a1[0]);
     }
-    double pkp[1];
-    all_sum<1>(a1, scratch, pkp);  // also publishes t
-    if (!(pkp[0] > 0.0)) break;
-    const double alpha = rw / pkp[0];
+    quick_sum<1>(a1, scr2);  // also publishes t
+    if (!(a1[0] > 0.0)) break;
+    if (th == T - 1) s_alpha = rw / a1[0];
+    if (th == T - 33) s_inv = 1.0 / rw;
+    for (int k = th; k < nb; k += T) x.q[k] = line_dot(S, k, x.t);
+    __syncthreads();
+    const double alpha = s_alpha, inv = s_inv;
     double a2[2] = {0.0, 0.0};
     for (int k = th; k < nb; k += T) {
-      const double s = line_dot(S, k, t);
-      z[k] = fma(alpha, p[k], z[k]);
-      const double rk = fma(-alpha, s, r[k]), wk = rk / diag[k];
-      r[k] = rk;
-      wv[k] = wk;
+      x.z[k] = fma(alpha, x.p[k], x.z[k]);
+      const double rk = fma(-alpha, x.q[k], x.r[k]), wk = rk * x.dinv[k];
+      x.r[k] = rk;
+      x.q[k] = wk;
       a2[0] = fma(rk, rk, a2[0]);
       a2[1] = fma(rk, wk, a2[1]);
     }
-    double s2[2];
-    all_sum<2>(a2, scratch, s2);  // every thread is done reading p and t
-    rnorm = sqrt(s2[0]);
-    const double beta = s2[1] / rw;
-    rw = s2[1];
-    for (int k = th; k < nb; k += T) p[k] = fma(beta, p[k], wv[k]);
+    quick_sum<2>(a2, scratch);
+    rr = a2[0];
+    const double beta = a2[1] * inv;
+    rw = a2[1];
+    for (int k = th; k < nb; k += T) x.p[k] = fma(beta, x.p[k], x.q[k]);
     __syncthreads();
     ++it;
   }
@@ -1525,65 +1624,116 @@ constexpr int kRefinePasses = 3;
 constexpr double kPassReduction = 1e-12;
 
 // S u = h (F = S') by refinement passes around pcg_sf; u holds the starting point on entry
-// and the solution on exit, w.kw[2..6] are used as scratch. Returns the conjugate-gradient
-// iterations; *rel receives ||h - S u|| / ||h|| at the end (0 when h = 0).
-__device__ int solve_square(const Lines& S, const Lines& F, int nb, const double* h, double* u,
-                            const AdjView& w, double* p, double* t, double* scratch, int max_it,
-                            double tol, double* rel) {
+// and the solution on exit. Returns the conjugate-gradient iterations; *rel receives
+// ||h - S u|| / ||h|| at the end (0 when h = 0).
+template <typename I>
+__device__ __forceinline__ int solve_square(const Lines<I>& S, const Lines<I>& F, int nb,
+                                            const double* h, double* u, const SqVectors& x,
+                                            double* scratch, int max_it, double tol,
+                                            double* rel) {
   const int T = blockDim.x, th = threadIdx.x;
-  double* const res = w.kw[2];
-  double* const z = w.kw[3];
-  double* const r = w.kw[4];
-  double* const wv = w.kw[5];
-  double* const diag = w.kw[6];
   double a0[1] = {0.0};
   for (int k = th; k < nb; k += T) {
     double d = 0.0;
-    for (int e = S.ptr[k]; e < S.ptr[k + 1]; ++e) d = fma(S.val[e], S.val[e], d);
-    diag[k] = d > 0.0 ? d : 1.0;
+    size_t e = static_cast<size_t>(S.base[k >> 5]) * 32 + (k & 31);
+    for (int q = 0; q < S.len[k]; ++q, e += 32) d = fma(S.val[e], S.val[e], d);
+    x.dinv[k] = d > 0.0 ? 1.0 / d : 1.0;
     a0[0] = fma(h[k], h[k], a0[0]);
   }
-  double hs[1];
-  all_sum<1>(a0, scratch, hs);
-  const double hnorm = sqrt(hs[0]);
+  quick_sum<1>(a0, scratch);
+  const double hnorm = sqrt(a0[0]);
   int its = 0;
   for (int pass = 0;; ++pass) {
     double a1[1] = {0.0};
     for (int k = th; k < nb; k += T) {
       const double rk = h[k] - line_dot(S, k, u);
-      res[k] = rk;
+      x.r[k] = rk;
       a1[0] = fma(rk, rk, a1[0]);
     }
-    double rs[1];
-    all_sum<1>(a1, scratch, rs);
-    const double rnorm = sqrt(rs[0]);
+    quick_sum<1>(a1, scratch + 64);
+    const double rnorm = sqrt(a1[0]);
     *rel = hnorm > 0.0 ? rnorm / hnorm : 0.0;
     if (*rel <= tol || pass == kRefinePasses) break;
     // A pass reduces its own residual to the final target, and by kPassReduction at least:
     // a solve started next to the answer (a polish from the PDHG point, or from a neighbour's
     // vertex, sankhya_gb300_batch_set_point) must still solve its small correction to full
     // accuracy, or two neighbouring solves carry different errors of the correction's size.
-    its += pcg_sf(S, F, nb, res, z, r, wv, diag, p, t, scratch, max_it,
-                  fmin(tol * hnorm / rnorm, kPassReduction));
-    for (int k = th; k < nb; k += T) u[k] += line_dot(F, k, z);
+    its += pcg_sf(S, F, nb, x, scratch, max_it, fmin(tol * hnorm / rnorm, kPassReduction));
+    __syncthreads();  // z is complete
+    for (int k = th; k < nb; k += T) u[k] += line_dot(F, k, x.z);
     __syncthreads();
   }
   return its;
 }
 
-// The two gathered vectors of a solve: shared memory when |B| fits, else w.kw[7], w.kw[8].
-struct Gathered {
-  double *p, *t;
-};
-
-__device__ Gathered gathered(const AdjointBuffers& a, const AdjView& w, double* s_vec, int nb) {
-  if (nb <= a.smem_vec) return Gathered{s_vec, s_vec + a.smem_vec};
-  return Gathered{w.kw[7], w.kw[8]};
+// The solve with the storage this LP gets (see above). `first` is the LP's first solve, which fills the shared copies;
+// `rows` solves with A_RB (S = rows), otherwise with its transpose.
+__device__ int solve_basis(const AdjointBuffers& a, const AdjView& w, unsigned char* smem, int nb,
+                           bool first, bool rows, const double* h, double* u, double* scratch,
+                           double* rel) {
+  const int T = blockDim.x, th = threadIdx.x;
+  const int slices = (nb + 31) / 32;
+  const size_t vec = static_cast<size_t>(kSqVectors) * nb * sizeof(double);
+  const size_t er = static_cast<size_t>(w.krb[slices]) * 32, ec = static_cast<size_t>(w.kcb[slices]) * 32;
+  const size_t mat = (er + ec) * (sizeof(double) + sizeof(unsigned short));
+  const size_t meta = 2 * (static_cast<size_t>(slices) + 1 + nb) * sizeof(int);
+  const size_t room = static_cast<size_t>(a.smem_bytes);
+  if (nb <= 65535 && vec + mat + meta <= room) {
+    double* const d = reinterpret_cast<double*>(smem);
+    const SqVectors x{d, d + nb, d + 2 * nb, d + 3 * nb, d + 4 * nb, d + 5 * nb};
+    double* const rv = d + kSqVectors * nb;
+    double* const cv = rv + er;
+    int* const rl = reinterpret_cast<int*>(cv + ec);
+    int* const cl = rl + nb;
+    unsigned* const rb = reinterpret_cast<unsigned*>(cl + nb);
+    unsigned* const cb = rb + slices + 1;
+    unsigned short* const ri = reinterpret_cast<unsigned short*>(cb + slices + 1);
+    unsigned short* const ci = ri + er;
+    if (first) {
+      // Padding is copied too; no line reads it.
+      for (size_t e = th; e < er; e += T) {
+        rv[e] = w.krv[e];
+        ri[e] = static_cast<unsigned short>(w.kri[e]);
+      }
+      for (size_t e = th; e < ec; e += T) {
+        cv[e] = w.kcv[e];
+        ci[e] = static_cast<unsigned short>(w.kci[e]);
+      }
+      for (int k = th; k < nb; k += T) {
+        rl[k] = w.krl[k];
+        cl[k] = w.kcl[k];
+      }
+      for (int k = th; k <= slices; k += T) {
+        rb[k] = w.krb[k];
+        cb[k] = w.kcb[k];
+      }
+      __syncthreads();
+    }
+    const Lines<unsigned short> r{rl, rb, ri, rv}, c{cl, cb, ci, cv};
+    return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
+                        a.cg_tolerance, rel);
+  }
+  const Lines<int> r{w.krl, w.krb, w.kri, w.krv}, c{w.kcl, w.kcb, w.kci, w.kcv};
+  if (vec <= room) {
+    double* const d = reinterpret_cast<double*>(smem);
+    const SqVectors x{d, d + nb, d + 2 * nb, d + 3 * nb, d + 4 * nb, d + 5 * nb};
+    return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
+                        a.cg_tolerance, rel);
+  }
+  if (2 * static_cast<size_t>(nb) * sizeof(double) <= room) {
+    double* const d = reinterpret_cast<double*>(smem);
+    const SqVectors x{d, d + nb, w.kw[4], w.kw[5], w.kw[6], w.kw[7]};
+    return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
+                        a.cg_tolerance, rel);
+  }
+  const SqVectors x{w.kw[2], w.kw[3], w.kw[4], w.kw[5], w.kw[6], w.kw[7]};
+  return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
+                      a.cg_tolerance, rel);
 }
 
-__global__ void __launch_bounds__(kAdjThreads, 2) k_batch_adjoint(BatchBuffers b,
+__global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b,
                                                                    AdjointBuffers a) {
-  extern __shared__ double s_vec[];
+  extern __shared__ __align__(16) unsigned char s_mem[];
   __shared__ double scratch[kBScratch];
   __shared__ int s_item;
   __shared__ LpView s_view;
@@ -1610,8 +1760,6 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_adjoint(BatchBuffers b
       for (int j = t; j < v.n; j += T) w.dc[j] = w.dl[j] = w.du[j] = 0.0;
       for (int i = t; i < v.m; i += T) w.drl[i] = w.dru[i] = 0.0;
     } else {
-      const Gathered g = gathered(a, w, s_vec, nb);
-      const Lines csr{w.krp, w.kri, w.krv}, csc{w.kcp, w.kci, w.kcv};
       double* const h = w.kw[0];
       double* const u = w.kw[1];
       // q: A_RB q = g_y[R] (the reported multipliers are -y and satisfy A_RB' y_R = c_B).
@@ -1620,8 +1768,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_adjoint(BatchBuffers b
         u[k] = 0.0;
       }
       __syncthreads();
-      it1 = solve_square(csr, csc, nb, h, u, w, g.p, g.t, scratch, a.max_iterations,
-                         a.cg_tolerance, &res1);
+      it1 = solve_basis(a, w, s_mem, nb, true, true, h, u, scratch, &res1);
       for (int j = t; j < v.n; j += T) {
         const int q = w.cpos[j];
         w.dc[j] = fma(w.gf, v.best_x[j], q >= 0 ? u[q] : 0.0);
@@ -1633,8 +1780,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_adjoint(BatchBuffers b
         u[k] = 0.0;
       }
       __syncthreads();
-      it2 = solve_square(csc, csr, nb, h, u, w, g.p, g.t, scratch, a.max_iterations,
-                         a.cg_tolerance, &res2);
+      it2 = solve_basis(a, w, s_mem, nb, false, false, h, u, scratch, &res2);
       for (int i = t; i < v.m; i += T) {
         const signed char st = w.rs[i];
         const double yrep = -v.best_y[i];  // the reported multiplier
@@ -1682,9 +1828,9 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_adjoint(BatchBuffers b
 // and status are rewritten.
 // AdjointOutcome.status: 0 polished, 1 degenerate, 2 a solve did not converge, 4 not a
 // converged solve, 5 the polished point failed the feasibility checks.
-__global__ void __launch_bounds__(kAdjThreads, 2) k_batch_polish(BatchBuffers b,
+__global__ void __launch_bounds__(kAdjThreads, 1) k_batch_polish(BatchBuffers b,
                                                                   AdjointBuffers a) {
-  extern __shared__ double s_vec[];
+  extern __shared__ __align__(16) unsigned char s_mem[];
   __shared__ double scratch[kBScratch];
   __shared__ int s_item;
   __shared__ LpView s_view;
@@ -1719,8 +1865,6 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_polish(BatchBuffers b,
       }
       continue;
     }
-    const Gathered g = gathered(a, w, s_vec, nb);
-    const Lines csr{w.krp, w.kri, w.krv}, csc{w.kcp, w.kci, w.kcv};
     double* const h = w.kw[0];
     double* const u = w.kw[1];
     // x_B from b_R - A_RN x_N, starting at the reported x_B.
@@ -1737,8 +1881,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_polish(BatchBuffers b,
     __syncthreads();
     int it1 = 0, it2 = 0;
     double res1 = 0.0, res2 = 0.0;
-    it1 = solve_square(csr, csc, nb, h, u, w, g.p, g.t, scratch, a.max_iterations,
-                       a.cg_tolerance, &res1);
+    it1 = solve_basis(a, w, s_mem, nb, true, true, h, u, scratch, &res1);
     for (int j = t; j < v.n; j += T) {
       const signed char st = w.cs[j];
       v.xu[1][j] = st == 0 ? u[w.cpos[j]] : (st == 1 ? v.l[j] : v.u[j]);
@@ -1750,8 +1893,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_polish(BatchBuffers b,
       u[k] = -v.best_y[w.rrow[k]];
     }
     __syncthreads();
-    it2 = solve_square(csc, csr, nb, h, u, w, g.p, g.t, scratch, a.max_iterations,
-                       a.cg_tolerance, &res2);
+    it2 = solve_basis(a, w, s_mem, nb, false, false, h, u, scratch, &res2);
     for (int i = t; i < v.m; i += T) {
       const int q = w.rpos[i];
       v.yu[1][i] = q >= 0 ? -u[q] : 0.0;  // the solver's sign
@@ -1843,39 +1985,35 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_batch_polish(BatchBuffers b,
 
 }  // namespace
 
-namespace {
-size_t adjoint_smem_bytes(int smem_vec) {
-  return 2 * static_cast<size_t>(smem_vec) * sizeof(double);
-}
-}  // namespace
-
 void launch_batch_adjoint(const BatchBuffers& b, const AdjointBuffers& a, int grid,
                           cudaStream_t s) {
-  const size_t bytes = adjoint_smem_bytes(a.smem_vec);
   // A failure here stays the last error, which the caller's launch check reports.
   cudaFuncSetAttribute(k_batch_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(bytes));
-  k_batch_adjoint<<<grid, kAdjThreads, bytes, s>>>(b, a);
+                       a.smem_bytes);
+  k_batch_adjoint<<<grid, a.threads, a.smem_bytes, s>>>(b, a);
 }
 
 void launch_batch_polish(const BatchBuffers& b, const AdjointBuffers& a, int grid,
                          cudaStream_t s) {
-  const size_t bytes = adjoint_smem_bytes(a.smem_vec);
   // A failure here stays the last error, which the caller's launch check reports.
-  cudaFuncSetAttribute(k_batch_polish, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(bytes));
-  k_batch_polish<<<grid, kAdjThreads, bytes, s>>>(b, a);
+  cudaFuncSetAttribute(k_batch_polish, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_bytes);
+  k_batch_polish<<<grid, a.threads, a.smem_bytes, s>>>(b, a);
 }
 
-int adjoint_blocks_per_sm(int smem_vec) {
-  const size_t bytes = adjoint_smem_bytes(smem_vec);
+int adjoint_max_smem() {
+  return std::min(max_dynamic_smem(reinterpret_cast<const void*>(k_batch_adjoint)),
+                  max_dynamic_smem(reinterpret_cast<const void*>(k_batch_polish)));
+}
+
+int adjoint_blocks_per_sm(int threads, int smem_bytes) {
   int per_sm = 1 << 30;
   for (const void* f : {reinterpret_cast<const void*>(k_batch_adjoint),
                         reinterpret_cast<const void*>(k_batch_polish)}) {
     int n = 0;
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(bytes)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, kAdjThreads, bytes) !=
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, threads,
+                                                      static_cast<size_t>(smem_bytes)) !=
             cudaSuccess) {
       cudaGetLastError();
       n = 1;
