@@ -38,11 +38,18 @@ __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Lets the next kernel in the stream, where it was launched with launch_after, be placed as soon as
+// every block of this one has called it (or left): its blocks then load what no kernel writes (the
+// matrix) while this one works, and wait in grid_dependency_wait() for its end.
+__device__ __forceinline__ void grid_dependency_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Launches kernel<<<grid, threads, smem, s>>>(args...) with programmatic stream
-// serialization: its blocks are placed on the SMs as the previous kernel's blocks leave them,
-// instead of after the whole kernel and its launch; the kernel must call
-// grid_dependency_wait() before its first read of the previous kernel's results. Returns the
-// launch's error.
+// serialization: its blocks are placed on the SMs as the previous kernel's blocks leave them (or
+// call grid_dependency_launch), instead of after the whole kernel and its launch; the kernel
+// must call grid_dependency_wait() before its first read of anything an earlier kernel of the
+// stream writes, and before its first write. Returns the launch's error.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_after(void (*kernel)(Params...), int grid, int threads, int smem,
                                 cudaStream_t s, Args... args) {

@@ -669,25 +669,33 @@ void Engine::load(const sankhya_gb300_lp& lp) {
 }
 
 // One FP64 sliced layout: planned on the host (plan_slices) and uploaded; its indices and values
-// are filled on the device from the compressed layout. Windows are kept where they hold at
-// least 95% of the entries: a gather that misses stalls its warp on L2, and a block without a
-// window leaves its shared memory to L1, which then serves the gathers better. A capacity set
-// through SANKHYA_GB300_WINDOW_CAP (window_cap >= 0) keeps its windows whatever their share.
-// A fixed rule, not a timing: the blocks decide the order of the partial sums, so they must not
-// vary from run to run.
+// are filled on the device from the compressed layout. A window is kept only where it holds the
+// whole gathered vector in kFullWindow bytes: larger ones, and partial ones, leave the block too
+// little L1 for the operands and hold its warps at every copy (column pass of the 500,000 x 1M
+// block-angular LP: 72.8 us with windows that hold 97.7% of the entries, 54.7 us without; a solve
+// of 50 x 100 is 4% slower with its 1.6 KB window, within the noise at 32 KB). A capacity set
+// through SANKHYA_GB300_WINDOW_CAP (window_cap >= 0) keeps its windows whatever their share. A
+// fixed rule, not a timing: runs must not vary.
 void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* lidx, int lines,
                          int extent, int pass, int window_cap) {
+  constexpr int kFullWindow = 32 * 1024;
   cudaStream_t s = stream_;
-  int wmax = fp64_window_capacity(pass);
-  if (window_cap >= 0) wmax = std::min(wmax, window_cap);
-  const SlicePlan P = plan_slices(lptr, lidx, lines, extent, wmax, window_cap >= 0 ? 0.0 : 0.95,
-                                  num_sms_, pass == 0 ? 1 : 2);
+  const int elem = static_cast<int>(pass == 0 ? sizeof(double) : sizeof(double2));
+  int wmax = std::min(fp64_window_capacity(pass), kFullWindow / elem);
+  if (window_cap >= 0) {
+    wmax = std::min(wmax, window_cap);
+  } else if (((extent + 3) & ~3) > wmax) {
+    wmax = 0;
+  }
+  const SlicePlan P =
+      plan_slices(lptr, lidx, lines, extent, wmax, 0.0, num_sms_, pass == 0 ? 1 : 2);
   D.meta.upload(P.meta.data(), P.meta.size(), s);
   D.base.upload(P.base.data(), P.base.size(), s);
   D.items.upload(P.items.data(), P.items.size(), s);
   D.longs.upload(P.longs.data(), P.longs.size(), s);
   D.segs.upload(P.segs.data(), P.segs.size(), s);
   D.seg_start.upload(P.seg_start.data(), P.seg_start.size(), s);
+  D.block_start.upload(P.block_start.data(), P.block_start.size(), s);
   const size_t e = static_cast<size_t>(P.entries);
   D.idx.allocate(e);
   D.raw.allocate(e);
@@ -711,6 +719,7 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
   S.nchunks = P.nchunks;
   S.nrows = lines;
   S.wmax = P.wmax;
+  S.block_start = D.block_start.ptr;
   S.grid = P.grid;
   S.threads = P.threads;
 }

@@ -116,7 +116,7 @@ class Engine {
   struct SliceDev {
     DeviceArray<unsigned short> meta;
     DeviceArray<unsigned int> base;
-    DeviceArray<int> idx, seg_start;
+    DeviceArray<int> idx, seg_start, block_start;
     DeviceArray<double> raw, scaled;
     DeviceArray<SliceItem> items;
     DeviceArray<LongRow> longs;
@@ -219,7 +219,7 @@ struct SlicePlan {
   std::vector<SliceItem> items;
   std::vector<LongRow> longs;
   std::vector<SliceSeg> segs;
-  std::vector<int> seg_start;
+  std::vector<int> seg_start, block_start;
 };
 SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, int extent, int wmax,
                       double window_min, int sms, int np);

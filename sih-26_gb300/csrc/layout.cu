@@ -350,8 +350,8 @@ SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, in
   const long long nnz = lines > 0 ? ptr[lines] : 0;
   p.nslices = ngroups * kGroupSlices;
   p.meta.assign(static_cast<size_t>(p.nslices) * 32, kNoRow);
-  p.base.assign(static_cast<size_t>(p.nslices), 0);
-  std::vector<double> cost(static_cast<size_t>(ngroups) + 1, 0.0);
+  p.base.assign(static_cast<size_t>(p.nslices) + 1, 0);
+  std::vector<double> cost(static_cast<size_t>(p.nslices) + 1, 0.0);
   std::vector<Tile> groups(static_cast<size_t>(ngroups));
   long long rows32 = 0;  // entries stored so far, / 32
   long long lentries = 0;
@@ -380,18 +380,18 @@ SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, in
         continue;
       }
       meta[start[kSliceLong - len]++] =
-          static_cast<unsigned short>((r - r0) | (static_cast<unsigned>(len) << 8));
+          static_cast<unsigned short>(static_cast<unsigned>(r - r0) | (static_cast<unsigned>(len) << 8));
     }
-    double c = 0.0;
     for (int q = 0; q < kGroupSlices; ++q) {
       const unsigned short head = meta[q * 32];
       const int width = head == kNoRow ? 0 : head >> 8;
       p.base[static_cast<size_t>(g) * kGroupSlices + q] = static_cast<unsigned>(rows32);
       rows32 += width;
-      c += static_cast<double>(width) * np + 12.0;
+      const size_t at = static_cast<size_t>(g) * kGroupSlices + q;
+      cost[at + 1] = cost[at] + static_cast<double>(width) * np + 12.0;
     }
-    cost[static_cast<size_t>(g) + 1] = cost[static_cast<size_t>(g)] + c;
   }
+  p.base[static_cast<size_t>(p.nslices)] = static_cast<unsigned>(rows32);
   p.long_base = rows32 * 32;
   p.entries = p.long_base + lentries;
 
@@ -407,43 +407,48 @@ SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, in
   p.staged = nnz > 0 ? static_cast<double>(covered) / static_cast<double>(nnz) : 0.0;
   for (const int2& w : windows) p.wmax = std::max(p.wmax, w.y);
 
-  // Blocks: one per SM, cut where the running cost passes the next share; a block has as many
-  // warps as its slices or items keep busy, at most kSliceThreads threads.
-  const int G = std::max(1, std::min(std::max(ngroups, static_cast<int>(p.items.size())), sms));
+  // Blocks: at most one per SM and not under four slices each (a small matrix spreads over the
+  // SMs: the FP64 pipe of each is the bound even there), cut where the running cost passes the
+  // next share; a block has as many warps as its slices or items keep busy, at most
+  // kSliceThreads threads.
+  const int wanted = (std::max(p.nslices, static_cast<int>(p.items.size())) + 3) / 4;
+  const int G = std::max(1, std::min(wanted, sms));
   p.grid = G;
   p.seg_start.assign(static_cast<size_t>(G) + 1, 0);
-  int g0 = 0, most = 1;
+  p.block_start.assign(static_cast<size_t>(G) + 1, p.nslices);
+  int s0 = 0, most = 1;
   for (int b = 0; b < G; ++b) {
     p.seg_start[static_cast<size_t>(b)] = static_cast<int>(p.segs.size());
-    const double upto = cost[static_cast<size_t>(ngroups)] * (b + 1) / G;
-    int g1 = g0;
-    while (g1 < ngroups && (b + 1 == G || cost[static_cast<size_t>(g1) + 1] <= upto * (1 + 1e-12) ||
-                            (cost[static_cast<size_t>(g1)] + cost[static_cast<size_t>(g1) + 1]) < 2.0 * upto)) {
-      ++g1;
+    p.block_start[static_cast<size_t>(b)] = s0;
+    const double upto = cost[static_cast<size_t>(p.nslices)] * (b + 1) / G;
+    int s1 = s0;
+    while (s1 < p.nslices &&
+           (b + 1 == G ||
+            cost[static_cast<size_t>(s1)] + cost[static_cast<size_t>(s1) + 1] < 2.0 * upto)) {
+      ++s1;
     }
-    most = std::max(most, (g1 - g0) * kGroupSlices);
-    for (int g = g0; g < g1;) {
-      int e = g + 1;
-      while (e < g1 && group_win[static_cast<size_t>(e)] == group_win[static_cast<size_t>(g)]) ++e;
-      SliceSeg sg{g * kGroupSlices, e * kGroupSlices, 0, 0};
-      if (group_win[static_cast<size_t>(g)] >= 0) {
-        sg.lo = windows[static_cast<size_t>(group_win[static_cast<size_t>(g)])].x;
-        sg.len = windows[static_cast<size_t>(group_win[static_cast<size_t>(g)])].y;
+    most = std::max(most, s1 - s0);
+    const auto window = [&](int s) { return group_win[static_cast<size_t>(s / kGroupSlices)]; };
+    for (int s = s0; s < s1;) {
+      int e = s + 1;
+      while (e < s1 && window(e) == window(s)) ++e;
+      SliceSeg sg{s, e, 0, 0};
+      if (window(s) >= 0) {
+        sg.lo = windows[static_cast<size_t>(window(s))].x;
+        sg.len = windows[static_cast<size_t>(window(s))].y;
       }
       p.segs.push_back(sg);
-      g = e;
+      s = e;
     }
     // A block of items only still visits them: they belong to its first segment.
     if (static_cast<int>(p.segs.size()) == p.seg_start[static_cast<size_t>(b)]) {
       p.segs.push_back(SliceSeg{0, 0, 0, 0});
     }
-    g0 = g1;
+    s0 = s1;
   }
   p.seg_start[static_cast<size_t>(G)] = static_cast<int>(p.segs.size());
   most = std::max(most, (static_cast<int>(p.items.size()) + G - 1) / G);
-  int warps = 4;
-  while (warps * 32 < kSliceThreads && warps < most) warps *= 2;
-  p.threads = warps * 32;
+  p.threads = std::min(kSliceThreads, std::max(128, (most + 3) / 4 * 128));
   return p;
 }
 

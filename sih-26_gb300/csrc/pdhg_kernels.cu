@@ -35,6 +35,9 @@ namespace {
 long long g_launches = 0;
 
 constexpr int kScratch = 16 * (kSliceThreads / 32);
+// Entry rows per piece of the passes that gather a pair per entry (row pass of the 500,000 x 1M
+// block-angular LP: 86.5 us with 8, 86.6 with 6, 90.7 with 4; Zipf rows 60.3, 62.8, 63.8 us).
+constexpr int kPairPiece = kPiece;
 
 // Per-device state: whether the kernels' shared-memory limits are set on the device, and
 // its occupancy and SM count (an engine on device 1 needs its own opt-in).
@@ -86,16 +89,20 @@ __device__ bool fp64_stop_test(const Ctl* c, const Residuals& r) {
 __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
   extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
-  grid_dependency_wait();  // the previous kernel's results (launch_after)
+  SliceStart<kPiece> start;
+  start_slices(b.csc, start);
+  grid_dependency_wait();  // the previous kernels' results (launch_after)
   Ctl* ctl = b.ctl;
   // Every control field the pass reads, loaded together before the first test.
   const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
   const bool add = ctl->pending_add != 0;
   const long long iteration = ctl->iteration, limit = ctl->iteration_limit;
   const double omega = ctl->omega, eta = ctl->eta;
-  if (done != kRunning || eval_now != 0) return;
-  if (iteration >= limit) {  // src/pdhg/pdhg.cpp:206
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->done = kIterationLimit;
+  if (done != kRunning || eval_now != 0 || iteration >= limit) {
+    // src/pdhg/pdhg.cpp:206
+    if (done == kRunning && eval_now == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+      ctl->done = kIterationLimit;
+    }
     return;
   }
   const double* __restrict__ x = b.x[cur];
@@ -129,7 +136,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
     b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
     mv[0] = fma(d, d, mv[0]);
   };
-  if (!run_slices<true, 1, 5>(b.csc, y, fetch, dsmem, b.chunk_primal, mac, load, epi) &&
+  if (!run_slices<true, 1, 5>(b.csc, start, y, fetch, dsmem, b.chunk_primal, mac, load, epi) &&
       threadIdx.x == 0) {
     raise_error(ctl);
   }
@@ -157,7 +164,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
 __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
   extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
-  grid_dependency_wait();  // the previous kernel's results (launch_after)
+  SliceStart<kPairPiece> start;
+  start_slices(b.csr, start);
+  grid_dependency_wait();  // the previous kernels' results (launch_after)
   Ctl* ctl = b.ctl;
   const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
   const bool add = ctl->pending_add != 0;
@@ -199,7 +208,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
     acc2[0] = fma(d, d, acc2[0]);
     acc2[1] = fma(d, s[1], acc2[1]);
   };
-  if (!run_slices<true, 2, 4>(b.csr, xd, fetch, dsmem, b.chunk_dual, mac, load, epi) &&
+  if (!run_slices<true, 2, 4>(b.csr, start, xd, fetch, dsmem, b.chunk_dual, mac, load, epi) &&
       threadIdx.x == 0) {
     raise_error(ctl);
   }
@@ -328,7 +337,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_eval_cols(EvalBuffers e) {
       acc[3 * q + 2] += cj * xc[q];
     }
   };
-  run_slices<false, 2, 0, double2>(e.csc, nullptr, fetch, nullptr, e.chunk_cols, mac, load, epi);
+  SliceStart<kPairPiece> start;
+  start_slices(e.csc, start);
+  run_slices<false, 2, 0, double2>(e.csc, start, nullptr, fetch, nullptr, e.chunk_cols, mac, load, epi);
   double out[8], mout[2];
   block_sum<8>(acc, scratch, out);
   block_max<2>(cmax, scratch, mout);
@@ -410,7 +421,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_eval_rows1(EvalBuffers e) 
       }
     }
   };
-  run_slices<false, 2, 0, double2>(e.csr, nullptr, fetch, nullptr, e.chunk_rows, mac, load, epi);
+  SliceStart<kPairPiece> start;
+  start_slices(e.csr, start);
+  run_slices<false, 2, 0, double2>(e.csr, start, nullptr, fetch, nullptr, e.chunk_rows, mac, load, epi);
   double mout[2], sums[2];
   block_max<2>(cmax, scratch, mout);
   block_sum<2>(acc, scratch, sums);
@@ -503,8 +516,8 @@ __global__ void k_eval_apply(EvalBuffers e) {
 
 // ---- Setup kernels (src/la/scaling.cpp) ----------------------------------------------------
 
-// The scaling rounds run on the sliced layouts: one lane per line, every load and store of the
-// values coalesced, a line's magnitudes taken in ascending index order, the reference's
+// The scaling rounds run on the sliced layouts: every load and store of the values coalesced, a
+// line's magnitudes added in ascending index order, the reference's
 // accumulation order. (One thread per line on the compressed layouts read 32 scattered
 // entries per load: 101 us for the factors of one layout and 123 us to apply them on the
 // 500,000 x 1M block-angular LP, and 1.35 and 2.5 ms where a Zipf row of 6,674 entries held one
@@ -539,19 +552,28 @@ __device__ __forceinline__ double pass_factor(double acc) {
 
 constexpr int kScaleThreads = 256;
 
+// Maximum and minimum of non-negative doubles by their bits (which order as the values do): the
+// integer pipe's, where FP64 compares would take as long as the rounds' multiplications.
+__device__ __forceinline__ double max_magnitude(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+__device__ __forceinline__ double min_magnitude(double a, double b) {
+  return __longlong_as_double(min(__double_as_longlong(a), __double_as_longlong(b)));
+}
+
 template <int MODE, bool APPLY>
 __global__ void __launch_bounds__(kScaleThreads) k_scale_round(ScaleArgs a) {
   __shared__ double scratch[2 * (kScaleThreads / 32)];
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int warp = static_cast<int>(threadIdx.x) >> 5;
   const int slice_blocks = (a.S.nslices + kScaleThreads / 32 - 1) / (kScaleThreads / 32);
-  double mm[2] = {0.0, -HUGE_VAL};  // kScaleNone: max, max of -magnitude
+  double most = 0.0, least = HUGE_VAL;  // kScaleNone: the magnitudes' range
   const auto take = [&](double mag, double& acc) {
-    if (MODE == kScaleMax) acc = dmax(acc, mag);
+    if (MODE == kScaleMax) acc = max_magnitude(acc, mag);
     if (MODE == kScaleSum) acc = acc + mag;
     if (MODE == kScaleNone) {
-      mm[0] = dmax(mm[0], mag);
-      mm[1] = dmax(mm[1], -mag);
+      most = max_magnitude(most, mag);
+      least = min_magnitude(least, mag);
     }
   };
   if (static_cast<int>(blockIdx.x) < slice_blocks) {
@@ -628,7 +650,7 @@ __global__ void __launch_bounds__(kScaleThreads) k_scale_round(ScaleArgs a) {
     }
   }
   if (MODE == kScaleNone && a.minmax != nullptr) {
-    double out[2];
+    double mm[2] = {most, -least}, out[2];
     block_max<2>(mm, scratch, out);
     if (threadIdx.x == 0) {
       a.minmax[2 * blockIdx.x] = out[0];
@@ -740,7 +762,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_spmv(SliceSet a, const dou
     y[r] = v;
     if (NORM) sq[0] = fma(v, v, sq[0]);
   };
-  run_slices<false, 1, 0, double>(a, nullptr, fetch, nullptr, chunk, mac, load, epi);
+  SliceStart<kPiece> start;
+  start_slices(a, start);
+  run_slices<false, 1, 0, double>(a, start, nullptr, fetch, nullptr, chunk, mac, load, epi);
   if (NORM) {
     if (!arrive_last<1>(sq, scratch, part, ticket)) return;
     sq[0] = 0.0;
@@ -852,10 +876,11 @@ long long kernel_launch_count() { return g_launches; }
 
 int fp64_window_capacity(int pass) {
   configure_fp64_kernels();
-  return pass == 0 ? window_capacity(reinterpret_cast<const void*>(k_primal), kSliceBarBytes,
-                                     sizeof(double))
-                   : window_capacity(reinterpret_cast<const void*>(k_dual), kSliceBarBytes,
-                                     sizeof(double2));
+  return pass == 0
+             ? window_capacity(reinterpret_cast<const void*>(k_primal), kSliceBarBytes,
+                               sizeof(double))
+             : window_capacity(reinterpret_cast<const void*>(k_dual), kSliceBarBytes,
+                               sizeof(double2));
 }
 
 void launch_primal_pass(const StepBuffers& b, cudaStream_t s) {

@@ -39,6 +39,9 @@ std::string qp_format(const char* fmt, ...) {
   return buf;
 }
 
+// Steps of both power iterations (src/qp/qp_condat_vu.cpp:74-143).
+constexpr int kQpPowerSteps = 20;
+
 bool valid_lanes(int g) { return g == 1 || g == 2 || g == 4 || g == 8 || g == 16 || g == 32; }
 
 }  // namespace
@@ -55,7 +58,11 @@ QpEngine::QpEngine(int device) : device_(device) {
   SGB_CUDA(cudaMallocHost(&hist_host_, sizeof(QpHist) * kQpMaxPeriods));
   ctl_.allocate(1);
   hist_.allocate(kQpMaxPeriods);
+  SGB_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device));
   dot_part_.allocate(kQpDotBlocks);
+  norms_.allocate(2 * (kQpPowerSteps + 1));
+  product_ticket_.allocate(1);
+  SGB_CUDA(cudaMemset(product_ticket_.ptr, 0, sizeof(unsigned int)));
   dot_out_.allocate(1);
 }
 
@@ -152,6 +159,9 @@ void QpEngine::load(const sankhya_gb300_qp_problem& p) {
   nnz_q_ = qz;
   col_len_ = h.col_len;
   row_len_ = h.row_len;
+  q_starts_ = h.q_starts;
+  a_row_starts_ = h.row_starts;
+  a_col_starts_.assign(lp.col_starts, lp.col_starts + n + 1);
 
   cudaStream_t s = stream_;
   const size_t z = static_cast<size_t>(nnz);
@@ -175,8 +185,40 @@ void QpEngine::load(const sankhya_gb300_qp_problem& p) {
   loaded_ = true;
 }
 
-void QpEngine::layout(int col_lanes, int row_lanes) {
-  if (col_lanes == col_lanes_ && row_lanes == row_lanes_) return;
+void QpEngine::plan_sliced(SliceDev& D, const int* starts1, const int* starts2, int count) {
+  cudaStream_t s = stream_;
+  QpSlices P;
+  qp_build_slices(starts1, starts2, count, num_sms_, &P);
+  D.meta.upload(P.meta.data(), P.meta.size(), s);
+  D.base1.upload(P.base1.data(), P.base1.size(), s);
+  D.base2.upload(P.base2.data(), P.base2.size(), s);
+  D.block_start.upload(P.block_start.data(), P.block_start.size(), s);
+  const size_t e1 = static_cast<size_t>(P.base1.back()) * 32;
+  const size_t e2 = static_cast<size_t>(P.base2.back()) * 32;
+  D.idx1.allocate(e1);
+  D.val1.allocate(e1);
+  D.idx2.allocate(e2);
+  D.val2.allocate(e2);
+  SGB_CUDA(cudaStreamSynchronize(s));  // the plan's arrays end here
+  QpSliceSet& S = D.view;
+  S = QpSliceSet{};
+  S.meta = D.meta.ptr;
+  S.base1 = D.base1.ptr;
+  S.base2 = D.base2.ptr;
+  S.idx1 = D.idx1.ptr;
+  S.idx2 = D.idx2.ptr;
+  S.val1 = D.val1.ptr;
+  S.val2 = D.val2.ptr;
+  S.block_start = D.block_start.ptr;
+  S.nslices = P.nslices;
+  S.blocks = P.nslices > 0 ? static_cast<int>(P.block_start.size()) - 1 : 0;
+}
+
+void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_sliced) {
+  if (col_lanes == col_lanes_ && row_lanes == row_lanes_ && cols_sliced == cols_sliced_ &&
+      rows_sliced == rows_sliced_) {
+    return;
+  }
   cudaStream_t s = stream_;
   std::vector<QpChunk> cc, rc;
   qp_build_chunks(col_len_, col_lanes, &cc, &nlong_cols_);
@@ -194,10 +236,32 @@ void QpEngine::layout(int col_lanes, int row_lanes) {
                                        kQpThreads);
   row_short_blocks_ = static_cast<int>((static_cast<long long>(m_) * row_lanes + kQpThreads - 1) /
                                        kQpThreads);
+  col_slices_.view = QpSliceSet{};
+  row_slices_.view = QpSliceSet{};
+  if (cols_sliced) {
+    plan_sliced(col_slices_, q_starts_.data(), a_col_starts_.data(), n_);
+    col_short_blocks_ = col_slices_.view.blocks;
+  }
+  if (rows_sliced) {
+    plan_sliced(row_slices_, nullptr, a_row_starts_.data(), m_);
+    row_short_blocks_ = row_slices_.view.blocks;
+  }
   obj_part_.allocate_padded(static_cast<size_t>(col_short_blocks_), 1, s);
-  SGB_CUDA(cudaStreamSynchronize(s));
   col_lanes_ = col_lanes;
   row_lanes_ = row_lanes;
+  cols_sliced_ = cols_sliced;
+  rows_sliced_ = rows_sliced;
+  const QpDev d = dev();
+  if (cols_sliced) {
+    qp_launch_slice_fill(d, true, col_slices_.idx1.ptr, col_slices_.val1.ptr,
+                         col_slices_.idx2.ptr, col_slices_.val2.ptr, s);
+  }
+  if (rows_sliced) {
+    qp_launch_slice_fill(d, false, nullptr, nullptr, row_slices_.idx2.ptr, row_slices_.val2.ptr, s);
+  }
+  SGB_CUDA(cudaGetLastError());
+  product_part_.allocate(2 * static_cast<size_t>(qp_product_blocks(d)));
+  SGB_CUDA(cudaStreamSynchronize(s));
   destroy_graph();
 }
 
@@ -210,6 +274,8 @@ QpDev QpEngine::dev() const {
   d.stage = stage_;
   d.sense = sense_;
   d.offset = offset_;
+  d.cols = col_slices_.view;
+  d.rows = row_slices_.view;
   d.a_cs = a_cs_.ptr;
   d.a_ri = a_ri_.ptr;
   d.a_cv = a_cv_.ptr;
@@ -246,16 +312,8 @@ QpDev QpEngine::dev() const {
   return d;
 }
 
-double QpEngine::dot(const double* a, const double* b, int n) {
-  qp_launch_dot(a, b, n, dot_part_.ptr, dot_out_.ptr, stream_);
-  double out = 0.0;
-  SGB_CUDA(cudaMemcpyAsync(&out, dot_out_.ptr, sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  SGB_CUDA(cudaStreamSynchronize(stream_));
-  return out;
-}
-
 // ||A||: src/qp/qp_condat_vu.cpp:74-103 (std::mt19937(26119 + seed), uniform on [-1, 1],
-// twenty steps of v <- A'A v / |v|, estimate |A'A v|^(1/2)).
+// twenty steps of v <- A'A v / |v|, estimate |A'A v|^(1/2)). norms_[2 k] is |v_k|^2.
 double QpEngine::spectral_norm(unsigned seed) {
   if (m_ == 0 || n_ == 0 || nnz_a_ == 0) return 0.0;
   std::mt19937 rng(26119u + seed);
@@ -264,16 +322,22 @@ double QpEngine::spectral_norm(unsigned seed) {
   for (double& value : v) value = unit(rng);
   SGB_CUDA(cudaMemcpyAsync(vec_n_.ptr, v.data(), v.size() * sizeof(double),
                            cudaMemcpyHostToDevice, stream_));
+  const QpDev d = dev();
+  qp_launch_dot(vec_n_.ptr, vec_n_.ptr, n_, dot_part_.ptr, norms_.ptr, stream_);
+  for (int k = 0; k < kQpPowerSteps; ++k) {
+    qp_launch_product(d, kQpRows, vec_n_.ptr, norms_.ptr + 2 * k, vec_m_.ptr,
+                      qp_auto_lanes(double(nnz_a_) / m_), nullptr, nullptr, nullptr, stream_);
+    qp_launch_product(d, kQpCols, vec_m_.ptr, nullptr, vec_n_.ptr,
+                      qp_auto_lanes(double(nnz_a_) / n_), norms_.ptr + 2 * k + 2,
+                      product_part_.ptr, product_ticket_.ptr, stream_);
+  }
+  double host[2 * (kQpPowerSteps + 1)];
+  SGB_CUDA(cudaMemcpyAsync(host, norms_.ptr, sizeof(host), cudaMemcpyDeviceToHost, stream_));
+  SGB_CUDA(cudaStreamSynchronize(stream_));
   double estimate = 0.0;
-  for (int iteration = 0; iteration < 20; ++iteration) {
-    const double norm2 = dot(vec_n_.ptr, vec_n_.ptr, n_);
-    if (std::sqrt(norm2) <= 0.0) return 0.0;
-    qp_launch_scale(vec_n_.ptr, n_, dot_out_.ptr, stream_);
-    qp_launch_spmv(m_, a_rs_.ptr, a_ci_.ptr, a_rv_.ptr, vec_n_.ptr, vec_m_.ptr,
-                   qp_auto_lanes(double(nnz_a_) / m_), stream_);
-    qp_launch_spmv(n_, a_cs_.ptr, a_ri_.ptr, a_cv_.ptr, vec_m_.ptr, vec_n_.ptr,
-                   qp_auto_lanes(double(nnz_a_) / n_), stream_);
-    estimate = std::sqrt(std::sqrt(dot(vec_n_.ptr, vec_n_.ptr, n_)));
+  for (int k = 0; k < kQpPowerSteps; ++k) {
+    if (std::sqrt(host[2 * k]) <= 0.0) return 0.0;
+    estimate = std::sqrt(std::sqrt(host[2 * k + 2]));
   }
   return estimate;
 }
@@ -290,24 +354,28 @@ double QpEngine::hessian_norm(unsigned seed) {
                            cudaMemcpyHostToDevice, stream_));
   double* a = vec_n_.ptr;
   double* b = col_dual_.ptr;  // scratch until the report
-  double estimate = 0.0;
-  for (int iteration = 0; iteration < 20; ++iteration) {
-    const double norm2 = dot(a, a, n_);
-    if (std::sqrt(norm2) <= 0.0) return 0.0;
-    qp_launch_scale(a, n_, dot_out_.ptr, stream_);
-    qp_launch_spmv(n_, q_rs_.ptr, q_ci_.ptr, q_v_.ptr, a, b, qp_auto_lanes(double(nnz_q_) / n_),
-                   stream_);
-    estimate = std::fabs(dot(b, a, n_));
+  const QpDev d = dev();
+  qp_launch_dot(a, a, n_, dot_part_.ptr, norms_.ptr, stream_);
+  for (int k = 0; k < kQpPowerSteps; ++k) {
+    qp_launch_product(d, kQpHessian, a, norms_.ptr + 2 * k, b,
+                      qp_auto_lanes(double(nnz_q_) / n_), norms_.ptr + 2 * k + 2,
+                      product_part_.ptr, product_ticket_.ptr, stream_);
     std::swap(a, b);
+  }
+  double host[2 * (kQpPowerSteps + 1)];
+  SGB_CUDA(cudaMemcpyAsync(host, norms_.ptr, sizeof(host), cudaMemcpyDeviceToHost, stream_));
+  SGB_CUDA(cudaStreamSynchronize(stream_));
+  double estimate = 0.0;
+  for (int k = 0; k < kQpPowerSteps; ++k) {
+    if (std::sqrt(host[2 * k]) <= 0.0) return 0.0;
+    estimate = std::fabs(host[2 * k + 3]);
   }
   return estimate;
 }
 
 void QpEngine::build_graph(int periods) {
-  if (graph_ != nullptr && graph_periods_ == periods && graph_col_lanes_ == col_lanes_ &&
-      graph_row_lanes_ == row_lanes_ && graph_stage_ == stage_) {
-    return;
-  }
+  // A change of the layout has destroyed the graph.
+  if (graph_ != nullptr && graph_periods_ == periods && graph_stage_ == stage_) return;
   destroy_graph();
   const QpDev d = dev();
   QpCtl* ctl = ctl_.ptr;
@@ -334,8 +402,6 @@ void QpEngine::build_graph(int periods) {
   SGB_CUDA(inst);
   graph_nodes_ = qp_kernel_launch_count() - before;
   graph_periods_ = periods;
-  graph_col_lanes_ = col_lanes_;
-  graph_row_lanes_ = row_lanes_;
   graph_stage_ = stage_;
 }
 
@@ -347,16 +413,20 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
   if (!(p.tolerance > 0.0) || std::isnan(p.time_limit)) {
     throw EngineError{SANKHYA_GB300_ERROR_OPTION, "qp_tolerance must be positive"};
   }
-  const int col_lanes = p.column_lanes > 0 ? p.column_lanes
-                                           : qp_auto_lanes(n_ > 0 ? double(nnz_a_ + nnz_q_) / n_ : 1.0);
-  const int row_lanes = p.row_lanes > 0 ? p.row_lanes
-                                        : qp_auto_lanes(m_ > 0 ? double(nnz_a_) / m_ : 1.0);
+  // With the lanes left to the engine, a side that one lane per item would do runs on sliced
+  // items; lanes that are asked for, or staging, run on the compressed arrays.
+  const double col_mean = n_ > 0 ? double(nnz_a_ + nnz_q_) / n_ : 1.0;
+  const double row_mean = m_ > 0 ? double(nnz_a_) / m_ : 1.0;
+  const int col_lanes = p.column_lanes > 0 ? p.column_lanes : qp_auto_lanes(col_mean);
+  const int row_lanes = p.row_lanes > 0 ? p.row_lanes : qp_auto_lanes(row_mean);
+  const bool cols_sliced = p.column_lanes <= 0 && col_lanes == 1 && p.staging == 0;
+  const bool rows_sliced = p.row_lanes <= 0 && row_lanes == 1 && p.staging == 0;
   if (!valid_lanes(col_lanes) || !valid_lanes(row_lanes)) {
     throw EngineError{SANKHYA_GB300_ERROR_OPTION, "lanes must be 1, 2, 4, 8, 16 or 32"};
   }
   SGB_CUDA(cudaSetDevice(device_));
   solved_ = false;
-  layout(col_lanes, row_lanes);
+  layout(col_lanes, row_lanes, cols_sliced, rows_sliced);
   stage_ = p.staging ? 1 : 0;
   // Check periods per graph: about 2 ms of work by the bytes an iteration moves, at most 20.
   int periods = p.periods_per_poll;

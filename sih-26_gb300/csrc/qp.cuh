@@ -7,7 +7,8 @@
 // and every 50 iterations measures the worst row violation of A x and the worst
 // |x - proj_box(x - gradient)|, stopping when both are within qp_tolerance.
 //
-// Here one iteration is two kernels:
+// Here one iteration is two kernels, on sliced items where lanes are not asked for (qp_layout.hpp:
+// every matrix load of a warp contiguous) and else on the compressed arrays:
 //   column pass  for each column j: (Qx)_j over row j of the full symmetric Q and (A'y)_j over
 //                column j of A, then the projected step and the extrapolation (x' to the
 //                other buffer of a pair, xbar);
@@ -25,6 +26,7 @@
 
 #include "common.cuh"
 #include "qp_layout.hpp"
+#include "slices.cuh"
 
 namespace sgb {
 
@@ -64,12 +66,26 @@ struct QpHist {
   double primal, dual, objective;
 };
 
+// A sliced layout on the device (qp_layout.hpp); nslices = 0 when the passes run on the compressed
+// arrays. The second part of a column slice is A's, the first Q's.
+struct QpSliceSet {
+  const unsigned* meta;
+  const unsigned *base1, *base2;
+  const int *idx1, *idx2;
+  const double *val1, *val2;
+  const int* block_start;
+  int nslices, blocks;
+};
+// The threads of a block on sliced items.
+constexpr int kQpSliceThreads = 768;  // 85 registers a thread
+
 // Everything the kernels read, by value.
 struct QpDev {
   int m, n;
   int col_lanes, row_lanes;
   int stage;  // one-lane passes stage the warp's matrix slice in shared memory
   double sense, offset;
+  QpSliceSet cols, rows;
   // A by columns (CSC) and by rows (CSR); Q as the full symmetric matrix by rows.
   const int* a_cs;
   const int* a_ri;
@@ -118,15 +134,22 @@ void qp_launch_decide(const QpDev& d, QpCtl* ctl, int k, int p, cudaStream_t s);
 // base += iterations of the graph (capped at the limit) unless done.
 void qp_launch_advance(QpCtl* ctl, int graph_iterations, cudaStream_t s);
 
-// Setup: out = M v over the rows of a CSR (`lanes` threads per row, 1..32); sum of a[i] * b[i]
-// into *out in a fixed order (partials of kQpDotBlocks blocks, then one block);
-// v /= sqrt(*norm2).
+// Setup. The sliced copies of the compressed arrays (col: by columns, else by rows).
+void qp_launch_slice_fill(const QpDev& d, bool cols, int* idx1, double* val1, int* idx2,
+                          double* val2, cudaStream_t s);
+// Power steps: out = M (v / sqrt(*norm2)) with M = A (kQpRows), A' (kQpCols) or Q (kQpHessian).
+// next[0] receives sum out^2 and next[1] sum out v / sqrt(*norm2) (Q only), in a fixed order, from
+// `part` (2 doubles per block, qp_product_blocks) and `ticket` (zero on entry and exit); next may
+// be null (A). norm2 null: v is used as it is. Without slices `lanes` threads share an item.
+enum QpSide { kQpRows = 0, kQpCols = 1, kQpHessian = 2 };
+int qp_product_blocks(const QpDev& d);
+void qp_launch_product(const QpDev& d, int side, const double* v, const double* norm2, double* out,
+                       int lanes, double* next, double* part, unsigned int* ticket,
+                       cudaStream_t s);
+// Sum of a[i] * b[i] into *out in a fixed order (partials of kQpDotBlocks blocks, then one block).
 constexpr int kQpDotBlocks = 304;
-void qp_launch_spmv(int rows, const int* starts, const int* index, const double* values,
-                    const double* v, double* out, int lanes, cudaStream_t s);
 void qp_launch_dot(const double* a, const double* b, int n, double* partials, double* out,
                    cudaStream_t s);
-void qp_launch_scale(double* v, int n, const double* norm2, cudaStream_t s);
 // row_dual = -sense * y.
 void qp_launch_row_dual(const QpDev& d, double* row_dual, cudaStream_t s);
 // x0 = proj_box(0) (src/qp/qp_condat_vu.cpp:213-217), y = 0.

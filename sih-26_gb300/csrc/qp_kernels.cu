@@ -24,6 +24,8 @@
 
 #include <algorithm>
 
+#include "chunks.cuh"
+
 namespace sgb {
 namespace {
 
@@ -168,26 +170,133 @@ __device__ __forceinline__ void staged_column_sums(const QpDev& d, const double*
   *aty = sa;
 }
 
+// ---- Sliced items -----------------------------------------------------------------------------
+// A lane's item in slice s: its meta word, unpacked.
+struct QpPlace {
+  int item, len1, len2;  // item valid where `has`
+  bool has;
+  __device__ __forceinline__ void set(int s, unsigned m) {
+    has = m != kQpNoItem;
+    item = (s / (kQpGroup / 32)) * kQpGroup + static_cast<int>(m & 127u);
+    len1 = has ? static_cast<int>((m >> 8) & 255u) : 0;
+    len2 = has ? static_cast<int>(m >> 16) : 0;
+  }
+};
+
+__device__ __forceinline__ unsigned qp_meta(const QpSliceSet& S, int s, int s1) {
+  return s < s1 ? __ldg(S.meta + static_cast<size_t>(s) * 32 + (threadIdx.x & 31)) : kQpNoItem;
+}
+
+// A warp's walk over its block's slices: the slice at hand, and the first piece of what is summed
+// next (slices.cuh). PART 0 is the first part and then the second of each slice, 1 and 2 one part.
+template <int PART>
+struct QpWalk {
+  int s, s1;
+  QpPlace p;
+  size_t at1, at2;
+  PieceIndices<kPiece> ix;
+  unsigned m;  // of the next slice
+  unsigned b1, b2;
+
+  __device__ __forceinline__ void fetch(const QpSliceSet& S, int next) {
+    m = kQpNoItem;
+    b1 = b2 = 0;
+    if (next < s1) {
+      m = __ldg(S.meta + static_cast<size_t>(next) * 32 + (threadIdx.x & 31));
+      if (PART != 2) b1 = __ldg(S.base1 + next);
+      if (PART != 1) b2 = __ldg(S.base2 + next);
+    }
+  }
+  __device__ __forceinline__ void unpack() {
+    p.set(s, m);
+    at1 = static_cast<size_t>(b1) * 32 + (threadIdx.x & 31);
+    at2 = static_cast<size_t>(b2) * 32 + (threadIdx.x & 31);
+  }
+  __device__ __forceinline__ void start(const QpSliceSet& S) {
+    const bool mine = static_cast<int>(blockIdx.x) < S.blocks;
+    s = mine ? __ldg(S.block_start + blockIdx.x) + static_cast<int>(threadIdx.x >> 5) : 0;
+    s1 = mine ? __ldg(S.block_start + blockIdx.x + 1) : 0;
+    fetch(S, s);
+    unpack();
+    if (PART == 2) {
+      ix.load(S.idx2 + at2, p.len2);
+    } else {
+      ix.load(S.idx1 + at1, p.len1);
+    }
+    fetch(S, s + kQpSliceThreads / 32);
+  }
+  // The next slice's first piece, once its record has arrived.
+  __device__ __forceinline__ void after(const QpSliceSet& S, const int** idx, int* left) const {
+    QpPlace n;
+    n.set(0, m);
+    if (PART == 2) {
+      *idx = S.idx2 + static_cast<size_t>(b2) * 32 + (threadIdx.x & 31);
+      *left = n.len2;
+    } else {
+      *idx = S.idx1 + static_cast<size_t>(b1) * 32 + (threadIdx.x & 31);
+      *left = n.len1;
+    }
+  }
+  // The item's sums over the parts of PART, FMA-accumulated in entry order.
+  __device__ __forceinline__ void sums(const QpSliceSet& S, const double* __restrict__ v1,
+                                       const double* __restrict__ v2, double* sum1,
+                                       double* sum2) {
+    const int* ni;
+    int nl;
+    after(S, &ni, &nl);
+    double a1 = 0.0, a2 = 0.0;
+    if (PART != 2) {
+      slice_sum<double>(S.idx1 + at1, S.val1 + at1, p.len1, __reduce_max_sync(0xffffffffu, p.len1),
+                        ix, PART == 0 ? S.idx2 + at2 : ni, PART == 0 ? p.len2 : nl,
+                        [&](int c) { return __ldg(v1 + c); },
+                        [&](double v, double g) { a1 = fma(v, g, a1); });
+    }
+    if (PART != 1) {
+      slice_sum<double>(S.idx2 + at2, S.val2 + at2, p.len2, __reduce_max_sync(0xffffffffu, p.len2),
+                        ix, ni, nl, [&](int c) { return __ldg(v2 + c); },
+                        [&](double v, double g) { a2 = fma(v, g, a2); });
+    }
+    *sum1 = a1;
+    *sum2 = a2;
+  }
+  __device__ __forceinline__ void advance(const QpSliceSet& S) {
+    s += kQpSliceThreads / 32;
+    unpack();
+    fetch(S, s + kQpSliceThreads / 32);
+  }
+};
+
 // ---- Column pass ------------------------------------------------------------------------
+
+// The epilogue's operands of column j.
+struct ColumnOps {
+  double x, c, lower, upper;
+  __device__ __forceinline__ void load(const QpDev& d, const double* xv, int j) {
+    x = xv[j];
+    c = d.cost[j];
+    lower = d.col_lower[j];
+    upper = d.col_upper[j];
+  }
+};
 
 // The epilogue of column j, run by one lane. Returns the check's residual (check form) and the
 // objective term c_j x_j + 0.5 x_j (Qx)_j (check and report forms).
 template <int MODE>
 __device__ __forceinline__ void column_epilogue(const QpDev& d, double tau, int j,
-                                                const double* x, double* xn, double qx,
+                                                const ColumnOps& o, double* xn, double qx,
                                                 double aty, double* residual, double* obj) {
-  const double xj = x[j];
-  const double c = d.cost[j];  // sense c; qx is (sense Q x)_j
+  const double xj = o.x;
+  const double c = o.c;  // sense c; qx is (sense Q x)_j
   if (MODE == kQpStep) {
     const double g = qp_gradient(c, qx, aty);
     const double t = __dsub_rn(xj, __dmul_rn(tau, g));
-    const double xnj = box(t, d.col_lower[j], d.col_upper[j]);
+    const double xnj = box(t, o.lower, o.upper);
     xn[j] = xnj;
     d.xbar[j] = fma(2.0, xnj, -xj);
   } else {
     if (MODE == kQpCheck) {
       const double g = qp_gradient(c, qx, aty);
-      const double stepped = box(__dsub_rn(xj, g), d.col_lower[j], d.col_upper[j]);
+      const double stepped = box(__dsub_rn(xj, g), o.lower, o.upper);
       *residual = fabs(__dsub_rn(xj, stepped));
     } else {
       // c + Qx = sense (sense c + sense Qx), exactly.
@@ -198,18 +307,55 @@ __device__ __forceinline__ void column_epilogue(const QpDev& d, double tau, int 
   }
 }
 
+// G = 0: the short columns on sliced items, in blocks of kQpSliceThreads.
+template <int G>
+constexpr int qp_threads() {
+  return G == 0 ? kQpSliceThreads : kQpThreads;
+}
+
 template <int G, int MODE>
-__global__ void __launch_bounds__(kQpThreads) k_qp_column(QpDev d, QpCtl* ctl, int k, int src) {
+__global__ void __launch_bounds__(qp_threads<G>()) k_qp_column(QpDev d, QpCtl* ctl, int k, int src) {
+  // The first entries are under way before the wait: no kernel of the solve writes the matrix.
+  QpWalk<0> walk;
+  if (G == 0) walk.start(d.cols);
+  grid_dependency_launch();
   grid_dependency_wait();
   if (MODE != kQpReport && qp_skip(ctl, k)) return;
   const double tau = ctl->tau;
   const double* x = src ? d.x1 : d.x0;
   double* xn = src ? d.x0 : d.x1;
   const int lane32 = threadIdx.x & 31;
-  if (static_cast<int>(blockIdx.x) < d.col_short_blocks) {
+  if (G == 0 && static_cast<int>(blockIdx.x) < d.col_short_blocks) {
+    double residual = 0.0, obj = 0.0;
+    for (; walk.s < walk.s1; walk.advance(d.cols)) {
+      const QpPlace p = walk.p;
+      ColumnOps o;
+      if (p.has) o.load(d, x, p.item);
+      double qx, aty, r = 0.0, t = 0.0;
+      walk.sums(d.cols, x, d.y, &qx, &aty);
+      if (p.has) column_epilogue<MODE>(d, tau, p.item, o, xn, qx, aty, &r, &t);
+      if (MODE != kQpStep) {
+        residual = r > residual ? r : residual;
+        obj += t;
+      }
+    }
+    if (MODE != kQpStep) {
+      __shared__ double scratch[kQpSliceThreads / 32];
+      if (MODE == kQpCheck) {
+        const double w = warp_max(residual);
+        if (lane32 == 0) max_bits(&ctl->dual_bits, w);
+      }
+      double v[1] = {obj}, total[1];
+      block_sum<1>(v, scratch, total);
+      if (threadIdx.x == 0) d.obj_part[blockIdx.x] = total[0];
+    }
+    return;
+  }
+  if (G > 0 && static_cast<int>(blockIdx.x) < d.col_short_blocks) {
     // Short columns: G lanes per column, in column order.
+    constexpr int kG = G > 0 ? G : 1;
     const int gid = static_cast<int>(blockIdx.x) * kQpThreads + static_cast<int>(threadIdx.x);
-    const int j = gid / G, lane = gid % G;
+    const int j = gid / kG, lane = gid % kG;
     int qb = 0, qe = 0, ab = 0, ae = 0;
     bool active = j < d.n;
     if (active) {
@@ -217,7 +363,7 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_column(QpDev d, QpCtl* ctl, i
       qe = d.q_rs[j + 1];
       ab = d.a_cs[j];
       ae = d.a_cs[j + 1];
-      if ((qe - qb) + (ae - ab) > kQpLongPerLane * G) {  // a long column: the chunk path's
+      if ((qe - qb) + (ae - ab) > kQpLongPerLane * kG) {  // a long column: the chunk path's
         active = false;
         qb = qe = ab = ae = 0;
       }
@@ -229,13 +375,17 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_column(QpDev d, QpCtl* ctl, i
       qx = seq_dot(d.q_v, d.q_ci, x, qb, qe, 0.0);
       aty = seq_dot(d.a_cv, d.a_ri, d.y, ab, ae, 0.0);
     } else {
-      for (int e = qb + lane; e < qe; e += G) qx = fma(d.q_v[e], x[d.q_ci[e]], qx);
-      for (int e = ab + lane; e < ae; e += G) aty = fma(d.a_cv[e], d.y[d.a_ri[e]], aty);
-      qx = group_sum<G>(qx);
-      aty = group_sum<G>(aty);
+      for (int e = qb + lane; e < qe; e += kG) qx = fma(d.q_v[e], x[d.q_ci[e]], qx);
+      for (int e = ab + lane; e < ae; e += kG) aty = fma(d.a_cv[e], d.y[d.a_ri[e]], aty);
+      qx = group_sum<kG>(qx);
+      aty = group_sum<kG>(aty);
     }
     double residual = 0.0, obj = 0.0;
-    if (active && lane == 0) column_epilogue<MODE>(d, tau, j, x, xn, qx, aty, &residual, &obj);
+    if (active && lane == 0) {
+      ColumnOps o;
+      o.load(d, x, j);
+      column_epilogue<MODE>(d, tau, j, o, xn, qx, aty, &residual, &obj);
+    }
     if (MODE != kQpStep) {
       __shared__ double scratch[kQpThreads / 32];
       if (MODE == kQpCheck) {
@@ -251,7 +401,7 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_column(QpDev d, QpCtl* ctl, i
   // Long columns: one warp per chunk of the column's entries (row j of Q, then column j of
   // A); the last chunk of a column to finish adds the chunks' sums in order and runs its
   // epilogue.
-  const int w = (static_cast<int>(blockIdx.x) - d.col_short_blocks) * (kQpThreads / 32) +
+  const int w = (static_cast<int>(blockIdx.x) - d.col_short_blocks) * (qp_threads<G>() / 32) +
                 static_cast<int>(threadIdx.x >> 5);
   if (w >= d.ncol_chunks) return;
   const QpChunk ch = d.col_chunks[w];
@@ -290,7 +440,9 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_column(QpDev d, QpCtl* ctl, i
   }
   if (lane32 == 0) {
     double residual = 0.0, obj = 0.0;
-    column_epilogue<MODE>(d, tau, j, x, xn, qx, aty, &residual, &obj);
+    ColumnOps o;
+    o.load(d, x, j);
+    column_epilogue<MODE>(d, tau, j, o, xn, qx, aty, &residual, &obj);
     if (MODE == kQpCheck) max_bits(&ctl->dual_bits, residual);
     if (MODE != kQpStep) d.long_col_obj[ch.slot] = obj;
   }
@@ -298,36 +450,69 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_column(QpDev d, QpCtl* ctl, i
 
 // ---- Row pass ---------------------------------------------------------------------------
 
+// The epilogue's operands of row i.
+struct RowOps {
+  double y, lower, upper;
+  __device__ __forceinline__ void load(const QpDev& d, int i) {
+    y = d.y[i];
+    lower = d.row_lower[i];
+    upper = d.row_upper[i];
+  }
+};
+
 template <int MODE>
 __device__ __forceinline__ double row_epilogue(const QpDev& d, double sigma, double inv_sigma,
-                                               int i, double ax) {
+                                               int i, const RowOps& o, double ax) {
   if (MODE == kQpStep) {
     // y' = v - sigma proj(v / sigma), v = y + sigma (A xbar)_i (src/qp/qp_condat_vu.cpp:270-276).
-    const double v = __dadd_rn(d.y[i], __dmul_rn(sigma, ax));
-    const double p = box(divide(v, sigma, inv_sigma), d.row_lower[i], d.row_upper[i]);
+    const double v = __dadd_rn(o.y, __dmul_rn(sigma, ax));
+    const double p = box(divide(v, sigma, inv_sigma), o.lower, o.upper);
     d.y[i] = __dsub_rn(v, __dmul_rn(sigma, p));
     return 0.0;
   }
-  const double projected = box(ax, d.row_lower[i], d.row_upper[i]);
+  const double projected = box(ax, o.lower, o.upper);
   return fabs(__dsub_rn(ax, projected));
 }
 
 template <int G, int MODE>
-__global__ void __launch_bounds__(kQpThreads) k_qp_row(QpDev d, QpCtl* ctl, int k, int src) {
+__global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl, int k, int src) {
+  QpWalk<2> walk;
+  if (G == 0) walk.start(d.rows);
+  grid_dependency_launch();
   grid_dependency_wait();
   if (qp_skip(ctl, k)) return;
   const double sigma = ctl->sigma, inv_sigma = ctl->inv_sigma;
   const double* v = MODE == kQpStep ? d.xbar : (src ? d.x1 : d.x0);
   const int lane32 = threadIdx.x & 31;
-  if (static_cast<int>(blockIdx.x) < d.row_short_blocks) {
+  if (G == 0 && static_cast<int>(blockIdx.x) < d.row_short_blocks) {
+    double residual = 0.0;
+    for (; walk.s < walk.s1; walk.advance(d.rows)) {
+      const QpPlace p = walk.p;
+      RowOps o;
+      if (p.has) o.load(d, p.item);
+      double none, ax;
+      walk.sums(d.rows, nullptr, v, &none, &ax);
+      if (p.has) {
+        const double r = row_epilogue<MODE>(d, sigma, inv_sigma, p.item, o, ax);
+        residual = r > residual ? r : residual;
+      }
+    }
+    if (MODE == kQpCheck) {
+      const double w = warp_max(residual);
+      if (lane32 == 0) max_bits(&ctl->primal_bits, w);
+    }
+    return;
+  }
+  if (G > 0 && static_cast<int>(blockIdx.x) < d.row_short_blocks) {
+    constexpr int kG = G > 0 ? G : 1;
     const int gid = static_cast<int>(blockIdx.x) * kQpThreads + static_cast<int>(threadIdx.x);
-    const int i = gid / G, lane = gid % G;
+    const int i = gid / kG, lane = gid % kG;
     int b = 0, e = 0;
     bool active = i < d.m;
     if (active) {
       b = d.a_rs[i];
       e = d.a_rs[i + 1];
-      if (e - b > kQpLongPerLane * G) {
+      if (e - b > kQpLongPerLane * kG) {
         active = false;
         b = e = 0;
       }
@@ -338,18 +523,22 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_row(QpDev d, QpCtl* ctl, int 
     } else if (G == 1) {
       ax = seq_dot(d.a_rv, d.a_ci, v, b, e, 0.0);
     } else {
-      for (int q = b + lane; q < e; q += G) ax = fma(d.a_rv[q], v[d.a_ci[q]], ax);
-      ax = group_sum<G>(ax);
+      for (int q = b + lane; q < e; q += kG) ax = fma(d.a_rv[q], v[d.a_ci[q]], ax);
+      ax = group_sum<kG>(ax);
     }
     double residual = 0.0;
-    if (active && lane == 0) residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, ax);
+    if (active && lane == 0) {
+      RowOps o;
+      o.load(d, i);
+      residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, o, ax);
+    }
     if (MODE == kQpCheck) {
       const double w = warp_max(residual);
       if (lane32 == 0) max_bits(&ctl->primal_bits, w);
     }
     return;
   }
-  const int w = (static_cast<int>(blockIdx.x) - d.row_short_blocks) * (kQpThreads / 32) +
+  const int w = (static_cast<int>(blockIdx.x) - d.row_short_blocks) * (qp_threads<G>() / 32) +
                 static_cast<int>(threadIdx.x >> 5);
   if (w >= d.nrow_chunks) return;
   const QpChunk ch = d.row_chunks[w];
@@ -374,7 +563,9 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_row(QpDev d, QpCtl* ctl, int 
     }
   }
   if (lane32 == 0) {
-    const double residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, ax);
+    RowOps o;
+    o.load(d, i);
+    const double residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, o, ax);
     if (MODE == kQpCheck) max_bits(&ctl->primal_bits, residual);
   }
 }
@@ -400,6 +591,7 @@ __device__ double objective_total(const QpDev& d) {
 }
 
 __global__ void __launch_bounds__(kQpThreads) k_qp_decide(QpDev d, QpCtl* ctl, int k, int p) {
+  grid_dependency_launch();
   grid_dependency_wait();
   if (qp_skip(ctl, k)) return;
   const double obj = objective_total(d);
@@ -422,12 +614,14 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_decide(QpDev d, QpCtl* ctl, i
 }
 
 __global__ void k_qp_objective(QpDev d, QpCtl* ctl) {
+  grid_dependency_launch();
   grid_dependency_wait();
   const double obj = objective_total(d);
   if (threadIdx.x == 0) ctl->objective = obj;
 }
 
 __global__ void k_qp_advance(QpCtl* ctl, int graph_iterations) {
+  grid_dependency_launch();
   grid_dependency_wait();
   if (ctl->done) return;
   const long long next = ctl->base + graph_iterations;
@@ -436,26 +630,119 @@ __global__ void k_qp_advance(QpCtl* ctl, int graph_iterations) {
 
 // ---- Setup --------------------------------------------------------------------------------
 
-// G lanes per row, grid-stride over the rows (a long row is walked by its G lanes: the setup
-// products run forty times per solve).
-template <int G>
-__global__ void __launch_bounds__(kQpThreads) k_qp_spmv(int rows, const int* starts,
-                                                        const int* index, const double* values,
-                                                        const double* v, double* out) {
-  const int lane = static_cast<int>(threadIdx.x) % G;
-  const int groups = static_cast<int>(gridDim.x) * (kQpThreads / G);
-  const int first = (static_cast<int>(blockIdx.x) * kQpThreads + static_cast<int>(threadIdx.x)) / G;
-  // Every group runs the same number of rounds, so the lanes of a warp stay together for the
-  // shuffles of group_sum.
-  const int rounds = (rows + groups - 1) / groups;
-  for (int q = 0; q < rounds; ++q) {
-    const int r = first + q * groups;
-    double s = 0.0;
-    if (r < rows) {
-      for (int e = starts[r] + lane; e < starts[r + 1]; e += G) s = fma(values[e], v[index[e]], s);
+// The sliced copy of one part, a warp per slice.
+__global__ void __launch_bounds__(kQpThreads) k_qp_slice_fill(QpSliceSet S, int part,
+                                                              const int* starts, const int* index,
+                                                              const double* values, int* idx,
+                                                              double* val) {
+  const int s = static_cast<int>(blockIdx.x) * kQpWarps + static_cast<int>(threadIdx.x >> 5);
+  if (s >= S.nslices) return;
+  QpPlace p;
+  p.set(s, qp_meta(S, s, S.nslices));
+  if (!p.has) return;
+  const int len = part == 1 ? p.len1 : p.len2;
+  const size_t at =
+      static_cast<size_t>(part == 1 ? S.base1[s] : S.base2[s]) * 32 + (threadIdx.x & 31);
+  const int from = starts[p.item];
+  for (int k = 0; k < len; ++k) {
+    idx[at + static_cast<size_t>(k) * 32] = index[from + k];
+    val[at + static_cast<size_t>(k) * 32] = values[from + k];
+  }
+}
+
+// One product of the power iterations (qp_launch_product): the short items on the slices and a
+// warp per long item, or, without slices, `lanes` threads per item; the vector is normalised where an
+// item's sum leaves the warp, so no pass over it is spent on that.
+template <int SIDE>
+__global__ void __launch_bounds__(kQpSliceThreads, 1) k_qp_product(QpDev d, const double* v,
+                                                                const double* norm2, double* out,
+                                                                int lanes, double* next,
+                                                                double* part,
+                                                                unsigned int* ticket) {
+  __shared__ double scratch[2 * (kQpSliceThreads / 32)];
+  __shared__ double s_inv;
+  const QpSliceSet& S = SIDE == kQpRows ? d.rows : d.cols;
+  const int count = SIDE == kQpRows ? d.m : d.n;
+  const int* starts = SIDE == kQpRows ? d.a_rs : (SIDE == kQpCols ? d.a_cs : d.q_rs);
+  const int* index = SIDE == kQpRows ? d.a_ci : (SIDE == kQpCols ? d.a_ri : d.q_ci);
+  const double* values = SIDE == kQpRows ? d.a_rv : (SIDE == kQpCols ? d.a_cv : d.q_v);
+  QpWalk<SIDE == kQpHessian ? 1 : 2> walk;
+  if (S.nslices > 0) walk.start(S);
+  if (threadIdx.x == 0) s_inv = norm2 != nullptr ? 1.0 / sqrt(*norm2) : 1.0;
+  __syncthreads();
+  const double inv = s_inv;
+  const int lane = threadIdx.x & 31;
+  constexpr int kWarps = kQpSliceThreads / 32;
+  const int warps = static_cast<int>(gridDim.x) * kWarps;
+  const int warp = static_cast<int>(blockIdx.x) * kWarps + static_cast<int>(threadIdx.x >> 5);
+  double acc[2] = {0.0, 0.0};  // sum out^2, sum out (v inv)
+  const auto put = [&](int item, double sum) {
+    const double o = sum * inv;
+    out[item] = o;
+    if (next != nullptr) {
+      acc[0] = fma(o, o, acc[0]);
+      if (SIDE == kQpHessian) acc[1] = fma(o, v[item] * inv, acc[1]);
     }
-    s = group_sum<G>(s);
-    if (r < rows && lane == 0) out[r] = s;
+  };
+  if (S.nslices > 0) {
+    for (; walk.s < walk.s1; walk.advance(S)) {
+      const QpPlace p = walk.p;
+      double sum1, sum2;
+      walk.sums(S, v, v, &sum1, &sum2);
+      if (p.has) put(p.item, SIDE == kQpHessian ? sum1 : sum2);
+    }
+    const QpChunk* chunks = SIDE == kQpRows ? d.row_chunks : d.col_chunks;
+    const int nchunks = SIDE == kQpRows ? d.nrow_chunks : d.ncol_chunks;
+    for (int c = warp; c < nchunks; c += warps) {
+      if (chunks[c].begin != 0) continue;
+      const int item = chunks[c].item;
+      double sum = 0.0;
+      for (int e = starts[item] + lane; e < starts[item + 1]; e += 32) {
+        sum = fma(values[e], v[index[e]], sum);
+      }
+      sum = warp_sum(sum);
+      if (lane == 0) put(item, sum);
+    }
+  } else {
+    // Every warp runs the same number of rounds, so its lanes stay together for the sums.
+    const int per = 32 / lanes, sub = lane & (lanes - 1);
+    for (long long i0 = static_cast<long long>(warp) * per; i0 < count;
+         i0 += static_cast<long long>(warps) * per) {
+      const int item = static_cast<int>(i0) + lane / lanes;
+      double sum = 0.0;
+      if (item < count) {
+        for (int e = starts[item] + sub; e < starts[item + 1]; e += lanes) {
+          sum = fma(values[e], v[index[e]], sum);
+        }
+      }
+      for (int o = lanes >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (item < count && sub == 0) put(item, sum);
+    }
+  }
+  if (next == nullptr) return;
+  double total[2];
+  block_sum<2>(acc, scratch, total);
+  __shared__ int s_last;
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = total[0];
+    part[2 * blockIdx.x + 1] = total[1];
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  acc[0] = acc[1] = 0.0;
+  for (int b = static_cast<int>(threadIdx.x); b < static_cast<int>(gridDim.x);
+       b += kQpSliceThreads) {
+    acc[0] += __ldcg(part + 2 * b);
+    acc[1] += __ldcg(part + 2 * b + 1);
+  }
+  block_sum<2>(acc, scratch, total);
+  if (threadIdx.x == 0) {
+    next[0] = total[0];
+    next[1] = total[1];
+    *ticket = 0u;
   }
 }
 
@@ -481,14 +768,6 @@ __global__ void __launch_bounds__(kQpThreads) k_qp_dot_final(const double* parti
   if (threadIdx.x == 0) *out = total[0];
 }
 
-__global__ void k_qp_scale(double* v, int n, const double* norm2) {
-  const double norm = sqrt(*norm2);
-  for (int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); i < n;
-       i += static_cast<int>(gridDim.x * blockDim.x)) {
-    v[i] = __ddiv_rn(v[i], norm);
-  }
-}
-
 __global__ void k_qp_row_dual(QpDev d, double* row_dual) {
   for (int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); i < d.m;
        i += static_cast<int>(gridDim.x * blockDim.x)) {
@@ -512,10 +791,15 @@ int grid_for(int n) { return n <= 0 ? 0 : std::min((n + kQpThreads - 1) / kQpThr
 
 template <int MODE>
 void column_pass(const QpDev& d, QpCtl* ctl, int k, int src, cudaStream_t s) {
-  const int grid = d.col_short_blocks + (d.ncol_chunks + 7) / 8;
+  const bool sliced = d.cols.nslices > 0;
+  const int warps = (sliced ? kQpSliceThreads : kQpThreads) / 32;
+  const int grid = d.col_short_blocks + (d.ncol_chunks + warps - 1) / warps;
   if (grid == 0) return;
   const int smem = d.stage ? kQpStageBytes : 0;
-  switch (d.col_lanes) {
+  switch (sliced ? 0 : d.col_lanes) {
+    case 0:
+      launch_after(k_qp_column<0, MODE>, grid, kQpSliceThreads, 0, s, d, ctl, k, src);
+      break;
     case 1: launch_after(k_qp_column<1, MODE>, grid, kQpThreads, smem, s, d, ctl, k, src); break;
     case 2: launch_after(k_qp_column<2, MODE>, grid, kQpThreads, 0, s, d, ctl, k, src); break;
     case 4: launch_after(k_qp_column<4, MODE>, grid, kQpThreads, 0, s, d, ctl, k, src); break;
@@ -528,10 +812,15 @@ void column_pass(const QpDev& d, QpCtl* ctl, int k, int src, cudaStream_t s) {
 
 template <int MODE>
 void row_pass(const QpDev& d, QpCtl* ctl, int k, int src, cudaStream_t s) {
-  const int grid = d.row_short_blocks + (d.nrow_chunks + 7) / 8;
+  const bool sliced = d.rows.nslices > 0;
+  const int warps = (sliced ? kQpSliceThreads : kQpThreads) / 32;
+  const int grid = d.row_short_blocks + (d.nrow_chunks + warps - 1) / warps;
   if (grid == 0) return;
   const int smem = d.stage ? kQpStageBytes : 0;
-  switch (d.row_lanes) {
+  switch (sliced ? 0 : d.row_lanes) {
+    case 0:
+      launch_after(k_qp_row<0, MODE>, grid, kQpSliceThreads, 0, s, d, ctl, k, src);
+      break;
     case 1: launch_after(k_qp_row<1, MODE>, grid, kQpThreads, smem, s, d, ctl, k, src); break;
     case 2: launch_after(k_qp_row<2, MODE>, grid, kQpThreads, 0, s, d, ctl, k, src); break;
     case 4: launch_after(k_qp_row<4, MODE>, grid, kQpThreads, 0, s, d, ctl, k, src); break;
@@ -570,19 +859,43 @@ void qp_launch_advance(QpCtl* ctl, int graph_iterations, cudaStream_t s) {
   ++g_qp_launches;
 }
 
-void qp_launch_spmv(int rows, const int* starts, const int* index, const double* values,
-                    const double* v, double* out, int lanes, cudaStream_t s) {
-  if (rows <= 0) return;
-  const long long threads = static_cast<long long>(rows) * lanes;
-  const int grid = static_cast<int>(std::min<long long>((threads + kQpThreads - 1) / kQpThreads, 8192));
-  switch (lanes) {
-    case 1: k_qp_spmv<1><<<grid, kQpThreads, 0, s>>>(rows, starts, index, values, v, out); break;
-    case 2: k_qp_spmv<2><<<grid, kQpThreads, 0, s>>>(rows, starts, index, values, v, out); break;
-    case 4: k_qp_spmv<4><<<grid, kQpThreads, 0, s>>>(rows, starts, index, values, v, out); break;
-    case 8: k_qp_spmv<8><<<grid, kQpThreads, 0, s>>>(rows, starts, index, values, v, out); break;
-    case 16: k_qp_spmv<16><<<grid, kQpThreads, 0, s>>>(rows, starts, index, values, v, out); break;
-    default: k_qp_spmv<32><<<grid, kQpThreads, 0, s>>>(rows, starts, index, values, v, out); break;
+int qp_product_blocks(const QpDev& d) {
+  constexpr int kWarps = kQpSliceThreads / 32;
+  // A sliced side's blocks each take their own slices; otherwise the warps stride over the items.
+  const int warps = std::max({d.ncol_chunks, d.nrow_chunks, d.cols.nslices > 0 ? 0 : d.n / 32,
+                              d.rows.nslices > 0 ? 0 : d.m / 32, 1});
+  return std::max({std::min((warps + kWarps - 1) / kWarps, 2048), d.cols.blocks, d.rows.blocks});
+}
+
+void qp_launch_product(const QpDev& d, int side, const double* v, const double* norm2, double* out,
+                       int lanes, double* next, double* part, unsigned int* ticket,
+                       cudaStream_t s) {
+  const int grid = qp_product_blocks(d);
+  const auto launch = [&](auto kernel) {
+    kernel<<<grid, kQpSliceThreads, 0, s>>>(d, v, norm2, out, lanes, next, part, ticket);
+  };
+  if (side == kQpRows) {
+    launch(k_qp_product<kQpRows>);
+  } else if (side == kQpCols) {
+    launch(k_qp_product<kQpCols>);
+  } else {
+    launch(k_qp_product<kQpHessian>);
   }
+  ++g_qp_launches;
+}
+
+void qp_launch_slice_fill(const QpDev& d, bool cols, int* idx1, double* val1, int* idx2,
+                          double* val2, cudaStream_t s) {
+  const QpSliceSet& S = cols ? d.cols : d.rows;
+  if (S.nslices == 0) return;
+  const int grid = (S.nslices + kQpWarps - 1) / kQpWarps;
+  if (cols) {
+    k_qp_slice_fill<<<grid, kQpThreads, 0, s>>>(S, 1, d.q_rs, d.q_ci, d.q_v, idx1, val1);
+    ++g_qp_launches;
+  }
+  k_qp_slice_fill<<<grid, kQpThreads, 0, s>>>(S, 2, cols ? d.a_cs : d.a_rs,
+                                              cols ? d.a_ri : d.a_ci, cols ? d.a_cv : d.a_rv,
+                                              idx2, val2);
   ++g_qp_launches;
 }
 
@@ -591,12 +904,6 @@ void qp_launch_dot(const double* a, const double* b, int n, double* partials, do
   k_qp_dot_partial<<<kQpDotBlocks, kQpThreads, 0, s>>>(a, b, n, partials);
   k_qp_dot_final<<<1, kQpThreads, 0, s>>>(partials, out);
   g_qp_launches += 2;
-}
-
-void qp_launch_scale(double* v, int n, const double* norm2, cudaStream_t s) {
-  if (n <= 0) return;
-  k_qp_scale<<<grid_for(n), kQpThreads, 0, s>>>(v, n, norm2);
-  ++g_qp_launches;
 }
 
 void qp_launch_row_dual(const QpDev& d, double* row_dual, cudaStream_t s) {

@@ -159,6 +159,81 @@ inline void qp_build_chunks(const std::vector<int>& len, int lanes, std::vector<
   }
 }
 
+// ---- Sliced items ----------------------------------------------------------------------------
+// The one-lane passes' layout of the matrix: a slice is 32 items that one warp sums, one item per
+// lane, with lane l's k-th entry at 32 (base + k) + l, so that a slice's entries are one run.
+// Items of at most kQpLongPerLane entries are dealt to slices by length, longest first, inside
+// groups of kQpGroup consecutive items: a warp takes as long as its longest item. A column's
+// entries are its row of Q and its column of A, stored apart; a row has the second part only.
+constexpr int kQpGroup = 128;
+constexpr unsigned kQpNoItem = 0xffffffffu;
+
+struct QpSlices {
+  int nslices = 0;
+  // Per slice and lane: the item's place in its group (7 bits), its entries of the first part
+  // (from bit 8) and of the second (from bit 16); kQpNoItem where there is no short item.
+  std::vector<unsigned> meta;
+  std::vector<unsigned> base1, base2;  // per slice: first entry / 32 of each part; nslices + 1
+  std::vector<int> block_start;        // block b's slices: [block_start[b], block_start[b + 1])
+};
+
+// starts1 may be null (no first part). At most `blocks` blocks, cut by cost (entry rows, and an
+// epilogue's worth per slice), of at least four slices on average.
+inline void qp_build_slices(const int* starts1, const int* starts2, int count, int blocks,
+                            QpSlices* out) {
+  const int groups = (count + kQpGroup - 1) / kQpGroup, per = kQpGroup / 32;
+  out->nslices = groups * per;
+  const size_t ns = static_cast<size_t>(out->nslices);
+  out->meta.assign(ns * 32, kQpNoItem);
+  out->base1.assign(ns + 1, 0);
+  out->base2.assign(ns + 1, 0);
+  unsigned t1 = 0, t2 = 0;
+  const auto len1 = [&](int i) { return starts1 != nullptr ? starts1[i + 1] - starts1[i] : 0; };
+  const auto len2 = [&](int i) { return starts2[i + 1] - starts2[i]; };
+  for (int g = 0; g < groups; ++g) {
+    const int i0 = g * kQpGroup, i1 = std::min(count, i0 + kQpGroup);
+    int start[kQpLongPerLane + 2] = {0};
+    for (int i = i0; i < i1; ++i) {
+      const int len = len1(i) + len2(i);
+      if (len <= kQpLongPerLane) ++start[kQpLongPerLane - len + 1];
+    }
+    for (int k = 0; k <= kQpLongPerLane; ++k) start[k + 1] += start[k];
+    unsigned* meta = out->meta.data() + static_cast<size_t>(g) * kQpGroup;
+    for (int i = i0; i < i1; ++i) {
+      const int a = len1(i), b = len2(i);
+      if (a + b > kQpLongPerLane) continue;
+      meta[start[kQpLongPerLane - a - b]++] = static_cast<unsigned>(i - i0) |
+                                              static_cast<unsigned>(a) << 8 |
+                                              static_cast<unsigned>(b) << 16;
+    }
+    for (int s = 0; s < per; ++s) {
+      unsigned w1 = 0, w2 = 0;
+      for (int l = 0; l < 32; ++l) {
+        const unsigned m = meta[s * 32 + l];
+        if (m == kQpNoItem) continue;
+        w1 = std::max(w1, (m >> 8) & 255u);
+        w2 = std::max(w2, m >> 16);
+      }
+      t1 += w1;
+      t2 += w2;
+      out->base1[static_cast<size_t>(g) * per + s + 1] = t1;
+      out->base2[static_cast<size_t>(g) * per + s + 1] = t2;
+    }
+  }
+  const int G = std::max(1, std::min(blocks, (out->nslices + 3) / 4));
+  const auto cost = [&](int s) {
+    return static_cast<double>(out->base1[static_cast<size_t>(s)]) +
+           static_cast<double>(out->base2[static_cast<size_t>(s)]) + 8.0 * s;
+  };
+  out->block_start.assign(static_cast<size_t>(G) + 1, out->nslices);
+  int s = 0;
+  for (int b = 0; b < G; ++b) {
+    out->block_start[static_cast<size_t>(b)] = s;
+    const double upto = cost(out->nslices) * (b + 1) / G;
+    while (s < out->nslices && b + 1 < G && cost(s) + cost(s + 1) < 2.0 * upto) ++s;
+  }
+}
+
 // Lanes per item from the mean entries per item: the smallest power of two that leaves each
 // lane at most 32 entries of a typical item. The passes wait on memory and on the FP64 pipe,
 // where a lane that sits out the epilogue costs as much as a working one, so few lanes win:

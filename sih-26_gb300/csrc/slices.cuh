@@ -1,10 +1,11 @@
 // slices.cuh -- sliced rows: the FP64 sparse-product engine.
 //
 // A SLICE is 32 rows (of the CSR copy, or columns of the CSC copy) that one warp sums, one row
-// per lane, with the entries stored so that lane l's k-th entry is at base + 32 k + l: every
-// matrix load of a warp is one contiguous 256-byte (values) or 128-byte (indices) run. A lane
-// walks its own row in ascending index order with FMA, so every short row is summed in the
-// reference's order.
+// per lane, with the entries stored so that lane l's k-th entry is at base + 32 k + l: a slice's
+// entries are one contiguous run. A lane walks its own row in ascending index order with FMA, so
+// every short row is summed in the reference's order. (Splitting the rows of a small matrix over
+// 2 to 8 lanes to shorten their walk was slower at every size tried, down to 50 x 100: the lanes
+// that sit out the epilogue cost the FP64 pipe as much as working ones.)
 //
 // Rows are dealt to slices inside GROUPS of kGroupRows consecutive rows, longest first, so the
 // rows of a slice have nearly the same length: GB300 retires two FP64 lane operations per clock
@@ -20,14 +21,21 @@
 // pieces of kSlicePiece entries when it is longer than that; the pieces of a row are combined in
 // order by the kernel's last block.
 //
-// WINDOWS. A random 8-byte gather from L1 or L2 costs a tag lookup and a sector each, 32 per
-// warp-wide gather at about one per clock per SM; from shared memory a warp-wide gather of
-// doubles costs about 7 clocks of bank conflicts. So a block keeps a window [lo, lo + len) of
-// the gathered vector in shared memory where the layout's windows hold at least 95% of its
-// entries (build_windows over the groups), copied in by one bulk copy per segment of groups.
+// PIECES. A warp takes a slice in pieces of up to kPiece entry rows: a piece's values and gathers are
+// requested together, then the next piece's indices (of this slice, or the first of the warp's
+// next), then the products are added, so a warp waits for memory once per piece. The first
+// indices are requested before the kernel may read anything that an earlier one wrote, since the
+// matrix never changes between the kernels of a graph. Each count of rows has its own code:
+// predicated-off FP64 instructions hold the pipe like working ones.
 //
-// Block b owns a contiguous run of groups, cut by cost, and its warps take the run's slices in
-// turn: every sum and every block partial is taken in a fixed order, so runs are
+// WINDOWS. A random 8-byte gather from L1 or L2 costs a tag lookup and a sector each, 32 per
+// warp-wide gather at one per clock per SM; from shared memory a warp-wide gather of
+// doubles costs about 7 clocks of bank conflicts. So a block keeps a window [lo, lo + len) of
+// the gathered vector in shared memory where the layout's windows hold enough of its entries
+// (build_windows over the groups; Engine::plan_sliced), copied in by one bulk copy per segment of
+// groups.
+//
+// Block b owns a contiguous run of slices, cut by cost, and its warps take them in turn: every sum and every block partial is taken in a fixed order, so runs are
 // bit-reproducible. Warps do not wait for one another except where the window changes. Every
 // wait is bounded: a wait that gives up raises the block's abort flag, the block's remaining
 // slices are skipped, a copy still in flight is given a bounded time to land, and the caller
@@ -47,7 +55,8 @@ constexpr int kGroupRows = 128;
 constexpr int kGroupSlices = kGroupRows / 32;
 constexpr int kSliceLong = 64;     // entries past which a row is long
 constexpr int kSlicePiece = kCap;  // entries per piece of a long row
-constexpr int kSliceThreads = 1024;  // the largest block of a slice kernel
+constexpr int kSliceThreads = 768;   // the largest block of a slice kernel: 85 registers a thread
+constexpr int kPiece = 8;            // entry rows (32 entries each) per piece, at most
 constexpr unsigned short kNoRow = 0xffff;
 
 // A piece of a long row (or all of it): entries [begin, begin + count) of the layout's long
@@ -69,20 +78,21 @@ struct SliceSet {
   // Per slice and lane: the row's place in its group (7 bits) and its length (from bit 8), or
   // kNoRow (no row, or a long one).
   const unsigned short* meta;
-  const unsigned int* base;  // per slice: first entry / 32
+  const unsigned int* base;  // per slice: first entry / 32; nslices + 1
   const int* idx;
   const double* val;
   const SliceItem* items;
   const LongRow* longs;      // rows of several pieces
   const SliceSeg* segs;
   const int* seg_start;      // per block: its segments [seg_start[b], seg_start[b + 1])
+  const int* block_start;    // per block: its slices [block_start[b], block_start[b + 1])
   long long long_base;       // first entry of the long region
   int nslices, nitems, nlong, nchunks, nrows;
   int wmax;                  // window capacity in gathered elements (0: none)
   int grid, threads;
 };
 
-// Shared memory of a slice kernel's window: the mbarrier, then the window.
+// Dynamic shared memory of a slice kernel with a window: its mbarrier, then the window.
 constexpr int kSliceBarBytes = 128;
 template <typename G>
 __host__ __device__ constexpr int slice_smem(int wmax) {
@@ -94,48 +104,102 @@ __device__ __forceinline__ int slice_row(int s, unsigned m) {
   return (s / kGroupSlices) * kGroupRows + static_cast<int>(m & 127u);
 }
 
-// One slice. `m` is the lane's meta word and `base` the slice's first entry / 32. A lane loads
-// the indices and values of kBatch entries, then gathers them, then accumulates: two memory
-// latencies per kBatch entries.
-constexpr int kSliceBatch = 4;
-
-template <int NP, int NR, typename G, typename Get, typename Mac, typename Load, typename Epi>
-__device__ __forceinline__ void slice_step(const SliceSet& S, int s, unsigned m, unsigned base,
-                                           Get get, Mac mac, Load load, Epi epi) {
-  const int lane = static_cast<int>(threadIdx.x) & 31;
-  const bool has = m != kNoRow;
-  const int len = has ? static_cast<int>(m >> 8) : 0;
-  const int row = slice_row(s, m);
-  double ops[NR > 0 ? NR : 1];
-  if (has) load(row, ops);
-  const int width = __shfl_sync(0xffffffffu, len, 0);  // lane 0 holds the longest row
-  const size_t at = static_cast<size_t>(base) * 32 + static_cast<size_t>(lane);
-  const int* __restrict__ ip = S.idx + at;
-  const double* __restrict__ vp = S.val + at;
-  double acc[NP];
+// The indices of a lane's next piece: its first P of `left` entries from `idx` on.
+template <int P>
+struct PieceIndices {
+  int c[P];
+  __device__ __forceinline__ void load(const int* __restrict__ idx, int left) {
 #pragma unroll
-  for (int q = 0; q < NP; ++q) acc[q] = 0.0;
-  for (int k = 0; k < width; k += kSliceBatch) {
-    int c[kSliceBatch];
-    double v[kSliceBatch];
-#pragma unroll
-    for (int u = 0; u < kSliceBatch; ++u) {
-      const bool in = k + u < len;
-      c[u] = in ? ld_stream(ip + (k + u) * 32) : -1;
-      v[u] = in ? ld_stream(vp + (k + u) * 32) : 0.0;
-    }
-    G g[kSliceBatch];
-#pragma unroll
-    for (int u = 0; u < kSliceBatch; ++u) g[u] = c[u] >= 0 ? get(c[u]) : G{};
-#pragma unroll
-    for (int u = 0; u < kSliceBatch; ++u) {
-      if (k + u < width) mac(v[u], g[u], acc);
-    }
+    for (int u = 0; u < P; ++u) c[u] = u < left ? ld_stream(idx + u * 32) : 0;
   }
-  if (has) epi(row, acc, ops);
+};
+
+// N entry rows: the lane's `left` entries' values from `val` on, gathered with get(c) and added with
+// mac(v, g); `p` holds the piece's indices on entry and the next piece's on exit.
+template <int N, typename G, int P, typename Get, typename Mac>
+__device__ __forceinline__ void slice_piece(const double* __restrict__ val, int left,
+                                            PieceIndices<P>& p, const int* next_idx, int next_left,
+                                            Get get, Mac mac) {
+  if constexpr (N <= P) {
+    double v[N > 0 ? N : 1];
+    G g[N > 0 ? N : 1];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const bool in = u < left;
+      v[u] = in ? ld_stream(val + u * 32) : 0.0;
+      g[u] = in ? get(p.c[u]) : G{};
+    }
+    p.load(next_idx, next_left);
+#pragma unroll
+    for (int u = 0; u < N; ++u) mac(v[u], g[u]);
+  }
+}
+
+// A lane's `len` entries of a slice `width` entry rows wide, the first at idx / val; `p` as above,
+// (next_idx, next_left) the first piece of what the warp sums next.
+template <typename G, int P, typename Get, typename Mac>
+__device__ __forceinline__ void slice_sum(const int* idx, const double* val, int len, int width,
+                                          PieceIndices<P>& p, const int* next_idx, int next_left,
+                                          Get get, Mac mac) {
+  static_assert(P <= 8, "a case per count");
+  int k = 0;
+  do {
+    const bool more = k + P < width;
+    const int* ni = more ? idx + (k + P) * 32 : next_idx;
+    const int nl = more ? len - k - P : next_left;
+    const double* v = val + k * 32;
+    const int left = len - k;
+    switch (min(width - k, P)) {
+      case 0: p.load(ni, nl); break;
+      case 1: slice_piece<1, G>(v, left, p, ni, nl, get, mac); break;
+      case 2: slice_piece<2, G>(v, left, p, ni, nl, get, mac); break;
+      case 3: slice_piece<3, G>(v, left, p, ni, nl, get, mac); break;
+      case 4: slice_piece<4, G>(v, left, p, ni, nl, get, mac); break;
+      case 5: slice_piece<5, G>(v, left, p, ni, nl, get, mac); break;
+      case 6: slice_piece<6, G>(v, left, p, ni, nl, get, mac); break;
+      case 7: slice_piece<7, G>(v, left, p, ni, nl, get, mac); break;
+      default: slice_piece<8, G>(v, left, p, ni, nl, get, mac); break;
+    }
+    k += P;
+  } while (k < width);
+}
+
+// A lane's place in slice s of a layout: its meta word and the slice's first entry.
+struct SlicePlace {
+  unsigned m;
+  size_t at;
+  int len;
+  __device__ __forceinline__ void load(const SliceSet& S, int s, int s1) {
+    const int lane = static_cast<int>(threadIdx.x) & 31;
+    m = kNoRow;
+    at = 0;
+    if (s < s1) {
+      m = __ldg(S.meta + static_cast<size_t>(s) * 32 + lane);
+      at = static_cast<size_t>(__ldg(S.base + s)) * 32 + lane;
+    }
+    len = m != kNoRow ? static_cast<int>(m >> 8) : 0;
+  }
+};
+
+// What a warp holds of its first slice when its kernel starts to wait for the ones before it.
+template <int P>
+struct SliceStart {
+  int s, s1;
+  SlicePlace place;
+  PieceIndices<P> indices;
+};
+
+template <int P>
+__device__ __forceinline__ void start_slices(const SliceSet& S, SliceStart<P>& st) {
+  st.s = __ldg(S.block_start + blockIdx.x) + (static_cast<int>(threadIdx.x) >> 5);
+  st.s1 = __ldg(S.block_start + blockIdx.x + 1);
+  st.place.load(S, st.s, st.s1);
+  st.indices.load(S.idx + st.place.at, st.place.len);
 }
 
 // One long item, by the whole warp.
+constexpr int kSliceBatch = 4;
+
 template <int NP, int NR, typename G, typename Get, typename Mac, typename Load, typename Epi>
 __device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& it,
                                            double* chunk_part, Get get, Mac mac, Load load,
@@ -182,15 +246,14 @@ __device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& i
 //   load(row, ops), epi(row, acc, ops) the row's NR operands and its epilogue
 // WIN is false in kernels that stage no window whatever the layout has. Returns false -- in
 // every thread -- if a wait gave up (only a staged window waits).
-template <bool WIN, int NP, int NR, typename G, typename Fetch, typename Mac, typename Load,
+template <bool WIN, int NP, int NR, typename G, int P, typename Fetch, typename Mac, typename Load,
           typename Epi>
-__device__ __forceinline__ bool run_slices(const SliceSet& S, const G* vec, Fetch fetch,
-                                           unsigned char* dsmem, double* chunk_part, Mac mac,
-                                           Load load, Epi epi) {
+__device__ __forceinline__ bool run_slices(const SliceSet& S, SliceStart<P>& st, const G* vec,
+                                           Fetch fetch, unsigned char* dsmem, double* chunk_part,
+                                           Mac mac, Load load, Epi epi) {
   __shared__ volatile int s_abort;
   const int W = static_cast<int>(blockDim.x) >> 5;
   const int warp = static_cast<int>(threadIdx.x) >> 5;
-  const int lane = static_cast<int>(threadIdx.x) & 31;
   uint64_t* bar = reinterpret_cast<uint64_t*>(dsmem);
   G* win = reinterpret_cast<G*>(dsmem + kSliceBarBytes);
   const bool windowed = WIN && S.wmax > 0;
@@ -204,8 +267,11 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, const G* vec, Fetc
   }
   bool pending = false;  // thread 0: a copy issued and not yet seen complete
   uint32_t phase = 0;
-  const int g0 = S.seg_start[blockIdx.x], g1 = S.seg_start[blockIdx.x + 1];
+  const int g0 = __ldg(S.seg_start + blockIdx.x), g1 = __ldg(S.seg_start + blockIdx.x + 1);
   bool ok = true;
+  int s = st.s;
+  SlicePlace p = st.place;
+  PieceIndices<P> ix = st.indices;
   for (int g = g0; g < g1; ++g) {
     const SliceSeg sg = S.segs[g];
     if (WIN && sg.len > 0) {
@@ -228,10 +294,10 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, const G* vec, Fetc
     }
     if (!ok) break;
     const int lo = sg.lo;
-    const unsigned len = static_cast<unsigned>(sg.len);
+    const unsigned wlen = static_cast<unsigned>(sg.len);
     auto get = [&](int c) {
       const unsigned o = static_cast<unsigned>(c - lo);
-      return WIN && o < len ? win[o] : fetch(c);
+      return WIN && o < wlen ? win[o] : fetch(c);
     };
     if (g == g0) {
       for (int i = static_cast<int>(blockIdx.x) + warp * static_cast<int>(gridDim.x);
@@ -239,25 +305,25 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, const G* vec, Fetc
         slice_item<NP, NR, G>(S, S.items[i], chunk_part, get, mac, load, epi);
       }
     }
-    // The next slice's meta word and base are loaded while this one is worked on.
-    int s = sg.s0 + warp;
-    unsigned m = kNoRow, base = 0;
-    if (s < sg.s1) {
-      m = __ldg(S.meta + static_cast<size_t>(s) * 32 + lane);
-      base = __ldg(S.base + s);
-    }
     for (; s < sg.s1; s += W) {
-      const unsigned cm = m, cb = base;
-      const int sn = s + W;
-      if (sn < sg.s1) {
-        m = __ldg(S.meta + static_cast<size_t>(sn) * 32 + lane);
-        base = __ldg(S.base + sn);
-      }
-      slice_step<NP, NR, G>(S, s, cm, cb, get, mac, load, epi);
+      const bool has = p.m != kNoRow;
+      const int row = slice_row(s, p.m);
+      SlicePlace next;  // on its way while this slice is summed
+      next.load(S, s + W, st.s1);
+      double ops[NR > 0 ? NR : 1];
+      if (has) load(row, ops);
+      double acc[NP];
+#pragma unroll
+      for (int q = 0; q < NP; ++q) acc[q] = 0.0;
+      const int width = __shfl_sync(0xffffffffu, p.len, 0);  // lane 0 holds the longest row
+      slice_sum<G>(S.idx + p.at, S.val + p.at, p.len, width, ix, S.idx + next.at, next.len, get,
+                   [&](double v, G gv) { mac(v, gv, acc); });
+      if (has) epi(row, acc, ops);
+      p = next;
     }
   }
   if (!windowed || ok) return true;
-  // A copy still in flight must land before the block exits (bounded).
+  // A window copy still in flight must land too (bounded).
   if (threadIdx.x == 0 && pending) mbar_wait_bounded(bar, phase ^ 1u);
   __syncthreads();
   return false;

@@ -38,6 +38,9 @@ static void check(const std::vector<int>& len, int extent, int wmax, double wind
     if (place[static_cast<size_t>(at)]++) fail("two entries at one place", at, 0);
   };
   if (p.nslices % kGroupSlices != 0 || p.nslices * 32LL < lines) fail("slices", p.nslices, lines);
+  if (static_cast<int>(p.base.size()) != p.nslices + 1 || p.base[p.nslices] * 32LL != p.long_base) {
+    fail("bases", static_cast<long long>(p.base.size()), p.nslices);
+  }
   for (int s = 0; s < p.nslices; ++s) {
     int before = kSliceLong;
     for (int l = 0; l < 32; ++l) {
@@ -51,6 +54,7 @@ static void check(const std::vector<int>& len, int extent, int wmax, double wind
       if (row >= lines) fail("row", row, lines);
       if (n != len[row]) fail("length", n, len[row]);
       if (n > before) fail("longest first", s, l);
+      if (n > static_cast<int>(p.base[s + 1] - p.base[s])) fail("width", s, n);
       before = n;
       ++seen[row];
       for (int k = 0; k < n; ++k) put(static_cast<long long>(p.base[s]) * 32 + 32LL * k + l);
@@ -90,6 +94,7 @@ static void check(const std::vector<int>& len, int extent, int wmax, double wind
   int at = 0;
   for (int b = 0; b < p.grid; ++b) {
     if (p.seg_start[b + 1] <= p.seg_start[b]) fail("block without a segment", b, 0);
+    if (p.block_start[b] != at) fail("block start", p.block_start[b], at);
     for (int g = p.seg_start[b]; g < p.seg_start[b + 1]; ++g) {
       const SliceSeg& sg = p.segs[g];
       if (sg.s1 > sg.s0) {
@@ -102,6 +107,7 @@ static void check(const std::vector<int>& len, int extent, int wmax, double wind
       }
     }
   }
+  if (p.block_start[p.grid] != p.nslices) fail("last block", p.block_start[p.grid], p.nslices);
   if (at != p.nslices) fail("slices covered", at, p.nslices);
 }
 

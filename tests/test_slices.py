@@ -98,3 +98,23 @@ def test_slices_match_the_oracle(oracle, m, n, longest):
     scale = max(1.0, np.abs(ref.col_value).max())
     assert np.abs(px - ref.col_value).max() <= 1e-9 * scale
     assert np.abs(py - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,per_column,band", [(0, 33, 0, 2), (1, 1, 1, 0), (31, 33, 3, 1),
+                                                 (128, 129, 5, 0), (40, 300, 20, 30)])
+def test_qp_slices_match_the_oracle(oracle, m, n, per_column, band):
+    """The QP passes on sliced items (lanes left to the engine) around a slice and a group, with
+    no rows, and with columns on both sides of the long-item limit: the oracle's status and
+    iteration count, and its point within 1e-9 of its scale, as every QP parity test."""
+    from sankhya_gb300.model import random_qp
+
+    qp = random_qp(17 + n, m, n, per_column=per_column, hessian_band=band)
+    ref = oracle.solve_qp(qp, tolerance=1e-8, iteration_limit=1500)
+    with capi.QpEngine(0) as eng:
+        eng.load(qp)
+        got = eng.solve(tolerance=1e-8, iteration_limit=1500)
+        x, d, y = eng.solution()
+    assert (got.status_name, got.iterations) == (ref.status_name, ref.iterations)
+    for a, b in ((x, ref.col_value), (d, ref.col_dual), (y, ref.row_dual)):
+        assert np.all(np.abs(a - b) <= 1e-9 * max(1.0, np.abs(b).max() if len(b) else 0.0))
