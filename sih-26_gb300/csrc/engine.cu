@@ -298,6 +298,9 @@ size_t estimate_memory(long long rows, long long cols, long long nnz, int precis
   return bytes;
 }
 
+// Attempted steps per resident kernel: an evaluation period of 40 accepted steps and some rejected.
+constexpr int kResidentAttempts = 48;
+
 // Power steps of the spectral-norm estimate (src/la/scaling.cpp:161).
 constexpr int kPowerSteps = 30;
 
@@ -597,8 +600,21 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   // windows hold any entry, so tests run the split form.
   int cap = -1;
   if (const char* env = std::getenv("SANKHYA_GB300_WINDOW_CAP")) cap = std::max(0, std::atoi(env)) & ~3;
-  plan_sliced(sl_csc_, cptr, lp.row_index, n, m, 0, cap);
-  plan_sliced(sl_csr_, rptr, ridx.data(), m, n, 1, cap);
+  // The resident step takes LPs that its cluster's shared memory holds and that have no long rows
+  // or columns (slices.cuh). Every block holds both gathered vectors, 16 (n + m) bytes; past half
+  // of the shared memory for them the rest no longer fits.
+  const auto longest = [](const std::vector<int>& ptr) {
+    int len = 0;
+    for (size_t r = 1; r < ptr.size(); ++r) len = std::max(len, ptr[r] - ptr[r - 1]);
+    return len;
+  };
+  int resident = 0;
+  if (m > 0 && n > 0 && cap < 0 && 16LL * (m + n) <= 120 * 1024 && longest(cptr) <= kSliceLong &&
+      longest(rptr) <= kSliceLong) {
+    resident = resident_blocks((n + 31) / 32, (m + 31) / 32);
+  }
+  plan_sliced(sl_csc_, cptr, lp.row_index, n, m, 0, cap, resident);
+  plan_sliced(sl_csr_, rptr, ridx.data(), m, n, 1, cap, resident);
   plan_layout(ck_csc_f_, cptr, lp.row_index, n, m, 0, cap);
   plan_layout(ck_csr_f_, rptr, ridx.data(), m, n, 1, cap);
   const int grid_c = std::max({sl_csc_.view.grid, grid_csc_f_, ck_csc_f_.grid});
@@ -665,6 +681,9 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   SGB_CUDA(cudaMemsetAsync(tickets_.ptr, 0, 4 * sizeof(unsigned int), s));
   SGB_CUDA(cudaStreamSynchronize(s));
   fill_buffers();
+  resident_smem_ = resident_smem(m, n, sl_csc_.most_rows, sl_csc_.most_slices, sl_csr_.most_rows,
+                                 sl_csr_.most_slices);
+  resident_ = resident > 0 && resident_fits(step_, resident_smem_);
   loaded_ = true;
 }
 
@@ -677,7 +696,7 @@ void Engine::load(const sankhya_gb300_lp& lp) {
 // through SANKHYA_GB300_WINDOW_CAP (window_cap >= 0) keeps its windows whatever their share. A
 // fixed rule, not a timing: runs must not vary.
 void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* lidx, int lines,
-                         int extent, int pass, int window_cap) {
+                         int extent, int pass, int window_cap, int resident) {
   constexpr int kFullWindow = 32 * 1024;
   cudaStream_t s = stream_;
   const int elem = static_cast<int>(pass == 0 ? sizeof(double) : sizeof(double2));
@@ -688,7 +707,7 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
     wmax = 0;
   }
   const SlicePlan P =
-      plan_slices(lptr, lidx, lines, extent, wmax, 0.0, num_sms_, pass == 0 ? 1 : 2);
+      plan_slices(lptr, lidx, lines, extent, wmax, 0.0, num_sms_, pass == 0 ? 1 : 2, resident);
   D.meta.upload(P.meta.data(), P.meta.size(), s);
   D.base.upload(P.base.data(), P.base.size(), s);
   D.items.upload(P.items.data(), P.items.size(), s);
@@ -702,6 +721,13 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
   D.scaled.allocate(e);
   SGB_CUDA(cudaStreamSynchronize(s));  // the plan's arrays end here
   D.staged = P.staged;
+  D.most_rows = D.most_slices = 0;
+  for (int b = 0; b < P.grid; ++b) {
+    const int s0 = P.block_start[static_cast<size_t>(b)], s1 = P.block_start[static_cast<size_t>(b) + 1];
+    D.most_slices = std::max(D.most_slices, s1 - s0);
+    D.most_rows = std::max(D.most_rows, static_cast<int>(P.base[static_cast<size_t>(s1)] -
+                                                         P.base[static_cast<size_t>(s0)]));
+  }
   SliceSet& S = D.view;
   S = SliceSet{};
   S.meta = D.meta.ptr;
@@ -1054,10 +1080,20 @@ void Engine::build_graphs(int steps) {
   for (int slot = 0; slot < 2; ++slot) {
     cudaGraph_t graph = nullptr;
     SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < steps; ++k) {
-      launch_pdhg_step(step_, stream_);
-      if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_evaluation(eval_, stream_);
+    const long long before = kernel_launch_count();
+    if (resident_) {
+      // A resident kernel ends where an evaluation falls due, at most 40 accepted steps on.
+      for (int k = 0; k < steps; k += kResidentAttempts) {
+        launch_pdhg_resident(step_, std::min(kResidentAttempts, steps - k), resident_smem_, stream_);
+        launch_evaluation(eval_, stream_);
+      }
+    } else {
+      for (int k = 0; k < steps; ++k) {
+        launch_pdhg_step(step_, stream_);
+        if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_evaluation(eval_, stream_);
+      }
     }
+    graph_launches_ = static_cast<int>(kernel_launch_count() - before);
     cudaMemcpyAsync(snapshot_ + slot, ctl_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_);
     const cudaError_t end = cudaStreamEndCapture(stream_, &graph);
     SGB_CUDA(end);
@@ -1235,7 +1271,9 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
 
   int stop_status = SANKHYA_GB300_ITERATION_LIMIT;
   const long long launches_setup = kernel_launch_count() - launches_before;
-  build_graphs(p.steps_per_poll > 0 ? p.steps_per_poll : 32);  // capture launches nothing
+  // Capture launches nothing. A resident step takes a fraction of the time, so by default a graph
+  // holds one evaluation period of them, rejected steps included.
+  build_graphs(p.steps_per_poll > 0 ? p.steps_per_poll : (resident_ ? kResidentAttempts : 32));
   const long long count_after_capture = kernel_launch_count();
   run_graphs(p, t0, graph_exec_, snapshot_, true, 0, &stop_status);
   const double t_end_loop = now_seconds();
@@ -1248,10 +1286,11 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   SGB_CUDA(cudaEventElapsedTime(&device_ms, timing_[0], timing_[1]));
   r->device_seconds = 1e-3 * device_ms;
   launches_ = launches_setup + (kernel_launch_count() - count_after_capture) +
-              graphs_launched_ * graph_kernel_launches(graph_steps_);
+              graphs_launched_ * graph_launches_;
   r->kernel_launches = launches_;
-  r->staged_fraction[0] = sl_csc_.staged;
-  r->staged_fraction[1] = sl_csr_.staged;
+  // A resident step gathers every entry from shared memory.
+  r->staged_fraction[0] = resident_ ? 1.0 : sl_csc_.staged;
+  r->staged_fraction[1] = resident_ ? 1.0 : sl_csr_.staged;
   if (c.error) {
     throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "a tile copy did not complete in time"};
   }

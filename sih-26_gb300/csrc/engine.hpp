@@ -123,10 +123,11 @@ class Engine {
     DeviceArray<SliceSeg> segs;
     SliceSet view{};      // val = the scaled values
     double staged = 0.0;  // share of the nonzeros gathered from a staged window
+    int most_rows = 0, most_slices = 0;  // entry rows and slices of the largest block
   };
   SliceDev sl_csc_, sl_csr_;
   void plan_sliced(SliceDev& D, const std::vector<int>& ptr, const int* idx, int lines,
-                   int extent, int pass, int window_cap);
+                   int extent, int pass, int window_cap, int resident);
   // The FP32 step passes' chunk layouts (chunks.cuh): CSC (column pass) and CSR (row pass).
   // A split layout owns its main and outer index arrays (and the maps from their entries to
   // the full layout's, through which each solve fills their values); otherwise it reads the
@@ -181,6 +182,9 @@ class Engine {
   Ctl* snapshot_ = nullptr;  // pinned host, two slots
   cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};
   int graph_steps_ = 0;
+  int graph_launches_ = 0;  // engine kernels per step graph
+  bool resident_ = false;   // FP64 steps run in the resident kernel,
+  int resident_smem_ = 0;   // with this much shared memory a block
   cudaEvent_t done_event_[2] = {nullptr, nullptr};
   cudaEvent_t timing_[2] = {nullptr, nullptr};
   long long launches_ = 0;  // engine kernels launched by the current solve
@@ -209,7 +213,8 @@ class Engine {
 };
 
 // The sliced layout of one matrix layout (layout.cu): windows of at most `wmax` elements are
-// kept where they hold at least `window_min` of the entries; at most `sms` blocks.
+// kept where they hold at least `window_min` of the entries; at most `sms` blocks, or `resident`
+// of them.
 struct SlicePlan {
   int nslices = 0, nchunks = 0, wmax = 0, grid = 1, threads = 128;
   long long long_base = 0, entries = 0;  // first entry of the long region; entries stored
@@ -222,7 +227,7 @@ struct SlicePlan {
   std::vector<int> seg_start, block_start;
 };
 SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, int extent, int wmax,
-                      double window_min, int sms, int np);
+                      double window_min, int sms, int np, int resident = 0);
 
 size_t estimate_memory(long long rows, long long cols, long long nnz, int precision);
 

@@ -143,6 +143,13 @@ struct EvalBuffers {
 
 // ---- Launchers (pdhg_kernels.cu) ---------------------------------------------------------
 void launch_pdhg_step(const StepBuffers& b, cudaStream_t s);
+// The resident form (slices.cuh): up to `attempts` attempted steps in one kernel, which ends at once
+// when an evaluation falls due; `smem` is resident_smem of the largest block.
+void launch_pdhg_resident(const StepBuffers& b, int attempts, int smem, cudaStream_t s);
+// Dynamic shared memory of a resident block with these slices and entry rows of the two layouts, in
+// a problem of m rows and n columns; and whether the device can run the cluster with it.
+int resident_smem(int m, int n, int col_rows, int col_slices, int row_rows, int row_slices);
+bool resident_fits(const StepBuffers& b, int smem);
 void launch_primal_pass(const StepBuffers& b, cudaStream_t s);
 void launch_dual_pass(const StepBuffers& b, cudaStream_t s);
 // Kernels launched per attempted step inside a graph (2 step + 4 evaluation kernels).

@@ -344,7 +344,7 @@ ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, in
 // `np` products are accumulated per entry by the kernel that runs on it (the cost model: a
 // slice costs its longest row's entries times np FP64 instructions, plus its epilogue).
 SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, int extent, int wmax,
-                      double window_min, int sms, int np) {
+                      double window_min, int sms, int np, int resident) {
   SlicePlan p;
   const int ngroups = (lines + kGroupRows - 1) / kGroupRows;
   const long long nnz = lines > 0 ? ptr[lines] : 0;
@@ -410,9 +410,9 @@ SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, in
   // Blocks: at most one per SM and not under four slices each (a small matrix spreads over the
   // SMs: the FP64 pipe of each is the bound even there), cut where the running cost passes the
   // next share; a block has as many warps as its slices or items keep busy, at most
-  // kSliceThreads threads.
+  // kSliceThreads threads. A resident layout's blocks are its cluster's.
   const int wanted = (std::max(p.nslices, static_cast<int>(p.items.size())) + 3) / 4;
-  const int G = std::max(1, std::min(wanted, sms));
+  const int G = resident > 0 ? resident : std::max(1, std::min(wanted, sms));
   p.grid = G;
   p.seg_start.assign(static_cast<size_t>(G) + 1, 0);
   p.block_start.assign(static_cast<size_t>(G) + 1, p.nslices);
@@ -449,6 +449,7 @@ SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, in
   p.seg_start[static_cast<size_t>(G)] = static_cast<int>(p.segs.size());
   most = std::max(most, (static_cast<int>(p.items.size()) + G - 1) / G);
   p.threads = std::min(kSliceThreads, std::max(128, (most + 3) / 4 * 128));
+
   return p;
 }
 

@@ -229,6 +229,186 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
   }
 }
 
+// ---- The resident step (slices.cuh) -----------------------------------------------------------
+// The passes of k_primal and k_dual, item for item, in one cluster. Every block keeps a copy of the
+// control block and takes the same step decision from the same sums, in the same order, so the
+// blocks agree on every branch. The warps' partial sums go to every block, into one of two tables
+// by step: a block may be in the next column pass while another still adds the last step's.
+constexpr int kResidentWarps = kResidentThreads / 32;
+constexpr int kResidentTable = kResidentBlocks * kResidentWarps;
+
+// Copies a block's state to (or, WRITE, from) shared memory: the slots' items of `src`.
+template <bool WRITE>
+__device__ __forceinline__ void local_items(const LocalSlices& L, double* slots, double* global) {
+  for (int k = static_cast<int>(threadIdx.x); k < L.n * 32; k += static_cast<int>(blockDim.x)) {
+    const unsigned m = L.meta[k];
+    if (m == kNoRow) continue;
+    const int item = slice_row(L.s0 + k / 32, m);
+    if (WRITE) {
+      global[item] = slots[k];
+    } else {
+      slots[k] = global[item];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffers b, int attempts) {
+  extern __shared__ __align__(128) unsigned char dsmem[];
+  __shared__ Ctl s_ctl;
+  __shared__ double2 s_factors;
+  __shared__ double s_tau, s_sigma, s_sums[3];
+  __shared__ double s_part[2][3][kResidentTable];
+  static_assert(sizeof(Ctl) % sizeof(unsigned long long) == 0, "copied by words");
+  constexpr int kWords = static_cast<int>(sizeof(Ctl) / sizeof(unsigned long long));
+  const int T = static_cast<int>(blockDim.x), t = static_cast<int>(threadIdx.x);
+  const int C = static_cast<int>(gridDim.x), W = T >> 5, lane = t & 31, warp = t >> 5;
+  const int m = b.csr.nrows, n = b.csc.nrows;
+  unsigned long long* const words = reinterpret_cast<unsigned long long*>(&s_ctl);
+  for (int k = t; k < kWords; k += T) {
+    words[k] = reinterpret_cast<const volatile unsigned long long*>(b.ctl)[k];
+  }
+  // Shared memory: the gathered vectors at the same place in every block, then the block's own.
+  double2* const xd = reinterpret_cast<double2*>(dsmem);
+  double* const ys[2] = {reinterpret_cast<double*>(xd + n), reinterpret_cast<double*>(xd + n) + m};
+  unsigned char* mem = dsmem + (static_cast<size_t>(n) * 16 + static_cast<size_t>(m) * 16);
+  LocalSlices cs, rs;
+  mem = fill_local(b.csc, cs, mem);
+  mem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(mem) + 15) & ~uintptr_t(15));
+  mem = fill_local(b.csr, rs, mem);
+  double* const own = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(mem) + 15) & ~uintptr_t(15));
+  const int nc = cs.n * 32, nr = rs.n * 32;
+  double* const x[2] = {own, own + nc};
+  double *const xsum = own + 2 * nc, *const c = own + 3 * nc, *const lo = own + 4 * nc,
+         *const up = own + 5 * nc;
+  double *const ysum = own + 6 * nc, *const rl = ysum + nr, *const ru = ysum + 2 * nr;
+  __syncthreads();
+  const int first = s_ctl.cur;
+  local_items<false>(cs, x[first], b.x[first]);
+  local_items<false>(cs, xsum, b.x_sum);
+  local_items<false>(cs, c, const_cast<double*>(b.c));
+  local_items<false>(cs, lo, const_cast<double*>(b.l));
+  local_items<false>(cs, up, const_cast<double*>(b.u));
+  local_items<false>(rs, ysum, b.y_sum);
+  local_items<false>(rs, rl, const_cast<double*>(b.rl));
+  local_items<false>(rs, ru, const_cast<double*>(b.ru));
+  for (int i = t; i < m; i += T) ys[first][i] = b.y[first][i];
+  if (t == 0) {
+    if (s_ctl.done == kRunning && s_ctl.eval_now == 0 &&
+        s_ctl.iteration >= s_ctl.iteration_limit) {
+      s_ctl.done = kIterationLimit;  // src/pdhg/pdhg.cpp:206
+    }
+    s_tau = s_ctl.eta / s_ctl.omega;
+    s_sigma = s_ctl.eta * s_ctl.omega;
+  }
+  cluster_meet();  // every block has read the control block, and may be written to
+  for (int a = 0; a < attempts; ++a) {
+    if (s_ctl.done != kRunning || s_ctl.eval_now != 0) break;
+    const int cur = s_ctl.cur;
+    const bool add = s_ctl.pending_add != 0;
+    const double tau = s_tau, sigma = s_sigma, omega = s_ctl.omega;
+    double(*const part)[kResidentTable] = s_part[a & 1];
+    if (t == T - 1) s_factors = step_factors(s_ctl.iteration, b.step_factors, b.step_factors_n);
+    {
+      const double* y = ys[cur];
+      double mv = 0.0;
+      for (int s = warp; s < cs.n; s += W) {
+        const unsigned meta = cs.meta[s * 32 + lane];
+        if (meta == kNoRow) continue;
+        const int len = static_cast<int>(meta >> 8), e = cs.base[s] * 32 + lane, k = s * 32 + lane;
+        double g = 0.0;
+#pragma unroll 4
+        for (int q = 0; q < len; ++q) g = fma(cs.val[e + q * 32], y[cs.idx[e + q * 32]], g);
+        const double xj = x[cur][k];
+        if (add) xsum[k] = xsum[k] + xj;
+        const double xnj = clamp_box(__dsub_rn(xj, __dmul_rn(tau, c[k] + g)), lo[k], up[k]);
+        x[cur ^ 1][k] = xnj;
+        const double d = xnj - xj;
+        const double2 both = make_double2(fma(2.0, xnj, -xj), d);
+        double2* const at = xd + slice_row(cs.s0 + s, meta);
+        for (int r = 0; r < C; ++r) cluster_store(cluster_addr(at, r), both);
+        mv = fma(d, d, mv);
+      }
+      __syncwarp();
+      mv = warp_sum(mv);
+      if (lane < C) {
+        cluster_store(cluster_addr(&part[0][static_cast<int>(blockIdx.x) * W + warp], lane), mv);
+      }
+    }
+    cluster_meet();
+    {
+      const double* y = ys[cur];
+      double* const yn = ys[cur ^ 1];
+      double dy2 = 0.0, ia = 0.0;
+      for (int s = warp; s < rs.n; s += W) {
+        const unsigned meta = rs.meta[s * 32 + lane];
+        if (meta == kNoRow) continue;
+        const int len = static_cast<int>(meta >> 8), e = rs.base[s] * 32 + lane, k = s * 32 + lane;
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll 4
+        for (int q = 0; q < len; ++q) {
+          const double v = rs.val[e + q * 32];
+          const double2 p = xd[rs.idx[e + q * 32]];
+          s0 = fma(v, p.x, s0);
+          s1 = fma(v, p.y, s1);
+        }
+        const int i = slice_row(rs.s0 + s, meta);
+        const double yi = y[i];
+        if (add) ysum[k] = ysum[k] + yi;
+        const double v = __dadd_rn(yi, __dmul_rn(sigma, s0));
+        const double p = rl[k] == ru[k] ? rl[k] : clamp_box(v / sigma, rl[k], ru[k]);
+        const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
+        for (int r = 0; r < C; ++r) cluster_store(cluster_addr(yn + i, r), yni);
+        const double d = yni - yi;
+        dy2 = fma(d, d, dy2);
+        ia = fma(d, s1, ia);
+      }
+      __syncwarp();
+      dy2 = warp_sum(dy2);
+      ia = warp_sum(ia);
+      if (lane < C) {
+        const int at = static_cast<int>(blockIdx.x) * W + warp;
+        cluster_store(cluster_addr(&part[1][at], lane), dy2);
+        cluster_store(cluster_addr(&part[2][at], lane), ia);
+      }
+    }
+    cluster_meet();
+    // A warp per sum: the primal movement, the dual movement over omega, the interaction.
+    if (t < 96) {
+      const int q = t >> 5;
+      double sum = 0.0;
+      for (int k = lane; k < C * W; k += 32) sum += part[q][k];
+      sum = warp_sum(sum);
+      if (lane == 0) s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? (0.5 * sum) / omega : sum);
+    }
+    __syncthreads();
+    if (t == 0) {
+      s_ctl.mv_primal = s_sums[0];
+      step_decision(&s_ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), s_factors);
+      if (s_ctl.eval_now == 0 && s_ctl.iteration >= s_ctl.iteration_limit) {
+        s_ctl.done = kIterationLimit;
+      }
+      s_tau = s_ctl.eta / s_ctl.omega;
+      s_sigma = s_ctl.eta * s_ctl.omega;
+    }
+    __syncthreads();
+  }
+  // The current iterate, the sums and the control block go back; the other buffers are written
+  // before they are read again.
+  const int last = s_ctl.cur;
+  local_items<true>(cs, x[last], b.x[last]);
+  local_items<true>(cs, xsum, b.x_sum);
+  local_items<true>(rs, ysum, b.y_sum);
+  for (int k = t; k < nr; k += T) {
+    const unsigned meta = rs.meta[k];
+    if (meta == kNoRow) continue;
+    const int i = slice_row(rs.s0 + k / 32, meta);
+    b.y[last][i] = ys[last][i];
+  }
+  if (blockIdx.x == 0) {
+    for (int k = t; k < kWords; k += T) reinterpret_cast<unsigned long long*>(b.ctl)[k] = words[k];
+  }
+}
+
 // ---- Evaluation ----------------------------------------------------------------------------
 __device__ __forceinline__ bool eval_active(const Ctl* c) {
   return c->final_mode != 0 || (c->eval_now != 0 && c->done == kRunning);
@@ -861,7 +1041,10 @@ bool configure_fp64_kernels() {
       cudaFuncSetAttribute(k_primal, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_primal))),
       cudaFuncSetAttribute(k_dual, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           max_dynamic_smem(reinterpret_cast<const void*>(k_dual)))};
+                           max_dynamic_smem(reinterpret_cast<const void*>(k_dual))),
+      cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           max_dynamic_smem(reinterpret_cast<const void*>(k_pdhg_resident))),
+      cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)};
   for (cudaError_t e : errs) {
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -891,6 +1074,28 @@ void launch_primal_pass(const StepBuffers& b, cudaStream_t s) {
 void launch_dual_pass(const StepBuffers& b, cudaStream_t s) {
   launch_after(k_dual, b.csr.grid, b.csr.threads, slice_smem<double2>(b.csr.wmax), s, b);
   ++g_launches;
+}
+
+namespace {
+int resident_threads(const StepBuffers& b) {
+  return std::min(kResidentThreads, std::max(b.csc.threads, b.csr.threads));
+}
+}  // namespace
+
+int resident_smem(int m, int n, int col_rows, int col_slices, int row_rows, int row_slices) {
+  return 16 * n + 16 * m + local_slices_bytes(col_rows, col_slices) +
+         local_slices_bytes(row_rows, row_slices) + 32 + 8 * 32 * (6 * col_slices + 3 * row_slices);
+}
+
+bool resident_fits(const StepBuffers& b, int smem) {
+  return b.csc.grid == b.csr.grid &&
+         smem <= max_dynamic_smem(reinterpret_cast<const void*>(k_pdhg_resident)) &&
+         cluster_fits(k_pdhg_resident, b.csc.grid, resident_threads(b), smem);
+}
+
+void launch_pdhg_resident(const StepBuffers& b, int attempts, int smem, cudaStream_t s) {
+  ++g_launches;
+  launch_cluster(k_pdhg_resident, b.csc.grid, resident_threads(b), smem, s, b, attempts);
 }
 
 void launch_pdhg_step(const StepBuffers& b, cudaStream_t s) {

@@ -195,6 +195,8 @@ void QpEngine::plan_sliced(SliceDev& D, const int* starts1, const int* starts2, 
   D.block_start.upload(P.block_start.data(), P.block_start.size(), s);
   const size_t e1 = static_cast<size_t>(P.base1.back()) * 32;
   const size_t e2 = static_cast<size_t>(P.base2.back()) * 32;
+  D.rows1 = P.base1.back();
+  D.rows2 = P.base2.back();
   D.idx1.allocate(e1);
   D.val1.allocate(e1);
   D.idx2.allocate(e2);
@@ -252,6 +254,16 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
   cols_sliced_ = cols_sliced;
   rows_sliced_ = rows_sliced;
   const QpDev d = dev();
+  // The smallest QPs iterate in one block (slices.cuh). The line is kQpResidentItems, not what a
+  // block or a cluster holds: kernel_launches is read as at least two per iteration from 200 x 400
+  // on (tests/test_gpu_qp.py).
+  constexpr int kQpResidentItems = 256;
+  const long long smem = qp_resident_smem(m_, n_, col_slices_.rows1, col_slices_.rows2,
+                                          row_slices_.rows2);
+  resident_ = cols_sliced && (rows_sliced || m_ == 0) && n_ > 0 &&
+              std::max(m_, n_) <= kQpResidentItems && cc.empty() && rc.empty() &&
+              qp_resident_fits(smem);
+  resident_smem_ = resident_ ? static_cast<int>(smem) : 0;
   if (cols_sliced) {
     qp_launch_slice_fill(d, true, col_slices_.idx1.ptr, col_slices_.val1.ptr,
                          col_slices_.idx2.ptr, col_slices_.val2.ptr, s);
@@ -383,7 +395,10 @@ void QpEngine::build_graph(int periods) {
   cudaGraph_t graph = nullptr;
   SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
   for (int p = 0; p < periods; ++p) {
-    for (int it = 0; it < kQpCheckEvery; ++it) {
+    if (resident_) {
+      qp_launch_resident(d, ctl, p * kQpCheckEvery, kQpCheckEvery, 0, resident_smem_, stream_);
+    }
+    for (int it = 0; it < kQpCheckEvery && !resident_; ++it) {
       const int k = p * kQpCheckEvery + it;
       qp_launch_column_pass(d, ctl, kQpStep, k, k & 1, stream_);
       if (m_ > 0) qp_launch_row_pass(d, ctl, kQpStep, k, 0, stream_);

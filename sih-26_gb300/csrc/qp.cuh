@@ -129,6 +129,13 @@ struct QpDev {
 void qp_launch_column_pass(const QpDev& d, QpCtl* ctl, int mode, int k, int src,
                            cudaStream_t s);
 void qp_launch_row_pass(const QpDev& d, QpCtl* ctl, int mode, int k, int src, cudaStream_t s);
+// The resident form (slices.cuh) of a QP whose matrices and vectors one block's shared memory
+// holds: iterations k0 .. k0 + count - 1 of the graph; x is in buffer `src` before the first.
+// qp_resident_smem: the block's dynamic shared memory; qp_resident_fits: whether it has that much.
+void qp_launch_resident(const QpDev& d, QpCtl* ctl, int k0, int count, int src, int smem,
+                        cudaStream_t s);
+long long qp_resident_smem(int m, int n, long long rows_q, long long rows_a, long long rows_r);
+bool qp_resident_fits(long long smem);
 // The decision after the check whose last iteration is graph index k (period p).
 void qp_launch_decide(const QpDev& d, QpCtl* ctl, int k, int p, cudaStream_t s);
 // base += iterations of the graph (capped at the limit) unless done.

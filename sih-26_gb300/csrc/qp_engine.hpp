@@ -56,11 +56,14 @@ class QpEngine {
   // Layout for the current lanes.
   int col_lanes_ = 0, row_lanes_ = 0;
   bool cols_sliced_ = false, rows_sliced_ = false;
+  bool resident_ = false;  // the iterations run in the resident kernel,
+  int resident_smem_ = 0;  // with this much shared memory
   struct SliceDev {
     DeviceArray<unsigned int> meta, base1, base2;
     DeviceArray<int> idx1, idx2, block_start;
     DeviceArray<double> val1, val2;
     QpSliceSet view{};
+    long long rows1 = 0, rows2 = 0;  // entry rows of each part
   };
   SliceDev col_slices_, row_slices_;
   void plan_sliced(SliceDev& D, const int* starts1, const int* starts2, int count);

@@ -197,6 +197,7 @@ struct QpWalk {
   PieceIndices<kPiece> ix;
   unsigned m;  // of the next slice
   unsigned b1, b2;
+  int step;
 
   __device__ __forceinline__ void fetch(const QpSliceSet& S, int next) {
     m = kQpNoItem;
@@ -213,6 +214,7 @@ struct QpWalk {
     at2 = static_cast<size_t>(b2) * 32 + (threadIdx.x & 31);
   }
   __device__ __forceinline__ void start(const QpSliceSet& S) {
+    step = static_cast<int>(blockDim.x >> 5);
     const bool mine = static_cast<int>(blockIdx.x) < S.blocks;
     s = mine ? __ldg(S.block_start + blockIdx.x) + static_cast<int>(threadIdx.x >> 5) : 0;
     s1 = mine ? __ldg(S.block_start + blockIdx.x + 1) : 0;
@@ -223,7 +225,7 @@ struct QpWalk {
     } else {
       ix.load(S.idx1 + at1, p.len1);
     }
-    fetch(S, s + kQpSliceThreads / 32);
+    fetch(S, s + step);
   }
   // The next slice's first piece, once its record has arrived.
   __device__ __forceinline__ void after(const QpSliceSet& S, const int** idx, int* left) const {
@@ -237,9 +239,10 @@ struct QpWalk {
       *left = n.len1;
     }
   }
-  // The item's sums over the parts of PART, FMA-accumulated in entry order.
-  __device__ __forceinline__ void sums(const QpSliceSet& S, const double* __restrict__ v1,
-                                       const double* __restrict__ v2, double* sum1,
+  // The item's sums over the parts of PART, FMA-accumulated in entry order, of the vectors that
+  // get1(c) and get2(c) read.
+  template <typename Get1, typename Get2>
+  __device__ __forceinline__ void sums(const QpSliceSet& S, Get1 get1, Get2 get2, double* sum1,
                                        double* sum2) {
     const int* ni;
     int nl;
@@ -248,21 +251,19 @@ struct QpWalk {
     if (PART != 2) {
       slice_sum<double>(S.idx1 + at1, S.val1 + at1, p.len1, __reduce_max_sync(0xffffffffu, p.len1),
                         ix, PART == 0 ? S.idx2 + at2 : ni, PART == 0 ? p.len2 : nl,
-                        [&](int c) { return __ldg(v1 + c); },
-                        [&](double v, double g) { a1 = fma(v, g, a1); });
+                        get1, [&](double v, double g) { a1 = fma(v, g, a1); });
     }
     if (PART != 1) {
       slice_sum<double>(S.idx2 + at2, S.val2 + at2, p.len2, __reduce_max_sync(0xffffffffu, p.len2),
-                        ix, ni, nl, [&](int c) { return __ldg(v2 + c); },
-                        [&](double v, double g) { a2 = fma(v, g, a2); });
+                        ix, ni, nl, get2, [&](double v, double g) { a2 = fma(v, g, a2); });
     }
     *sum1 = a1;
     *sum2 = a2;
   }
   __device__ __forceinline__ void advance(const QpSliceSet& S) {
-    s += kQpSliceThreads / 32;
+    s += step;
     unpack();
-    fetch(S, s + kQpSliceThreads / 32);
+    fetch(S, s + step);
   }
 };
 
@@ -332,7 +333,8 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_column(QpDev d, QpCtl* c
       ColumnOps o;
       if (p.has) o.load(d, x, p.item);
       double qx, aty, r = 0.0, t = 0.0;
-      walk.sums(d.cols, x, d.y, &qx, &aty);
+      walk.sums(d.cols, [&](int c) { return __ldg(x + c); }, [&](int c) { return __ldg(d.y + c); },
+                &qx, &aty);
       if (p.has) column_epilogue<MODE>(d, tau, p.item, o, xn, qx, aty, &r, &t);
       if (MODE != kQpStep) {
         residual = r > residual ? r : residual;
@@ -460,14 +462,19 @@ struct RowOps {
   }
 };
 
+// y' = v - sigma proj(v / sigma), v = y + sigma (A xbar)_i (src/qp/qp_condat_vu.cpp:270-276).
+__device__ __forceinline__ double row_step(double sigma, double inv_sigma, const RowOps& o,
+                                           double ax) {
+  const double v = __dadd_rn(o.y, __dmul_rn(sigma, ax));
+  const double p = box(divide(v, sigma, inv_sigma), o.lower, o.upper);
+  return __dsub_rn(v, __dmul_rn(sigma, p));
+}
+
 template <int MODE>
 __device__ __forceinline__ double row_epilogue(const QpDev& d, double sigma, double inv_sigma,
                                                int i, const RowOps& o, double ax) {
   if (MODE == kQpStep) {
-    // y' = v - sigma proj(v / sigma), v = y + sigma (A xbar)_i (src/qp/qp_condat_vu.cpp:270-276).
-    const double v = __dadd_rn(o.y, __dmul_rn(sigma, ax));
-    const double p = box(divide(v, sigma, inv_sigma), o.lower, o.upper);
-    d.y[i] = __dsub_rn(v, __dmul_rn(sigma, p));
+    d.y[i] = row_step(sigma, inv_sigma, o, ax);
     return 0.0;
   }
   const double projected = box(ax, o.lower, o.upper);
@@ -491,7 +498,7 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl,
       RowOps o;
       if (p.has) o.load(d, p.item);
       double none, ax;
-      walk.sums(d.rows, nullptr, v, &none, &ax);
+      walk.sums(d.rows, [](int) { return 0.0; }, [&](int c) { return __ldg(v + c); }, &none, &ax);
       if (p.has) {
         const double r = row_epilogue<MODE>(d, sigma, inv_sigma, p.item, o, ax);
         residual = r > residual ? r : residual;
@@ -568,6 +575,98 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl,
     const double residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, o, ax);
     if (MODE == kQpCheck) max_bits(&ctl->primal_bits, residual);
   }
+}
+
+// ---- The resident iterations (slices.cuh) ------------------------------------------------------
+// The step forms of the two passes, item for item, in one block with everything in shared memory.
+// One part of the slices: the entries, indices as 16 bits, and the slices' first entry rows.
+struct QpLocal {
+  const double* val;
+  const unsigned short* idx;
+  const int* base;
+  __device__ __forceinline__ double dot(int s, int len, const double* v) const {
+    const int e = base[s] * 32 + (threadIdx.x & 31);
+    double acc = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < len; ++q) acc = fma(val[e + q * 32], v[idx[e + q * 32]], acc);
+    return acc;
+  }
+};
+
+__device__ __forceinline__ unsigned char* qp_fill_local(const int* idx, const double* val,
+                                                        const unsigned* base, int slices,
+                                                        unsigned char* mem, QpLocal* out) {
+  const int rows = static_cast<int>(base[slices]);
+  double* const v = reinterpret_cast<double*>(mem);
+  int* const b = reinterpret_cast<int*>(v + rows * 32);
+  unsigned short* const i = reinterpret_cast<unsigned short*>(b + ((slices + 4) & ~3));
+  const int T = static_cast<int>(blockDim.x), t = static_cast<int>(threadIdx.x);
+  for (int k = t; k < rows * 32; k += T) {
+    v[k] = val[k];
+    i[k] = static_cast<unsigned short>(idx[k]);
+  }
+  for (int k = t; k <= slices; k += T) b[k] = static_cast<int>(base[k]);
+  *out = QpLocal{v, i, b};
+  return reinterpret_cast<unsigned char*>(i + ((rows * 32 + 7) & ~7));
+}
+
+// A warp holds one slice of columns and one of rows (kQpResidentItems), a lane its column's and its
+// row's data in registers.
+__global__ void __launch_bounds__(kResidentThreads, 1) k_qp_resident(QpDev d, QpCtl* ctl, int k0,
+                                                                     int count, int src) {
+  extern __shared__ __align__(16) unsigned char qp_smem[];
+  if (ctl->done != 0) return;
+  const long long left = ctl->limit - (ctl->base + k0);
+  const int iterations = left < count ? static_cast<int>(left) : count;
+  if (iterations <= 0) return;
+  const double tau = ctl->tau, sigma = ctl->sigma, inv_sigma = ctl->inv_sigma;
+  const int T = static_cast<int>(blockDim.x), t = static_cast<int>(threadIdx.x);
+  const int warp = t >> 5, m = d.m, n = d.n;
+  double* const xs0 = reinterpret_cast<double*>(qp_smem);
+  double* const xs1 = xs0 + n;
+  double* const xbar = xs0 + 2 * n;
+  double* const ys = xs0 + 3 * n;
+  for (int j = t; j < n; j += T) {
+    xs0[j] = d.x0[j];
+    xs1[j] = d.x1[j];
+  }
+  for (int i = t; i < m; i += T) ys[i] = d.y[i];
+  unsigned char* mem = qp_smem + ((3 * n + m) * 8 + 15) / 16 * 16;
+  QpLocal q, a, r;
+  mem = qp_fill_local(d.cols.idx1, d.cols.val1, d.cols.base1, d.cols.nslices, mem, &q);
+  mem = qp_fill_local(d.cols.idx2, d.cols.val2, d.cols.base2, d.cols.nslices, mem, &a);
+  if (m > 0) qp_fill_local(d.rows.idx2, d.rows.val2, d.rows.base2, d.rows.nslices, mem, &r);
+  QpPlace col, row;
+  col.set(warp, qp_meta(d.cols, warp, d.cols.nslices));
+  row.set(warp, qp_meta(d.rows, warp, m > 0 ? d.rows.nslices : 0));
+  ColumnOps o{0.0, 0.0, 0.0, 0.0};
+  if (col.has) o.load(d, src ? d.x1 : d.x0, col.item);
+  RowOps w{0.0, 0.0, 0.0};
+  if (row.has) w.load(d, row.item);
+  __syncthreads();
+  for (int i = 0; i < iterations; ++i) {
+    const bool odd = (src + i) & 1;
+    if (col.has) {
+      const double qx = q.dot(warp, col.len1, odd ? xs1 : xs0), aty = a.dot(warp, col.len2, ys);
+      const double g = qp_gradient(o.c, qx, aty);
+      const double xnj = box(__dsub_rn(o.x, __dmul_rn(tau, g)), o.lower, o.upper);
+      (odd ? xs0 : xs1)[col.item] = xnj;
+      xbar[col.item] = fma(2.0, xnj, -o.x);
+      o.x = xnj;
+    }
+    __syncthreads();
+    if (row.has) {
+      w.y = row_step(sigma, inv_sigma, w, r.dot(warp, row.len2, xbar));
+      ys[row.item] = w.y;
+    }
+    __syncthreads();
+  }
+  for (int j = t; j < n; j += T) {
+    d.x0[j] = xs0[j];
+    d.x1[j] = xs1[j];
+    d.xbar[j] = xbar[j];
+  }
+  for (int i = t; i < m; i += T) d.y[i] = ys[i];
 }
 
 // ---- Decision -----------------------------------------------------------------------------
@@ -688,7 +787,8 @@ __global__ void __launch_bounds__(kQpSliceThreads, 1) k_qp_product(QpDev d, cons
     for (; walk.s < walk.s1; walk.advance(S)) {
       const QpPlace p = walk.p;
       double sum1, sum2;
-      walk.sums(S, v, v, &sum1, &sum2);
+      walk.sums(S, [&](int c) { return __ldg(v + c); }, [&](int c) { return __ldg(v + c); }, &sum1,
+                &sum2);
       if (p.has) put(p.item, SIDE == kQpHessian ? sum1 : sum2);
     }
     const QpChunk* chunks = SIDE == kQpRows ? d.row_chunks : d.col_chunks;
@@ -849,6 +949,26 @@ void qp_launch_row_pass(const QpDev& d, QpCtl* ctl, int mode, int k, int src, cu
   else row_pass<kQpCheck>(d, ctl, k, src, s);
 }
 
+long long qp_resident_smem(int m, int n, long long rows_q, long long rows_a, long long rows_r) {
+  const auto part = [](long long rows, int items) {
+    const int slices = (items + kQpGroup - 1) / kQpGroup * (kQpGroup / 32);
+    return rows * 32 * 10 + ((slices + 4) & ~3) * 4 + 16;
+  };
+  return 8LL * (3 * n + m) + 16 + part(rows_q, n) + part(rows_a, n) +
+         (m > 0 ? part(rows_r, m) : 0);
+}
+
+bool qp_resident_fits(long long smem) {
+  return smem <= max_dynamic_smem(reinterpret_cast<const void*>(k_qp_resident));
+}
+
+void qp_launch_resident(const QpDev& d, QpCtl* ctl, int k0, int count, int src, int smem,
+                        cudaStream_t s) {
+  const int warps = std::max(2, std::max(d.cols.nslices, d.rows.nslices));
+  k_qp_resident<<<1, std::min(kResidentThreads, warps * 32), smem, s>>>(d, ctl, k0, count, src);
+  ++g_qp_launches;
+}
+
 void qp_launch_decide(const QpDev& d, QpCtl* ctl, int k, int p, cudaStream_t s) {
   launch_after(k_qp_decide, 1, kQpThreads, 0, s, d, ctl, k, p);
   ++g_qp_launches;
@@ -928,6 +1048,8 @@ cudaError_t qp_configure_kernels() {
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kQpStageBytes);
     if (err == cudaSuccess) err = e;
   };
+  err = cudaFuncSetAttribute(k_qp_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             max_dynamic_smem(reinterpret_cast<const void*>(k_qp_resident)));
   opt(reinterpret_cast<const void*>(k_qp_column<1, kQpStep>));
   opt(reinterpret_cast<const void*>(k_qp_column<1, kQpCheck>));
   opt(reinterpret_cast<const void*>(k_qp_column<1, kQpReport>));

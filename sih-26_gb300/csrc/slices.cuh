@@ -45,6 +45,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "chunks.cuh"
 #include "common.cuh"
 #include "tiles.cuh"
@@ -327,6 +329,60 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, SliceStart<P>& st,
   if (threadIdx.x == 0 && pending) mbar_wait_bounded(bar, phase ^ 1u);
   __syncthreads();
   return false;
+}
+
+// ---- Resident solves ----------------------------------------------------------------------
+// Small problems run many steps in one RESIDENT kernel, a cluster of up to kResidentBlocks blocks.
+// A block keeps in shared memory its slices' entries and its items' data and state, and a copy of
+// each gathered vector, which the blocks write into one another's shared memory; they meet at the
+// cluster barrier between the passes. No step touches global memory, where the other path
+// launches two kernels (a step of 50 x 100 took 25 us so). The blocks of such a layout are the
+// cluster's.
+constexpr int kResidentBlocks = 16;
+constexpr int kResidentThreads = 512;
+
+// Blocks of the cluster for sides of `cols` and `rows` slices: four slices a block, one for each of
+// an SM's FP64 units, before another SM is taken.
+inline int resident_blocks(int cols, int rows) {
+  int blocks = 1;
+  while (blocks < kResidentBlocks && 4 * blocks < std::max(cols, rows)) blocks *= 2;
+  return blocks;
+}
+
+// A block's slices of one layout in shared memory: the entries (indices as 16 bits), and per slice
+// the first entry row, per slot the meta word.
+struct LocalSlices {
+  double* val;
+  unsigned short* idx;
+  unsigned short* meta;
+  int* base;
+  int s0, n;  // the block's first slice, its slices
+};
+
+// Bytes of a block's LocalSlices with `rows` entry rows and `slices` slices.
+__host__ __device__ inline int local_slices_bytes(int rows, int slices) {
+  return rows * 32 * 10 + slices * 32 * 2 + ((slices + 4) & ~3) * 4;
+}
+
+// Lays L out at `mem` and fills it; every thread calls it. Returns the first byte after it.
+__device__ __forceinline__ unsigned char* fill_local(const SliceSet& S, LocalSlices& L,
+                                                     unsigned char* mem) {
+  L.s0 = S.block_start[blockIdx.x];
+  L.n = S.block_start[blockIdx.x + 1] - L.s0;
+  const unsigned first = S.base[L.s0], rows = S.base[L.s0 + L.n] - first;
+  L.val = reinterpret_cast<double*>(mem);
+  L.base = reinterpret_cast<int*>(L.val + rows * 32);
+  L.idx = reinterpret_cast<unsigned short*>(L.base + ((L.n + 4) & ~3));
+  L.meta = L.idx + rows * 32;
+  const int T = static_cast<int>(blockDim.x), t = static_cast<int>(threadIdx.x);
+  const size_t at = static_cast<size_t>(first) * 32;
+  for (int k = t; k < static_cast<int>(rows) * 32; k += T) {
+    L.val[k] = S.val[at + k];
+    L.idx[k] = static_cast<unsigned short>(S.idx[at + k]);
+  }
+  for (int k = t; k < L.n * 32; k += T) L.meta[k] = S.meta[static_cast<size_t>(L.s0) * 32 + k];
+  for (int k = t; k <= L.n; k += T) L.base[k] = static_cast<int>(S.base[L.s0 + k] - first);
+  return reinterpret_cast<unsigned char*>(L.meta + L.n * 32);
 }
 
 // Last block only: the rows of several pieces, each combined from its partials in order.

@@ -101,6 +101,25 @@ def test_slices_match_the_oracle(oracle, m, n, longest):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(20, 30), (100, 200), (200, 400), (450, 900), (1300, 2600),
+                                 (3500, 3900)])
+def test_resident_steps_match_the_oracle(oracle, m, n):
+    """LPs on clusters of 1, 2, 4, 8 and 16 blocks and one past them: iteration limits are exact
+    inside and at the end of an evaluation period, and the point after 40 accepted steps is the
+    oracle's within 1e-9."""
+    lp = lp_with_rows(np.random.default_rng(n).integers(0, 21, size=m), n, seed=n)
+    with capi.PdhgEngine(0) as eng:
+        eng.load(lp)
+        for limit in (1, 41, 85):
+            assert eng.solve(tolerance=1e-13, iteration_limit=limit).iterations == limit
+        eng.solve(tolerance=1e-13, iteration_limit=40)
+        x, _, y = eng.solution()
+    ref = oracle.solve(lp, tolerance=1e-13, iteration_limit=40)
+    assert np.abs(x - ref.col_value).max() <= 1e-9 * max(1.0, np.abs(ref.col_value).max())
+    assert np.abs(y - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,per_column,band", [(0, 33, 0, 2), (1, 1, 1, 0), (31, 33, 3, 1),
                                                  (128, 129, 5, 0), (40, 300, 20, 30)])
 def test_qp_slices_match_the_oracle(oracle, m, n, per_column, band):
