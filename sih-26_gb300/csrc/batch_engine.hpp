@@ -45,6 +45,11 @@ class BatchEngine {
   // four LPs per SM, spread over the size order) and returns the fastest.
   void autotune(BatchBuffers b, bool mixed, int* lanes, int* threads);
   void ensure_adjoint_buffers();
+  // The reported points on the host: LPs [points_first_, points_end_) in page-locked memory, their
+  // x, reduced costs and y one after another. Forgotten when a solve, a polish or a set point
+  // changes them.
+  void fetch_points(int index);
+  void forget_points();
   AdjointBuffers adjoint_buffers();
   void finish_adjoint(double* const* dl_dc, double* const* dl_drl, double* const* dl_dru,
                       double* const* dl_dl, double* const* dl_du,
@@ -85,6 +90,9 @@ class BatchEngine {
   DeviceArray<float> v0_, v1_, v_sum_, v_rst_, gu_, gl_, yhat_, vc0_, vc1_, v_best_;
   DeviceArray<long long> refinements_;
   BatchBuffers buffers_{};  // of the last solve
+  double* points_host_ = nullptr;
+  size_t points_capacity_ = 0, points_n_ = 0;
+  int points_first_ = -1, points_end_ = -1;
   // Adjoint (allocated on first use).
   bool adjoint_ready_ = false;
   DeviceArray<double> a_gx_, a_gy_, a_gf_, a_dc_, a_dl_, a_du_, a_drl_, a_dru_;

@@ -59,9 +59,14 @@ void cuda_check(cudaError_t err, const char* what, const char* file, int line) {
 
 template <typename T>
 void DeviceArray<T>::allocate(size_t n) {
-  release();
+  const bool keep = n > 0 && n <= capacity &&
+                    (capacity <= kKeepFactor * n || capacity * sizeof(T) <= kKeepBytes);
+  if (!keep) {
+    release();
+    if (n > 0) SGB_CUDA(cudaMalloc(&ptr, n * sizeof(T)));
+    capacity = n;
+  }
   count = n;
-  if (n > 0) SGB_CUDA(cudaMalloc(&ptr, n * sizeof(T)));
 }
 template <typename T>
 void DeviceArray<T>::upload(const T* host, size_t n, cudaStream_t s) {
@@ -83,7 +88,7 @@ template <typename T>
 void DeviceArray<T>::release() {
   if (ptr != nullptr) cudaFree(ptr);
   ptr = nullptr;
-  count = 0;
+  count = capacity = 0;
 }
 template struct DeviceArray<int>;
 template struct DeviceArray<int2>;
@@ -475,7 +480,7 @@ void Engine::require_loaded() const {
 
 // Model::validate's structural and numeric checks (src/core/model.cpp:175-183 and the bound
 // checks) on an LP handed across the boundary.
-void validate_lp(const sankhya_gb300_lp& lp) {
+void validate_lp(const sankhya_gb300_lp& lp, bool matrix_known) {
   if (lp.rows < 0 || lp.cols < 0 || lp.col_starts == nullptr) {
     throw EngineError{SANKHYA_GB300_ERROR_ARGUMENT, "bad LP dimensions or null column starts"};
   }
@@ -484,12 +489,12 @@ void validate_lp(const sankhya_gb300_lp& lp) {
   if (lp.col_starts[0] != 0 || nnz < 0) {
     throw EngineError{SANKHYA_GB300_ERROR_MODEL, "column starts must begin at 0"};
   }
-  for (int j = 0; j < n; ++j) {
+  for (int j = 0; j < n && !matrix_known; ++j) {
     if (lp.col_starts[j + 1] < lp.col_starts[j]) {
       throw EngineError{SANKHYA_GB300_ERROR_MODEL, "column starts are not monotone"};
     }
   }
-  for (long long k = 0; k < nnz; ++k) {
+  for (long long k = 0; k < nnz && !matrix_known; ++k) {
     const int i = lp.row_index[k];
     if (i < 0 || i >= m) {
       throw EngineError{SANKHYA_GB300_ERROR_MODEL, format("row index %d out of range", i)};
@@ -505,7 +510,7 @@ void validate_lp(const sankhya_gb300_lp& lp) {
         std::isnan(lp.col_upper[j]) || lp.col_lower[j] > lp.col_upper[j]) {
       throw EngineError{SANKHYA_GB300_ERROR_MODEL, format("column %d has a bad cost or bound", j)};
     }
-    for (int k = lp.col_starts[j] + 1; k < lp.col_starts[j + 1]; ++k) {
+    for (int k = lp.col_starts[j] + 1; k < lp.col_starts[j + 1] && !matrix_known; ++k) {
       if (lp.row_index[k] <= lp.row_index[k - 1]) {
         throw EngineError{SANKHYA_GB300_ERROR_MODEL,
                           format("column %d: row indices are not strictly ascending", j)};
@@ -532,6 +537,9 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   const int m = lp.rows, n = lp.cols;
   const long long nnz = lp.col_starts[n];
   SGB_CUDA(cudaSetDevice(device_));
+  // The arrays are reused (DeviceArray): no work on the last LP may be left, on the caller's
+  // streams included (spmv_noalloc).
+  SGB_CUDA(cudaDeviceSynchronize());
   destroy_graphs();
   loaded_ = solved_ = scaled_ = mixed_ready_ = false;
   m_ = m;
@@ -719,7 +727,6 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
   D.idx.allocate(e);
   D.raw.allocate(e);
   D.scaled.allocate(e);
-  SGB_CUDA(cudaStreamSynchronize(s));  // the plan's arrays end here
   D.staged = P.staged;
   D.most_rows = D.most_slices = 0;
   for (int b = 0; b < P.grid; ++b) {

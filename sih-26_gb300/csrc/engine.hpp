@@ -33,10 +33,17 @@ struct EngineError {
 void cuda_check(cudaError_t err, const char* what, const char* file, int line);
 #define SGB_CUDA(call) ::sgb::cuda_check((call), #call, __FILE__, __LINE__)
 
+// A device allocation. allocate() keeps the one it has where that is large enough and not more than
+// kKeepFactor times too large (or kKeepBytes), so an engine that is loaded again with a problem of
+// like size allocates nothing; a much smaller problem gives the memory back. The contents are
+// undefined after it either way. The caller sees to it that no work on the old contents is left.
+constexpr size_t kKeepFactor = 4, kKeepBytes = 1u << 20;
+
 template <typename T>
 struct DeviceArray {
   T* ptr = nullptr;
   size_t count = 0;
+  size_t capacity = 0;
   DeviceArray() = default;
   DeviceArray(const DeviceArray&) = delete;
   DeviceArray& operator=(const DeviceArray&) = delete;
@@ -252,8 +259,9 @@ ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, in
                       int wmax, int grid, int elem_bytes, double split_min, double full_min,
                       int outer_round_cap);
 
-// Throws EngineError (ARGUMENT / MODEL) when an LP is malformed.
-void validate_lp(const sankhya_gb300_lp& lp);
+// Throws EngineError (ARGUMENT / MODEL) when an LP is malformed. `matrix_known`: the same arrays
+// have passed already (a batch's LPs may share them), so their entries are not walked again.
+void validate_lp(const sankhya_gb300_lp& lp, bool matrix_known = false);
 
 // Row tiles of a CSR / CSC pattern (see tiles.cuh).
 void build_tiles(const std::vector<int>& ptr, int lines, int lanes, int threads,

@@ -141,6 +141,7 @@ void QpEngine::load(const sankhya_gb300_qp_problem& p) {
   }
 
   SGB_CUDA(cudaSetDevice(device_));
+  SGB_CUDA(cudaStreamSynchronize(stream_));  // the arrays are reused (DeviceArray)
   destroy_graph();
   loaded_ = solved_ = false;
   col_lanes_ = row_lanes_ = 0;
@@ -201,7 +202,6 @@ void QpEngine::plan_sliced(SliceDev& D, const int* starts1, const int* starts2, 
   D.val1.allocate(e1);
   D.idx2.allocate(e2);
   D.val2.allocate(e2);
-  SGB_CUDA(cudaStreamSynchronize(s));  // the plan's arrays end here
   QpSliceSet& S = D.view;
   S = QpSliceSet{};
   S.meta = D.meta.ptr;

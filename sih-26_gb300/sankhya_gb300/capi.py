@@ -48,6 +48,13 @@ class CLp(ctypes.Structure):
                 ("sense", ctypes.c_double), ("objective_offset", ctypes.c_double)]
 
 
+# The same layout as a numpy record, pointers as addresses.
+_LP_RECORD = np.dtype([("rows", np.int32), ("cols", np.int32)] +
+                      [(name, np.uintp) for name, _ in CLp._fields_[2:10]] +
+                      [("sense", np.float64), ("objective_offset", np.float64)])
+assert _LP_RECORD.itemsize == ctypes.sizeof(CLp)
+
+
 class CParams(ctypes.Structure):
     _fields_ = [("tolerance", ctypes.c_double), ("iteration_limit", ctypes.c_int64),
                 ("time_limit", ctypes.c_double), ("restart", ctypes.c_int32),
@@ -509,13 +516,15 @@ class BatchEngine:
 
     def load(self, lps):
         lps = [lp.contiguous() for lp in lps]
-        arr = (CLp * len(lps))()
-        for k, lp in enumerate(lps):
-            arr[k] = CLp(lp.rows, lp.cols, _ptr(lp.col_starts, ctypes.c_int32),
-                         _ptr(lp.row_index, ctypes.c_int32), _ptr(lp.values), _ptr(lp.col_cost),
-                         _ptr(lp.col_lower), _ptr(lp.col_upper), _ptr(lp.row_lower),
-                         _ptr(lp.row_upper), lp.sense, lp.objective_offset)
-        _check(self._lib.sankhya_gb300_batch_load(self._h, len(lps), arr))
+        # The structs as one numpy record array: ten ctypes pointers per LP cost more than the
+        # load itself (304 nodes: 4.5 ms).
+        arr = np.array([(lp.rows, lp.cols, lp.col_starts.ctypes.data, lp.row_index.ctypes.data,
+                         lp.values.ctypes.data, lp.col_cost.ctypes.data, lp.col_lower.ctypes.data,
+                         lp.col_upper.ctypes.data, lp.row_lower.ctypes.data,
+                         lp.row_upper.ctypes.data, lp.sense, lp.objective_offset)
+                        for lp in lps], dtype=_LP_RECORD)
+        _check(self._lib.sankhya_gb300_batch_load(
+            self._h, len(lps), ctypes.cast(arr.ctypes.data, ctypes.POINTER(CLp))))
         self._lps = lps
 
     def solve(self, tolerance: float = 1e-4, iteration_limit: int = -1, restart: bool = True,
