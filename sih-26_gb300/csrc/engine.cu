@@ -906,11 +906,7 @@ void Engine::fill_buffers() {
   e.n = n_;
 }
 
-void Engine::precondition(long long seed) {
-  (void)seed;
-  cudaStream_t s = stream_;
-  launch_fill(dr_.ptr, m_, 1.0, s);
-  launch_fill(dc_.ptr, n_, 1.0, s);
+ScalingBuffers Engine::scaling_buffers() const {
   ScalingBuffers b{};
   b.csr = sl_csr_.view;
   b.csc = sl_csc_.view;
@@ -927,11 +923,46 @@ void Engine::precondition(long long seed) {
   b.minmax = minmax_.ptr;
   b.minmax_out = minmax_.ptr + 2 * scale_blocks(b.csc);
   b.nnz = nnz_;
-  launch_scaling(b, s);
+  return b;
+}
+
+void Engine::precondition(long long seed) {
+  (void)seed;
+  cudaStream_t s = stream_;
+  launch_fill(dr_.ptr, m_, 1.0, s);
+  launch_fill(dc_.ptr, n_, 1.0, s);
+  launch_scaling(scaling_buffers(), s);
   launch_scale_vectors(m_, n_, cost_.ptr, l_.ptr, u_.ptr, rl_.ptr, ru_.ptr, dr_.ptr, dc_.ptr,
                        cs_.ptr, ls_.ptr, us_.ptr, rls_.ptr, rus_.ptr, s);
   SGB_CUDA(cudaGetLastError());
   scaled_ = true;
+}
+
+double Engine::scale_and_norm(long long seed) {
+  if (!resident_ || nnz_ == 0) {
+    precondition(seed);
+    return power_iteration(seed);
+  }
+  draw_power_start(seed);
+  ResidentSetup r{};
+  r.scaling = scaling_buffers();
+  r.cost = cost_.ptr;
+  r.l = l_.ptr;
+  r.u = u_.ptr;
+  r.rl = rl_.ptr;
+  r.ru = ru_.ptr;
+  r.cs = cs_.ptr;
+  r.ls = ls_.ptr;
+  r.us = us_.ptr;
+  r.rls = rls_.ptr;
+  r.rus = rus_.ptr;
+  r.start = power_v_.ptr;
+  r.norms = power_norms_.ptr;
+  r.steps = kPowerSteps;
+  launch_resident_setup(r, resident_threads(step_), resident_smem_, stream_);
+  SGB_CUDA(cudaGetLastError());
+  scaled_ = true;
+  return norm_from_steps();
 }
 
 // The scaled values in the compressed layouts' order, for scaling() and the FP32 copies.
@@ -955,17 +986,36 @@ void Engine::fill_split_values() {
   }
 }
 
-// src/la/scaling.cpp:161-194 on the device. The start vector is the reference's own
-// std::mt19937(seed) + uniform_real_distribution(-1, 1) stream, drawn on the host.
-double Engine::power_iteration(long long seed) {
-  if (m_ == 0 || n_ == 0 || nnz_ == 0) return 1.0;
-  cudaStream_t s = stream_;
+// The power iteration's start vector: the reference's own std::mt19937(seed) +
+// uniform_real_distribution(-1, 1) stream, drawn on the host.
+void Engine::draw_power_start(long long seed) {
   std::mt19937 rng(static_cast<unsigned>(seed) + 1u);
   std::uniform_real_distribution<double> spread(-1.0, 1.0);
   std::vector<double> v(static_cast<size_t>(n_));
   for (double& value : v) value = spread(rng);
   SGB_CUDA(cudaMemcpyAsync(power_v_.ptr, v.data(), v.size() * sizeof(double),
-                           cudaMemcpyHostToDevice, s));
+                           cudaMemcpyHostToDevice, stream_));
+}
+
+// The estimate from the steps' |v_k|^2 (power_norms_[2 k]).
+double Engine::norm_from_steps() {
+  std::vector<double> host(2 * (kPowerSteps + 1));
+  SGB_CUDA(cudaMemcpyAsync(host.data(), power_norms_.ptr, host.size() * sizeof(double),
+                           cudaMemcpyDeviceToHost, stream_));
+  SGB_CUDA(cudaStreamSynchronize(stream_));
+  double norm = 0.0;
+  for (int step = 0; step < kPowerSteps; ++step) {
+    if (std::sqrt(host[2 * step]) == 0.0) return 1.0;
+    norm = std::sqrt(std::sqrt(host[2 * step + 2]));
+  }
+  return norm > 0.0 ? norm * 1.01 : 1.0;
+}
+
+// src/la/scaling.cpp:161-194 on the device.
+double Engine::power_iteration(long long seed) {
+  if (m_ == 0 || n_ == 0 || nnz_ == 0) return 1.0;
+  cudaStream_t s = stream_;
+  draw_power_start(seed);
   const int grid = std::min(num_sms_ * 4, std::max(1, (n_ + 255) / 256));
   // norms[2 k] = |v_k|^2 and norms[2 k + 1] = 1 / |v_k|, where v_{k+1} = A' (A v_k / |v_k|): the
   // start is normalised where its product is formed, one multiplication per row.
@@ -978,24 +1028,14 @@ double Engine::power_iteration(long long seed) {
                      scalars_.ptr, norms + 2 * step + 2, s);
   }
   SGB_CUDA(cudaGetLastError());
-  std::vector<double> host(2 * (kPowerSteps + 1));
-  SGB_CUDA(cudaMemcpyAsync(host.data(), norms, host.size() * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
-  SGB_CUDA(cudaStreamSynchronize(s));
-  double norm = 0.0;
-  for (int step = 0; step < kPowerSteps; ++step) {
-    if (std::sqrt(host[2 * step]) == 0.0) return 1.0;
-    norm = std::sqrt(std::sqrt(host[2 * step + 2]));
-  }
-  return norm > 0.0 ? norm * 1.01 : 1.0;
+  return norm_from_steps();
 }
 
 void Engine::scaling(long long seed, double* row_scale, double* col_scale, double* scaled_values,
                      double* spectral_norm) {
   require_loaded();
   SGB_CUDA(cudaSetDevice(device_));
-  precondition(seed);
-  const double norm = power_iteration(seed);
+  const double norm = scale_and_norm(seed);
   cudaStream_t s = stream_;
   if (scaled_values) unslice_scaled();
   if (row_scale) SGB_CUDA(cudaMemcpyAsync(row_scale, dr_.ptr, m_ * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1174,8 +1214,7 @@ void Engine::final_evaluation() {
 void Engine::setup(const sankhya_gb300_params& p, sankhya_gb300_result* r, double* norm) {
   Trace trace("pdhg scaling");
   cudaStream_t s = stream_;
-  precondition(p.random_seed);
-  *norm = power_iteration(p.random_seed);
+  *norm = scale_and_norm(p.random_seed);
   double mm[2] = {0.0, 0.0};
   SGB_CUDA(cudaMemcpyAsync(mm, minmax_.ptr + 2 * scale_blocks(sl_csc_.view), 2 * sizeof(double),
                            cudaMemcpyDeviceToHost, s));

@@ -81,6 +81,11 @@ class Engine {
   void require_loaded() const;
   void precondition(long long seed);
   double power_iteration(long long seed);
+  ScalingBuffers scaling_buffers() const;
+  // The preconditioning and the spectral-norm estimate, over launches or resident.
+  double scale_and_norm(long long seed);
+  void draw_power_start(long long seed);
+  double norm_from_steps();
   void init_iterates(const sankhya_gb300_params& p);
   void build_graphs(int steps);
   void build_mixed_graphs(int steps);

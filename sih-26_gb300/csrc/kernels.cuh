@@ -183,6 +183,20 @@ struct ScalingBuffers {
   long long nnz;
 };
 int scale_blocks(const SliceSet& S);
+// The setup of a resident LP in one kernel: the preconditioner, the scaled vectors (cs, ls, us, rls,
+// rus as launch_scale_vectors forms them) and the power iteration of `steps` steps from `start`
+// (n entries). norms[2 k] = |v_k|^2 for k = 0 .. steps, as the power iteration over launches leaves
+// them. `smem` and the cluster are the resident step's.
+struct ResidentSetup {
+  ScalingBuffers scaling;
+  const double *cost, *l, *u, *rl, *ru;
+  double *cs, *ls, *us, *rls, *rus;
+  const double* start;
+  double* norms;
+  int steps;
+};
+void launch_resident_setup(const ResidentSetup& r, int threads, int smem, cudaStream_t s);
+int resident_threads(const StepBuffers& b);
 void launch_scaling(const ScalingBuffers& b, cudaStream_t s);
 // The sliced copy of a compressed layout's indices and values, and the values back.
 void launch_slice_fill(const SliceSet& S, const int* ptr, const int* idx, const double* val,

@@ -732,6 +732,22 @@ __device__ __forceinline__ double pass_factor(double acc) {
 
 constexpr int kScaleThreads = 256;
 
+// The scaled data of one column or row (src/la/scaling.cpp:124-145). An absent bound is stored as
+// an IEEE infinity (the reference keeps +-1e30 as is and tests it with is_finite_bound each time),
+// so the step kernels project with min/max.
+__device__ __forceinline__ void scale_column(double d, double cost, double l, double u, double* cs,
+                                             double* ls, double* us) {
+  *cs = cost * d;
+  const double inv = 1.0 / d;
+  *ls = finite_bound(l) ? l * inv : -HUGE_VAL;
+  *us = finite_bound(u) ? u * inv : HUGE_VAL;
+}
+__device__ __forceinline__ void scale_row(double d, double rl, double ru, double* rls,
+                                          double* rus) {
+  *rls = finite_bound(rl) ? rl * d : -HUGE_VAL;
+  *rus = finite_bound(ru) ? ru * d : HUGE_VAL;
+}
+
 // Maximum and minimum of non-negative doubles by their bits (which order as the values do): the
 // integer pipe's, where FP64 compares would take as long as the rounds' multiplications.
 __device__ __forceinline__ double max_magnitude(double a, double b) {
@@ -905,20 +921,202 @@ __global__ void k_scale_vectors(int m, int n, const double* cost, const double* 
                                 double* us, double* rls, double* rus) {
   const int total = m > n ? m : n;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
-    // An absent bound is stored as an IEEE infinity (the reference keeps +-1e30 as is and
-    // tests it with is_finite_bound each time), so the step kernels project with min/max.
-    if (k < n) {
-      const double d = dc[k];
-      cs[k] = cost[k] * d;
-      const double inv = 1.0 / d;
-      ls[k] = finite_bound(l[k]) ? l[k] * inv : -HUGE_VAL;
-      us[k] = finite_bound(u[k]) ? u[k] * inv : HUGE_VAL;
+    if (k < n) scale_column(dc[k], cost[k], l[k], u[k], cs + k, ls + k, us + k);
+    if (k < m) scale_row(dr[k], rl[k], ru[k], rls + k, rus + k);
+  }
+}
+
+// The whole setup of a resident LP, in its cluster (slices.cuh): every block scales its slices of
+// both layouts in shared memory, the lines' factors and then the power iteration's vectors copied
+// to every block as they are formed: latency alone, two cluster barriers a step. A call on 50 x 100
+// (80 iterations) takes 1.29 ms so, 1.70 ms with the eighty-odd launches of the other path.
+template <bool SUM>
+__device__ __forceinline__ void local_factors(const LocalSlices& L, double* factors, int C) {
+  const int W = static_cast<int>(blockDim.x) >> 5, warp = static_cast<int>(threadIdx.x) >> 5;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  for (int s = warp; s < L.n; s += W) {
+    const unsigned meta = L.meta[s * 32 + lane];
+    if (meta == kNoRow) continue;
+    const int len = static_cast<int>(meta >> 8), e = L.base[s] * 32 + lane;
+    double acc = 0.0;
+    for (int q = 0; q < len; ++q) {
+      const double mag = fabs(L.val[e + q * 32]);
+      acc = SUM ? acc + mag : max_magnitude(acc, mag);
     }
-    if (k < m) {
-      const double d = dr[k];
-      rls[k] = finite_bound(rl[k]) ? rl[k] * d : -HUGE_VAL;
-      rus[k] = finite_bound(ru[k]) ? ru[k] * d : HUGE_VAL;
+    const double f = pass_factor(acc);
+    double* const at = factors + slice_row(L.s0 + s, meta);
+    for (int r = 0; r < C; ++r) cluster_store(cluster_addr(at, r), f);
+  }
+}
+
+// Applies a round's factors to the block's slices and to its lines' accumulated scale.
+__device__ __forceinline__ void local_apply(const LocalSlices& L, const double* line,
+                                            const double* other, double* scale, int line_is_row) {
+  const int W = static_cast<int>(blockDim.x) >> 5, warp = static_cast<int>(threadIdx.x) >> 5;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  for (int s = warp; s < L.n; s += W) {
+    const unsigned meta = L.meta[s * 32 + lane];
+    if (meta == kNoRow) continue;
+    const int len = static_cast<int>(meta >> 8), e = L.base[s] * 32 + lane;
+    const double lp = line[slice_row(L.s0 + s, meta)];
+    for (int q = 0; q < len; ++q) {
+      L.val[e + q * 32] = scaled_value(L.val[e + q * 32], lp, other[L.idx[e + q * 32]], line_is_row);
     }
+    scale[s * 32 + lane] *= lp;
+  }
+}
+
+// The block's lines' sums of the matrix times v, times `by`, to every block's `out`; returns this
+// thread's sum of their squares.
+__device__ __forceinline__ double local_product(const LocalSlices& L, const double* v, double by,
+                                                double* out, int C) {
+  const int W = static_cast<int>(blockDim.x) >> 5, warp = static_cast<int>(threadIdx.x) >> 5;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  double sq = 0.0;
+  for (int s = warp; s < L.n; s += W) {
+    const unsigned meta = L.meta[s * 32 + lane];
+    if (meta == kNoRow) continue;
+    const int len = static_cast<int>(meta >> 8), e = L.base[s] * 32 + lane;
+    double acc = 0.0;
+#pragma unroll 4
+    for (int q = 0; q < len; ++q) acc = fma(L.val[e + q * 32], v[L.idx[e + q * 32]], acc);
+    acc *= by;
+    double* const at = out + slice_row(L.s0 + s, meta);
+    for (int r = 0; r < C; ++r) cluster_store(cluster_addr(at, r), acc);
+    sq = fma(acc, acc, sq);
+  }
+  return sq;
+}
+
+__global__ void __launch_bounds__(kResidentThreads, 1) k_resident_setup(ResidentSetup r) {
+  extern __shared__ __align__(128) unsigned char dsmem[];
+  __shared__ double s_part[2][2][kResidentTable];
+  __shared__ double s_norm2, s_inv;
+  const ScalingBuffers& b = r.scaling;
+  const int T = static_cast<int>(blockDim.x), t = static_cast<int>(threadIdx.x);
+  const int C = static_cast<int>(gridDim.x), W = T >> 5, lane = t & 31, warp = t >> 5;
+  const int m = b.csr.nrows, n = b.csc.nrows;
+  double* const fc[2] = {reinterpret_cast<double*>(dsmem), reinterpret_cast<double*>(dsmem) + n};
+  double* const fr[2] = {fc[1] + n, fc[1] + n + m};
+  SliceSet csc = b.csc, csr = b.csr;
+  csc.val = b.csc_raw;
+  csr.val = b.csr_raw;
+  LocalSlices cs, rs;
+  unsigned char* mem = fill_local(csc, cs, dsmem + static_cast<size_t>(m + n) * 16);
+  mem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(mem) + 15) & ~uintptr_t(15));
+  mem = fill_local(csr, rs, mem);
+  double* const dc = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(mem) + 15) & ~uintptr_t(15));
+  double* const dr = dc + cs.n * 32;
+  for (int k = t; k < cs.n * 32; k += T) dc[k] = 1.0;
+  for (int k = t; k < rs.n * 32; k += T) dr[k] = 1.0;
+  cluster_meet();
+  local_factors<false>(cs, fc[0], C);
+  local_factors<false>(rs, fr[0], C);
+  cluster_meet();
+  for (int round = 0; round < 11; ++round) {
+    const int now = round & 1, then = now ^ 1;
+    local_apply(cs, fc[now], fr[now], dc, 0);
+    local_apply(rs, fr[now], fc[now], dr, 1);
+    // A lane takes the next factor of the lines it has just scaled.
+    if (round < 9) {
+      local_factors<false>(cs, fc[then], C);
+      local_factors<false>(rs, fr[then], C);
+    } else if (round == 9) {
+      local_factors<true>(cs, fc[then], C);
+      local_factors<true>(rs, fr[then], C);
+    }
+    cluster_meet();
+  }
+  // The scaled matrix, the scales and the scaled vectors go out; the magnitudes' range.
+  double most = 0.0, least = HUGE_VAL;
+  for (int side = 0; side < 2; ++side) {
+    const LocalSlices& L = side ? rs : cs;
+    const SliceSet& S = side ? csr : csc;
+    double* const out = side ? b.csr_val : b.csc_val;
+    const size_t at = static_cast<size_t>(S.base[L.s0]) * 32;
+    for (int s = warp; s < L.n; s += W) {
+      const unsigned meta = L.meta[s * 32 + lane];
+      if (meta == kNoRow) continue;
+      const int len = static_cast<int>(meta >> 8), e = L.base[s] * 32 + lane;
+      for (int q = 0; q < len; ++q) {
+        const double v = L.val[e + q * 32];
+        out[at + static_cast<size_t>(e + q * 32)] = v;
+        if (side == 0) {
+          most = max_magnitude(most, fabs(v));
+          least = min_magnitude(least, fabs(v));
+        }
+      }
+      const int item = slice_row(L.s0 + s, meta);
+      if (side == 0) {
+        const double d = dc[s * 32 + lane];
+        b.dc[item] = d;
+        scale_column(d, r.cost[item], r.l[item], r.u[item], r.cs + item, r.ls + item, r.us + item);
+      } else {
+        const double d = dr[s * 32 + lane];
+        b.dr[item] = d;
+        scale_row(d, r.rl[item], r.ru[item], r.rls + item, r.rus + item);
+      }
+    }
+  }
+  __syncwarp();
+  most = warp_max(most);
+  least = -warp_max(-least);
+  if (lane == 0) {
+    const int at = static_cast<int>(blockIdx.x) * W + warp;
+    cluster_store(cluster_addr(&s_part[0][0][at], 0), most);
+    cluster_store(cluster_addr(&s_part[0][1][at], 0), -least);
+  }
+  // The power iteration (src/la/scaling.cpp:161-194): v in fc[0], A v in fr[0], every block's copy
+  // of the start its own.
+  double* const v = fc[0];
+  double* const av = fr[0];
+  double sq = 0.0;
+  for (int j = t; j < n; j += T) {
+    v[j] = r.start[j];
+    sq = fma(v[j], v[j], sq);
+  }
+  sq = warp_sum(sq);
+  if (lane == 0) s_part[1][0][warp] = sq;
+  cluster_meet();
+  if (blockIdx.x == 0 && t < 32) {
+    double a = 0.0, c = -HUGE_VAL;
+    for (int k = lane; k < C * W; k += 32) {
+      a = dmax(a, s_part[0][0][k]);
+      c = dmax(c, s_part[0][1][k]);
+    }
+    a = warp_max(a);
+    c = warp_max(c);
+    if (lane == 0) {
+      b.minmax_out[0] = a;
+      b.minmax_out[1] = b.nnz > 0 ? -c : 0.0;
+    }
+  }
+  int entries = W;  // of the table that holds the current |v|^2
+  for (int step = 0;; ++step) {
+    const double* const table = s_part[(step + 1) & 1][0];
+    if (t < 32) {
+      double sum = 0.0;
+      for (int k = lane; k < entries; k += 32) sum += table[k];
+      sum = warp_sum(sum);
+      if (lane == 0) {
+        s_norm2 = sum;
+        s_inv = 1.0 / sqrt(sum);
+      }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && t == 0) r.norms[2 * step] = s_norm2;
+    if (step == r.steps) break;
+    local_product(rs, v, s_inv, av, C);
+    cluster_meet();
+    double out = local_product(cs, av, 1.0, v, C);
+    __syncwarp();
+    out = warp_sum(out);
+    if (lane < C) {
+      cluster_store(cluster_addr(&s_part[step & 1][0][static_cast<int>(blockIdx.x) * W + warp], lane),
+                    out);
+    }
+    entries = C * W;
+    cluster_meet();
   }
 }
 
@@ -1044,7 +1242,10 @@ bool configure_fp64_kernels() {
                            max_dynamic_smem(reinterpret_cast<const void*>(k_dual))),
       cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_pdhg_resident))),
-      cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)};
+      cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+      cudaFuncSetAttribute(k_resident_setup, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           max_dynamic_smem(reinterpret_cast<const void*>(k_resident_setup))),
+      cudaFuncSetAttribute(k_resident_setup, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)};
   for (cudaError_t e : errs) {
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -1076,11 +1277,14 @@ void launch_dual_pass(const StepBuffers& b, cudaStream_t s) {
   ++g_launches;
 }
 
-namespace {
 int resident_threads(const StepBuffers& b) {
   return std::min(kResidentThreads, std::max(b.csc.threads, b.csr.threads));
 }
-}  // namespace
+
+void launch_resident_setup(const ResidentSetup& r, int threads, int smem, cudaStream_t s) {
+  ++g_launches;
+  launch_cluster(k_resident_setup, r.scaling.csc.grid, threads, smem, s, r);
+}
 
 int resident_smem(int m, int n, int col_rows, int col_slices, int row_rows, int row_slices) {
   return 16 * n + 16 * m + local_slices_bytes(col_rows, col_slices) +
@@ -1090,7 +1294,9 @@ int resident_smem(int m, int n, int col_rows, int col_slices, int row_rows, int 
 bool resident_fits(const StepBuffers& b, int smem) {
   return b.csc.grid == b.csr.grid &&
          smem <= max_dynamic_smem(reinterpret_cast<const void*>(k_pdhg_resident)) &&
-         cluster_fits(k_pdhg_resident, b.csc.grid, resident_threads(b), smem);
+         smem <= max_dynamic_smem(reinterpret_cast<const void*>(k_resident_setup)) &&
+         cluster_fits(k_pdhg_resident, b.csc.grid, resident_threads(b), smem) &&
+         cluster_fits(k_resident_setup, b.csc.grid, resident_threads(b), smem);
 }
 
 void launch_pdhg_resident(const StepBuffers& b, int attempts, int smem, cudaStream_t s) {

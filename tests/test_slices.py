@@ -120,6 +120,25 @@ def test_resident_steps_match_the_oracle(oracle, m, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(1, 1), (33, 31), (64, 256), (700, 700), (1500, 1400)])
+def test_resident_setup_gives_the_bits_of_the_launches(monkeypatch, m, n):
+    """Scaled in one cluster kernel or over launches (a window capacity turns the cluster off):
+    maxima, ascending sums and products are the same operations, so the scaled LP has the same bits;
+    the norm differs by the order of sums of 1,500 non-negative terms (1,500 * 2^-52 at most)."""
+    lp = lp_with_rows(np.random.default_rng(n).integers(1, min(n, 20) + 1, size=m), n, seed=n)
+    with capi.PdhgEngine(0) as eng:
+        eng.load(lp)
+        got = eng.scaling(3)
+    monkeypatch.setenv("SANKHYA_GB300_WINDOW_CAP", "0")
+    with capi.PdhgEngine(0) as eng:
+        eng.load(lp)
+        want = eng.scaling(3)
+    for g, w in zip(got[:-1], want[:-1]):
+        np.testing.assert_array_equal(g, w)
+    assert abs(got[-1] - want[-1]) <= 4e-13 * want[-1]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("m,n,per_column,band", [(0, 33, 0, 2), (1, 1, 1, 0), (31, 33, 3, 1),
                                                  (128, 129, 5, 0), (40, 300, 20, 30)])
 def test_qp_slices_match_the_oracle(oracle, m, n, per_column, band):
