@@ -131,6 +131,83 @@ inline bool cluster_fits(Kernel kernel, int blocks, int threads, int smem) {
   return n > 0;
 }
 
+// ---- A grid whose blocks meet --------------------------------------------------------------
+// A cooperative launch: all blocks run at once, so they may wait for one another. `counter` counts
+// arrivals over launches of the same grid (a multiple of gridDim.x between launches, 64 bits, so it
+// never wraps) and is zeroed with the control block it lives in.
+struct GridMeet {
+  unsigned long long* counter;
+  unsigned long long target;
+  // Before this block's first arrival the counter lacks at least that one of the launch's first
+  // meeting, so rounding it down gives the launch's start. All threads call it (only thread 0's
+  // value is used).
+  __device__ __forceinline__ void start(unsigned long long* c) {
+    counter = c;
+    target = 0;
+    if (threadIdx.x == 0) target = *reinterpret_cast<volatile unsigned long long*>(c) / gridDim.x * gridDim.x;
+  }
+  // All threads of all blocks meet: what each wrote before is visible to the others after (through
+  // ld_live, never through the read-only path). Returns false, in every thread of the block, if
+  // the others did not arrive within kMeetPolls polls (about a second) or `error` was raised.
+  __device__ __forceinline__ bool meet(int* error) {
+    constexpr int kMeetPolls = 1 << 21;
+    __shared__ int s_met;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      target += gridDim.x;
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(counter), "l"(1ull) : "memory");
+      unsigned long long now = 0;
+      int polls = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(counter) : "memory");
+      } while (now < target && ++polls < kMeetPolls);
+      s_met = now >= target;
+      if (now < target) *reinterpret_cast<volatile int*>(error) = 1;
+    }
+    __syncthreads();
+    return s_met != 0;
+  }
+};
+
+// A load of data that the running kernel writes.
+__device__ __forceinline__ double ld_live(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Launches kernel<<<blocks, threads, smem, s>>>(args...) cooperatively; returns the launch's error.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_grid(void (*kernel)(Params...), int blocks, int threads, int smem,
+                               cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+  cfg.blockDim = dim3(static_cast<unsigned>(threads));
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Whether `blocks` blocks of the kernel run at once on the current device.
+template <typename Kernel>
+inline bool grid_fits(Kernel kernel, int blocks, int threads, int smem) {
+  int dev = 0, sms = 0, able = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&able, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads,
+                                                    static_cast<size_t>(smem)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return able != 0 && blocks > 0 && blocks <= sms * per_sm;
+}
+
 __device__ __forceinline__ double clamp_box(double v, double lo, double hi) {
   return fmin(fmax(v, lo), hi);
 }

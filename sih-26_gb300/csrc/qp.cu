@@ -263,6 +263,10 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
   resident_ = cols_sliced && (rows_sliced || m_ == 0) && n_ > 0 &&
               std::max(m_, n_) <= kQpResidentItems && cc.empty() && rc.empty() &&
               qp_resident_fits(smem);
+  // Larger ones run a period's steps in one cooperative launch.
+  constexpr int kQpStepItems = 1024;
+  steps_ = !resident_ && std::max(m_, n_) > kQpStepItems && cols_sliced &&
+           (rows_sliced || m_ == 0) && qp_steps_fit(d);
   resident_smem_ = resident_ ? static_cast<int>(smem) : 0;
   if (cols_sliced) {
     qp_launch_slice_fill(d, true, col_slices_.idx1.ptr, col_slices_.val1.ptr,
@@ -398,7 +402,8 @@ void QpEngine::build_graph(int periods) {
     if (resident_) {
       qp_launch_resident(d, ctl, p * kQpCheckEvery, kQpCheckEvery, 0, resident_smem_, stream_);
     }
-    for (int it = 0; it < kQpCheckEvery && !resident_; ++it) {
+    if (steps_) qp_launch_steps(d, ctl, p * kQpCheckEvery, kQpCheckEvery, stream_);
+    for (int it = 0; it < kQpCheckEvery && !resident_ && !steps_; ++it) {
       const int k = p * kQpCheckEvery + it;
       qp_launch_column_pass(d, ctl, kQpStep, k, k & 1, stream_);
       if (m_ > 0) qp_launch_row_pass(d, ctl, kQpStep, k, 0, stream_);
@@ -527,6 +532,9 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
         if (now.done && h.iteration == now.iterations) continue;
         p.log(p.log_user, h.iteration, h.objective, h.primal, h.dual, qp_now() - t0);
       }
+    }
+    if (now.error != 0) {
+      throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "the blocks of a step kernel did not meet"};
     }
     base = now.base;
     if (now.done) {

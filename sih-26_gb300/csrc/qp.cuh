@@ -50,7 +50,7 @@ enum QpMode { kQpStep = 0, kQpCheck = 1, kQpReport = 2 };
 // Decision state, on the device.
 struct QpCtl {
   int done;   // the stopping test held
-  int error;  // unused by the kernels, cleared at load
+  int error;  // a grid's blocks did not meet (GridMeet)
   double tau, sigma, tolerance;  // the solve's step sizes and stopping tolerance
   double inv_sigma;              // RN(1 / sigma), for the row pass's division
   long long base;        // iterations completed before the running graph
@@ -59,6 +59,7 @@ struct QpCtl {
   unsigned long long primal_bits, dual_bits;  // running maxima of the running check
   double primal, dual, objective;  // the last check's residuals and objective
   long long checked;               // iteration of the last check (0: none)
+  unsigned long long arrivals;     // GridMeet's counter
 };
 
 struct QpHist {
@@ -136,6 +137,10 @@ void qp_launch_resident(const QpDev& d, QpCtl* ctl, int k0, int count, int src, 
                         cudaStream_t s);
 long long qp_resident_smem(int m, int n, long long rows_q, long long rows_a, long long rows_r);
 bool qp_resident_fits(long long smem);
+// Iterations k0 .. k0 + count - 1 of the graph (k0 even: x is in buffer 0) on sliced items in one
+// cooperative launch; qp_steps_fit: whether the device runs its blocks at once.
+void qp_launch_steps(const QpDev& d, QpCtl* ctl, int k0, int count, cudaStream_t s);
+bool qp_steps_fit(const QpDev& d);
 // The decision after the check whose last iteration is graph index k (period p).
 void qp_launch_decide(const QpDev& d, QpCtl* ctl, int k, int p, cudaStream_t s);
 // base += iterations of the graph (capped at the limit) unless done.

@@ -56,6 +56,7 @@ class QpEngine {
   // Layout for the current lanes.
   int col_lanes_ = 0, row_lanes_ = 0;
   bool cols_sliced_ = false, rows_sliced_ = false;
+  bool steps_ = false;     // a period's steps in one launch (qp_launch_steps)
   bool resident_ = false;  // the iterations run in the resident kernel,
   int resident_smem_ = 0;  // with this much shared memory
   struct SliceDev {

@@ -269,6 +269,12 @@ struct QpWalk {
 
 // ---- Column pass ------------------------------------------------------------------------
 
+// A gathered entry: of a vector that the running kernel does not write, or of one that it does.
+template <bool LIVE>
+__device__ __forceinline__ double gathered(const double* p) {
+  return LIVE ? ld_live(p) : __ldg(p);
+}
+
 // The epilogue's operands of column j.
 struct ColumnOps {
   double x, c, lower, upper;
@@ -308,6 +314,77 @@ __device__ __forceinline__ void column_epilogue(const QpDev& d, double tau, int 
   }
 }
 
+// Long columns: one warp per chunk of the column's entries (row j of Q, then column j of A); the
+// last chunk of a column to finish adds the chunks' sums in order and runs its epilogue. LIVE: the
+// vectors are the running kernel's own (ld_live).
+template <int MODE, bool LIVE>
+__device__ __forceinline__ void long_column(const QpDev& d, QpCtl* ctl, double tau, int w,
+                                            const double* x, double* xn) {
+  const int lane32 = threadIdx.x & 31;
+  const QpChunk ch = d.col_chunks[w];
+  const int j = ch.item;
+  const int qb = d.q_rs[j], lq = d.q_rs[j + 1] - qb, ab = d.a_cs[j];
+  double qx = 0.0, aty = 0.0;
+  for (int v = ch.begin + lane32; v < ch.end; v += 32) {
+    if (v < lq) {
+      qx = fma(d.q_v[qb + v], gathered<LIVE>(x + d.q_ci[qb + v]), qx);
+    } else {
+      const int e = ab + v - lq;
+      aty = fma(d.a_cv[e], gathered<LIVE>(d.y + d.a_ri[e]), aty);
+    }
+  }
+  qx = warp_sum(qx);
+  aty = warp_sum(aty);
+  int last = 1;
+  if (ch.count > 1) {
+    if (lane32 == 0) {
+      __stcg(&d.chunk_part[w], make_double2(qx, aty));
+      __threadfence();
+      last = atomicAdd(&d.col_tickets[ch.slot], 1u) == static_cast<unsigned>(ch.count - 1);
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (!last) return;
+    if (lane32 == 0) {
+      __threadfence();
+      qx = aty = 0.0;
+      for (int c = ch.first; c < ch.first + ch.count; ++c) {
+        const double2 p = __ldcg(&d.chunk_part[c]);
+        qx += p.x;
+        aty += p.y;
+      }
+      d.col_tickets[ch.slot] = 0u;
+    }
+  }
+  if (lane32 == 0) {
+    double residual = 0.0, obj = 0.0;
+    ColumnOps o;
+    o.load(d, x, j);
+    column_epilogue<MODE>(d, tau, j, o, xn, qx, aty, &residual, &obj);
+    if (MODE == kQpCheck) max_bits(&ctl->dual_bits, residual);
+    if (MODE != kQpStep) d.long_col_obj[ch.slot] = obj;
+  }
+}
+
+// The step form of the block's columns on sliced items.
+template <int MODE, bool LIVE>
+__device__ __forceinline__ void sliced_columns(const QpDev& d, QpWalk<0>& walk, double tau,
+                                               const double* x, double* xn, double* residual,
+                                               double* obj) {
+  for (; walk.s < walk.s1; walk.advance(d.cols)) {
+    const QpPlace p = walk.p;
+    ColumnOps o;
+    if (p.has) o.load(d, x, p.item);
+    double qx, aty, r = 0.0, t = 0.0;
+    walk.sums(d.cols, [&](int c) { return gathered<LIVE>(x + c); },
+              [&](int c) { return gathered<LIVE>(d.y + c); }, &qx, &aty);
+    if (p.has) column_epilogue<MODE>(d, tau, p.item, o, xn, qx, aty, &r, &t);
+    if (MODE != kQpStep) {
+      *residual = r > *residual ? r : *residual;
+      *obj += t;
+    }
+  }
+}
+
 // G = 0: the short columns on sliced items, in blocks of kQpSliceThreads.
 template <int G>
 constexpr int qp_threads() {
@@ -328,19 +405,7 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_column(QpDev d, QpCtl* c
   const int lane32 = threadIdx.x & 31;
   if (G == 0 && static_cast<int>(blockIdx.x) < d.col_short_blocks) {
     double residual = 0.0, obj = 0.0;
-    for (; walk.s < walk.s1; walk.advance(d.cols)) {
-      const QpPlace p = walk.p;
-      ColumnOps o;
-      if (p.has) o.load(d, x, p.item);
-      double qx, aty, r = 0.0, t = 0.0;
-      walk.sums(d.cols, [&](int c) { return __ldg(x + c); }, [&](int c) { return __ldg(d.y + c); },
-                &qx, &aty);
-      if (p.has) column_epilogue<MODE>(d, tau, p.item, o, xn, qx, aty, &r, &t);
-      if (MODE != kQpStep) {
-        residual = r > residual ? r : residual;
-        obj += t;
-      }
-    }
+    sliced_columns<MODE, false>(d, walk, tau, x, xn, &residual, &obj);
     if (MODE != kQpStep) {
       __shared__ double scratch[kQpSliceThreads / 32];
       if (MODE == kQpCheck) {
@@ -400,54 +465,9 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_column(QpDev d, QpCtl* c
     }
     return;
   }
-  // Long columns: one warp per chunk of the column's entries (row j of Q, then column j of
-  // A); the last chunk of a column to finish adds the chunks' sums in order and runs its
-  // epilogue.
   const int w = (static_cast<int>(blockIdx.x) - d.col_short_blocks) * (qp_threads<G>() / 32) +
                 static_cast<int>(threadIdx.x >> 5);
-  if (w >= d.ncol_chunks) return;
-  const QpChunk ch = d.col_chunks[w];
-  const int j = ch.item;
-  const int qb = d.q_rs[j], lq = d.q_rs[j + 1] - qb, ab = d.a_cs[j];
-  double qx = 0.0, aty = 0.0;
-  for (int v = ch.begin + lane32; v < ch.end; v += 32) {
-    if (v < lq) {
-      qx = fma(d.q_v[qb + v], x[d.q_ci[qb + v]], qx);
-    } else {
-      const int e = ab + v - lq;
-      aty = fma(d.a_cv[e], d.y[d.a_ri[e]], aty);
-    }
-  }
-  qx = warp_sum(qx);
-  aty = warp_sum(aty);
-  int last = 1;
-  if (ch.count > 1) {
-    if (lane32 == 0) {
-      __stcg(&d.chunk_part[w], make_double2(qx, aty));
-      __threadfence();
-      last = atomicAdd(&d.col_tickets[ch.slot], 1u) == static_cast<unsigned>(ch.count - 1);
-    }
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (!last) return;
-    if (lane32 == 0) {
-      __threadfence();
-      qx = aty = 0.0;
-      for (int c = ch.first; c < ch.first + ch.count; ++c) {
-        const double2 p = __ldcg(&d.chunk_part[c]);
-        qx += p.x;
-        aty += p.y;
-      }
-      d.col_tickets[ch.slot] = 0u;
-    }
-  }
-  if (lane32 == 0) {
-    double residual = 0.0, obj = 0.0;
-    ColumnOps o;
-    o.load(d, x, j);
-    column_epilogue<MODE>(d, tau, j, o, xn, qx, aty, &residual, &obj);
-    if (MODE == kQpCheck) max_bits(&ctl->dual_bits, residual);
-    if (MODE != kQpStep) d.long_col_obj[ch.slot] = obj;
-  }
+  if (w < d.ncol_chunks) long_column<MODE, false>(d, ctl, tau, w, x, xn);
 }
 
 // ---- Row pass ---------------------------------------------------------------------------
@@ -481,6 +501,62 @@ __device__ __forceinline__ double row_epilogue(const QpDev& d, double sigma, dou
   return fabs(__dsub_rn(ax, projected));
 }
 
+// Long rows, a warp per chunk, as the long columns.
+template <int MODE, bool LIVE>
+__device__ __forceinline__ void long_row(const QpDev& d, QpCtl* ctl, double sigma, double inv_sigma,
+                                         int w, const double* v) {
+  const int lane32 = threadIdx.x & 31;
+  const QpChunk ch = d.row_chunks[w];
+  const int i = ch.item, b = d.a_rs[i];
+  double ax = 0.0;
+  for (int q = ch.begin + lane32; q < ch.end; q += 32) {
+    ax = fma(d.a_rv[b + q], gathered<LIVE>(v + d.a_ci[b + q]), ax);
+  }
+  ax = warp_sum(ax);
+  int last = 1;
+  if (ch.count > 1) {
+    if (lane32 == 0) {
+      __stcg(&d.row_chunk_part[w], make_double2(ax, 0.0));
+      __threadfence();
+      last = atomicAdd(&d.row_tickets[ch.slot], 1u) == static_cast<unsigned>(ch.count - 1);
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (!last) return;
+    if (lane32 == 0) {
+      __threadfence();
+      ax = 0.0;
+      for (int c = ch.first; c < ch.first + ch.count; ++c) ax += __ldcg(&d.row_chunk_part[c]).x;
+      d.row_tickets[ch.slot] = 0u;
+    }
+  }
+  if (lane32 == 0) {
+    RowOps o;
+    o.load(d, i);
+    const double residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, o, ax);
+    if (MODE == kQpCheck) max_bits(&ctl->primal_bits, residual);
+  }
+}
+
+// The block's rows on sliced items; returns this thread's largest residual (check form).
+template <int MODE, bool LIVE>
+__device__ __forceinline__ double sliced_rows(const QpDev& d, QpWalk<2>& walk, double sigma,
+                                              double inv_sigma, const double* v) {
+  double residual = 0.0;
+  for (; walk.s < walk.s1; walk.advance(d.rows)) {
+    const QpPlace p = walk.p;
+    RowOps o;
+    if (p.has) o.load(d, p.item);
+    double none, ax;
+    walk.sums(d.rows, [](int) { return 0.0; }, [&](int c) { return gathered<LIVE>(v + c); }, &none,
+              &ax);
+    if (p.has) {
+      const double r = row_epilogue<MODE>(d, sigma, inv_sigma, p.item, o, ax);
+      residual = r > residual ? r : residual;
+    }
+  }
+  return residual;
+}
+
 template <int G, int MODE>
 __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl, int k, int src) {
   QpWalk<2> walk;
@@ -492,18 +568,7 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl,
   const double* v = MODE == kQpStep ? d.xbar : (src ? d.x1 : d.x0);
   const int lane32 = threadIdx.x & 31;
   if (G == 0 && static_cast<int>(blockIdx.x) < d.row_short_blocks) {
-    double residual = 0.0;
-    for (; walk.s < walk.s1; walk.advance(d.rows)) {
-      const QpPlace p = walk.p;
-      RowOps o;
-      if (p.has) o.load(d, p.item);
-      double none, ax;
-      walk.sums(d.rows, [](int) { return 0.0; }, [&](int c) { return __ldg(v + c); }, &none, &ax);
-      if (p.has) {
-        const double r = row_epilogue<MODE>(d, sigma, inv_sigma, p.item, o, ax);
-        residual = r > residual ? r : residual;
-      }
-    }
+    const double residual = sliced_rows<MODE, false>(d, walk, sigma, inv_sigma, v);
     if (MODE == kQpCheck) {
       const double w = warp_max(residual);
       if (lane32 == 0) max_bits(&ctl->primal_bits, w);
@@ -547,33 +612,47 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl,
   }
   const int w = (static_cast<int>(blockIdx.x) - d.row_short_blocks) * (qp_threads<G>() / 32) +
                 static_cast<int>(threadIdx.x >> 5);
-  if (w >= d.nrow_chunks) return;
-  const QpChunk ch = d.row_chunks[w];
-  const int i = ch.item, b = d.a_rs[i];
-  double ax = 0.0;
-  for (int q = ch.begin + lane32; q < ch.end; q += 32) ax = fma(d.a_rv[b + q], v[d.a_ci[b + q]], ax);
-  ax = warp_sum(ax);
-  int last = 1;
-  if (ch.count > 1) {
-    if (lane32 == 0) {
-      __stcg(&d.row_chunk_part[w], make_double2(ax, 0.0));
-      __threadfence();
-      last = atomicAdd(&d.row_tickets[ch.slot], 1u) == static_cast<unsigned>(ch.count - 1);
+  if (w < d.nrow_chunks) long_row<MODE, false>(d, ctl, sigma, inv_sigma, w, v);
+}
+
+// ---- The steps of a period in one launch ---------------------------------------------------------
+// Iterations k0 .. of the graph by one cooperative grid: blocks meet between the passes, and each
+// warp has its next pass's first entries under way while it waits. Between two launches lie the
+// drain of one, the start of the next and its first loads, some 7 us an item-free pass; a meeting
+// takes 1.3 us.
+__global__ void __launch_bounds__(kQpSliceThreads, 1) k_qp_steps(QpDev d, QpCtl* ctl, int k0,
+                                                                 int count) {
+  if (ctl->done != 0) return;
+  const long long left = ctl->limit - (ctl->base + k0);
+  const int iterations = left < count ? static_cast<int>(left) : count;
+  if (iterations <= 0) return;
+  const double tau = ctl->tau, sigma = ctl->sigma, inv_sigma = ctl->inv_sigma;
+  const int gw = static_cast<int>((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+  const int warps = static_cast<int>((blockDim.x >> 5) * gridDim.x);
+  GridMeet grid;
+  grid.start(&ctl->arrivals);
+  QpWalk<0> cols;
+  cols.start(d.cols);
+  for (int i = 0; i < iterations; ++i) {
+    const bool odd = (k0 + i) & 1;
+    const double* x = odd ? d.x1 : d.x0;
+    double* xn = odd ? d.x0 : d.x1;
+    for (int w = gw; w < d.ncol_chunks; w += warps) {
+      long_column<kQpStep, true>(d, ctl, tau, w, x, xn);
     }
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (!last) return;
-    if (lane32 == 0) {
-      __threadfence();
-      ax = 0.0;
-      for (int c = ch.first; c < ch.first + ch.count; ++c) ax += __ldcg(&d.row_chunk_part[c]).x;
-      d.row_tickets[ch.slot] = 0u;
+    sliced_columns<kQpStep, true>(d, cols, tau, x, xn, nullptr, nullptr);
+    if (d.m > 0) {
+      QpWalk<2> rows;
+      rows.start(d.rows);
+      if (!grid.meet(&ctl->error)) return;
+      for (int w = gw; w < d.nrow_chunks; w += warps) {
+        long_row<kQpStep, true>(d, ctl, sigma, inv_sigma, w, d.xbar);
+      }
+      sliced_rows<kQpStep, true>(d, rows, sigma, inv_sigma, d.xbar);
     }
-  }
-  if (lane32 == 0) {
-    RowOps o;
-    o.load(d, i);
-    const double residual = row_epilogue<MODE>(d, sigma, inv_sigma, i, o, ax);
-    if (MODE == kQpCheck) max_bits(&ctl->primal_bits, residual);
+    if (i + 1 == iterations) return;
+    cols.start(d.cols);
+    if (!grid.meet(&ctl->error)) return;
   }
 }
 
@@ -966,6 +1045,17 @@ void qp_launch_resident(const QpDev& d, QpCtl* ctl, int k0, int count, int src, 
                         cudaStream_t s) {
   const int warps = std::max(2, std::max(d.cols.nslices, d.rows.nslices));
   k_qp_resident<<<1, std::min(kResidentThreads, warps * 32), smem, s>>>(d, ctl, k0, count, src);
+  ++g_qp_launches;
+}
+
+bool qp_steps_fit(const QpDev& d) {
+  return d.cols.nslices > 0 && (d.m == 0 || d.rows.nslices > 0) &&
+         grid_fits(k_qp_steps, std::max(d.cols.blocks, d.rows.blocks), kQpSliceThreads, 0);
+}
+
+void qp_launch_steps(const QpDev& d, QpCtl* ctl, int k0, int count, cudaStream_t s) {
+  launch_grid(k_qp_steps, std::max(d.cols.blocks, d.rows.blocks), kQpSliceThreads, 0, s, d, ctl, k0,
+              count);
   ++g_qp_launches;
 }
 

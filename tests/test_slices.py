@@ -156,3 +156,24 @@ def test_qp_slices_match_the_oracle(oracle, m, n, per_column, band):
     assert (got.status_name, got.iterations) == (ref.status_name, ref.iterations)
     for a, b in ((x, ref.col_value), (d, ref.col_dual), (y, ref.row_dual)):
         assert np.all(np.abs(a - b) <= 1e-9 * max(1.0, np.abs(b).max() if len(b) else 0.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths,n,limit", [([], 1025, 60), ([1100, 600, 65, 64] + [3] * 700, 1100, 177),
+                                             ([7] * 6000, 9000, 101), ([2] * 1300, 40, 50)])
+def test_qp_steps_in_one_launch_match_the_oracle(oracle, lengths, n, limit):
+    """QPs past 1,024 items, whose check periods run in one cooperative launch: no rows, rows in
+    chunks, limits that end inside a period, more rows than columns; the oracle's iteration count,
+    and its point within 1e-9 of its scale, as every QP parity test."""
+    from sankhya_gb300.model import QP, banded_hessian
+
+    lp = lp_with_rows(lengths, n, seed=n)
+    qp = QP(lp, *banded_hessian(n, 2, seed=n))
+    ref = oracle.solve_qp(qp, tolerance=1e-12, iteration_limit=limit)
+    with capi.QpEngine(0) as eng:
+        eng.load(qp)
+        got = eng.solve(tolerance=1e-12, iteration_limit=limit)
+        x, d, y = eng.solution()
+    assert (got.status_name, got.iterations) == (ref.status_name, ref.iterations)
+    for a, b in ((x, ref.col_value), (d, ref.col_dual), (y, ref.row_dual)):
+        assert np.all(np.abs(a - b) <= 1e-9 * max(1.0, np.abs(b).max() if len(b) else 0.0))
