@@ -169,11 +169,11 @@ struct GridMeet {
   }
 };
 
-// A load of data that the running kernel writes.
-__device__ __forceinline__ double ld_live(const double* p) {
-  double v;
-  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
-  return v;
+// A load of data that the running kernel writes: an ordinary one, as the pointer is not __restrict__
+// (a volatile asm load would not be predicated but branched around).
+template <typename T>
+__device__ __forceinline__ T ld_live(const T* p) {
+  return *p;
 }
 
 // Launches kernel<<<blocks, threads, smem, s>>>(args...) cooperatively; returns the launch's error.
@@ -246,27 +246,64 @@ __device__ __forceinline__ T group_sum(T v) {
   return v;
 }
 
+// Sums of N values (a power of two) over a warp by halves: at each level a lane hands half of its
+// values to its partner and adds the partner's to the other half, so N values take N - 1 adds
+// and log2(32 / N) more, not 5 N. Afterwards lane l holds the total of value warp_sums_index<N>(l)
+// in v[0].
+template <int N, int O = 16>
+__device__ __forceinline__ void warp_sums(double* v) {
+  if constexpr (O > 0) {
+    constexpr int kHalf = N > 1 ? N / 2 : 1;
+    const bool high = (threadIdx.x & O) != 0;
+#pragma unroll
+    for (int k = 0; k < kHalf; ++k) {
+      if constexpr (N > 1) {
+        const double give = high ? v[k] : v[k + kHalf];
+        const double keep = high ? v[k + kHalf] : v[k];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+      } else {
+        v[k] += __shfl_xor_sync(0xffffffffu, v[k], O);
+      }
+    }
+    warp_sums<kHalf, O / 2>(v);
+  }
+}
+template <int N>
+__device__ __forceinline__ int warp_sums_index(int lane) {
+  int at = 0;
+#pragma unroll
+  for (int o = 16, half = N / 2; half > 0; o >>= 1, half >>= 1) at += (lane & o) ? half : 0;
+  return at;
+}
+
 // Block-wide sum of NV values per thread. `scratch` holds NV * (blockDim/32) doubles. Thread 0
-// receives the totals in out[]. All threads must call it.
+// receives the totals in out[]. All threads must call it. An FP64 addition holds the pipe of its
+// quarter of the SM for 64 cycles whatever its lanes add, so a warp whose values are all zero adds
+// nothing, the others add by halves, and each total is taken by a warp of its own: three sums over
+// 24 warps took 4.3 us as butterflies.
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* scratch, double (&out)[NV]) {
+  constexpr int kAll = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 4 : NV <= 8 ? 8 : 16;
+  static_assert(NV <= kAll, "at most 16 sums");
+  __shared__ double s_total[NV];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  long long bits = 0;
 #pragma unroll
-  for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
-  if (lane == 0) {
+  for (int q = 0; q < NV; ++q) bits |= __double_as_longlong(v[q]);
+  double w[kAll];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) scratch[q * nwarps + warp] = v[q];
+  for (int q = 0; q < kAll; ++q) w[q] = q < NV ? v[q] : 0.0;
+  if (__any_sync(0xffffffffu, bits != 0)) warp_sums<kAll>(w);
+  const int mine = warp_sums_index<kAll>(lane);
+  if ((lane & (32 / kAll - 1)) == 0 && mine < NV) scratch[mine * nwarps + warp] = w[0];
+  __syncthreads();
+  for (int q = warp; q < NV; q += nwarps) {
+    const double s = warp_sum(lane < nwarps ? scratch[q * nwarps + lane] : 0.0);
+    if (lane == 0) s_total[q] = s;
   }
   __syncthreads();
-  if (warp == 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double s = lane < nwarps ? scratch[q * nwarps + lane] : 0.0;
-      s = warp_sum(s);
-      out[q] = s;
-    }
-  }
-  __syncthreads();
+  for (int q = 0; q < NV; ++q) out[q] = s_total[q];
 }
 
 template <int NV>

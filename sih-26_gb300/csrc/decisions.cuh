@@ -65,16 +65,29 @@ __device__ inline double2 step_factors(long long iteration, const double2* table
   return (table != nullptr && e < n) ? table[e] : step_factors(e);
 }
 
+// What the decision of an attempt needs beside its sums, known when the attempt starts: a kernel that
+// waits for the sums forms it before.
+struct StepPrep {
+  double shrink, grown;    // shrink, grow * eta
+  double inv_omega;
+  int due[2];              // an evaluation falls due after a rejected, an accepted step
+  __device__ __forceinline__ void set(const Ctl* c, double2 factors) {
+    const long long k = c->iteration;
+    shrink = factors.x;
+    grown = factors.y * c->eta;
+    inv_omega = 1.0 / c->omega;
+    due[0] = k > 0 && k % 40 == 0;
+    due[1] = (k + 1) % 40 == 0;
+  }
+};
+
 __device__ inline void step_decision(Ctl* c, double movement, double interaction,
-                                     double2 factors) {
+                                     const StepPrep& p) {
   c->movement = movement;
   c->interaction = interaction;
   const bool no_information = interaction <= 0.0;
   const double limit = no_information ? __longlong_as_double(0x7ff0000000000000LL)
                                       : movement / interaction;
-  const double shrink = factors.x;
-  const double grow = factors.y;
-  const double proposed = dmin(shrink * limit, grow * c->eta);
   const bool accept = c->eta <= limit;
   if (accept) {
     c->cur ^= 1;
@@ -85,14 +98,21 @@ __device__ inline void step_decision(Ctl* c, double movement, double interaction
     c->pending_add = 0;
   }
   if (!no_information) {
-    double eta = proposed;
+    double eta = dmin(p.shrink * limit, p.grown);
     eta = eta < 1e-12 ? 1e-12 : (c->eta_ceiling < eta ? c->eta_ceiling : eta);
     c->eta = eta;
   }
   c->attempts += 1;
   c->accepted = accept;
   c->no_information = no_information;
-  c->eval_now = (c->iteration > 0) && ((c->iteration % 40) == 0 || no_information);
+  c->eval_now = p.due[accept ? 1 : 0] || (c->iteration > 0 && no_information);
+}
+
+__device__ inline void step_decision(Ctl* c, double movement, double interaction,
+                                     double2 factors) {
+  StepPrep p;
+  p.set(c, factors);
+  step_decision(c, movement, interaction, p);
 }
 
 __device__ inline void step_decision(Ctl* c, double movement, double interaction) {

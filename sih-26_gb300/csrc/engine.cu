@@ -685,6 +685,8 @@ void Engine::load(const sankhya_gb300_lp& lp) {
     step_factors_.allocate(static_cast<size_t>(kStepFactorTable));
     launch_step_factors(step_factors_.ptr, kStepFactorTable, s);
   }
+  part_steps_.allocate(3 * static_cast<size_t>(std::max(sl_csc_.view.grid, sl_csr_.view.grid)));
+  arrivals_.allocate(1);
   tickets_.allocate(4);
   SGB_CUDA(cudaMemsetAsync(tickets_.ptr, 0, 4 * sizeof(unsigned int), s));
   SGB_CUDA(cudaStreamSynchronize(s));
@@ -692,6 +694,13 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   resident_smem_ = resident_smem(m, n, sl_csc_.most_rows, sl_csc_.most_slices, sl_csr_.most_rows,
                                  sl_csr_.most_slices);
   resident_ = resident > 0 && resident_fits(step_, resident_smem_);
+  // Larger LPs run a period's steps in one cooperative launch (us a step, launches first: uniform
+  // 5,000 x 10,001 18.4 and 14.5, 60,000 x 120,001 32.0 and 28.8; blocks 320,000 x 640,000 90.5 and
+  // 88.0; Zipf rows with 200,000 entries 48.0 and 40.5). Not large ones with rows of several pieces
+  // (Zipf, 2 million entries: 68 and 75), whose blocks end far apart.
+  constexpr int kLongRowNnz = 1 << 20;
+  const bool pieces = sl_csc_.view.nlong + sl_csr_.view.nlong > 0;
+  steps_ = !resident_ && cap < 0 && (!pieces || nnz_ <= kLongRowNnz) && pdhg_steps_fit(step_);
   loaded_ = true;
 }
 
@@ -720,6 +729,7 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
   D.base.upload(P.base.data(), P.base.size(), s);
   D.items.upload(P.items.data(), P.items.size(), s);
   D.longs.upload(P.longs.data(), P.longs.size(), s);
+  D.tickets.allocate_padded(P.longs.size(), 1, s);
   D.segs.upload(P.segs.data(), P.segs.size(), s);
   D.seg_start.upload(P.seg_start.data(), P.seg_start.size(), s);
   D.block_start.upload(P.block_start.data(), P.block_start.size(), s);
@@ -843,6 +853,8 @@ void Engine::fill_buffers() {
   b.ctl = ctl_.ptr;
   b.csc = sl_csc_.view;
   b.csr = sl_csr_.view;
+  b.csc.tickets = sl_csc_.tickets.ptr;
+  b.csr.tickets = sl_csr_.tickets.ptr;
   b.x[0] = x0_.ptr;
   b.x[1] = x1_.ptr;
   b.y[0] = y0_.ptr;
@@ -862,6 +874,8 @@ void Engine::fill_buffers() {
   b.chunk_primal = chunk_primal_.ptr;
   b.chunk_dual = chunk_dual_.ptr;
   b.grid_primal = b.csc.grid;
+  b.part_steps = part_steps_.ptr;
+  b.arrivals = arrivals_.ptr;
 
   EvalBuffers& e = eval_;
   e.ctl = ctl_.ptr;
@@ -1113,6 +1127,7 @@ void Engine::init_iterates(const sankhya_gb300_params& p) {
   launch_fill(y_sum_.ptr, m_, 0.0, s);
   launch_fill(y_rst_.ptr, m_, 0.0, s);
   launch_fill(best_y_.ptr, m_, 0.0, s);
+  SGB_CUDA(cudaMemsetAsync(arrivals_.ptr, 0, sizeof(unsigned long long), s));
   if (n_ > 0) {
     SGB_CUDA(cudaMemcpyAsync(x_rst_.ptr, x0_.ptr, n_ * sizeof(double), cudaMemcpyDeviceToDevice, s));
     // best_x starts as the SCALED start point, as the reference's does (pdhg.cpp:190).
@@ -1128,10 +1143,15 @@ void Engine::build_graphs(int steps) {
     cudaGraph_t graph = nullptr;
     SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     const long long before = kernel_launch_count();
-    if (resident_) {
-      // A resident kernel ends where an evaluation falls due, at most 40 accepted steps on.
+    if (resident_ || steps_) {
+      // Both kernels end where an evaluation falls due, at most 40 accepted steps on.
       for (int k = 0; k < steps; k += kResidentAttempts) {
-        launch_pdhg_resident(step_, std::min(kResidentAttempts, steps - k), resident_smem_, stream_);
+        const int attempts = std::min(kResidentAttempts, steps - k);
+        if (resident_) {
+          launch_pdhg_resident(step_, attempts, resident_smem_, stream_);
+        } else {
+          launch_pdhg_steps(step_, attempts, stream_);
+        }
         launch_evaluation(eval_, stream_);
       }
     } else {
@@ -1319,7 +1339,7 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   const long long launches_setup = kernel_launch_count() - launches_before;
   // Capture launches nothing. A resident step takes a fraction of the time, so by default a graph
   // holds one evaluation period of them, rejected steps included.
-  build_graphs(p.steps_per_poll > 0 ? p.steps_per_poll : (resident_ ? kResidentAttempts : 32));
+  build_graphs(p.steps_per_poll > 0 ? p.steps_per_poll : (resident_ || steps_ ? kResidentAttempts : 32));
   const long long count_after_capture = kernel_launch_count();
   run_graphs(p, t0, graph_exec_, snapshot_, true, 0, &stop_status);
   const double t_end_loop = now_seconds();

@@ -131,6 +131,7 @@ class Engine {
     DeviceArray<int> idx, seg_start, block_start;
     DeviceArray<double> raw, scaled;
     DeviceArray<SliceItem> items;
+    DeviceArray<unsigned int> tickets;
     DeviceArray<LongRow> longs;
     DeviceArray<SliceSeg> segs;
     SliceSet view{};      // val = the scaled values
@@ -195,6 +196,9 @@ class Engine {
   cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};
   int graph_steps_ = 0;
   int graph_launches_ = 0;  // engine kernels per step graph
+  bool steps_ = false;      // FP64 steps run in launch_pdhg_steps' kernel
+  DeviceArray<double> part_steps_;
+  DeviceArray<unsigned long long> arrivals_;
   bool resident_ = false;   // FP64 steps run in the resident kernel,
   int resident_smem_ = 0;   // with this much shared memory a block
   cudaEvent_t done_event_[2] = {nullptr, nullptr};

@@ -109,6 +109,8 @@ struct StepBuffers {
   double* part_dual;     // [grid_dual * 2]
   double* chunk_primal;  // [csc.nchunks]
   double* chunk_dual;    // [csr.nchunks * 2]
+  double* part_steps;    // [3 * the larger grid] (k_pdhg_steps)
+  unsigned long long* arrivals;  // GridMeet's counter
   int grid_primal;
   // The step-size factors by iteration count (decisions.cuh, step_factors).
   const double2* step_factors;
@@ -197,6 +199,10 @@ struct ResidentSetup {
 };
 void launch_resident_setup(const ResidentSetup& r, int threads, int smem, cudaStream_t s);
 int resident_threads(const StepBuffers& b);
+// Up to `attempts` attempted steps in one cooperative launch, which ends early where an evaluation
+// falls due; pdhg_steps_fit: whether the device runs its blocks at once.
+void launch_pdhg_steps(const StepBuffers& b, int attempts, cudaStream_t s);
+bool pdhg_steps_fit(const StepBuffers& b);
 void launch_scaling(const ScalingBuffers& b, cudaStream_t s);
 // The sliced copy of a compressed layout's indices and values, and the values back.
 void launch_slice_fill(const SliceSet& S, const int* ptr, const int* idx, const double* val,

@@ -374,7 +374,8 @@ SlicePlan plan_slices(const std::vector<int>& ptr, const int* idx, int lines, in
         for (int c = 0; c < pieces; ++c) {
           const int b = c * kSlicePiece, e = std::min(len, b + kSlicePiece);
           p.items.push_back(SliceItem{r, pieces > 1 ? p.nchunks++ : -1,
-                                      static_cast<int>(lentries) + b, e - b});
+                                      static_cast<int>(lentries) + b, e - b,
+                                      pieces > 1 ? static_cast<int>(p.longs.size()) - 1 : -1});
         }
         lentries += len;
         continue;

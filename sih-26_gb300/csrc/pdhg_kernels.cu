@@ -85,6 +85,19 @@ __device__ bool fp64_stop_test(const Ctl* c, const Residuals& r) {
                                  (c->stop_at_request || meets_project_standard(r));
 }
 
+// The sum of get(0) .. get(n - 1) over a warp, in every lane: up to five per lane are read at once
+// and added as a tree, so 152 of them cost one latency and eight dependent additions.
+template <typename Get>
+__device__ __forceinline__ double table_sum(int n, Get get) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  double v[5];
+#pragma unroll
+  for (int u = 0; u < 5; ++u) v[u] = lane + 32 * u < n ? get(lane + 32 * u) : 0.0;
+  double sum = ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+  for (int k = lane + 160; k < n; k += 32) sum += get(k);
+  return warp_sum(sum);
+}
+
 // ---- k_primal ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
   extern __shared__ __align__(128) unsigned char dsmem[];
@@ -140,24 +153,11 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
       threadIdx.x == 0) {
     raise_error(ctl);
   }
-  if (b.csc.nlong == 0) {
-    // No long column to finish: each block publishes its partial, and k_dual's last block
-    // sums them in block order (primal_movement). No block of this pass waits for another.
-    double out[1];
-    block_sum<1>(mv, scratch, out);
-    if (threadIdx.x == 0) b.part_primal[blockIdx.x] = out[0];
-    return;
-  }
-  if (!arrive_last<1>(mv, scratch, b.part_primal, &ctl->ticket[kTicketPrimal])) return;
-  mv[0] = 0.0;
-  run_slice_long_rows<1, 5>(b.csc, b.chunk_primal, load, epi);
-  double longs[1], total[1];
-  block_sum<1>(mv, scratch, longs);
-  sum_partials<1>(b.part_primal, gridDim.x, scratch, total);
-  if (threadIdx.x == 0) {
-    ctl->mv_primal = 0.5 * omega * (total[0] + longs[0]);
-    ctl->ticket[kTicketPrimal] = 0;
-  }
+  // Each block publishes its partial, and k_dual's last block sums them in block order
+  // (primal_movement). No block of this pass waits for another.
+  double out[1];
+  block_sum<1>(mv, scratch, out);
+  if (threadIdx.x == 0) b.part_primal[blockIdx.x] = out[0];
 }
 
 // ---- k_dual ------------------------------------------------------------------------------
@@ -213,18 +213,15 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
     raise_error(ctl);
   }
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
-  acc2[0] = acc2[1] = 0.0;
-  run_slice_long_rows<2, 4>(b.csr, b.chunk_dual, load, epi);
-  double longs[2], total[2];
-  block_sum<2>(acc2, scratch, longs);
+  double total[2];
   sum_partials<2>(b.part_dual, gridDim.x, scratch, total);
   const double mv_primal =
-      primal_movement(b.csc.nlong == 0, b.part_primal, b.grid_primal, omega, ctl, scratch);
+      primal_movement(true, b.part_primal, b.grid_primal, omega, ctl, scratch);
   if (threadIdx.x == 0) {
     ctl->ticket[kTicketDual] = 0;
     if (ctl->done == kRunning) {
-      const double movement = mv_primal + (0.5 * (total[0] + longs[0])) / omega;
-      step_decision(ctl, movement, fabs(total[1] + longs[1]), factors);
+      const double movement = mv_primal + (0.5 * total[0]) / omega;
+      step_decision(ctl, movement, fabs(total[1]), factors);
     }
   }
 }
@@ -255,7 +252,7 @@ __device__ __forceinline__ void local_items(const LocalSlices& L, double* slots,
 __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffers b, int attempts) {
   extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ Ctl s_ctl;
-  __shared__ double2 s_factors;
+  __shared__ StepPrep s_prep;
   __shared__ double s_tau, s_sigma, s_sums[3];
   __shared__ double s_part[2][3][kResidentTable];
   static_assert(sizeof(Ctl) % sizeof(unsigned long long) == 0, "copied by words");
@@ -307,7 +304,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
     const bool add = s_ctl.pending_add != 0;
     const double tau = s_tau, sigma = s_sigma, omega = s_ctl.omega;
     double(*const part)[kResidentTable] = s_part[a & 1];
-    if (t == T - 1) s_factors = step_factors(s_ctl.iteration, b.step_factors, b.step_factors_n);
+    if (t == T - 1) {
+      s_prep.set(&s_ctl, step_factors(s_ctl.iteration, b.step_factors, b.step_factors_n));
+    }
     {
       const double* y = ys[cur];
       double mv = 0.0;
@@ -329,7 +328,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
         mv = fma(d, d, mv);
       }
       __syncwarp();
-      mv = warp_sum(mv);
+      if (__any_sync(0xffffffffu, mv != 0.0)) mv = warp_sum(mv);  // an idle warp adds nothing
       if (lane < C) {
         cluster_store(cluster_addr(&part[0][static_cast<int>(blockIdx.x) * W + warp], lane), mv);
       }
@@ -363,8 +362,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
         ia = fma(d, s1, ia);
       }
       __syncwarp();
-      dy2 = warp_sum(dy2);
-      ia = warp_sum(ia);
+      double both[2] = {dy2, ia};
+      if (__any_sync(0xffffffffu, dy2 != 0.0 || ia != 0.0)) {
+        warp_sums<2>(both);
+        dy2 = __shfl_sync(0xffffffffu, both[0], 0);
+        ia = __shfl_sync(0xffffffffu, both[0], 16);
+      }
       if (lane < C) {
         const int at = static_cast<int>(blockIdx.x) * W + warp;
         cluster_store(cluster_addr(&part[1][at], lane), dy2);
@@ -375,19 +378,17 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
     // A warp per sum: the primal movement, the dual movement over omega, the interaction.
     if (t < 96) {
       const int q = t >> 5;
-      double sum = 0.0;
-      for (int k = lane; k < C * W; k += 32) sum += part[q][k];
-      sum = warp_sum(sum);
-      if (lane == 0) s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? (0.5 * sum) / omega : sum);
+      const double sum = table_sum(C * W, [&](int k) { return part[q][k]; });
+      if (lane == 0) s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? 0.5 * sum * s_prep.inv_omega : sum);
     }
     __syncthreads();
     if (t == 0) {
       s_ctl.mv_primal = s_sums[0];
-      step_decision(&s_ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), s_factors);
+      step_decision(&s_ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), s_prep);
       if (s_ctl.eval_now == 0 && s_ctl.iteration >= s_ctl.iteration_limit) {
         s_ctl.done = kIterationLimit;
       }
-      s_tau = s_ctl.eta / s_ctl.omega;
+      s_tau = s_ctl.eta * s_prep.inv_omega;
       s_sigma = s_ctl.eta * s_ctl.omega;
     }
     __syncthreads();
@@ -405,6 +406,140 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
     b.y[last][i] = ys[last][i];
   }
   if (blockIdx.x == 0) {
+    for (int k = t; k < kWords; k += T) reinterpret_cast<unsigned long long*>(b.ctl)[k] = words[k];
+  }
+}
+
+// ---- The steps of a period in one launch ---------------------------------------------------------
+// k_primal and k_dual, item for item, by one cooperative grid whose blocks meet between the passes;
+// every block takes the step decision from the same partials. The next pass's first entries are
+// under way while a block waits. Operands a thread reads of its own rows it wrote itself; gathered
+// vectors are read with ld_live.
+__global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, int attempts) {
+  __shared__ double scratch[3 * (kSliceThreads / 32)];
+  __shared__ Ctl s_ctl;
+  __shared__ StepPrep s_prep;
+  __shared__ double s_tau, s_sigma, s_sums[3];
+  constexpr int kWords = static_cast<int>(sizeof(Ctl) / sizeof(unsigned long long));
+  const int t = static_cast<int>(threadIdx.x), T = static_cast<int>(blockDim.x);
+  const int block = static_cast<int>(blockIdx.x), G = static_cast<int>(gridDim.x);
+  const int lane = t & 31;
+  unsigned long long* const words = reinterpret_cast<unsigned long long*>(&s_ctl);
+  for (int k = t; k < kWords; k += T) {
+    words[k] = reinterpret_cast<const volatile unsigned long long*>(b.ctl)[k];
+  }
+  GridMeet grid;
+  grid.start(b.arrivals);
+  __syncthreads();
+  if (t == 0) {
+    if (s_ctl.done == kRunning && s_ctl.eval_now == 0 &&
+        s_ctl.iteration >= s_ctl.iteration_limit) {
+      s_ctl.done = kIterationLimit;  // src/pdhg/pdhg.cpp:206
+    }
+    s_tau = s_ctl.eta / s_ctl.omega;
+    s_sigma = s_ctl.eta * s_ctl.omega;
+  }
+  __syncthreads();
+  SliceStart<kPiece> cols;
+  if (block < b.csc.grid) start_slices(b.csc, cols);
+  for (int a = 0; a < attempts; ++a) {
+    if (s_ctl.done != kRunning || s_ctl.eval_now != 0) break;
+    const int cur = s_ctl.cur;
+    const bool add = s_ctl.pending_add != 0;
+    const double* y = b.y[cur];
+    double sums[3] = {0.0, 0.0, 0.0};  // dx^2, dy^2, dy (A dx)
+    if (t == T - 1) {
+      s_prep.set(&s_ctl, step_factors(s_ctl.iteration, b.step_factors, b.step_factors_n));
+    }
+    {
+      const double* x = b.x[cur];
+      double* xn = b.x[cur ^ 1];
+      const double tau = s_tau;
+      auto fetch = [&](int i) { return ld_live(y + i); };
+      auto mac = [](double v, double g, double* acc) { acc[0] = fma(v, g, acc[0]); };
+      auto load = [&](int j, double* o) {
+        o[0] = x[j];
+        o[1] = b.c[j];
+        o[2] = b.l[j];
+        o[3] = b.u[j];
+        o[4] = add ? b.x_sum[j] : 0.0;
+      };
+      auto epi = [&](int j, const double* s, const double* o) {
+        const double xj = o[0];
+        if (add) b.x_sum[j] = o[4] + xj;
+        const double gradient = o[1] + s[0];
+        const double xnj = clamp_box(__dsub_rn(xj, __dmul_rn(tau, gradient)), o[2], o[3]);
+        xn[j] = xnj;
+        const double d = xnj - xj;
+        b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
+        sums[0] = fma(d, d, sums[0]);
+      };
+      if (block < b.csc.grid) {
+        run_slices<false, 1, 5>(b.csc, cols, y, fetch, nullptr, b.chunk_primal, mac, load, epi);
+      }
+    }
+    {
+      SliceStart<kPairPiece> rows;
+      if (block < b.csr.grid) start_slices(b.csr, rows);
+      if (!grid.meet(&b.ctl->error)) return;
+      const double2* xd = b.xd;
+      double* yn = b.y[cur ^ 1];
+      const double sigma = s_sigma;
+      auto fetch = [&](int j) { return ld_live(xd + j); };
+      auto mac = [](double v, double2 p, double* acc) {
+        acc[0] = fma(v, p.x, acc[0]);
+        acc[1] = fma(v, p.y, acc[1]);
+      };
+      auto load = [&](int i, double* o) {
+        o[0] = y[i];
+        o[1] = b.rl[i];
+        o[2] = b.ru[i];
+        o[3] = add ? b.y_sum[i] : 0.0;
+      };
+      auto epi = [&](int i, const double* s, const double* o) {
+        const double yi = o[0];
+        if (add) b.y_sum[i] = o[3] + yi;
+        const double v = __dadd_rn(yi, __dmul_rn(sigma, s[0]));
+        const double p = o[1] == o[2] ? o[1] : clamp_box(v / sigma, o[1], o[2]);
+        const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
+        yn[i] = yni;
+        const double d = yni - yi;
+        sums[1] = fma(d, d, sums[1]);
+        sums[2] = fma(d, s[1], sums[2]);
+      };
+      if (block < b.csr.grid) {
+        run_slices<false, 2, 4>(b.csr, rows, xd, fetch, nullptr, b.chunk_dual, mac, load, epi);
+      }
+    }
+    double part[3];
+    block_sum<3>(sums, scratch, part);
+    if (t == 0) {
+      for (int q = 0; q < 3; ++q) b.part_steps[3 * block + q] = part[q];
+    }
+    if (block < b.csc.grid) start_slices(b.csc, cols);
+    if (!grid.meet(&b.ctl->error)) return;
+    // A warp per sum: the primal movement, the dual movement over omega, the interaction.
+    if (t < 96) {
+      const int q = t >> 5;
+      const double sum = table_sum(G, [&](int k) { return __ldcg(b.part_steps + 3 * k + q); });
+      if (lane == 0) {
+        s_sums[q] = q == 0 ? 0.5 * s_ctl.omega * sum
+                           : (q == 1 ? 0.5 * sum * s_prep.inv_omega : sum);
+      }
+    }
+    __syncthreads();
+    if (t == 0) {
+      s_ctl.mv_primal = s_sums[0];
+      step_decision(&s_ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), s_prep);
+      if (s_ctl.eval_now == 0 && s_ctl.iteration >= s_ctl.iteration_limit) {
+        s_ctl.done = kIterationLimit;
+      }
+      s_tau = s_ctl.eta * s_prep.inv_omega;
+      s_sigma = s_ctl.eta * s_ctl.omega;
+    }
+    __syncthreads();
+  }
+  if (block == 0) {
     for (int k = t; k < kWords; k += T) reinterpret_cast<unsigned long long*>(b.ctl)[k] = words[k];
   }
 }
@@ -1110,7 +1245,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident_setup(Resident
     cluster_meet();
     double out = local_product(cs, av, 1.0, v, C);
     __syncwarp();
-    out = warp_sum(out);
+    if (__any_sync(0xffffffffu, out != 0.0)) out = warp_sum(out);
     if (lane < C) {
       cluster_store(cluster_addr(&s_part[step & 1][0][static_cast<int>(blockIdx.x) * W + warp], lane),
                     out);
@@ -1302,6 +1437,15 @@ bool resident_fits(const StepBuffers& b, int smem) {
 void launch_pdhg_resident(const StepBuffers& b, int attempts, int smem, cudaStream_t s) {
   ++g_launches;
   launch_cluster(k_pdhg_resident, b.csc.grid, resident_threads(b), smem, s, b, attempts);
+}
+
+bool pdhg_steps_fit(const StepBuffers& b) {
+  return grid_fits(k_pdhg_steps, std::max(b.csc.grid, b.csr.grid), kSliceThreads, 0);
+}
+
+void launch_pdhg_steps(const StepBuffers& b, int attempts, cudaStream_t s) {
+  ++g_launches;
+  launch_grid(k_pdhg_steps, std::max(b.csc.grid, b.csr.grid), kSliceThreads, 0, s, b, attempts);
 }
 
 void launch_pdhg_step(const StepBuffers& b, cudaStream_t s) {

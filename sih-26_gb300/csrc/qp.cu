@@ -263,7 +263,9 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
   resident_ = cols_sliced && (rows_sliced || m_ == 0) && n_ > 0 &&
               std::max(m_, n_) <= kQpResidentItems && cc.empty() && rc.empty() &&
               qp_resident_fits(smem);
-  // Larger ones run a period's steps in one cooperative launch.
+  // Larger ones run a period's steps in one cooperative launch. Up to about 1,200 columns two short
+  // launches with a few blocks each are as fast (6.7 us an iteration at 1,000 columns; 7.1 us at
+  // 1,200 in one launch).
   constexpr int kQpStepItems = 1024;
   steps_ = !resident_ && std::max(m_, n_) > kQpStepItems && cols_sliced &&
            (rows_sliced || m_ == 0) && qp_steps_fit(d);

@@ -617,9 +617,9 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl,
 
 // ---- The steps of a period in one launch ---------------------------------------------------------
 // Iterations k0 .. of the graph by one cooperative grid: blocks meet between the passes, and each
-// warp has its next pass's first entries under way while it waits. Between two launches lie the
-// drain of one, the start of the next and its first loads, some 7 us an item-free pass; a meeting
-// takes 1.3 us.
+// warp has its next pass's first entries under way while it waits. A meeting takes 1.6 us of 152
+// blocks; between two launches lie the drain of one, the start of the next and its first loads.
+// An iteration over uniform rows: 8.9 us at 20,000 x 40,003 (14 us with launches), 14.2 us at 60,000.
 __global__ void __launch_bounds__(kQpSliceThreads, 1) k_qp_steps(QpDev d, QpCtl* ctl, int k0,
                                                                  int count) {
   if (ctl->done != 0) return;

@@ -68,6 +68,7 @@ struct SliceItem {
   int slot;
   int begin;
   int count;
+  int longs;  // slot >= 0: the row's LongRow
 };
 
 // Consecutive slices of one block that gather from the same window (len = 0: none).
@@ -85,6 +86,9 @@ struct SliceSet {
   const double* val;
   const SliceItem* items;
   const LongRow* longs;      // rows of several pieces
+  // Per such row, zero between passes: the warp that brings its last partial finishes the row. Null
+  // in the kernels that leave these rows to run_slice_long_rows.
+  unsigned int* tickets;
   const SliceSeg* segs;
   const int* seg_start;      // per block: its segments [seg_start[b], seg_start[b + 1])
   const int* block_start;    // per block: its slices [block_start[b], block_start[b + 1])
@@ -232,12 +236,33 @@ __device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& i
   __syncwarp();
 #pragma unroll
   for (int q = 0; q < NP; ++q) acc[q] = warp_sum(acc[q]);
-  if (lane != 0) return;
   if (it.slot < 0) {
-    epi(it.row, acc, ops);
-  } else {
+    if (lane == 0) epi(it.row, acc, ops);
+    return;
+  }
+  if (lane == 0) {
 #pragma unroll
     for (int q = 0; q < NP; ++q) chunk_part[it.slot * NP + q] = acc[q];
+  }
+  if (S.tickets == nullptr) return;
+  const LongRow lr = S.longs[it.longs];
+  int last = 0;
+  if (lane == 0) {
+    __threadfence();
+    last = atomicAdd(S.tickets + it.longs, 1u) == static_cast<unsigned>(lr.nchunks - 1);
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    acc[q] = 0.0;
+    for (int c = lane; c < lr.nchunks; c += 32) acc[q] += __ldcg(chunk_part + (lr.chunk0 + c) * NP + q);
+    acc[q] = warp_sum(acc[q]);
+  }
+  if (lane == 0) {
+    S.tickets[it.longs] = 0u;
+    load(it.row, ops);
+    epi(it.row, acc, ops);
   }
 }
 
@@ -269,13 +294,15 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, SliceStart<P>& st,
   }
   bool pending = false;  // thread 0: a copy issued and not yet seen complete
   uint32_t phase = 0;
-  const int g0 = __ldg(S.seg_start + blockIdx.x), g1 = __ldg(S.seg_start + blockIdx.x + 1);
+  // Without windows a block's slices are one segment.
+  const int g0 = windowed ? __ldg(S.seg_start + blockIdx.x) : 0;
+  const int g1 = windowed ? __ldg(S.seg_start + blockIdx.x + 1) : 1;
   bool ok = true;
   int s = st.s;
   SlicePlace p = st.place;
   PieceIndices<P> ix = st.indices;
   for (int g = g0; g < g1; ++g) {
-    const SliceSeg sg = S.segs[g];
+    const SliceSeg sg = windowed ? S.segs[g] : SliceSeg{0, st.s1, 0, 0};
     if (WIN && sg.len > 0) {
       if (g != g0) __syncthreads();  // every warp is done with the window held
       if (threadIdx.x == 0) {
@@ -302,8 +329,7 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, SliceStart<P>& st,
       return WIN && o < wlen ? win[o] : fetch(c);
     };
     if (g == g0) {
-      for (int i = static_cast<int>(blockIdx.x) + warp * static_cast<int>(gridDim.x);
-           i < S.nitems; i += W * static_cast<int>(gridDim.x)) {
+      for (int i = static_cast<int>(blockIdx.x) + warp * S.grid; i < S.nitems; i += W * S.grid) {
         slice_item<NP, NR, G>(S, S.items[i], chunk_part, get, mac, load, epi);
       }
     }

@@ -177,3 +177,23 @@ def test_qp_steps_in_one_launch_match_the_oracle(oracle, lengths, n, limit):
     assert (got.status_name, got.iterations) == (ref.status_name, ref.iterations)
     for a, b in ((x, ref.col_value), (d, ref.col_dual), (y, ref.row_dual)):
         assert np.all(np.abs(a - b) <= 1e-9 * max(1.0, np.abs(b).max() if len(b) else 0.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths,n", [([2100, 4100, 65, 64] + [3] * 500, 4300), ([6] * 5000, 8000),
+                                       ([2] * 9000, 60)])
+def test_pdhg_steps_in_one_launch_match_the_oracle(oracle, lengths, n):
+    """LPs past the resident kernel, whose steps run in one cooperative launch: rows of several
+    pieces, more blocks for one side than for the other; iteration limits are exact inside and at
+    the end of an evaluation period, and the point after 40 accepted steps is the oracle's within
+    1e-9."""
+    lp = lp_with_rows(lengths, n, seed=n)
+    with capi.PdhgEngine(0) as eng:
+        eng.load(lp)
+        for limit in (1, 41, 85):
+            assert eng.solve(tolerance=1e-13, iteration_limit=limit).iterations == limit
+        eng.solve(tolerance=1e-13, iteration_limit=40)
+        x, _, y = eng.solution()
+    ref = oracle.solve(lp, tolerance=1e-13, iteration_limit=40)
+    assert np.abs(x - ref.col_value).max() <= 1e-9 * max(1.0, np.abs(ref.col_value).max())
+    assert np.abs(y - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
