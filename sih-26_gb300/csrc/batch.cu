@@ -201,6 +201,10 @@ void BatchEngine::load(int count, const sankhya_gb300_lp* lps) {
   d_order_.upload(order.data(), order.size(), s);
   order_ = order;
   d_queue_.allocate(4);
+  if (step_factors_.ptr == nullptr) {
+    step_factors_.allocate(static_cast<size_t>(kBatchStepFactors));
+    launch_step_factors(step_factors_.ptr, kBatchStepFactors, s);
+  }
   csc_ptr_.upload(cptr.data(), cptr.size(), s);
   csc_idx_.upload(cidx.data(), cidx.size(), s);
   csc_raw_.upload(cval.data(), cval.size(), s);
@@ -331,6 +335,8 @@ void BatchEngine::solve(const sankhya_gb300_params& p, sankhya_gb300_batch_item*
   b.ray = ray_.ptr;
   b.outcome = outcome_.ptr;
   b.tolerance = p.tolerance;
+  b.step_factors = step_factors_.ptr;
+  b.step_factors_n = kBatchStepFactors;
   b.iteration_limit = p.iteration_limit < 0 ? 1000000 : p.iteration_limit;
   b.use_restarts = p.restart != 0;
   b.stop_at_request = p.stop_at_request != 0;

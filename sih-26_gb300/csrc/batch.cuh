@@ -76,6 +76,8 @@ struct BatchBuffers {
   const BatchInstance* instances;
   const int* order;           // instance solve order (largest first)
   unsigned int* queue;        // [0] next matrix, [1] next instance (reset by the host)
+  const double2* step_factors;  // by iteration count (decisions.cuh), below step_factors_n
+  long long step_factors_n;
   // Matrix arrays (offsets from BatchMatrix).
   const int *csc_ptr, *csc_idx, *csr_ptr, *csr_idx;
   const double *csc_raw, *csr_raw;

@@ -10,6 +10,9 @@
 
 namespace sgb {
 
+// Entries of a batch's step-size factor table.
+constexpr long long kBatchStepFactors = 1LL << 16;
+
 class BatchEngine {
  public:
   explicit BatchEngine(int device);
@@ -72,6 +75,7 @@ class BatchEngine {
   DeviceArray<BatchMatrix> d_mats_, d_mats_out_;
   DeviceArray<BatchInstance> d_inst_;
   DeviceArray<int> d_order_;
+  DeviceArray<double2> step_factors_;  // for iteration counts below kBatchStepFactors (1 MB)
   DeviceArray<unsigned int> d_queue_;
   DeviceArray<int> csc_ptr_, csc_idx_, csr_ptr_, csr_idx_;
   DeviceArray<double> csc_raw_, csr_raw_, csc_s_, csr_s_;

@@ -238,15 +238,32 @@ __device__ bool batch_stop_test(const Ctl* c, const Residuals& r) {
                                  (c->stop_at_request || meets_project_standard(r));
 }
 
+// An attempt's step sizes and its decision's other inputs, formed once per block: a division in
+// every thread, or a power in the deciding one, held the FP64 pipe longer than a pass's sums.
+struct BatchStep {
+  StepPrep prep;
+  double tau, sigma;
+  // Two threads share the divisions; the caller synchronises the block after.
+  __device__ __forceinline__ void set(const BatchBuffers& b, const Ctl* c) {
+    if (threadIdx.x == 0) {
+      tau = c->eta / c->omega;
+      sigma = c->eta * c->omega;
+    }
+    if (threadIdx.x == blockDim.x - 1) {
+      prep.set(c, step_factors(c->iteration, b.step_factors, b.step_factors_n));
+    }
+  }
+};
+
 // The primal step over the LP's columns (k_primal's arithmetic).
-__device__ void b_primal(const LpView& v, Ctl* c, double* scratch) {
+__device__ void b_primal(const LpView& v, const BatchStep& step, Ctl* c, double* scratch) {
   const int T = blockDim.x;
   const int cur = c->cur;
   const double* x = v.x[cur];
   double* xn = v.x[cur ^ 1];
   const double* y = v.y[cur];
   const double omega = c->omega;
-  const double tau = c->eta / omega;
+  const double tau = step.tau;
   const bool add = c->pending_add != 0;
   double mv[1] = {0.0};
   // `lanes` threads per column: lane s sums entries s, s + lanes, ... in order.
@@ -275,13 +292,12 @@ __device__ void b_primal(const LpView& v, Ctl* c, double* scratch) {
 }
 
 // The dual step over the LP's rows (k_dual's arithmetic) and the step decision.
-__device__ void b_dual(const LpView& v, Ctl* c, double* scratch) {
+__device__ void b_dual(const LpView& v, const BatchStep& step, Ctl* c, double* scratch) {
   const int T = blockDim.x;
   const int cur = c->cur;
   const double* y = v.y[cur];
   double* yn = v.y[cur ^ 1];
-  const double omega = c->omega;
-  const double sigma = c->eta * omega;
+  const double sigma = step.sigma, inv_sigma = step.prep.inv_sigma;
   const bool add = c->pending_add != 0;
   double acc2[2] = {0.0, 0.0};
   const int L = v.lanes, G = T / L, sub = threadIdx.x & (L - 1);
@@ -302,7 +318,7 @@ __device__ void b_dual(const LpView& v, Ctl* c, double* scratch) {
     if (add) v.y_sum[i] += yi;
     const double rl = v.rls[i], ru = v.rus[i];
     const double vv = __dadd_rn(yi, __dmul_rn(sigma, s0));
-    const double p = rl == ru ? rl : clamp_box(vv / sigma, rl, ru);
+    const double p = row_projection(vv, sigma, inv_sigma, rl, ru);
     const double yni = __dsub_rn(vv, __dmul_rn(sigma, p));
     yn[i] = yni;
     const double d = yni - yi;
@@ -312,8 +328,8 @@ __device__ void b_dual(const LpView& v, Ctl* c, double* scratch) {
   double tot[2];
   block_sum<2>(acc2, scratch, tot);
   if (threadIdx.x == 0 && c->done == kRunning) {
-    const double movement = c->mv_primal + (0.5 * tot[0]) / omega;
-    step_decision(c, movement, fabs(tot[1]));
+    const double movement = c->mv_primal + 0.5 * tot[0] * step.prep.inv_omega;
+    step_decision(c, movement, fabs(tot[1]), step.prep);
   }
   __syncthreads();
 }
@@ -575,6 +591,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 2) k_batch_solve(BatchBuffer
   __shared__ int s_item;
   __shared__ Ctl s_ctl;
   __shared__ LpView s_view;
+  __shared__ BatchStep s_step;
   __shared__ int s_infeasible;
   __shared__ double s_farkas;
   const int T = blockDim.x, t = threadIdx.x;
@@ -644,10 +661,11 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 2) k_batch_solve(BatchBuffer
         c->do_restart = 0;
         if (c->iteration >= c->iteration_limit) c->done = kIterationLimit;
       }
+      s_step.set(b, c);
       __syncthreads();
       if (c->done != kRunning) break;
-      b_primal(v, c, scratch);
-      b_dual(v, c, scratch);
+      b_primal(v, s_step, c, scratch);
+      b_dual(v, s_step, c, scratch);
       if (c->eval_now && c->done == kRunning) {
         b_evaluate(v, c, scratch, false);
         if (b.detect_infeasibility && c->done == kRunning) {
@@ -742,14 +760,15 @@ __device__ bool batch_round_stop(const Ctl* c, const Residuals& r) {
 }
 
 // The FP32 column pass (k_primal_f's arithmetic).
-__device__ void bm_primal(const LpView& v, const MixView& f, Ctl* c, double* scratch) {
+__device__ void bm_primal(const LpView& v, const MixView& f, const BatchStep& step, Ctl* c,
+                          double* scratch) {
   const int T = blockDim.x;
   const int cur = c->cur;
   const float* u = f.u[cur];
   float* un = f.u[cur ^ 1];
   const float* vv = f.v[cur];
   const double omega = c->omega;
-  const float tau = static_cast<float>(c->eta / omega);
+  const float tau = static_cast<float>(step.tau);
   const bool add = c->pending_add != 0;
   float mvf = 0.0f;
   const int L = v.lanes, G = T / L, sub = threadIdx.x & (L - 1);
@@ -777,13 +796,13 @@ __device__ void bm_primal(const LpView& v, const MixView& f, Ctl* c, double* scr
 }
 
 // The FP32 row pass with the correction-form prox (k_dual_f's arithmetic) and the decision.
-__device__ void bm_dual(const LpView& v, const MixView& f, Ctl* c, double* scratch) {
+__device__ void bm_dual(const LpView& v, const MixView& f, const BatchStep& step, Ctl* c,
+                        double* scratch) {
   const int T = blockDim.x;
   const int cur = c->cur;
   const float* vv = f.v[cur];
   float* vn = f.v[cur ^ 1];
-  const double omega = c->omega;
-  const float sigma = static_cast<float>(c->eta * omega);
+  const float sigma = static_cast<float>(step.sigma);
   const float inv_sigma = 1.0f / sigma;
   const bool add = c->pending_add != 0;
   float a0 = 0.0f, a1 = 0.0f;
@@ -822,8 +841,8 @@ __device__ void bm_dual(const LpView& v, const MixView& f, Ctl* c, double* scrat
   double acc[2] = {static_cast<double>(a0), static_cast<double>(a1)}, tot[2];
   block_sum<2>(acc, scratch, tot);
   if (threadIdx.x == 0 && c->done == kRunning) {
-    const double movement = c->mv_primal + (0.5 * tot[0]) / omega;
-    step_decision(c, movement, fabs(tot[1]));
+    const double movement = c->mv_primal + 0.5 * tot[0] * step.prep.inv_omega;
+    step_decision(c, movement, fabs(tot[1]), step.prep);
   }
   __syncthreads();
 }
@@ -974,6 +993,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 2) k_batch_solve_mixed(Batch
   __shared__ Ctl s_ctl;  // the inner loop's control block
   __shared__ Ctl s_fin;  // the exact evaluation's
   __shared__ LpView s_view;
+  __shared__ BatchStep s_step;
   __shared__ MixView s_mix;
   __shared__ double s_r[8];  // round scalars: [0] dp [1] dd [2] target [3..5] measures
   __shared__ int s_flags[4];  // [0] converged [1] stop [2] infeasible [3] round source
@@ -1142,10 +1162,11 @@ __global__ void __launch_bounds__(kBatchMaxThreads, 2) k_batch_solve_mixed(Batch
           c->do_restart = 0;
           if (c->iteration >= c->iteration_limit) c->done = kIterationLimit;
         }
+        s_step.set(b, c);
         __syncthreads();
         if (c->done != kRunning) break;
-        bm_primal(v, f, c, scratch);
-        bm_dual(v, f, c, scratch);
+        bm_primal(v, f, s_step, c, scratch);
+        bm_dual(v, f, s_step, c, scratch);
         if (c->eval_now && c->done == kRunning) bm_evaluate(v, f, c, scratch);
       }
       // Move the anchor: to the current iterate at a restart, else to the best candidate.

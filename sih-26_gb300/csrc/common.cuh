@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <string.h>
 #include <stdint.h>
 
 #include <cmath>
@@ -208,9 +209,50 @@ inline bool grid_fits(Kernel kernel, int blocks, int threads, int smem) {
   return able != 0 && blocks > 0 && blocks <= sms * per_sm;
 }
 
-__device__ __forceinline__ double clamp_box(double v, double lo, double hi) {
-  return fmin(fmax(v, lo), hi);
+// A key whose order as an integer is the order of the doubles (a negative zero before a positive
+// one, a NaN outside both infinities). An FP64 compare holds GB300's FP64 pipe as long as an FP64
+// addition does; the projections of the steps compare keys on the integer units instead.
+__host__ __device__ __forceinline__ long long order_key(double v) {
+#ifdef __CUDA_ARCH__
+  const long long i = __double_as_longlong(v);
+#else
+  long long i;
+  memcpy(&i, &v, sizeof(i));
+#endif
+  return i ^ ((i >> 63) & 0x7fffffffffffffffLL);
 }
+__host__ __device__ __forceinline__ bool nan_key(long long key) {
+  return key > 0x7ff0000000000000LL || key < ~0x7ff0000000000000LL;
+}
+
+// min(max(v, lo), hi), for bounds that are not NaN; a NaN v gives lo as fmax would.
+__host__ __device__ __forceinline__ double clamp_box(double v, double lo, double hi) {
+  const long long kv = order_key(v), kl = order_key(lo);
+  const bool low = kv < kl || nan_key(kv);
+  const double r = low ? lo : v;
+  return (low ? kl : kv) > order_key(hi) ? hi : r;
+}
+// The same projection with a NaN v left as it is.
+__host__ __device__ __forceinline__ double clamp_box_or_nan(double v, double lo, double hi) {
+  const long long kv = order_key(v);
+  if (nan_key(kv)) return v;
+  return kv < order_key(lo) ? lo : (kv > order_key(hi) ? hi : v);
+}
+
+// v / sigma from inv = RN(1 / sigma): Markstein's correction of the product with the correctly
+// rounded reciprocal (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q = v (1/sigma), r = v - sigma q exactly by
+// FMA, q + r (1/sigma) rounded once, which is the correctly rounded quotient for operands and
+// results in the normal range (tests/host/qp_division_check.c holds it to IEEE division). Three FP64
+// instructions where a division takes a dozen. An exact first product (r = 0) or a residual that is
+// not a number keeps the product.
+__device__ __forceinline__ double divide(double v, double sigma, double inv) {
+  const double q = __dmul_rn(v, inv);
+  const double r = fma(-q, sigma, v);
+  const long long size = __double_as_longlong(r) & 0x7fffffffffffffffLL;
+  return size == 0 || size > 0x7ff0000000000000LL ? q : fma(r, inv, q);
+}
+
 __device__ __forceinline__ float clamp_box(float v, float lo, float hi) {
   return fminf(fmaxf(v, lo), hi);
 }

@@ -65,17 +65,25 @@ __device__ inline double2 step_factors(long long iteration, const double2* table
   return (table != nullptr && e < n) ? table[e] : step_factors(e);
 }
 
+// The projection of v / sigma on [rl, ru]. On an equality row it is the bound whatever v is.
+__device__ __forceinline__ double row_projection(double v, double sigma, double inv_sigma, double rl,
+                                                 double ru) {
+  if (__double_as_longlong(rl) == __double_as_longlong(ru)) return rl;
+  return clamp_box(divide(v, sigma, inv_sigma), rl, ru);
+}
+
 // What the decision of an attempt needs beside its sums, known when the attempt starts: a kernel that
 // waits for the sums forms it before.
 struct StepPrep {
   double shrink, grown;    // shrink, grow * eta
-  double inv_omega;
+  double inv_omega, inv_sigma;  // sigma = eta * omega
   int due[2];              // an evaluation falls due after a rejected, an accepted step
   __device__ __forceinline__ void set(const Ctl* c, double2 factors) {
     const long long k = c->iteration;
     shrink = factors.x;
     grown = factors.y * c->eta;
     inv_omega = 1.0 / c->omega;
+    inv_sigma = 1.0 / (c->eta * c->omega);
     due[0] = k > 0 && k % 40 == 0;
     due[1] = (k + 1) % 40 == 0;
   }

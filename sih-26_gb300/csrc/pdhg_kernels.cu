@@ -179,7 +179,11 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
   const double* __restrict__ y = b.y[cur];
   double* __restrict__ yn = b.y[cur ^ 1];
   const double2* __restrict__ xd = b.xd;
+  __shared__ double s_inv_sigma;
   const double sigma = eta * omega;
+  if (threadIdx.x == 0) s_inv_sigma = 1.0 / sigma;
+  __syncthreads();
+  const double inv_sigma = s_inv_sigma;
   double acc2[2] = {0.0, 0.0};  // sum dy^2, sum dy (A dx)
   auto fetch = [&](int j) { return __ldg(xd + j); };
   auto mac = [](double v, double2 p, double* acc) {
@@ -196,12 +200,10 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
   auto epi = [&](int i, const double* s, const double* o) {
     const double yi = o[0];
     if (add) b.y_sum[i] = o[3] + yi;
-    const double rl = o[1], ru = o[2];
     // Unfused, as the reference rounds it (src/pdhg/pdhg.cpp:244-245): a fused
-    // v - sigma * (v / sigma) would leave the division's rounding error on a free row. On
-    // an equality row the projection is the bound whatever v is, so no division is needed.
+    // v - sigma * (v / sigma) would leave the division's rounding error on a free row.
     const double v = __dadd_rn(yi, __dmul_rn(sigma, s[0]));
-    const double p = rl == ru ? rl : clamp_box(v / sigma, rl, ru);
+    const double p = row_projection(v, sigma, inv_sigma, o[1], o[2]);
     const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
     yn[i] = yni;
     const double d = yni - yi;
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
         const double yi = y[i];
         if (add) ysum[k] = ysum[k] + yi;
         const double v = __dadd_rn(yi, __dmul_rn(sigma, s0));
-        const double p = rl[k] == ru[k] ? rl[k] : clamp_box(v / sigma, rl[k], ru[k]);
+        const double p = row_projection(v, sigma, s_prep.inv_sigma, rl[k], ru[k]);
         const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
         for (int r = 0; r < C; ++r) cluster_store(cluster_addr(yn + i, r), yni);
         const double d = yni - yi;
@@ -484,7 +486,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
       if (!grid.meet(&b.ctl->error)) return;
       const double2* xd = b.xd;
       double* yn = b.y[cur ^ 1];
-      const double sigma = s_sigma;
+      const double sigma = s_sigma, inv_sigma = s_prep.inv_sigma;
       auto fetch = [&](int j) { return ld_live(xd + j); };
       auto mac = [](double v, double2 p, double* acc) {
         acc[0] = fma(v, p.x, acc[0]);
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
         const double yi = o[0];
         if (add) b.y_sum[i] = o[3] + yi;
         const double v = __dadd_rn(yi, __dmul_rn(sigma, s[0]));
-        const double p = o[1] == o[2] ? o[1] : clamp_box(v / sigma, o[1], o[2]);
+        const double p = row_projection(v, sigma, inv_sigma, o[1], o[2]);
         const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
         yn[i] = yni;
         const double d = yni - yi;

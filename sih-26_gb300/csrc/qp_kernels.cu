@@ -14,12 +14,8 @@
 //   - the cost and Q are stored times the sense (exact), so the gradient
 //     (sense c + sense Qx) + A'y is two additions with the same bits;
 //   - 2 x' - x is one FMA (2 x' is exact);
-//   - v / sigma is Markstein's correction of the product with the correctly rounded
-//     reciprocal (P. Markstein, "Computation of elementary functions on the IBM RISC
-//     System/6000 processor", IBM J. Res. Dev. 34(1), 1990): q = v (1/sigma), r = v - sigma q
-//     exactly by FMA, q + r (1/sigma) rounded once, which is the correctly rounded quotient
-//     for operands and results in the normal range (tests/host/qp_division_check.c holds it to
-//     IEEE division).
+//   - v / sigma is divide() (common.cuh), the correctly rounded quotient from the reciprocal;
+//   - the projections compare on the integer units (clamp_box_or_nan).
 #include "qp.cuh"
 
 #include <algorithm>
@@ -40,15 +36,7 @@ __device__ __forceinline__ double qp_gradient(double cmin, double qxmin, double 
 // proj_[lo, hi](v) for bounds stored with absent sides as infinities: the reference's project
 // (src/qp/qp_condat_vu.cpp:60-64), a NaN left as it is.
 __device__ __forceinline__ double box(double v, double lo, double hi) {
-  return v < lo ? lo : (v > hi ? hi : v);
-}
-
-// v / sigma from inv = RN(1 / sigma) (Markstein's correction, see the file header); an exact
-// first product or a non-finite residual keeps the product.
-__device__ __forceinline__ double divide(double v, double sigma, double inv) {
-  const double q = __dmul_rn(v, inv);
-  const double r = fma(-q, sigma, v);
-  return (r == 0.0 || r != r) ? q : fma(r, inv, q);
+  return clamp_box_or_nan(v, lo, hi);
 }
 
 // A residual into a running maximum held as the bit pattern of a non-negative double (the
