@@ -666,8 +666,8 @@ void Engine::load(const sankhya_gb300_lp& lp) {
     a->allocate(static_cast<size_t>(m) + kPad);
   }
   const int pgrid = std::max(grid_c, grid_r) + num_sms_ * 8;
-  part_primal_.allocate(static_cast<size_t>(grid_c));
-  part_dual_.allocate(static_cast<size_t>(grid_r) * 2);
+  part_primal_.allocate(static_cast<size_t>(grid_c) + sl_csc_.view.nlong);
+  part_dual_.allocate(2 * (static_cast<size_t>(grid_r) + sl_csr_.view.nlong));
   part_rows0_.allocate(static_cast<size_t>(grid_r) * kEvalRowSlots);
   part_cols_.allocate(static_cast<size_t>(grid_c + 1) * kEvalColSlots);
   part_rows1_.allocate(static_cast<size_t>(grid_r) * kEvalRowSlots);
@@ -685,7 +685,10 @@ void Engine::load(const sankhya_gb300_lp& lp) {
     step_factors_.allocate(static_cast<size_t>(kStepFactorTable));
     launch_step_factors(step_factors_.ptr, kStepFactorTable, s);
   }
-  part_steps_.allocate(3 * static_cast<size_t>(std::max(sl_csc_.view.grid, sl_csr_.view.grid)));
+  const size_t step_parts = 3 * (static_cast<size_t>(std::max(sl_csc_.view.grid, sl_csr_.view.grid)) +
+                                 2 * sl_csc_.view.nlong + sl_csr_.view.nlong);
+  part_steps_.allocate(step_parts);
+  SGB_CUDA(cudaMemsetAsync(part_steps_.ptr, 0, step_parts * sizeof(double), s));
   arrivals_.allocate(1);
   tickets_.allocate(4);
   SGB_CUDA(cudaMemsetAsync(tickets_.ptr, 0, 4 * sizeof(unsigned int), s));
@@ -873,7 +876,6 @@ void Engine::fill_buffers() {
   b.part_dual = part_dual_.ptr;
   b.chunk_primal = chunk_primal_.ptr;
   b.chunk_dual = chunk_dual_.ptr;
-  b.grid_primal = b.csc.grid;
   b.part_steps = part_steps_.ptr;
   b.arrivals = arrivals_.ptr;
 

@@ -105,13 +105,12 @@ struct StepBuffers {
   // 16-byte element per entry: a scattered gather costs a cache sector whatever it reads.
   double2* xd;
   const double *c, *l, *u, *rl, *ru;  // scaled problem
-  double* part_primal;   // [grid_primal]
-  double* part_dual;     // [grid_dual * 2]
+  double* part_primal;   // [csc.grid + csc.nlong]
+  double* part_dual;     // [(csr.grid + csr.nlong) * 2]
   double* chunk_primal;  // [csc.nchunks]
   double* chunk_dual;    // [csr.nchunks * 2]
-  double* part_steps;    // [3 * the larger grid] (k_pdhg_steps)
+  double* part_steps;    // [(the larger grid + 2 csc.nlong + csr.nlong) * 3] (k_pdhg_steps)
   unsigned long long* arrivals;  // GridMeet's counter
-  int grid_primal;
   // The step-size factors by iteration count (decisions.cuh, step_factors).
   const double2* step_factors;
   long long step_factors_n;

@@ -149,7 +149,15 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
     b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
     mv[0] = fma(d, d, mv[0]);
   };
-  if (!run_slices<true, 1, 5>(b.csc, start, y, fetch, dsmem, b.chunk_primal, mac, load, epi) &&
+  auto finish = [&](int l, int j, const double* s, const double* o) {
+    const double sum = mv[0];
+    mv[0] = 0.0;
+    epi(j, s, o);
+    b.part_primal[b.csc.grid + l] = mv[0];
+    mv[0] = sum;
+  };
+  if (!run_slices<true, 1, 5>(b.csc, start, y, fetch, dsmem, b.chunk_primal, mac, load, epi,
+                              finish) &&
       threadIdx.x == 0) {
     raise_error(ctl);
   }
@@ -210,15 +218,25 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
     acc2[0] = fma(d, d, acc2[0]);
     acc2[1] = fma(d, s[1], acc2[1]);
   };
-  if (!run_slices<true, 2, 4>(b.csr, start, xd, fetch, dsmem, b.chunk_dual, mac, load, epi) &&
+  auto finish = [&](int l, int i, const double* s, const double* o) {
+    const double sums[2] = {acc2[0], acc2[1]};
+    acc2[0] = acc2[1] = 0.0;
+    epi(i, s, o);
+    for (int q = 0; q < 2; ++q) {
+      b.part_dual[2 * (b.csr.grid + l) + q] = acc2[q];
+      acc2[q] = sums[q];
+    }
+  };
+  if (!run_slices<true, 2, 4>(b.csr, start, xd, fetch, dsmem, b.chunk_dual, mac, load, epi,
+                              finish) &&
       threadIdx.x == 0) {
     raise_error(ctl);
   }
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
   double total[2];
-  sum_partials<2>(b.part_dual, gridDim.x, scratch, total);
-  const double mv_primal =
-      primal_movement(true, b.part_primal, b.grid_primal, omega, ctl, scratch);
+  sum_partials<2>(b.part_dual, b.csr.grid + b.csr.nlong, scratch, total);
+  const double mv_primal = primal_movement(true, b.part_primal, b.csc.grid + b.csc.nlong, omega, ctl,
+                                           scratch);
   if (threadIdx.x == 0) {
     ctl->ticket[kTicketDual] = 0;
     if (ctl->done == kRunning) {
@@ -476,8 +494,16 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
         b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
         sums[0] = fma(d, d, sums[0]);
       };
+      auto finish = [&](int l, int j, const double* s, const double* o) {
+        const double sum = sums[0];
+        sums[0] = 0.0;
+        epi(j, s, o);
+        b.part_steps[3 * (G + (a & 1) * b.csc.nlong + l)] = sums[0];
+        sums[0] = sum;
+      };
       if (block < b.csc.grid) {
-        run_slices<false, 1, 5>(b.csc, cols, y, fetch, nullptr, b.chunk_primal, mac, load, epi);
+        run_slices<false, 1, 5>(b.csc, cols, y, fetch, nullptr, b.chunk_primal, mac, load, epi,
+                                finish);
       }
     }
     {
@@ -509,8 +535,18 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
         sums[1] = fma(d, d, sums[1]);
         sums[2] = fma(d, s[1], sums[2]);
       };
+      auto finish = [&](int l, int i, const double* s, const double* o) {
+        const double keep[2] = {sums[1], sums[2]};
+        sums[1] = sums[2] = 0.0;
+        epi(i, s, o);
+        for (int q = 1; q < 3; ++q) {
+          b.part_steps[3 * (G + 2 * b.csc.nlong + l) + q] = sums[q];
+          sums[q] = keep[q - 1];
+        }
+      };
       if (block < b.csr.grid) {
-        run_slices<false, 2, 4>(b.csr, rows, xd, fetch, nullptr, b.chunk_dual, mac, load, epi);
+        run_slices<false, 2, 4>(b.csr, rows, xd, fetch, nullptr, b.chunk_dual, mac, load, epi,
+                                finish);
       }
     }
     double part[3];
@@ -523,7 +559,13 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
     // A warp per sum: the primal movement, the dual movement over omega, the interaction.
     if (t < 96) {
       const int q = t >> 5;
-      const double sum = table_sum(G, [&](int k) { return __ldcg(b.part_steps + 3 * k + q); });
+      // The blocks', the long columns' of this attempt (a block still at the last decision reads the
+      // other half) and the long rows'; entries that a column or a row does not have stay zero.
+      const int nc = b.csc.nlong;
+      const double sum = table_sum(G + nc + b.csr.nlong, [&](int k) {
+        const int skip = k < G ? 0 : (k < G + nc ? (a & 1) * nc : nc);
+        return __ldcg(b.part_steps + 3 * (k + skip) + q);
+      });
       if (lane == 0) {
         s_sums[q] = q == 0 ? 0.5 * s_ctl.omega * sum
                            : (q == 1 ? 0.5 * sum * s_prep.inv_omega : sum);

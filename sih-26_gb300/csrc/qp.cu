@@ -223,8 +223,9 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
   }
   cudaStream_t s = stream_;
   std::vector<QpChunk> cc, rc;
-  qp_build_chunks(col_len_, col_lanes, &cc, &nlong_cols_);
-  qp_build_chunks(row_len_, row_lanes, &rc, &nlong_rows_);
+  const int chunk = nnz_a_ > kQpShortChunkNnz ? kQpMidChunk : kQpShortChunk;
+  qp_build_chunks(col_len_, col_lanes, &cc, &nlong_cols_, chunk);
+  qp_build_chunks(row_len_, row_lanes, &rc, &nlong_rows_, chunk);
   ncol_chunks_ = static_cast<int>(cc.size());
   nrow_chunks_ = static_cast<int>(rc.size());
   col_chunks_.upload(cc.data(), cc.size(), s);
@@ -278,7 +279,8 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
     qp_launch_slice_fill(d, false, nullptr, nullptr, row_slices_.idx2.ptr, row_slices_.val2.ptr, s);
   }
   SGB_CUDA(cudaGetLastError());
-  product_part_.allocate(2 * static_cast<size_t>(qp_product_blocks(d)));
+  product_part_.allocate(2 * (static_cast<size_t>(qp_product_blocks(d)) +
+                              std::max(nlong_cols_, nlong_rows_)));
   SGB_CUDA(cudaStreamSynchronize(s));
   destroy_graph();
 }
@@ -323,6 +325,7 @@ QpDev QpEngine::dev() const {
   d.row_tickets = row_tickets_.ptr;
   d.long_col_obj = long_col_obj_.ptr;
   d.nlong_cols = nlong_cols_;
+  d.nlong_rows = nlong_rows_;
   d.obj_part = obj_part_.ptr;
   d.col_short_blocks = col_short_blocks_;
   d.row_short_blocks = row_short_blocks_;
@@ -439,10 +442,13 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
   // items; lanes that are asked for, or staging, run on the compressed arrays.
   const double col_mean = n_ > 0 ? double(nnz_a_ + nnz_q_) / n_ : 1.0;
   const double row_mean = m_ > 0 ? double(nnz_a_) / m_ : 1.0;
-  const int col_lanes = p.column_lanes > 0 ? p.column_lanes : qp_auto_lanes(col_mean);
-  const int row_lanes = p.row_lanes > 0 ? p.row_lanes : qp_auto_lanes(row_mean);
-  const bool cols_sliced = p.column_lanes <= 0 && col_lanes == 1 && p.staging == 0;
-  const bool rows_sliced = p.row_lanes <= 0 && row_lanes == 1 && p.staging == 0;
+  int col_lanes = p.column_lanes > 0 ? p.column_lanes : qp_auto_lanes(col_mean);
+  int row_lanes = p.row_lanes > 0 ? p.row_lanes : qp_auto_lanes(row_mean);
+  // Slices hold items of up to 64 entries, so a mean of up to 64 (two lanes by the rule) runs on them.
+  const bool cols_sliced = p.column_lanes <= 0 && col_lanes <= 2 && p.staging == 0;
+  const bool rows_sliced = p.row_lanes <= 0 && row_lanes <= 2 && p.staging == 0;
+  if (cols_sliced) col_lanes = 1;
+  if (rows_sliced) row_lanes = 1;
   if (!valid_lanes(col_lanes) || !valid_lanes(row_lanes)) {
     throw EngineError{SANKHYA_GB300_ERROR_OPTION, "lanes must be 1, 2, 4, 8, 16 or 32"};
   }

@@ -117,7 +117,7 @@ struct QpDev {
   unsigned int* col_tickets;
   unsigned int* row_tickets;
   double* long_col_obj;      // objective terms of the long columns, by slot
-  int nlong_cols;
+  int nlong_cols, nlong_rows;
   // Check partials.
   double* obj_part;          // per short-path block of the column pass
   int col_short_blocks, row_short_blocks;
@@ -151,7 +151,7 @@ void qp_launch_slice_fill(const QpDev& d, bool cols, int* idx1, double* val1, in
                           double* val2, cudaStream_t s);
 // Power steps: out = M (v / sqrt(*norm2)) with M = A (kQpRows), A' (kQpCols) or Q (kQpHessian).
 // next[0] receives sum out^2 and next[1] sum out v / sqrt(*norm2) (Q only), in a fixed order, from
-// `part` (2 doubles per block, qp_product_blocks) and `ticket` (zero on entry and exit); next may
+// `part` (2 doubles per block, qp_product_blocks, and per long item) and `ticket` (zero on entry and exit); next may
 // be null (A). norm2 null: v is used as it is. Without slices `lanes` threads share an item.
 enum QpSide { kQpRows = 0, kQpCols = 1, kQpHessian = 2 };
 int qp_product_blocks(const QpDev& d);

@@ -16,6 +16,11 @@ namespace sgb {
 // Entries a chunk of a long row or column holds at most, and the lanes past which an item is
 // long: an item with more than kQpLongPerLane entries per lane goes to the chunked path.
 constexpr int kQpChunk = 2048;
+// The chunks of the passes, by the entries of A: a warp's chunk is a chain of loads, and a chunk costs
+// a partial and a ticket. us an iteration of rows drawn by Zipf's law with chunks of 256, 512, 1,024
+// and 2,048: 16.8, 17.4, 18.9, 21.4 (200,000 entries); 39.8, 35.7, 32.5, 34.3 (2 million).
+constexpr int kQpShortChunk = 512, kQpMidChunk = 1024;
+constexpr long long kQpShortChunkNnz = 1LL << 20;
 constexpr int kQpLongPerLane = 64;
 
 // One chunk of a long row or column: entries [begin, end) of the item's entry sequence (for
@@ -140,20 +145,20 @@ inline void qp_build_layout(const sankhya_gb300_qp_problem& p, QpHostLayout* out
   }
 }
 
-// The chunks of the items longer than kQpLongPerLane * lanes entries, in item order; *nlong
-// receives the number of such items (their slots are 0 .. *nlong - 1 in item order).
+// The chunks, of at most `chunk` entries, of the items longer than kQpLongPerLane * lanes entries, in
+// item order; *nlong receives the number of such items (their slots are 0 .. *nlong - 1 in item
+// order).
 inline void qp_build_chunks(const std::vector<int>& len, int lanes, std::vector<QpChunk>* out,
-                            int* nlong) {
+                            int* nlong, int chunk = kQpChunk) {
   out->clear();
   *nlong = 0;
   for (int item = 0; item < static_cast<int>(len.size()); ++item) {
     const int l = len[item];
     if (l <= kQpLongPerLane * lanes) continue;
-    const int count = (l + kQpChunk - 1) / kQpChunk;
+    const int count = (l + chunk - 1) / chunk;
     const int first = static_cast<int>(out->size());
     for (int c = 0; c < count; ++c) {
-      out->push_back(QpChunk{item, c * kQpChunk, std::min(l, (c + 1) * kQpChunk), first, count,
-                             *nlong});
+      out->push_back(QpChunk{item, c * chunk, std::min(l, (c + 1) * chunk), first, count, *nlong});
     }
     ++*nlong;
   }

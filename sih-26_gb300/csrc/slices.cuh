@@ -204,12 +204,13 @@ __device__ __forceinline__ void start_slices(const SliceSet& S, SliceStart<P>& s
 }
 
 // One long item, by the whole warp.
-constexpr int kSliceBatch = 4;
+constexpr int kSliceBatch = 8;
 
-template <int NP, int NR, typename G, typename Get, typename Mac, typename Load, typename Epi>
+template <int NP, int NR, typename G, typename Get, typename Mac, typename Load, typename Epi,
+          typename Finish>
 __device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& it,
                                            double* chunk_part, Get get, Mac mac, Load load,
-                                           Epi epi) {
+                                           Epi epi, Finish finish) {
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int* __restrict__ ip = S.idx + S.long_base + it.begin;
   const double* __restrict__ vp = S.val + S.long_base + it.begin;
@@ -262,7 +263,7 @@ __device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& i
   if (lane == 0) {
     S.tickets[it.longs] = 0u;
     load(it.row, ops);
-    epi(it.row, acc, ops);
+    finish(it.longs, it.row, acc, ops);
   }
 }
 
@@ -271,13 +272,20 @@ __device__ __forceinline__ void slice_item(const SliceSet& S, const SliceItem& i
 //   windows they are staged from `vec`, the same vector
 //   mac(v, g, acc) adds the entry's products
 //   load(row, ops), epi(row, acc, ops) the row's NR operands and its epilogue
+//   finish(l, row, acc, ops) the epilogue of row l of S.longs, where S.tickets is set. Which warp runs
+//   it varies, so what it adds to a sum goes to a place of its own.
 // WIN is false in kernels that stage no window whatever the layout has. Returns false -- in
 // every thread -- if a wait gave up (only a staged window waits).
+struct NoFinish {
+  template <typename... Args>
+  __device__ __forceinline__ void operator()(Args...) const {}
+};
+
 template <bool WIN, int NP, int NR, typename G, int P, typename Fetch, typename Mac, typename Load,
-          typename Epi>
+          typename Epi, typename Finish = NoFinish>
 __device__ __forceinline__ bool run_slices(const SliceSet& S, SliceStart<P>& st, const G* vec,
                                            Fetch fetch, unsigned char* dsmem, double* chunk_part,
-                                           Mac mac, Load load, Epi epi) {
+                                           Mac mac, Load load, Epi epi, Finish finish = Finish()) {
   __shared__ volatile int s_abort;
   const int W = static_cast<int>(blockDim.x) >> 5;
   const int warp = static_cast<int>(threadIdx.x) >> 5;
@@ -330,7 +338,7 @@ __device__ __forceinline__ bool run_slices(const SliceSet& S, SliceStart<P>& st,
     };
     if (g == g0) {
       for (int i = static_cast<int>(blockIdx.x) + warp * S.grid; i < S.nitems; i += W * S.grid) {
-        slice_item<NP, NR, G>(S, S.items[i], chunk_part, get, mac, load, epi);
+        slice_item<NP, NR, G>(S, S.items[i], chunk_part, get, mac, load, epi, finish);
       }
     }
     for (; s < sg.s1; s += W) {

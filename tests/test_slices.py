@@ -112,8 +112,12 @@ def test_resident_steps_match_the_oracle(oracle, m, n):
         eng.load(lp)
         for limit in (1, 41, 85):
             assert eng.solve(tolerance=1e-13, iteration_limit=limit).iterations == limit
-        eng.solve(tolerance=1e-13, iteration_limit=40)
-        x, _, y = eng.solution()
+        points = []
+        for _ in range(2):
+            eng.solve(tolerance=1e-13, iteration_limit=40)
+            points.append(eng.solution())
+        x, _, y = points[0]
+        assert all(np.array_equal(a, b) for a, b in zip(*points))
     ref = oracle.solve(lp, tolerance=1e-13, iteration_limit=40)
     assert np.abs(x - ref.col_value).max() <= 1e-9 * max(1.0, np.abs(ref.col_value).max())
     assert np.abs(y - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
@@ -159,12 +163,13 @@ def test_qp_slices_match_the_oracle(oracle, m, n, per_column, band):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("lengths,n,limit", [([], 1025, 60), ([1100, 600, 65, 64] + [3] * 700, 1100, 177),
+@pytest.mark.parametrize("lengths,n,limit", [([40] * 900, 1500, 60), ([], 1025, 60), ([1100, 600, 65, 64] + [3] * 700, 1100, 177),
                                              ([7] * 6000, 9000, 101), ([2] * 1300, 40, 50)])
 def test_qp_steps_in_one_launch_match_the_oracle(oracle, lengths, n, limit):
     """QPs past 1,024 items, whose check periods run in one cooperative launch: no rows, rows in
-    chunks, limits that end inside a period, more rows than columns; the oracle's iteration count,
-    and its point within 1e-9 of its scale, as every QP parity test."""
+    chunks, rows of more than 32 entries, limits that end inside a period, more rows than columns;
+    the oracle's iteration count, its point within 1e-9 of its scale, as every QP parity test, and
+    the same bits twice."""
     from sankhya_gb300.model import QP, banded_hessian
 
     lp = lp_with_rows(lengths, n, seed=n)
@@ -174,6 +179,8 @@ def test_qp_steps_in_one_launch_match_the_oracle(oracle, lengths, n, limit):
         eng.load(qp)
         got = eng.solve(tolerance=1e-12, iteration_limit=limit)
         x, d, y = eng.solution()
+        eng.solve(tolerance=1e-12, iteration_limit=limit)
+        assert all(np.array_equal(a, b) for a, b in zip(eng.solution(), (x, d, y)))
     assert (got.status_name, got.iterations) == (ref.status_name, ref.iterations)
     for a, b in ((x, ref.col_value), (d, ref.col_dual), (y, ref.row_dual)):
         assert np.all(np.abs(a - b) <= 1e-9 * max(1.0, np.abs(b).max() if len(b) else 0.0))
@@ -192,8 +199,12 @@ def test_pdhg_steps_in_one_launch_match_the_oracle(oracle, lengths, n):
         eng.load(lp)
         for limit in (1, 41, 85):
             assert eng.solve(tolerance=1e-13, iteration_limit=limit).iterations == limit
-        eng.solve(tolerance=1e-13, iteration_limit=40)
-        x, _, y = eng.solution()
+        points = []
+        for _ in range(2):
+            eng.solve(tolerance=1e-13, iteration_limit=40)
+            points.append(eng.solution())
+        x, _, y = points[0]
+        assert all(np.array_equal(a, b) for a, b in zip(*points))
     ref = oracle.solve(lp, tolerance=1e-13, iteration_limit=40)
     assert np.abs(x - ref.col_value).max() <= 1e-9 * max(1.0, np.abs(ref.col_value).max())
     assert np.abs(y - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
