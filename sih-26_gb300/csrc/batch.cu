@@ -1,6 +1,7 @@
 // batch.cu -- BatchEngine: packs the LPs of a batch into device arrays (one copy per distinct
 // matrix) and runs the scaling and solve launches of batch_kernels.cu.
 #include "batch_engine.hpp"
+#include "dense_lu.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -654,8 +655,7 @@ void BatchEngine::adjoint(const double* const* dl_dx, const double* const* dl_dy
                            cudaMemcpyHostToDevice, s));
   AdjointBuffers a = adjoint_buffers();
   SGB_CUDA(cudaMemsetAsync(d_queue_.ptr + 2, 0, sizeof(unsigned int), s));
-  const int grid = std::max(
-      1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a.threads, a.smem_bytes)));
+  const int grid = adjoint_grid(&a);
   launch_batch_adjoint(buffers_, a, grid, s);
   SGB_CUDA(cudaGetLastError());
   finish_adjoint(dl_dc, dl_drl, dl_dru, dl_dl, dl_du, info);
@@ -684,6 +684,7 @@ void BatchEngine::ensure_adjoint_buffers() {
   long long nz = 0;
   const size_t room = static_cast<size_t>(adjoint_max_smem());
   size_t need = 0, likely = 0;
+  int widest = 1;
   for (int k = 0; k < count_; ++k) {
     const BatchInstance& I = inst_[static_cast<size_t>(k)];
     const BatchMatrix& M = mats_[static_cast<size_t>(I.matrix)];
@@ -692,6 +693,7 @@ void BatchEngine::ensure_adjoint_buffers() {
     // Shared memory that holds the LP's solves whatever its basis, and with a basis of half
     // its entries (solve_basis: six vectors, both matrices, the slices' records).
     const size_t d = static_cast<size_t>(std::min(I.m, I.n));
+    widest = std::max(widest, std::min(I.m, I.n));
     const size_t z = static_cast<size_t>(M.nnz);
     need = std::max(need, 64 * d + 20 * (z + 64 * 16) + 256);
     likely = std::max(likely, 64 * d + 11 * z);
@@ -700,6 +702,13 @@ void BatchEngine::ensure_adjoint_buffers() {
   // memory want more warps in flight.
   a_smem_ = static_cast<int>(std::min(room, need)) & ~15;
   a_threads_ = likely <= room ? 256 : kAdjThreads;
+  // Bases that a block factors densely (dense_lu.cuh) are solved so, all of the batch's or none.
+  a_lu_size_ = 0;
+  if (widest <= kLuMost && static_cast<size_t>(lu_smem(lu_size(widest))) <= room) {
+    a_lu_size_ = lu_size(widest);
+    a_smem_ = std::max(a_smem_, (lu_smem(a_lu_size_) + 15) & ~15);
+    a_threads_ = kLuThreads;
+  }
   const size_t Z = static_cast<size_t>(std::max(nz, 1LL));
   a_kci_.allocate(Z);
   a_kri_.allocate(Z);
@@ -713,6 +722,27 @@ void BatchEngine::ensure_adjoint_buffers() {
   a_rs_.allocate(M);
   a_out_.allocate(static_cast<size_t>(count_));
   adjoint_ready_ = true;
+}
+
+// The blocks of an adjoint or polish launch; with them the LU workspaces, one per block. Without the
+// memory for those the solves run by conjugate gradients.
+int BatchEngine::adjoint_grid(AdjointBuffers* a) {
+  const int grid = std::max(
+      1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a->threads, a->smem_bytes)));
+  a->lu = nullptr;
+  a->lu_size = a_lu_size_;
+  if (a_lu_size_ > 0) {
+    const size_t each = static_cast<size_t>(a_lu_size_) * a_lu_size_;
+    size_t free_bytes = 0, total = 0;
+    const bool room = a_lu_.capacity >= each * grid ||
+                      (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess &&
+                       each * grid * sizeof(float) < free_bytes / 2);
+    if (room) {
+      a_lu_.allocate(each * grid);
+      a->lu = a_lu_.ptr;
+    }
+  }
+  return grid;
 }
 
 AdjointBuffers BatchEngine::adjoint_buffers() {
@@ -807,8 +837,7 @@ void BatchEngine::polish(sankhya_gb300_batch_item* items, sankhya_gb300_adjoint_
   ensure_adjoint_buffers();
   AdjointBuffers a = adjoint_buffers();
   SGB_CUDA(cudaMemsetAsync(d_queue_.ptr + 3, 0, sizeof(unsigned int), s));
-  const int grid = std::max(
-      1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a.threads, a.smem_bytes)));
+  const int grid = adjoint_grid(&a);
   launch_batch_polish(buffers_, a, grid, s);
   SGB_CUDA(cudaGetLastError());
   std::vector<BatchOutcome> out(static_cast<size_t>(count_));

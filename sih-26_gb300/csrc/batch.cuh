@@ -134,6 +134,8 @@ struct AdjointBuffers {
   double cg_tolerance;
   int* tmp;                                        // m per LP
   int threads, smem_bytes;                         // of the launches
+  float* lu;                                       // lu_size^2 per block, or null (dense_lu.cuh)
+  int lu_size;
 };
 
 void launch_batch_scaling(const BatchBuffers& b, int grid, cudaStream_t s);

@@ -54,6 +54,7 @@ class BatchEngine {
   void fetch_points(int index);
   void forget_points();
   AdjointBuffers adjoint_buffers();
+  int adjoint_grid(AdjointBuffers* a);
   void finish_adjoint(double* const* dl_dc, double* const* dl_drl, double* const* dl_dru,
                       double* const* dl_dl, double* const* dl_du,
                       sankhya_gb300_adjoint_info* info);
@@ -75,6 +76,8 @@ class BatchEngine {
   DeviceArray<BatchMatrix> d_mats_, d_mats_out_;
   DeviceArray<BatchInstance> d_inst_;
   DeviceArray<int> d_order_;
+  DeviceArray<float> a_lu_;  // the adjoint's and the polish's LU workspaces
+  int a_lu_size_ = 0;        // columns each holds; 0: none
   DeviceArray<double2> step_factors_;  // for iteration counts below kBatchStepFactors (1 MB)
   DeviceArray<unsigned int> d_queue_;
   DeviceArray<int> csc_ptr_, csc_idx_, csr_ptr_, csr_idx_;

@@ -17,6 +17,7 @@
 #include "batch.cuh"
 #include "common.cuh"
 #include "decisions.cuh"
+#include "dense_lu.cuh"
 #include "kernels.cuh"
 #include "sankhya_gb300.h"
 
@@ -1556,24 +1557,26 @@ __device__ __forceinline__ double line_dot(const Lines<I>& L, int k, const doubl
   return s;
 }
 
-// Block-wide sums handed to every thread, in one barrier: each warp's total goes to `scratch`
-// (NV * 32 doubles, not in use by the reduction before this one), and every warp adds the
-// totals in the same order. The barrier also publishes what the threads wrote before it.
+// Block-wide sums (one or two) handed to every thread; the barriers also publish what the threads
+// wrote before. Few FP64 instructions, as in block_sum: both sums by halves in a warp, and one warp adds
+// the warps' totals, both at once, for all (16 warps that each added them held the FP64 pipe longer
+// than the extra barrier: 43% of an iteration's FP64 instructions on 1,000 basic columns).
 template <int NV>
 __device__ __forceinline__ void quick_sum(double (&v)[NV], double* scratch) {
+  static_assert(NV == 1 || NV == 2, "the warps' totals of one warp's lanes");
+  __shared__ double s_total[NV];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const double s = warp_sum(v[q]);
-    if (lane == 0) scratch[q * 32 + warp] = s;
+  warp_sums<NV>(v);
+  if ((lane & (32 / NV - 1)) == 0) scratch[warp_sums_index<NV>(lane) * nw + warp] = v[0];
+  __syncthreads();
+  if (warp == 0) {
+    double s = lane < NV * nw ? scratch[lane] : 0.0;
+    for (int o = nw >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((lane & (nw - 1)) == 0 && lane < NV * nw) s_total[lane / nw] = s;
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    double s = lane < nw ? scratch[q * 32 + lane] : 0.0;
-    for (int o = nw >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    v[q] = __shfl_sync(0xffffffffu, s, 0);
-  }
+  for (int q = 0; q < NV; ++q) v[q] = s_total[q];
 }
 
 // The vectors of a solve: p and t are gathered, dinv holds the reciprocal preconditioner.
@@ -1594,7 +1597,6 @@ __device__ __forceinline__ int pcg_sf(const Lines<I>& S, const Lines<I>& F, int 
                                       double tol) {
   __shared__ double s_alpha, s_inv;
   const int T = blockDim.x, th = threadIdx.x;
-  double* const scr2 = scratch + 64;
   double a0[2] = {0.0, 0.0};
   for (int k = th; k < nb; k += T) {
     const double rk = x.r[k], wk = rk * x.dinv[k];
@@ -1614,7 +1616,7 @@ __device__ __forceinline__ int pcg_sf(const Lines<I>& S, const Lines<I>& F, int 
       x.t[k] = s;
       a1[0] = fma(s, s, a1[0]);
     }
-    quick_sum<1>(a1, scr2);  // also publishes t
+    quick_sum<1>(a1, scratch);  // also publishes t
     if (!(a1[0] > 0.0)) break;
     if (th == T - 1) s_alpha = rw / a1[0];
     if (th == T - 33) s_inv = 1.0 / rw;
@@ -1687,11 +1689,125 @@ __device__ __forceinline__ int solve_square(const Lines<I>& S, const Lines<I>& F
   return its;
 }
 
-// The solve with the storage this LP gets (see above). `first` is the LP's first solve, which fills the shared copies;
-// `rows` solves with A_RB (S = rows), otherwise with its transpose.
+// The LP's basis in this block: its factors (dense_lu.cuh) and its copies in shared memory.
+struct BasisState {
+  int factored;  // 0 not yet, 1 the factors are in the block's workspace, -1 not to be had
+  bool copied;   // the matrices are in shared memory (the factors' pivots are not)
+};
+
+// S u = h (F = S') by refinement with the block's LU factors; u as for solve_square. Returns the
+// refinement steps, or -1 - steps where they did not reach tol, with u as it was. The residual is
+// followed until it stops falling, so that a solve is as accurate as its arithmetic allows.
+__device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjView& w,
+                                           unsigned char* smem, int nb, BasisState* state, bool rows,
+                                           const double* h, double* u, double* scratch,
+                                           double* rel) {
+  constexpr int kMostSteps = 30;
+  const int T = blockDim.x, th = threadIdx.x;
+  const int n = lu_size(nb);
+  const LuMem mem(smem, n);
+  float* const A = a.lu + static_cast<size_t>(blockIdx.x) * a.lu_size * a.lu_size;
+  const Lines<int> r{w.krl, w.krb, w.kri, w.krv}, c{w.kcl, w.kcb, w.kci, w.kcv};
+  const Lines<int>& S = rows ? r : c;
+  double* const keep = w.kw[2];
+  double* const res = w.kw[3];
+  double a0[1] = {0.0};
+  for (int k = th; k < nb; k += T) {
+    a0[0] = fma(h[k], h[k], a0[0]);
+    keep[k] = u[k];
+  }
+  quick_sum<1>(a0, scratch);
+  const double hnorm = sqrt(a0[0]);
+  double before = HUGE_VAL;
+  int steps = 0;
+  for (;; ++steps) {
+    double a1[1] = {0.0};
+    for (int k = th; k < nb; k += T) {
+      const double rk = h[k] - line_dot(S, k, u);
+      res[k] = rk;
+      a1[0] = fma(rk, rk, a1[0]);
+    }
+    quick_sum<1>(a1, scratch);
+    const double rnorm = sqrt(a1[0]);
+    *rel = hnorm > 0.0 ? rnorm / hnorm : 0.0;
+    if (steps == 0 && *rel <= a.cg_tolerance) return 0;
+    // Followed to where it no longer falls; a step that lost is taken back.
+    if (steps == kMostSteps || !(rnorm <= 0.9 * before)) {
+      if (steps > 0 && !(rnorm < before)) {
+        __syncthreads();
+        for (int k = th; k < nb; k += T) u[k] = w.kw[4][k];
+        *rel = hnorm > 0.0 ? before / hnorm : 0.0;
+        __syncthreads();
+      }
+      break;
+    }
+    if (rnorm == 0.0) break;
+    if (state->factored == 0) {
+      // The matrix by rows, padded with the identity.
+      const size_t quads = static_cast<size_t>(n) * n / 4;
+      for (size_t e = th; e < quads; e += T) {
+        reinterpret_cast<float4*>(A)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      __syncthreads();
+      for (int p = th; p < n; p += T) {
+        float* const row = A + static_cast<size_t>(p) * n;
+        if (p >= nb) {
+          row[p] = 1.0f;
+          continue;
+        }
+        size_t e = static_cast<size_t>(r.base[p >> 5]) * 32 + (p & 31);
+        for (int q = 0; q < r.len[p]; ++q, e += 32) row[r.idx[e]] = static_cast<float>(r.val[e]);
+      }
+      __syncthreads();
+      const bool ok = lu_factor(A, n, mem);
+      __syncthreads();
+      if (th == 0) state->factored = ok ? 1 : -1;
+      __syncthreads();
+      if (!ok) return -1 - steps;
+    }
+    float* const y = mem.lt;
+    const double inv = 1.0 / rnorm;
+    for (int k = th; k < n; k += T) {
+      const int at = rows ? mem.piv[k] : k;
+      y[k] = at < nb ? static_cast<float>(res[at] * inv) : 0.0f;
+    }
+    __syncthreads();
+    if (rows) {
+      lu_sweeps(A, n, mem.piv, y);
+    } else {
+      lu_sweeps_transposed(A, n, mem.piv, y);
+    }
+    for (int k = th; k < n; k += T) {
+      const int at = rows ? k : mem.piv[k];
+      if (at >= nb) continue;
+      w.kw[4][at] = u[at];
+      u[at] = fma(rnorm, static_cast<double>(y[k]), u[at]);
+    }
+    before = rnorm;
+    __syncthreads();
+  }
+  // Where rounding holds the residual up it passes the same test as the iterations' would.
+  if (*rel <= 100.0 * a.cg_tolerance) return steps;
+  for (int k = th; k < nb; k += T) u[k] = keep[k];
+  __syncthreads();
+  if (th == 0) state->factored = -1;
+  __syncthreads();
+  return -1 - steps;
+}
+
+// The solve of the LP's basis: with LU factors where the launch has a workspace for them
+// (AdjointBuffers::lu) and the basis is not too ill-conditioned for FP32 factors, else by conjugate
+// gradients with the storage this LP gets (see above). `rows` solves with A_RB (S = rows), otherwise
+// with its transpose. Returns the refinement steps or iterations.
 __device__ int solve_basis(const AdjointBuffers& a, const AdjView& w, unsigned char* smem, int nb,
-                           bool first, bool rows, const double* h, double* u, double* scratch,
+                           BasisState* state, bool rows, const double* h, double* u, double* scratch,
                            double* rel) {
+  if (a.lu != nullptr && state->factored >= 0 && !state->copied && nb <= a.lu_size) {
+    const int steps = solve_factored(a, w, smem, nb, state, rows, h, u, scratch, rel);
+    if (steps >= 0) return steps;
+  }
+  const bool first = !state->copied;
+  __syncthreads();  // read by all before it is set
   const int T = blockDim.x, th = threadIdx.x;
   const int slices = (nb + 31) / 32;
   const size_t vec = static_cast<size_t>(kSqVectors) * nb * sizeof(double);
@@ -1728,6 +1844,7 @@ __device__ int solve_basis(const AdjointBuffers& a, const AdjView& w, unsigned c
         rb[k] = w.krb[k];
         cb[k] = w.kcb[k];
       }
+      if (th == 0) state->copied = true;
       __syncthreads();
     }
     const Lines<unsigned short> r{rl, rb, ri, rv}, c{cl, cb, ci, cv};
@@ -1759,6 +1876,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b
   __shared__ int s_item;
   __shared__ LpView s_view;
   __shared__ AdjView s_adj;
+  __shared__ BasisState s_basis;
   const int T = blockDim.x, t = threadIdx.x;
   for (int wk = next_item(&b.queue[2], b.ninstances, &s_item); wk >= 0;
        wk = next_item(&b.queue[2], b.ninstances, &s_item)) {
@@ -1768,6 +1886,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b
     if (t == 0) {
       s_view = make_view(b, I, M);
       s_adj = make_adj_view(a, I, li);
+      s_basis = BasisState{0, false};
     }
     __syncthreads();
     const LpView& v = s_view;
@@ -1789,7 +1908,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b
         u[k] = 0.0;
       }
       __syncthreads();
-      it1 = solve_basis(a, w, s_mem, nb, true, true, h, u, scratch, &res1);
+      it1 = solve_basis(a, w, s_mem, nb, &s_basis, true, h, u, scratch, &res1);
       for (int j = t; j < v.n; j += T) {
         const int q = w.cpos[j];
         w.dc[j] = fma(w.gf, v.best_x[j], q >= 0 ? u[q] : 0.0);
@@ -1801,7 +1920,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b
         u[k] = 0.0;
       }
       __syncthreads();
-      it2 = solve_basis(a, w, s_mem, nb, false, false, h, u, scratch, &res2);
+      it2 = solve_basis(a, w, s_mem, nb, &s_basis, false, h, u, scratch, &res2);
       for (int i = t; i < v.m; i += T) {
         const signed char st = w.rs[i];
         const double yrep = -v.best_y[i];  // the reported multiplier
@@ -1856,6 +1975,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_polish(BatchBuffers b,
   __shared__ int s_item;
   __shared__ LpView s_view;
   __shared__ AdjView s_adj;
+  __shared__ BasisState s_basis;
   __shared__ Ctl s_ctl;
   const int T = blockDim.x, t = threadIdx.x;
   for (int wk = next_item(&b.queue[3], b.ninstances, &s_item); wk >= 0;
@@ -1866,6 +1986,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_polish(BatchBuffers b,
     if (t == 0) {
       s_view = make_view(b, I, M);
       s_adj = make_adj_view(a, I, li);
+      s_basis = BasisState{0, false};
     }
     __syncthreads();
     const LpView& v = s_view;
@@ -1902,7 +2023,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_polish(BatchBuffers b,
     __syncthreads();
     int it1 = 0, it2 = 0;
     double res1 = 0.0, res2 = 0.0;
-    it1 = solve_basis(a, w, s_mem, nb, true, true, h, u, scratch, &res1);
+    it1 = solve_basis(a, w, s_mem, nb, &s_basis, true, h, u, scratch, &res1);
     for (int j = t; j < v.n; j += T) {
       const signed char st = w.cs[j];
       v.xu[1][j] = st == 0 ? u[w.cpos[j]] : (st == 1 ? v.l[j] : v.u[j]);
@@ -1914,7 +2035,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_polish(BatchBuffers b,
       u[k] = -v.best_y[w.rrow[k]];
     }
     __syncthreads();
-    it2 = solve_basis(a, w, s_mem, nb, false, false, h, u, scratch, &res2);
+    it2 = solve_basis(a, w, s_mem, nb, &s_basis, false, h, u, scratch, &res2);
     for (int i = t; i < v.m; i += T) {
       const int q = w.rpos[i];
       v.yu[1][i] = q >= 0 ? -u[q] : 0.0;  // the solver's sign
