@@ -1557,6 +1557,25 @@ __device__ __forceinline__ double line_dot(const Lines<I>& L, int k, const doubl
   return s;
 }
 
+// h - line k's product with x, as if in twice the precision (Ogita, Rump and Oishi, "Accurate sum and
+// dot product", SIAM J. Sci. Comput. 26(6), 2005: Dot2): the products' and the sums' rounding errors
+// are formed exactly and added in the end.
+template <typename I>
+__device__ __forceinline__ double line_residual(const Lines<I>& L, int k, const double* x, double h) {
+  const int n = L.len[k];
+  size_t e = static_cast<size_t>(L.base[k >> 5]) * 32 + (k & 31);
+  double s = h, low = 0.0;
+  for (int q = 0; q < n; ++q, e += 32) {
+    const double v = L.val[e], g = x[L.idx[e]];
+    const double p = __dmul_rn(v, g), p_low = fma(v, g, -p);
+    const double sum = __dsub_rn(s, p), b = __dsub_rn(sum, s);
+    const double s_low = __dadd_rn(__dsub_rn(s, __dsub_rn(sum, b)), __dsub_rn(-p, b));
+    low = __dadd_rn(low, __dsub_rn(s_low, p_low));
+    s = sum;
+  }
+  return __dadd_rn(s, low);
+}
+
 // Block-wide sums (one or two) handed to every thread; the barriers also publish what the threads
 // wrote before. Few FP64 instructions, as in block_sum: both sums by halves in a warp, and one warp adds
 // the warps' totals, both at once, for all (16 warps that each added them held the FP64 pipe longer
@@ -1696,8 +1715,9 @@ struct BasisState {
 };
 
 // S u = h (F = S') by refinement with the block's LU factors; u as for solve_square. Returns the
-// refinement steps, or -1 - steps where they did not reach tol, with u as it was. The residual is
-// followed until it stops falling, so that a solve is as accurate as its arithmetic allows.
+// refinement steps, or -1 - steps where they did not reach tol, with u as it was. The residual, formed
+// to twice the precision, is followed until it stops falling: then u is the solution but for its own
+// rounding.
 __device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjView& w,
                                            unsigned char* smem, int nb, BasisState* state, bool rows,
                                            const double* h, double* u, double* scratch,
@@ -1723,7 +1743,7 @@ __device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjVie
   for (;; ++steps) {
     double a1[1] = {0.0};
     for (int k = th; k < nb; k += T) {
-      const double rk = h[k] - line_dot(S, k, u);
+      const double rk = line_residual(S, k, u, h[k]);
       res[k] = rk;
       a1[0] = fma(rk, rk, a1[0]);
     }
