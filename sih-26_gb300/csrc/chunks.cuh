@@ -4,14 +4,17 @@
 // CSC copy) holding at most CH nonzeros; a row longer than CH is cut into PIECES of CH
 // entries. Each warp of a block works through its own chunks, one at a time, with no
 // barrier between warps:
-//   1. its lanes load the chunk's indices and values straight from global memory, lane l
-//      taking entries l, l + 32, ... (every load coalesced, streamed past L1), and the
-//      per-row operands of the epilogue, lane l taking row r0 + l;
+//   1. its lanes load the chunk's indices and values straight from global memory, and the per-row
+//      operands of the epilogue, lane l taking row r0 + l. A chunk's entries are PACKED for this:
+//      kChunkCapF places a chunk, lane l's eight (entries l, l + 32, ...) in runs of 16 bytes a lane,
+//      so three or four loads bring what took sixteen of 4 bytes. Where the windows hold all entries
+//      the packed indices are 16 bits from the window's start, and the next chunk's entries are in
+//      flight while this one is summed (with 32-bit indices the registers for that would spill);
 //   2. they gather the vector entry of each nonzero -- from the block's staged WINDOW of the
 //      vector in shared memory, or from L2 when the window does not hold it -- and stage the
-//      (value, gathered) pairs in the warp's shared buffer;
+//      products in the warp's shared buffer;
 //   3. `L` lanes per row (the largest power of two with 32 / L >= rows) sum each row from
-//      the buffer with FMA, in a fixed order (lane s takes entries s, s + L, ...; then a fixed
+//      the buffer, in a fixed order (lane s takes entries s, s + L, ...; then a fixed
 //      xor tree), and the row's first lane runs the epilogue with the operands shuffled to
 //      it. A piece of a long row is summed by the whole warp into a piece partial; the last
 //      block of the kernel combines the pieces of each long row in order.
@@ -65,11 +68,13 @@ struct ChunkSeg {
 
 // A chunk record is a Tile: rows [r0, r1), entries [k0, k1); r1 < 0 marks a piece of a long
 // row whose partial goes to piece slot -r1 - 1.
-template <typename T>
 struct ChunkSet {
   const int* ptr;        // rows + 1 (main part)
-  const int* idx;        // nnz (+ kPad)
-  const T* val;          // nnz (+ kPad)
+  const int* idx;        // nnz (+ kPad): the pieces' entries
+  const float* val;      // nnz (+ kPad)
+  const float* pval;     // packed values, kChunkCapF per chunk
+  const void* pidx;      // packed indices: uint16 from the window's start, or int
+  int narrow;            // the packed indices are 16 bits
   const Tile* chunks;
   const ChunkSeg* segs;
   const int* seg_start;  // per block: its segments [seg_start[b], seg_start[b + 1])
@@ -81,13 +86,15 @@ struct ChunkSet {
   // Split layouts: the out-of-window entries as a CSR of their own. Block b sums the outer
   // entries of its rows in ROUNDS (row ranges orounds[oround_start[b] .. oround_start[b + 1]),
   // each with at most as many outer entries as the block's warp buffers hold); outer holds
-  // NP sums per row.
+  // a sum per row. A round's entries are stored by column, opos their places in the order of the
+  // rows (a round's start is optr of its first row).
   const int* optr;
   const int* oidx;
-  const T* oval;
+  const float* oval;
+  const unsigned short* opos;
   const int2* orounds;
   const int* oround_start;
-  T* outer;              // nullptr: not split
+  float* outer;          // nullptr: not split
 };
 
 // ---- PTX helpers ---------------------------------------------------------------------------
@@ -107,42 +114,27 @@ __device__ __forceinline__ double ld_stream(const double* p) {
   return v;
 }
 
-// Components of a gathered element.
-template <typename T>
-__device__ __forceinline__ void split_gathered(float g, T (&c)[1]) { c[0] = g; }
-template <typename T>
-__device__ __forceinline__ void split_gathered(double g, T (&c)[1]) { c[0] = g; }
-template <typename T>
-__device__ __forceinline__ void split_gathered(double2 g, T (&c)[2]) {
-  c[0] = g.x;
-  c[1] = g.y;
+__device__ __forceinline__ float4 ld_stream(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_stream(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
 }
 
-template <typename T>
-__device__ __forceinline__ T fma_t(T a, T b, T c);
-template <>
-__device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return fmaf(a, b, c); }
-template <>
-__device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return fma(a, b, c); }
-
-// Whether a layout's warps stage products (one FP32 multiply per entry, summed with adds) or
-// (value, gathered) pairs (summed with one FMA per entry and product). FP32 stages products:
-// half the shared-memory traffic. FP64 stages pairs: GB300 retires FP64 at a few operations
-// per clock per SM, so a multiply and an add per entry would cost twice the FMA.
-template <typename T>
-struct StageProducts {
-  static constexpr bool value = sizeof(T) == sizeof(float);
-};
-
-// Dynamic shared memory of a chunk kernel: per-warp buffers, the window barrier, the window.
-template <typename T, typename G, int NP, int CH>
-struct ChunkSmem {
-  static constexpr int kBufBytes =
-      CH * (StageProducts<T>::value ? NP : 1 + NP) * static_cast<int>(sizeof(T));
-  __host__ __device__ static constexpr int bytes(int warps, int wmax) {
-    return warps * kBufBytes + 128 + ((wmax * static_cast<int>(sizeof(G)) + 127) & ~127);
-  }
-};
+// Dynamic shared memory of a chunk kernel: per-warp buffers of products (half the shared-memory
+// traffic of value and gathered element), the window barrier, the window.
+constexpr int kChunkBufBytes = kChunkCapF * static_cast<int>(sizeof(float));
+__host__ __device__ constexpr int chunk_smem(int warps, int wmax) {
+  return warps * kChunkBufBytes + 128 + ((wmax * static_cast<int>(sizeof(float)) + 127) & ~127);
+}
 
 // Lanes per row for a chunk of R rows: the largest power of two L with 32 / L >= R.
 __device__ __forceinline__ int chunk_lanes(int R) {
@@ -150,187 +142,161 @@ __device__ __forceinline__ int chunk_lanes(int R) {
   return 32 >> p;
 }
 
-// One chunk: stream, gather, stage, sum, epilogue (all lanes of the warp call it).
-//   gather(col) -> G          the vector element of column col
+// A lane's eight packed entries of a chunk.
+template <bool NARROW>
+struct PackedEntries {
+  static constexpr int kEach = kChunkCapF / 32;
+  static_assert(kEach == 8, "two float4 and one or two uint4 a lane");
+  float4 a0, a1;
+  uint4 x0, x1;
+  __device__ __forceinline__ void load(const ChunkSet& cs, int chunk) {
+    const int lane = static_cast<int>(threadIdx.x) & 31;
+    const float4* v = reinterpret_cast<const float4*>(cs.pval) + static_cast<size_t>(chunk) * 64 + lane;
+    a0 = ld_stream(v);
+    a1 = ld_stream(v + 32);
+    const uint4* x = reinterpret_cast<const uint4*>(cs.pidx) +
+                     static_cast<size_t>(chunk) * (NARROW ? 32 : 64) + lane;
+    x0 = ld_stream(x);
+    if (!NARROW) x1 = ld_stream(x + 32);
+  }
+  __device__ __forceinline__ void unpack(float (&a)[kEach], int (&c)[kEach]) const {
+    a[0] = a0.x, a[1] = a0.y, a[2] = a0.z, a[3] = a0.w;
+    a[4] = a1.x, a[5] = a1.y, a[6] = a1.z, a[7] = a1.w;
+    if (NARROW) {
+      const unsigned w[4] = {x0.x, x0.y, x0.z, x0.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        c[2 * j] = static_cast<int>(w[j] & 0xffffu);
+        c[2 * j + 1] = static_cast<int>(w[j] >> 16);
+      }
+    } else {
+      c[0] = static_cast<int>(x0.x), c[1] = static_cast<int>(x0.y);
+      c[2] = static_cast<int>(x0.z), c[3] = static_cast<int>(x0.w);
+      c[4] = static_cast<int>(x1.x), c[5] = static_cast<int>(x1.y);
+      c[6] = static_cast<int>(x1.z), c[7] = static_cast<int>(x1.w);
+    }
+  }
+};
+
+// One chunk of whole rows: gather, stage, sum, epilogue (all lanes of the warp call it).
+//   gather(c) -> float        the vector element of packed index c
 //   load(row, ops)            the row's NR epilogue operands (lane-per-row, at chunk start)
 //   epi(row, sums, ops)       once per row, on the row's first lane
-template <int NP, int NR, typename T, typename G, int CH, bool OUTER, typename Gather,
-          typename Load, typename Epi>
-__device__ __forceinline__ void chunk_step(const int* __restrict__ ptr, const int* __restrict__ idx,
-                                           const T* __restrict__ val, const Tile& ch, T* buf,
-                                           const T* __restrict__ outer, double* piece_part,
-                                           Gather gather, Load load, Epi epi) {
-  constexpr int J = CH / 32;
+template <int NR, bool NARROW, bool OUTER, typename Gather, typename Load, typename Epi>
+__device__ __forceinline__ void chunk_step(const int* __restrict__ ptr, const Tile& ch,
+                                           const PackedEntries<NARROW>& e, float* buf,
+                                           const float* __restrict__ outer, Gather gather,
+                                           Load load, Epi epi) {
+  constexpr int J = kChunkCapF / 32;
   const int lane = static_cast<int>(threadIdx.x) & 31;
-  const bool piece = ch.r1 < 0;
-  const int R = piece ? 0 : ch.r1 - ch.r0;
-  const int n = ch.k1 - ch.k0;
-  int col[J];
-  T a[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    const int k = ch.k0 + lane + 32 * j;
-    const bool in = lane + 32 * j < n;
-    col[j] = in ? ld_stream(idx + k) : -1;
-    a[j] = in ? ld_stream(val + k) : T(0);
-  }
+  const int R = ch.r1 - ch.r0;
   int pr = 0;
-  T ops[NR > 0 ? NR : 1];
-  T out[NP];
-#pragma unroll
-  for (int q = 0; q < NP; ++q) out[q] = T(0);
-  if (!piece) {
-    if (lane <= R) pr = __ldg(ptr + ch.r0 + lane);
-    if (lane < R) {
-      load(ch.r0 + lane, ops);
-      if (OUTER) {
-#pragma unroll
-        for (int q = 0; q < NP; ++q) out[q] = outer[(ch.r0 + lane) * NP + q];
-      }
-    }
+  float ops[NR > 0 ? NR : 1];
+  float out = 0.0f;
+  if (lane <= R) pr = __ldg(ptr + ch.r0 + lane);
+  if (lane < R) {
+    load(ch.r0 + lane, ops);
+    if (OUTER) out = outer[ch.r0 + lane];
   }
-  constexpr bool kProducts = StageProducts<T>::value;
-  // Pairs: bv holds the values, bg the NP gathered components; products: bg the NP products.
-  T* bv = buf;
-  T* bg = kProducts ? buf : buf + CH;
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-    T c[NP];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) c[q] = T(0);
-    if (col[j] >= 0) split_gathered(gather(col[j]), c);
+  {
+    float a[J];
+    int c[J];
+    e.unpack(a, c);
     // Past the chunk's end the entry is a zero that no row reads.
-    if (kProducts) {
 #pragma unroll
-      for (int q = 0; q < NP; ++q) bg[q * CH + lane + 32 * j] = a[j] * c[q];
-    } else {
-      bv[lane + 32 * j] = a[j];
-#pragma unroll
-      for (int q = 0; q < NP; ++q) bg[q * CH + lane + 32 * j] = c[q];
-    }
+    for (int j = 0; j < J; ++j) buf[lane + 32 * j] = __fmul_rn(a[j], gather(c[j]));
   }
   __syncwarp();
-  // The sum of entry k's term q in order: an add of the staged product, or an FMA of the
-  // staged pair.
-  auto term = [&](int q, int k, T acc) {
-    return kProducts ? acc + bg[q * CH + k] : fma_t(bv[k], bg[q * CH + k], acc);
-  };
-  if (piece) {
-#pragma unroll
-    for (int q = 0; q < NP; ++q) {
-      T s = T(0);
-      for (int k = lane; k < n; k += 32) s = term(q, k, s);
-      const double d = warp_sum(static_cast<double>(s));
-      if (lane == 0) piece_part[(-ch.r1 - 1) * NP + q] = d;
-    }
-  } else {
-    const int L = chunk_lanes(R);
-    const int g = lane / L, sub = lane & (L - 1);
-    const int ra = __shfl_sync(0xffffffffu, pr, g & 31) - ch.k0;
-    const int re = __shfl_sync(0xffffffffu, pr, (g + 1) & 31) - ch.k0;
-    T s[NP];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) s[q] = T(0);
-    if (g < R) {
-      for (int k = ra + sub; k < re; k += L) {
-#pragma unroll
-        for (int q = 0; q < NP; ++q) s[q] = term(q, k, s[q]);
-      }
-    }
-    for (int o = L >> 1; o > 0; o >>= 1) {
-#pragma unroll
-      for (int q = 0; q < NP; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
-    }
-    T og[NR > 0 ? NR : 1];
-#pragma unroll
-    for (int q = 0; q < NR; ++q) og[q] = __shfl_sync(0xffffffffu, ops[q], g & 31);
-    if (OUTER) {
-#pragma unroll
-      for (int q = 0; q < NP; ++q) s[q] += __shfl_sync(0xffffffffu, out[q], g & 31);
-    }
-    if (g < R && sub == 0) epi(ch.r0 + g, s, og);
+  const int L = chunk_lanes(R);
+  const int g = lane / L, sub = lane & (L - 1);
+  const int ra = __shfl_sync(0xffffffffu, pr, g & 31) - ch.k0;
+  const int re = __shfl_sync(0xffffffffu, pr, (g + 1) & 31) - ch.k0;
+  float s[1] = {0.0f};
+  if (g < R) {
+#pragma unroll 4
+    for (int k = ra + sub; k < re; k += L) s[0] = s[0] + buf[k];
   }
+  for (int o = L >> 1; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+  float og[NR > 0 ? NR : 1];
+#pragma unroll
+  for (int q = 0; q < NR; ++q) og[q] = __shfl_sync(0xffffffffu, ops[q], g & 31);
+  if (OUTER) s[0] += __shfl_sync(0xffffffffu, out, g & 31);
+  if (g < R && sub == 0) epi(ch.r0 + g, s, og);
   __syncwarp();
+}
+
+// A piece of a long row: entries l, l + 32, ... per lane, products rounded before they are added.
+template <typename Gather>
+__device__ __forceinline__ void chunk_piece(const ChunkSet& cs, const Tile& ch, double* piece_part,
+                                            Gather gather) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  float s = 0.0f;
+#pragma unroll 4
+  for (int k = ch.k0 + lane; k < ch.k1; k += 32) {
+    s = __fadd_rn(s, __fmul_rn(ld_stream(cs.val + k), gather(ld_stream(cs.idx + k))));
+  }
+  const double d = warp_sum(static_cast<double>(s));
+  if (lane == 0) piece_part[-ch.r1 - 1] = d;
 }
 
 // The outer sums of a split layout's rows, for this block: in each round, every thread takes
 // outer entries e, e + blockDim, ... of the round's contiguous entry range (coalesced loads,
-// gathers from global memory) and stages their products (or pairs) in the warp buffers, then
+// gathers from global memory) and stages their products in the warp buffers at their places, then
 // every thread sums the rows r, r + blockDim, ... of the round in entry order into outer[r].
-// All threads call it; it ends with the block synchronised.
-template <int NP, typename T, typename G>
-__device__ __forceinline__ void outer_sums(const ChunkSet<T>& cs, const G* __restrict__ vec,
-                                           T* stage) {
-  constexpr bool kProducts = StageProducts<T>::value;
+// All threads call it; it ends with the block synchronised. An SM looks up about one line per clock,
+// and 32 random columns are 32 lines: by column, a warp's gathers fall on a few (1M x 2M
+// block-angular LP, 48% of the row pass's entries outside its windows: 79 us a pass in row order).
+__device__ __forceinline__ void outer_sums(const ChunkSet& cs, const float* __restrict__ vec,
+                                           float* stage) {
   const int B = static_cast<int>(blockDim.x);
   const int t = static_cast<int>(threadIdx.x);
   for (int q0 = cs.oround_start[blockIdx.x]; q0 < cs.oround_start[blockIdx.x + 1]; ++q0) {
     const int2 rr = cs.orounds[q0];
     const int e0 = __ldg(cs.optr + rr.x), e1 = __ldg(cs.optr + rr.y);
     const int count = e1 - e0;
-    // Stage: pairs put the value at [k] and component q at [(1 + q) * count + k]. A thread
-    // takes kOuterBatch entries at a time and issues all their index and value loads, then
-    // all their gathers, so it waits for two latencies per batch, not two per entry.
+    // A thread takes kOuterBatch entries at a time and issues all their index and value loads,
+    // then all their gathers, so it waits for two latencies per batch, not two per entry.
     constexpr int kOuterBatch = 8;
     for (int k0 = t; k0 < count; k0 += B * kOuterBatch) {
-      int ix[kOuterBatch];
-      T av[kOuterBatch];
+      int ix[kOuterBatch], at[kOuterBatch];
+      float av[kOuterBatch], g[kOuterBatch];
 #pragma unroll
       for (int u = 0; u < kOuterBatch; ++u) {
         const int k = k0 + u * B;
         ix[u] = k < count ? ld_stream(cs.oidx + e0 + k) : -1;
-        av[u] = k < count ? ld_stream(cs.oval + e0 + k) : T(0);
+        av[u] = k < count ? ld_stream(cs.oval + e0 + k) : 0.0f;
+        at[u] = k < count ? __ldg(cs.opos + e0 + k) : 0;
       }
-      G g[kOuterBatch];
 #pragma unroll
-      for (int u = 0; u < kOuterBatch; ++u) g[u] = ix[u] >= 0 ? __ldg(vec + ix[u]) : G{};
+      for (int u = 0; u < kOuterBatch; ++u) g[u] = ix[u] >= 0 ? __ldg(vec + ix[u]) : 0.0f;
 #pragma unroll
       for (int u = 0; u < kOuterBatch; ++u) {
         const int k = k0 + u * B;
         if (k >= count) break;
-        T c[NP];
-        split_gathered(g[u], c);
-        if (kProducts) {
-#pragma unroll
-          for (int q = 0; q < NP; ++q) stage[q * count + k] = av[u] * c[q];
-        } else {
-          stage[k] = av[u];
-#pragma unroll
-          for (int q = 0; q < NP; ++q) stage[(1 + q) * count + k] = c[q];
-        }
+        stage[at[u]] = __fmul_rn(av[u], g[u]);
       }
     }
     __syncthreads();
     for (int r = rr.x + t; r < rr.y; r += B) {
       const int a0 = __ldg(cs.optr + r) - e0, a1 = __ldg(cs.optr + r + 1) - e0;
-      T s[NP];
-#pragma unroll
-      for (int q = 0; q < NP; ++q) s[q] = T(0);
-      for (int k = a0; k < a1; ++k) {
-#pragma unroll
-        for (int q = 0; q < NP; ++q) {
-          s[q] = kProducts ? s[q] + stage[q * count + k]
-                           : fma_t(stage[k], stage[(1 + q) * count + k], s[q]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < NP; ++q) cs.outer[r * NP + q] = s[q];
+      float s = 0.0f;
+      for (int k = a0; k < a1; ++k) s = s + stage[k];
+      cs.outer[r] = s;
     }
     __syncthreads();
   }
 }
 
-template <bool OUTER, int NP, int NR, typename T, typename G, int CH, typename Load, typename Epi>
-__device__ __forceinline__ bool run_chunks_impl(const ChunkSet<T>& cs, const G* __restrict__ vec,
+template <bool NARROW, bool OUTER, int NR, typename Load, typename Epi>
+__device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float* __restrict__ vec,
                                                 unsigned char* dsmem, double* piece_part,
                                                 Load load, Epi epi) {
   __shared__ volatile int s_abort;
   const int W = static_cast<int>(blockDim.x) >> 5;
   const int warp = static_cast<int>(threadIdx.x) >> 5;
-  T* buf = reinterpret_cast<T*>(dsmem + warp * ChunkSmem<T, G, NP, CH>::kBufBytes);
-  uint64_t* winbar =
-      reinterpret_cast<uint64_t*>(dsmem + W * ChunkSmem<T, G, NP, CH>::kBufBytes);
-  G* win = reinterpret_cast<G*>(dsmem + W * ChunkSmem<T, G, NP, CH>::kBufBytes + 128);
+  float* buf = reinterpret_cast<float*>(dsmem + warp * kChunkBufBytes);
+  uint64_t* winbar = reinterpret_cast<uint64_t*>(dsmem + W * kChunkBufBytes);
+  float* win = reinterpret_cast<float*>(dsmem + W * kChunkBufBytes + 128);
   if (threadIdx.x == 0) {
     s_abort = 0;
     mbar_init(winbar, 1);
@@ -346,21 +312,28 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet<T>& cs, const G* 
   if (s0 < s1 && cs.segs[s0].len > 0 && threadIdx.x == 0) {
     const ChunkSeg sg = cs.segs[s0];
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(winbar, static_cast<uint32_t>(sg.len) * sizeof(G));
-    bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(G), winbar);
+    mbar_arrive_expect_tx(winbar, static_cast<uint32_t>(sg.len) * sizeof(float));
+    bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(float), winbar);
     pending = true;
   }
-  if (OUTER) outer_sums<NP>(cs, vec, reinterpret_cast<T*>(dsmem));
+  if (OUTER) outer_sums(cs, vec, reinterpret_cast<float*>(dsmem));
 
   for (int s = s0; s < s1; ++s) {
     const ChunkSeg sg = cs.segs[s];
+    // The warp's first chunk of the segment is on its way while the window is.
+    Tile ch{0, 0, 0, 0};
+    PackedEntries<NARROW> e;
+    if (sg.c0 + warp < sg.c1) {
+      if (NARROW) e.load(cs, sg.c0 + warp);
+      ch = cs.chunks[sg.c0 + warp];
+    }
     if (sg.len > 0) {
       if (s != s0) {
         __syncthreads();  // every warp is done with the slice held
         if (!s_abort && threadIdx.x == 0) {
           fence_proxy_async_smem();
-          mbar_arrive_expect_tx(winbar, static_cast<uint32_t>(sg.len) * sizeof(G));
-          bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(G), winbar);
+          mbar_arrive_expect_tx(winbar, static_cast<uint32_t>(sg.len) * sizeof(float));
+          bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(float), winbar);
           pending = true;
         }
       }
@@ -374,19 +347,28 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet<T>& cs, const G* 
       phase ^= 1u;
     }
     const int lo = sg.lo, len = sg.len;
-    auto gather = [&](int c) {
+    // Of column c, and of packed index c.
+    auto gather_column = [&](int c) {
       const unsigned o = static_cast<unsigned>(c - lo);
       return o < static_cast<unsigned>(len) ? win[o] : __ldg(vec + c);
     };
-    // The next chunk's record is loaded while this one is worked on: the stream loads of a
-    // chunk wait for its record.
-    Tile next = sg.c0 + warp < sg.c1 ? cs.chunks[sg.c0 + warp] : Tile{0, 0, 0, 0};
+    auto gather = [&](int c) { return NARROW ? win[c] : gather_column(c); };
     for (int c = sg.c0 + warp; c < sg.c1; c += W) {
       if (s_abort) break;
-      const Tile ch = next;
-      if (c + W < sg.c1) next = cs.chunks[c + W];
-      chunk_step<NP, NR, T, G, CH, OUTER>(cs.ptr, cs.idx, cs.val, ch, buf, cs.outer, piece_part,
-                                          gather, load, epi);
+      Tile next{0, 0, 0, 0};
+      PackedEntries<NARROW> ahead;
+      if (!NARROW) e.load(cs, c);
+      if (c + W < sg.c1) {
+        if (NARROW) ahead.load(cs, c + W);
+        next = cs.chunks[c + W];
+      }
+      if (ch.r1 < 0) {
+        chunk_piece(cs, ch, piece_part, gather_column);
+      } else {
+        chunk_step<NR, NARROW, OUTER>(cs.ptr, ch, e, buf, cs.outer, gather, load, epi);
+      }
+      ch = next;
+      if (NARROW) e = ahead;
     }
   }
   __syncthreads();
@@ -399,34 +381,31 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet<T>& cs, const G* 
 
 // Visit this block's chunks (kernel launched with a multiple of 32 threads, every thread
 // calls it). Returns false -- in every thread -- if a wait gave up.
-template <int NP, int NR, typename T, typename G, int CH, typename Load, typename Epi>
-__device__ __forceinline__ bool run_chunks(const ChunkSet<T>& cs, const G* __restrict__ vec,
+template <int NR, typename Load, typename Epi>
+__device__ __forceinline__ bool run_chunks(const ChunkSet& cs, const float* __restrict__ vec,
                                            unsigned char* dsmem, double* piece_part, Load load,
                                            Epi epi) {
+  if (cs.narrow) {
+    return cs.outer != nullptr
+               ? run_chunks_impl<true, true, NR>(cs, vec, dsmem, piece_part, load, epi)
+               : run_chunks_impl<true, false, NR>(cs, vec, dsmem, piece_part, load, epi);
+  }
   return cs.outer != nullptr
-             ? run_chunks_impl<true, NP, NR, T, G, CH>(cs, vec, dsmem, piece_part, load, epi)
-             : run_chunks_impl<false, NP, NR, T, G, CH>(cs, vec, dsmem, piece_part, load, epi);
+             ? run_chunks_impl<false, true, NR>(cs, vec, dsmem, piece_part, load, epi)
+             : run_chunks_impl<false, false, NR>(cs, vec, dsmem, piece_part, load, epi);
 }
 
 // Last block only: each long row combined from its piece partials in piece order (double),
 // then handed to the epilogue with its operands.
-template <int NP, int NR, typename T, typename Load, typename Epi>
-__device__ __forceinline__ void run_chunk_long_rows(const ChunkSet<T>& cs,
-                                                    const double* piece_part, Load load,
-                                                    Epi epi) {
+template <int NR, typename Load, typename Epi>
+__device__ __forceinline__ void run_chunk_long_rows(const ChunkSet& cs, const double* piece_part,
+                                                    Load load, Epi epi) {
   for (int l = threadIdx.x; l < cs.nlong; l += blockDim.x) {
     const LongRow lr = cs.longs[l];
-    double acc[NP];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) acc[q] = 0.0;
-    for (int c = 0; c < lr.nchunks; ++c) {
-#pragma unroll
-      for (int q = 0; q < NP; ++q) acc[q] += __ldcg(piece_part + (lr.chunk0 + c) * NP + q);
-    }
-    T s[NP];
-#pragma unroll
-    for (int q = 0; q < NP; ++q) s[q] = static_cast<T>(acc[q]);
-    T ops[NR > 0 ? NR : 1];
+    double acc = 0.0;
+    for (int c = 0; c < lr.nchunks; ++c) acc += __ldcg(piece_part + lr.chunk0 + c);
+    const float s[1] = {static_cast<float>(acc)};
+    float ops[NR > 0 ? NR : 1];
     load(lr.row, ops);
     epi(lr.row, s, ops);
   }

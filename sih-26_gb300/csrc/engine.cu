@@ -385,12 +385,28 @@ void Engine::allocate_mixed() {
   for (DeviceArray<double>* a : {&anchor_x_, &aty64_}) a->allocate(n);
   for (DeviceArray<double>* a : {&anchor_y_, &ax64_}) a->allocate(m);
   for (ChunkDev* D : {&ck_csc_f_, &ck_csr_f_}) {
+    const size_t places = static_cast<size_t>(D->nchunks) * kChunkCapF;
+    D->pval.allocate(places);
+    if (D->narrow) {
+      D->pidx16.allocate(places);
+    } else {
+      D->pidx32.allocate(places);
+    }
     if (!D->split) continue;
     D->fval.allocate_padded(static_cast<size_t>(D->nmain), kPad, s);
     D->foval.allocate_padded(static_cast<size_t>(D->nouter), kPad, s);
+    D->osorted.allocate(static_cast<size_t>(D->nouter) + 1);
+    D->opos.allocate(static_cast<size_t>(D->nouter) + 1);
+    D->fosorted.allocate(static_cast<size_t>(D->nouter) + 1);
+    launch_sort_outer(D->orounds.ptr, static_cast<int>(D->orounds.count), D->optr.ptr, D->oidx.ptr,
+                      D->osorted.ptr, D->opos.ptr, s);
     D->fouter.allocate_padded(static_cast<size_t>(D->nrows), kPad, s);
   }
   fill_mixed_buffers();
+  launch_pack_indices(mixed_.csc_k, ck_csc_f_.nchunks, ck_csc_f_.lo.ptr,
+                      const_cast<void*>(mixed_.csc_k.pidx), s);
+  launch_pack_indices(mixed_.csr_k, ck_csr_f_.nchunks, ck_csr_f_.lo.ptr,
+                      const_cast<void*>(mixed_.csr_k.pidx), s);
   mixed_ready_ = true;
 }
 
@@ -795,6 +811,13 @@ void Engine::plan_layout(ChunkDev& D, const std::vector<int>& lptr, const int* l
   D.coverage = P.coverage;
   D.smem = mixed_step_smem(pass, P.wmax);
   D.chunks.upload(P.chunks.data(), P.chunks.size(), s);
+  D.nchunks = static_cast<int>(P.chunks.size());
+  D.narrow = P.narrow;
+  if (D.narrow) {
+    D.lo.upload(P.lo.data(), P.lo.size(), s);
+  } else {
+    D.lo.release();
+  }
   D.longs.upload(P.longs.data(), P.longs.size(), s);
   D.segs.upload(P.segs.data(), P.segs.size(), s);
   D.seg_start.upload(P.seg_start.data(), P.seg_start.size(), s);
@@ -819,11 +842,17 @@ void Engine::plan_layout(ChunkDev& D, const std::vector<int>& lptr, const int* l
   D.fval.release();
   D.foval.release();
   D.fouter.release();
+  D.osorted.release();
+  D.opos.release();
+  D.fosorted.release();
+  D.pval.release();
+  D.pidx16.release();
+  D.pidx32.release();
 }
 
-ChunkSet<float> Engine::chunk_set(const ChunkDev& D, const int* full_ptr, const int* full_idx,
+ChunkSet Engine::chunk_set(const ChunkDev& D, const int* full_ptr, const int* full_idx,
                                   const float* full_val) const {
-  ChunkSet<float> c{};
+  ChunkSet c{};
   c.chunks = D.chunks.ptr;
   c.segs = D.segs.ptr;
   c.seg_start = D.seg_start.ptr;
@@ -832,15 +861,19 @@ ChunkSet<float> Engine::chunk_set(const ChunkDev& D, const int* full_ptr, const 
   c.npieces = D.npieces;
   c.nrows = D.nrows;
   c.wmax = D.wmax;
+  c.narrow = D.narrow ? 1 : 0;
+  c.pval = D.pval.ptr;
+  c.pidx = D.narrow ? static_cast<const void*>(D.pidx16.ptr) : static_cast<const void*>(D.pidx32.ptr);
   if (D.split) {
     c.ptr = D.ptr.ptr;
     c.idx = D.idx.ptr;
     c.optr = D.optr.ptr;
-    c.oidx = D.oidx.ptr;
+    c.oidx = D.osorted.ptr;
     c.orounds = D.orounds.ptr;
     c.oround_start = D.oround_start.ptr;
     c.val = D.fval.ptr;
-    c.oval = D.foval.ptr;
+    c.oval = D.fosorted.ptr;
+    c.opos = D.opos.ptr;
     c.outer = D.fouter.ptr;
   } else {
     c.ptr = full_ptr;
@@ -989,7 +1022,8 @@ void Engine::unslice_scaled() {
 }
 
 // The FP32 scaled values of the split chunk layouts' main and outer parts, gathered from the
-// full layouts' FP64 scaled values (each mixed solve, after the preconditioning).
+// full layouts' FP64 scaled values, and both layouts' packed values (each mixed solve, after the
+// preconditioning and the full layouts' FP32 copies).
 void Engine::fill_split_values() {
   cudaStream_t s = stream_;
   const std::pair<ChunkDev*, const double*> layouts[] = {{&ck_csc_f_, csc_s_.ptr},
@@ -999,7 +1033,11 @@ void Engine::fill_split_values() {
     if (!D.split) continue;
     launch_gather_values(l.second, D.map.ptr, D.fval.ptr, D.nmain, s);
     launch_gather_values(l.second, D.omap.ptr, D.foval.ptr, D.nouter, s);
+    launch_sort_outer_values(D.orounds.ptr, static_cast<int>(D.orounds.count), D.optr.ptr,
+                             D.opos.ptr, D.foval.ptr, D.fosorted.ptr, s);
   }
+  launch_pack_values(mixed_.csc_k, ck_csc_f_.nchunks, ck_csc_f_.pval.ptr, s);
+  launch_pack_values(mixed_.csr_k, ck_csr_f_.nchunks, ck_csr_f_.pval.ptr, s);
 }
 
 // The power iteration's start vector: the reference's own std::mt19937(seed) +

@@ -153,7 +153,16 @@ class Engine {
     DeviceArray<int> seg_start, oround_start;
     DeviceArray<int> ptr, idx, map, optr, oidx, omap;
     DeviceArray<float> fval, foval, fouter;
-    DeviceArray<double> pieces;  // piece partials (NP per piece)
+    DeviceArray<int> osorted;  // the outer entries by column within a round,
+    DeviceArray<unsigned short> opos;  // their places in the order of the rows
+    DeviceArray<float> fosorted;
+    DeviceArray<double> pieces;  // piece partials
+    // Packed entries, allocated and filled when the mixed method first runs; the values each solve.
+    DeviceArray<float> pval;
+    DeviceArray<unsigned short> pidx16;
+    DeviceArray<int> pidx32, lo;
+    bool narrow = false;
+    int nchunks = 0;
     int nlong = 0, npieces = 0, wmax = 0, grid = 1, smem = 0, nrows = 0;
     bool split = false;
     long long nmain = 0, nouter = 0;
@@ -164,7 +173,7 @@ class Engine {
   void plan_layout(ChunkDev& D, const std::vector<int>& ptr, const int* idx, int lines,
                    int extent, int pass, int window_cap);
   void fill_split_values();
-  ChunkSet<float> chunk_set(const ChunkDev& D, const int* full_ptr, const int* full_idx,
+  ChunkSet chunk_set(const ChunkDev& D, const int* full_ptr, const int* full_idx,
                             const float* full_val) const;
 
   // Pattern (shared by scaled and unscaled values).
@@ -263,6 +272,9 @@ struct ChunkPlan {
   std::vector<ChunkSeg> segs;
   std::vector<int> seg_start, oround_start;
   std::vector<int> ptr, idx, map, optr, oidx, omap;  // split layouts only
+  // The windows hold every entry of the (main) chunks of whole rows; lo: their starts by chunk.
+  bool narrow = false;
+  std::vector<int> lo;
 };
 ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, int extent, int cap,
                       int wmax, int grid, int elem_bytes, double split_min, double full_min,

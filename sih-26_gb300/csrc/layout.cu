@@ -298,6 +298,14 @@ ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, in
     }
   }
   p.seg_start[G] = static_cast<int>(p.segs.size());
+  p.lo.assign(static_cast<size_t>(T), 0);
+  p.narrow = p.wmax > 0 && p.wmax <= 65536 && (p.split || covered == nnz);
+  for (const ChunkSeg& sg : p.segs) {
+    for (int c = sg.c0; c < sg.c1; ++c) {
+      p.lo[static_cast<size_t>(c)] = sg.lo;
+      if (p.chunks[static_cast<size_t>(c)].r1 >= 0 && sg.len <= 0) p.narrow = false;
+    }
+  }
   // Outer rounds: block b sums the outer entries of rows [row_begin[b], row_begin[b + 1]),
   // where row_begin[b] is the first row of its first chunk. Its main chunks lie inside that
   // range (a piece of a long row may not, but pieces read no outer sum), and every row of it

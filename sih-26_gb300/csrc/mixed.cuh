@@ -30,7 +30,7 @@ namespace sgb {
 struct MixedBuffers {
   Ctl* ctl;                  // the inner loop's control block
   TileSet<float> csc, csr;   // scaled values in FP32 (evaluation tile layouts)
-  ChunkSet<float> csc_k, csr_k;  // the step passes' chunk layouts
+  ChunkSet csc_k, csr_k;  // the step passes' chunk layouts
   float* u[2];
   float* v[2];
   float* u_sum;
@@ -96,6 +96,17 @@ void launch_round_build(const RoundBuffers& r, cudaStream_t s);
 // xbar += u_best / dp (clamped to the box), ybar += v_best / dd; best_x = xbar Dc,
 // best_y = ybar Dr for the exact evaluation.
 void launch_round_update(const RoundBuffers& r, cudaStream_t s);
+// The packed entries of a layout's `count` chunks (chunks.cuh): the indices (lo: the chunks' windows'
+// starts, read where cs.narrow), once per load, and the values, once per solve.
+void launch_pack_indices(const ChunkSet& cs, int count, const int* lo, void* out, cudaStream_t s);
+void launch_pack_values(const ChunkSet& cs, int count, float* out, cudaStream_t s);
+// A split layout's outer entries by column within each round (chunks.cuh): columns and places once per
+// load, values once per solve.
+void launch_sort_outer(const int2* rounds, int nrounds, const int* optr, const int* oidx, int* out,
+                       unsigned short* opos, cudaStream_t s);
+void launch_sort_outer_values(const int2* rounds, int nrounds, const int* optr,
+                              const unsigned short* opos, const float* val, float* out,
+                              cudaStream_t s);
 void launch_to_float(const double* src, float* dst, long long count, cudaStream_t s);
 void launch_fill_float(float* v, int count, float value, cudaStream_t s);
 // Sets the dynamic shared-memory limits of the FP32 kernels on the current device (once per

@@ -29,9 +29,6 @@ constexpr int kChunkScratch = 2 * (kChunkThreads / 32);
 // for them).
 using EvalPipeF = TilePipe<float, 2, 0, kWideThreads>;
 constexpr int kSmemF = EvalPipeF::bytes();
-// The step passes' chunk geometry: 256 entries per chunk, one gathered float per entry (v in
-// the column pass, du in the row pass).
-using StepSmemF = ChunkSmem<float, float, 1, kChunkCapF>;
 
 // A value formed by thread 0 and handed to every thread of the block (all threads call it).
 template <typename F>
@@ -93,7 +90,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
     b.du[j] = d;
     mvf = fmaf(d, d, mvf);
   };
-  if (!run_chunks<1, 5, float, float, kChunkCapF>(b.csc_k, v, dsmem, b.piece_primal, load,
+  if (!run_chunks<5>(b.csc_k, v, dsmem, b.piece_primal, load,
                                                   epi) &&
       threadIdx.x == 0) {
     raise_error(ctl);
@@ -110,7 +107,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
   }
   if (!arrive_last<1>(mv, scratch, b.part_primal, &ctl->ticket[kTicketPrimal])) return;
   mvf = 0.0f;
-  run_chunk_long_rows<1, 5, float>(b.csc_k, b.piece_primal, load, epi);
+  run_chunk_long_rows<5>(b.csc_k, b.piece_primal, load, epi);
   mv[0] = static_cast<double>(mvf);
   double longs[1], total[1];
   block_sum<1>(mv, scratch, longs);
@@ -177,7 +174,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
     a0 = fmaf(d, d, a0);
     a1 = fmaf(d, adu, a1);
   };
-  if (!run_chunks<1, 6, float, float, kChunkCapF>(b.csr_k, b.du, dsmem, b.piece_dual, load,
+  if (!run_chunks<6>(b.csr_k, b.du, dsmem, b.piece_dual, load,
                                                   epi) &&
       threadIdx.x == 0) {
     raise_error(ctl);
@@ -185,7 +182,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
   double acc2[2] = {static_cast<double>(a0), static_cast<double>(a1)};
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
   a0 = a1 = 0.0f;
-  run_chunk_long_rows<1, 6, float>(b.csr_k, b.piece_dual, load, epi);
+  run_chunk_long_rows<6>(b.csr_k, b.piece_dual, load, epi);
   acc2[0] = a0;
   acc2[1] = a1;
   double longs[2], total[2];
@@ -539,6 +536,85 @@ __global__ void k_fill_float(float* v, int count, float value) {
   for (int k = grid_stride_begin(); k < count; k += gridDim.x * blockDim.x) v[k] = value;
 }
 
+// The packed entries of a chunk layout (chunks.cuh), a warp per chunk: the indices (narrow ones from
+// their window's start, lo[chunk]) and the values. Lane l's entry j of chunk c is at
+// packed_place(c, l, j): values and 32-bit indices in two runs of four a lane, narrow ones in one of
+// eight.
+__device__ __forceinline__ size_t packed_place(int c, int lane, int j) {
+  return static_cast<size_t>(c) * kChunkCapF + (j >> 2) * 128 + lane * 4 + (j & 3);
+}
+
+template <typename I>
+__global__ void k_pack_indices(const Tile* chunks, int count, const int* lo, const int* idx, I* out) {
+  const int c = static_cast<int>(blockIdx.x) * 8 + static_cast<int>(threadIdx.x >> 5);
+  if (c >= count) return;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const Tile ch = chunks[c];
+  const int n = ch.r1 < 0 ? 0 : ch.k1 - ch.k0;
+  const int from = sizeof(I) == 2 ? lo[c] : 0;
+  for (int j = 0; j < kChunkCapF / 32; ++j) {
+    const int k = lane + 32 * j;
+    const I at = k < n ? static_cast<I>(idx[ch.k0 + k] - from) : I(0);
+    out[sizeof(I) == 2 ? static_cast<size_t>(c) * kChunkCapF + lane * 8 + j
+                       : packed_place(c, lane, j)] = at;
+  }
+}
+
+__global__ void k_pack_values(const Tile* chunks, int count, const float* val, float* out) {
+  const int c = static_cast<int>(blockIdx.x) * 8 + static_cast<int>(threadIdx.x >> 5);
+  if (c >= count) return;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const Tile ch = chunks[c];
+  const int n = ch.r1 < 0 ? 0 : ch.k1 - ch.k0;
+  for (int j = 0; j < kChunkCapF / 32; ++j) {
+    const int k = lane + 32 * j;
+    out[packed_place(c, lane, j)] = k < n ? val[ch.k0 + k] : 0.0f;
+  }
+}
+
+// The outer entries of a round by column (chunks.cuh): a block's bitonic sort of (column, place).
+constexpr int kSortThreads = 512;
+__global__ void __launch_bounds__(kSortThreads) k_sort_outer(const int2* rounds, const int* optr,
+                                                             const int* oidx, int* out,
+                                                             unsigned short* opos) {
+  extern __shared__ unsigned long long keys[];
+  const int2 rr = rounds[blockIdx.x];
+  const int e0 = optr[rr.x], count = optr[rr.y] - e0;
+  int size = 2;
+  while (size < count) size *= 2;
+  for (int k = static_cast<int>(threadIdx.x); k < size; k += kSortThreads) {
+    keys[k] = k < count ? (static_cast<unsigned long long>(oidx[e0 + k]) << 16) | k : ~0ull;
+  }
+  __syncthreads();
+  for (int run = 2; run <= size; run *= 2) {
+    for (int gap = run / 2; gap > 0; gap /= 2) {
+      for (int k = static_cast<int>(threadIdx.x); k < size / 2; k += kSortThreads) {
+        const int i = 2 * k - (k & (gap - 1)), j = i + gap;
+        const unsigned long long a = keys[i], b = keys[j];
+        if ((a > b) == ((i & run) == 0)) {
+          keys[i] = b;
+          keys[j] = a;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int k = static_cast<int>(threadIdx.x); k < count; k += kSortThreads) {
+    out[e0 + k] = static_cast<int>(keys[k] >> 16);
+    opos[e0 + k] = static_cast<unsigned short>(keys[k] & 0xffffull);
+  }
+}
+
+// The outer values in that order, from those in the order of the rows.
+__global__ void k_sort_outer_values(const int2* rounds, const int* optr, const unsigned short* opos,
+                                    const float* val, float* out) {
+  const int2 rr = rounds[blockIdx.x];
+  const int e0 = optr[rr.x], count = optr[rr.y] - e0;
+  for (int k = static_cast<int>(threadIdx.x); k < count; k += static_cast<int>(blockDim.x)) {
+    out[e0 + k] = val[e0 + opos[e0 + k]];
+  }
+}
+
 int egrid(long long count) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -614,13 +690,13 @@ int mixed_window_capacity(int pass) {
   const void* k = pass == 0 ? reinterpret_cast<const void*>(k_primal_f)
                             : reinterpret_cast<const void*>(k_dual_f);
   const int budget =
-      std::min(max_dynamic_smem(k) - StepSmemF::bytes(kChunkThreads / 32, 0), kWindowBytesMax);
+      std::min(max_dynamic_smem(k) - chunk_smem(kChunkThreads / 32, 0), kWindowBytesMax);
   return budget > 0 ? (budget / static_cast<int>(sizeof(float))) & ~1023 : 0;
 }
 
 int mixed_step_smem(int pass, int wmax) {
   (void)pass;
-  return StepSmemF::bytes(kChunkThreads / 32, wmax);
+  return chunk_smem(kChunkThreads / 32, wmax);
 }
 
 // The two step passes are launched with programmatic stream serialization (launch_after):
@@ -656,6 +732,38 @@ void launch_round_build(const RoundBuffers& r, cudaStream_t s) {
 
 void launch_round_update(const RoundBuffers& r, cudaStream_t s) {
   k_round_update<<<egrid(r.m > r.n ? r.m : r.n), 256, 0, s>>>(r);
+}
+
+void launch_pack_indices(const ChunkSet& cs, int count, const int* lo, void* out, cudaStream_t s) {
+  if (count <= 0) return;
+  if (cs.narrow) {
+    k_pack_indices<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, lo, cs.idx,
+                                                   static_cast<unsigned short*>(out));
+  } else {
+    k_pack_indices<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, lo, cs.idx,
+                                                   static_cast<int*>(out));
+  }
+}
+
+void launch_pack_values(const ChunkSet& cs, int count, float* out, cudaStream_t s) {
+  if (count <= 0) return;
+  k_pack_values<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, cs.val, out);
+}
+
+void launch_sort_outer(const int2* rounds, int nrounds, const int* optr, const int* oidx, int* out,
+                       unsigned short* opos, cudaStream_t s) {
+  if (nrounds <= 0) return;
+  constexpr int kBytes = (kChunkThreads / 32) * kChunkCapF * static_cast<int>(sizeof(unsigned long long));
+  // A failure here stays the last error, which the caller's launch check reports.
+  cudaFuncSetAttribute(k_sort_outer, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
+  k_sort_outer<<<nrounds, kSortThreads, kBytes, s>>>(rounds, optr, oidx, out, opos);
+}
+
+void launch_sort_outer_values(const int2* rounds, int nrounds, const int* optr,
+                              const unsigned short* opos, const float* val, float* out,
+                              cudaStream_t s) {
+  if (nrounds <= 0) return;
+  k_sort_outer_values<<<nrounds, 256, 0, s>>>(rounds, optr, opos, val, out);
 }
 
 void launch_to_float(const double* src, float* dst, long long count, cudaStream_t s) {
