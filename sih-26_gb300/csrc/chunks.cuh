@@ -185,7 +185,7 @@ struct PackedEntries {
 template <int NR, bool NARROW, bool OUTER, typename Gather, typename Load, typename Epi>
 __device__ __forceinline__ void chunk_step(const int* __restrict__ ptr, const Tile& ch,
                                            const PackedEntries<NARROW>& e, float* buf,
-                                           const float* __restrict__ outer, Gather gather,
+                                           const float* outer, Gather gather,
                                            Load load, Epi epi) {
   constexpr int J = kChunkCapF / 32;
   const int lane = static_cast<int>(threadIdx.x) & 31;
@@ -246,8 +246,14 @@ __device__ __forceinline__ void chunk_piece(const ChunkSet& cs, const Tile& ch, 
 // All threads call it; it ends with the block synchronised. An SM looks up about one line per clock,
 // and 32 random columns are 32 lines: by column, a warp's gathers fall on a few (1M x 2M
 // block-angular LP, 48% of the row pass's entries outside its windows: 79 us a pass in row order).
-__device__ __forceinline__ void outer_sums(const ChunkSet& cs, const float* __restrict__ vec,
-                                           float* stage) {
+// LIVE: the running kernel writes the vector (ld_live).
+template <bool LIVE>
+__device__ __forceinline__ float element(const float* p) {
+  return LIVE ? ld_live(p) : __ldg(p);
+}
+
+template <bool LIVE>
+__device__ __forceinline__ void outer_sums(const ChunkSet& cs, const float* vec, float* stage) {
   const int B = static_cast<int>(blockDim.x);
   const int t = static_cast<int>(threadIdx.x);
   for (int q0 = cs.oround_start[blockIdx.x]; q0 < cs.oround_start[blockIdx.x + 1]; ++q0) {
@@ -268,7 +274,7 @@ __device__ __forceinline__ void outer_sums(const ChunkSet& cs, const float* __re
         at[u] = k < count ? __ldg(cs.opos + e0 + k) : 0;
       }
 #pragma unroll
-      for (int u = 0; u < kOuterBatch; ++u) g[u] = ix[u] >= 0 ? __ldg(vec + ix[u]) : 0.0f;
+      for (int u = 0; u < kOuterBatch; ++u) g[u] = ix[u] >= 0 ? element<LIVE>(vec + ix[u]) : 0.0f;
 #pragma unroll
       for (int u = 0; u < kOuterBatch; ++u) {
         const int k = k0 + u * B;
@@ -287,8 +293,22 @@ __device__ __forceinline__ void outer_sums(const ChunkSet& cs, const float* __re
   }
 }
 
-template <bool NARROW, bool OUTER, int NR, typename Load, typename Epi>
-__device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float* __restrict__ vec,
+// Starts a window's copy (thread 0). What the block has read of the buffer, and in a LIVE kernel what
+// others wrote of the vector, comes before it.
+template <bool LIVE>
+__device__ __forceinline__ void copy_window(float* win, const float* vec, const ChunkSeg& sg,
+                                            uint64_t* bar) {
+  if (LIVE) {
+    asm volatile("fence.proxy.async;" ::: "memory");
+  } else {
+    fence_proxy_async_smem();
+  }
+  mbar_arrive_expect_tx(bar, static_cast<uint32_t>(sg.len) * sizeof(float));
+  bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(float), bar);
+}
+
+template <bool LIVE, bool NARROW, bool OUTER, int NR, typename Load, typename Epi>
+__device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float* vec,
                                                 unsigned char* dsmem, double* piece_part,
                                                 Load load, Epi epi) {
   __shared__ volatile int s_abort;
@@ -310,13 +330,10 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
   // The first window copy is issued at once; a split layout sums its outer entries while it
   // is in flight.
   if (s0 < s1 && cs.segs[s0].len > 0 && threadIdx.x == 0) {
-    const ChunkSeg sg = cs.segs[s0];
-    fence_proxy_async_smem();
-    mbar_arrive_expect_tx(winbar, static_cast<uint32_t>(sg.len) * sizeof(float));
-    bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(float), winbar);
+    copy_window<LIVE>(win, vec, cs.segs[s0], winbar);
     pending = true;
   }
-  if (OUTER) outer_sums(cs, vec, reinterpret_cast<float*>(dsmem));
+  if (OUTER) outer_sums<LIVE>(cs, vec, reinterpret_cast<float*>(dsmem));
 
   for (int s = s0; s < s1; ++s) {
     const ChunkSeg sg = cs.segs[s];
@@ -331,9 +348,7 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
       if (s != s0) {
         __syncthreads();  // every warp is done with the slice held
         if (!s_abort && threadIdx.x == 0) {
-          fence_proxy_async_smem();
-          mbar_arrive_expect_tx(winbar, static_cast<uint32_t>(sg.len) * sizeof(float));
-          bulk_copy_g2s(win, vec + sg.lo, static_cast<uint32_t>(sg.len) * sizeof(float), winbar);
+          copy_window<LIVE>(win, vec, sg, winbar);
           pending = true;
         }
       }
@@ -350,7 +365,7 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
     // Of column c, and of packed index c.
     auto gather_column = [&](int c) {
       const unsigned o = static_cast<unsigned>(c - lo);
-      return o < static_cast<unsigned>(len) ? win[o] : __ldg(vec + c);
+      return o < static_cast<unsigned>(len) ? win[o] : element<LIVE>(vec + c);
     };
     auto gather = [&](int c) { return NARROW ? win[c] : gather_column(c); };
     for (int c = sg.c0 + warp; c < sg.c1; c += W) {
@@ -362,7 +377,7 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
         if (NARROW) ahead.load(cs, c + W);
         next = cs.chunks[c + W];
       }
-      if (ch.r1 < 0) {
+      if (!LIVE && ch.r1 < 0) {
         chunk_piece(cs, ch, piece_part, gather_column);
       } else {
         chunk_step<NR, NARROW, OUTER>(cs.ptr, ch, e, buf, cs.outer, gather, load, epi);
@@ -372,27 +387,39 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
     }
   }
   __syncthreads();
-  if (!s_abort) return true;
-  // A window copy still in flight must land before the block exits (bounded).
-  if (threadIdx.x == 0 && pending) mbar_wait_bounded(winbar, phase ^ 1u);
+  const bool ok = s_abort == 0;
+  // A window copy still in flight must land before the block exits (bounded). The next pass of the
+  // kernel initialises the barrier again.
+  if (threadIdx.x == 0) {
+    if (!ok && pending) mbar_wait_bounded(winbar, phase ^ 1u);
+    if (ok) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(winbar)) : "memory");
+  }
   __syncthreads();
-  return false;
+  return ok;
 }
 
 // Visit this block's chunks (kernel launched with a multiple of 32 threads, every thread
 // calls it). Returns false -- in every thread -- if a wait gave up.
 template <int NR, typename Load, typename Epi>
-__device__ __forceinline__ bool run_chunks(const ChunkSet& cs, const float* __restrict__ vec,
+__device__ __forceinline__ bool run_chunks(const ChunkSet& cs, const float* vec,
                                            unsigned char* dsmem, double* piece_part, Load load,
                                            Epi epi) {
   if (cs.narrow) {
     return cs.outer != nullptr
-               ? run_chunks_impl<true, true, NR>(cs, vec, dsmem, piece_part, load, epi)
-               : run_chunks_impl<true, false, NR>(cs, vec, dsmem, piece_part, load, epi);
+               ? run_chunks_impl<false, true, true, NR>(cs, vec, dsmem, piece_part, load, epi)
+               : run_chunks_impl<false, true, false, NR>(cs, vec, dsmem, piece_part, load, epi);
   }
   return cs.outer != nullptr
-             ? run_chunks_impl<false, true, NR>(cs, vec, dsmem, piece_part, load, epi)
-             : run_chunks_impl<false, false, NR>(cs, vec, dsmem, piece_part, load, epi);
+             ? run_chunks_impl<false, false, true, NR>(cs, vec, dsmem, piece_part, load, epi)
+             : run_chunks_impl<false, false, false, NR>(cs, vec, dsmem, piece_part, load, epi);
+}
+
+// The same in a kernel that writes the vector itself, for layouts of narrow indices without pieces or
+// outer entries.
+template <int NR, typename Load, typename Epi>
+__device__ __forceinline__ bool run_whole_chunks(const ChunkSet& cs, const float* vec,
+                                                 unsigned char* dsmem, Load load, Epi epi) {
+  return run_chunks_impl<true, true, false, NR>(cs, vec, dsmem, nullptr, load, epi);
 }
 
 // Last block only: each long row combined from its piece partials in piece order (double),

@@ -65,6 +65,19 @@ __device__ inline double2 step_factors(long long iteration, const double2* table
   return (table != nullptr && e < n) ? table[e] : step_factors(e);
 }
 
+// The sum of get(0) .. get(n - 1) over a warp, in every lane: up to five per lane are read at once
+// and added as a tree, so 152 of them cost one latency and eight dependent additions.
+template <typename Get>
+__device__ __forceinline__ double table_sum(int n, Get get) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  double v[5];
+#pragma unroll
+  for (int u = 0; u < 5; ++u) v[u] = lane + 32 * u < n ? get(lane + 32 * u) : 0.0;
+  double sum = ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+  for (int k = lane + 160; k < n; k += 32) sum += get(k);
+  return warp_sum(sum);
+}
+
 // The projection of v / sigma on [rl, ru]. On an equality row it is the bound whatever v is.
 __device__ __forceinline__ double row_projection(double v, double sigma, double inv_sigma, double rl,
                                                  double ru) {

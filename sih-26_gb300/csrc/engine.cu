@@ -402,7 +402,10 @@ void Engine::allocate_mixed() {
                       D->osorted.ptr, D->opos.ptr, s);
     D->fouter.allocate_padded(static_cast<size_t>(D->nrows), kPad, s);
   }
+  scaled_norms_.allocate(static_cast<size_t>(scaled_norms_size()));
+  part_steps_f_.allocate(3 * static_cast<size_t>(std::max(ck_csc_f_.grid, ck_csr_f_.grid)));
   fill_mixed_buffers();
+  steps_f_ = mixed_steps_fit(mixed_);
   launch_pack_indices(mixed_.csc_k, ck_csc_f_.nchunks, ck_csc_f_.lo.ptr,
                       const_cast<void*>(mixed_.csc_k.pidx), s);
   launch_pack_indices(mixed_.csr_k, ck_csr_f_.nchunks, ck_csr_f_.lo.ptr,
@@ -447,6 +450,8 @@ void Engine::fill_mixed_buffers() {
   b.step_factors_n = kStepFactorTable;
   b.part_primal = part_primal_.ptr;
   b.part_dual = part_dual_.ptr;
+  b.part_steps = part_steps_f_.ptr;
+  b.arrivals = arrivals_.ptr + 1;
   b.csc_k = chunk_set(ck_csc_f_, csc_ptr_.ptr, csc_idx_.ptr, csc_f_.ptr);
   b.csr_k = chunk_set(ck_csr_f_, csr_ptr_.ptr, csr_idx_.ptr, csr_f_.ptr);
   b.piece_primal = ck_csc_f_.pieces.ptr;
@@ -475,9 +480,20 @@ void Engine::build_mixed_graphs(int steps) {
   for (int slot = 0; slot < 2; ++slot) {
     cudaGraph_t graph = nullptr;
     SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < steps; ++k) {
-      launch_mixed_step(mixed_, stream_);
-      if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_mixed_evaluation(mixed_, stream_);
+    if (steps_f_) {
+      // The kernel ends where an evaluation falls due, at most 40 accepted steps on.
+      mgraph_launches_ = 0;
+      for (int k = 0; k < steps; k += kResidentAttempts) {
+        launch_mixed_steps(mixed_, std::min(kResidentAttempts, steps - k), stream_);
+        launch_mixed_evaluation(mixed_, stream_);
+        mgraph_launches_ += 5;
+      }
+    } else {
+      for (int k = 0; k < steps; ++k) {
+        launch_mixed_step(mixed_, stream_);
+        if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_mixed_evaluation(mixed_, stream_);
+      }
+      mgraph_launches_ = graph_kernel_launches(steps);
     }
     cudaMemcpyAsync(snapshot_mixed_ + slot, ctl_mixed_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost,
                     stream_);
@@ -705,7 +721,7 @@ void Engine::load(const sankhya_gb300_lp& lp) {
                                  2 * sl_csc_.view.nlong + sl_csr_.view.nlong);
   part_steps_.allocate(step_parts);
   SGB_CUDA(cudaMemsetAsync(part_steps_.ptr, 0, step_parts * sizeof(double), s));
-  arrivals_.allocate(1);
+  arrivals_.allocate(2);  // FP64 and mixed
   tickets_.allocate(4);
   SGB_CUDA(cudaMemsetAsync(tickets_.ptr, 0, 4 * sizeof(unsigned int), s));
   SGB_CUDA(cudaStreamSynchronize(s));
@@ -1167,7 +1183,6 @@ void Engine::init_iterates(const sankhya_gb300_params& p) {
   launch_fill(y_sum_.ptr, m_, 0.0, s);
   launch_fill(y_rst_.ptr, m_, 0.0, s);
   launch_fill(best_y_.ptr, m_, 0.0, s);
-  SGB_CUDA(cudaMemsetAsync(arrivals_.ptr, 0, sizeof(unsigned long long), s));
   if (n_ > 0) {
     SGB_CUDA(cudaMemcpyAsync(x_rst_.ptr, x0_.ptr, n_ * sizeof(double), cudaMemcpyDeviceToDevice, s));
     // best_x starts as the SCALED start point, as the reference's does (pdhg.cpp:190).
@@ -1274,6 +1289,7 @@ void Engine::final_evaluation() {
 void Engine::setup(const sankhya_gb300_params& p, sankhya_gb300_result* r, double* norm) {
   Trace trace("pdhg scaling");
   cudaStream_t s = stream_;
+  SGB_CUDA(cudaMemsetAsync(arrivals_.ptr, 0, 2 * sizeof(unsigned long long), s));
   *norm = scale_and_norm(p.random_seed);
   double mm[2] = {0.0, 0.0};
   SGB_CUDA(cudaMemcpyAsync(mm, minmax_.ptr + 2 * scale_blocks(sl_csc_.view), 2 * sizeof(double),
@@ -1425,32 +1441,20 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
   launch_project_start(n_, ls_.ptr, us_.ptr, anchor_x_.ptr, s);
   launch_fill(anchor_y_.ptr, m_, 0.0, s);
   extra_launches_ += 2;
-  {
-    // The scaled problem's norms, for the inner loop's relative residuals.
-    std::vector<double> h(static_cast<size_t>(std::max(m_, n_)));
-    double bs = 0.0, cs2 = 0.0;
-    std::vector<double> rl(static_cast<size_t>(m_)), ru(static_cast<size_t>(m_));
-    if (m_ > 0) {
-      SGB_CUDA(cudaMemcpyAsync(rl.data(), rls_.ptr, m_ * sizeof(double), cudaMemcpyDeviceToHost, s));
-      SGB_CUDA(cudaMemcpyAsync(ru.data(), rus_.ptr, m_ * sizeof(double), cudaMemcpyDeviceToHost, s));
-    }
-    if (n_ > 0) {
-      SGB_CUDA(cudaMemcpyAsync(h.data(), cs_.ptr, n_ * sizeof(double), cudaMemcpyDeviceToHost, s));
-    }
-    SGB_CUDA(cudaStreamSynchronize(s));
-    for (int i = 0; i < m_; ++i) {
-      const double b = !std::isinf(rl[i]) ? rl[i] : (!std::isinf(ru[i]) ? ru[i] : 0.0);
-      bs += b * b;
-    }
-    for (int j = 0; j < n_; ++j) cs2 += h[j] * h[j];
-    bound_norm_s_ = std::sqrt(bs);
-    cost_norm_s_ = std::sqrt(cs2);
-  }
+  // The scaled problem's norms, for the inner loop's relative residuals.
+  launch_scaled_norms(m_, n_, cs_.ptr, rls_.ptr, rus_.ptr, scaled_norms_.ptr, s);
+  extra_launches_ += 2;
+  double squares[2] = {0.0, 0.0};
+  SGB_CUDA(cudaMemcpyAsync(squares, scaled_norms_.ptr + scaled_norms_size() - 2, sizeof(squares),
+                           cudaMemcpyDeviceToHost, s));
+  SGB_CUDA(cudaStreamSynchronize(s));
+  cost_norm_s_ = std::sqrt(squares[0]);
+  bound_norm_s_ = std::sqrt(squares[1]);
   const double t_loop = now_seconds();
   r->setup_seconds = t_loop - t0;
   const long long launches_setup = kernel_launch_count() - launches_before;
 
-  const int steps = p.steps_per_poll > 0 ? p.steps_per_poll : 32;
+  const int steps = p.steps_per_poll > 0 ? p.steps_per_poll : (steps_f_ ? kResidentAttempts : 32);
   build_mixed_graphs(steps);
   const long long limit = p.iteration_limit < 0 ? 1000000 : p.iteration_limit;
   const double inf = std::numeric_limits<double>::infinity();
@@ -1614,7 +1618,7 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
   SGB_CUDA(cudaEventElapsedTime(&device_ms, timing_[0], timing_[1]));
   r->device_seconds = 1e-3 * device_ms;
   launches_ = launches_setup + extra_launches_ +
-              graphs_launched_ * graph_kernel_launches(mgraph_steps_);
+              graphs_launched_ * mgraph_launches_;
   r->kernel_launches = launches_;
   r->staged_fraction[0] = ck_csc_f_.staged;
   r->staged_fraction[1] = ck_csr_f_.staged;

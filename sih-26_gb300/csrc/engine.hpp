@@ -206,7 +206,9 @@ class Engine {
   int graph_steps_ = 0;
   int graph_launches_ = 0;  // engine kernels per step graph
   bool steps_ = false;      // FP64 steps run in launch_pdhg_steps' kernel
-  DeviceArray<double> part_steps_;
+  DeviceArray<double> part_steps_, part_steps_f_, scaled_norms_;
+  bool steps_f_ = false;    // the mixed method's steps run in launch_mixed_steps' kernel
+  int mgraph_launches_ = 0;
   DeviceArray<unsigned long long> arrivals_;
   bool resident_ = false;   // FP64 steps run in the resident kernel,
   int resident_smem_ = 0;   // with this much shared memory a block

@@ -52,6 +52,8 @@ struct MixedBuffers {
   float* v_best;
   double* part_primal;   // [grid_primal]
   double* part_dual;     // [grid_dual * 2]
+  double* part_steps;    // [3 * the larger step grid] (k_steps_f)
+  unsigned long long* arrivals;  // GridMeet's counter
   double* piece_primal;  // [csc_k.npieces]
   double* piece_dual;    // [csr_k.npieces]
   double* part_rows0;    // [grid_dual * kEvalRowSlots]
@@ -88,6 +90,11 @@ struct RoundBuffers {
 void launch_mixed_step(const MixedBuffers& b, cudaStream_t s);
 void launch_mixed_primal(const MixedBuffers& b, cudaStream_t s);
 void launch_mixed_dual(const MixedBuffers& b, cudaStream_t s);
+// Up to `attempts` attempted steps in one cooperative launch, which ends early where an evaluation
+// falls due; mixed_steps_fit: whether the layouts' windows hold the whole vectors and the device
+// runs its blocks at once.
+void launch_mixed_steps(const MixedBuffers& b, int attempts, cudaStream_t s);
+bool mixed_steps_fit(const MixedBuffers& b);
 void launch_mixed_evaluation(const MixedBuffers& b, cudaStream_t s);
 // Residual measures of the anchor (needs ax, aty computed): out[0..2].
 void launch_round_measure(const RoundBuffers& r, cudaStream_t s);
@@ -108,6 +115,11 @@ void launch_sort_outer_values(const int2* rounds, int nrounds, const int* optr,
                               const unsigned short* opos, const float* val, float* out,
                               cudaStream_t s);
 void launch_to_float(const double* src, float* dst, long long count, cudaStream_t s);
+// sum cs^2 and sum b^2 (b a row's finite side) in the last two of the scaled_norms_size() doubles of
+// `part`.
+int scaled_norms_size();
+void launch_scaled_norms(int m, int n, const double* cs, const double* rl, const double* ru,
+                         double* part, cudaStream_t s);
 void launch_fill_float(float* v, int count, float value, cudaStream_t s);
 // Sets the dynamic shared-memory limits of the FP32 kernels on the current device (once per
 // device); false if the device refused.

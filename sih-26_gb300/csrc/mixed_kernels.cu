@@ -49,29 +49,13 @@ __device__ __forceinline__ int grid_stride_begin() {
 }
 
 // ---- Inner step ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
-  __shared__ double scratch[kChunkScratch];
-  grid_dependency_wait();  // the previous kernel's results (launch_after)
-  Ctl* ctl = b.ctl;
-  // Every control field the pass reads, loaded together before the first test.
-  const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
-  const bool add = ctl->pending_add != 0;
-  const long long iteration = ctl->iteration, limit = ctl->iteration_limit;
-  const double omega = ctl->omega, eta = ctl->eta;
-  if (done != kRunning || eval_now != 0) return;
-  if (iteration >= limit) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->done = kIterationLimit;
-    return;
-  }
-  const float* __restrict__ u = b.u[cur];
-  float* __restrict__ un = b.u[cur ^ 1];
-  const float* __restrict__ v = b.v[cur];
-  // The step's FP32 scalar, formed once per block: GB300 runs FP64 at 1/64 of the FP32 rate,
-  // so an FP64 division in each of 1,024 threads would hold the FP64 pipe for thousands of
-  // cycles per SM at the start of every launch.
-  const float tau = block_scalar([&] { return static_cast<float>(eta / omega); });
-  float mvf = 0.0f;
+// The column pass of the block's chunks (or, longs, of the long columns): the squared movement is
+// added to mvf. False where a wait gave up. LIVE: one pass of many in the kernel (k_steps_f).
+template <bool LIVE>
+__device__ __forceinline__ bool primal_pass(const MixedBuffers& b, int cur, bool add, float tau,
+                                            unsigned char* dsmem, bool longs, float& mvf) {
+  const float* u = b.u[cur];
+  float* un = b.u[cur ^ 1];
   // Operands of column j: u, cf, lf, uf and (when the last step is still to be added) u_sum.
   auto load = [&](int j, float* o) {
     o[0] = u[j];
@@ -90,54 +74,23 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
     b.du[j] = d;
     mvf = fmaf(d, d, mvf);
   };
-  if (!run_chunks<5>(b.csc_k, v, dsmem, b.piece_primal, load,
-                                                  epi) &&
-      threadIdx.x == 0) {
-    raise_error(ctl);
+  if (LIVE) return run_whole_chunks<5>(b.csc_k, b.v[cur], dsmem, load, epi);
+  if (longs) {
+    run_chunk_long_rows<5>(b.csc_k, b.piece_primal, load, epi);
+    return true;
   }
-  double mv[1] = {static_cast<double>(mvf)};
-  if (b.csc_k.nlong == 0) {
-    // No long column to finish: each block publishes its partial, and the row pass's last
-    // block sums them in block order (primal_movement) when it takes the step decision. No
-    // block of this pass waits for another.
-    double out[1];
-    block_sum<1>(mv, scratch, out);
-    if (threadIdx.x == 0) b.part_primal[blockIdx.x] = out[0];
-    return;
-  }
-  if (!arrive_last<1>(mv, scratch, b.part_primal, &ctl->ticket[kTicketPrimal])) return;
-  mvf = 0.0f;
-  run_chunk_long_rows<5>(b.csc_k, b.piece_primal, load, epi);
-  mv[0] = static_cast<double>(mvf);
-  double longs[1], total[1];
-  block_sum<1>(mv, scratch, longs);
-  sum_partials<1>(b.part_primal, gridDim.x, scratch, total);
-  if (threadIdx.x == 0) {
-    ctl->mv_primal = 0.5 * omega * (total[0] + longs[0]);
-    ctl->ticket[kTicketPrimal] = 0;
-  }
+  return run_chunks<5>(b.csc_k, b.v[cur], dsmem, b.piece_primal, load, epi);
 }
 
-__global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
-  extern __shared__ __align__(16) unsigned char dsmem[];
-  __shared__ double scratch[kChunkScratch];
-  grid_dependency_wait();  // the previous kernel's results (launch_after)
-  Ctl* ctl = b.ctl;
-  const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
-  const bool add = ctl->pending_add != 0;
-  const double omega = ctl->omega, eta = ctl->eta;
-  if (done != kRunning || eval_now != 0) return;
-  // The step-size factors of this step, loaded now for the decision the last block takes.
-  const double2 factors = threadIdx.x == 0
-                              ? step_factors(ctl->iteration, b.step_factors, b.step_factors_n)
-                              : make_double2(0.0, 0.0);
-  const float* __restrict__ v = b.v[cur];
-  float* __restrict__ vn = b.v[cur ^ 1];
-  const float* __restrict__ au = b.au[cur];
-  float* __restrict__ aun = b.au[cur ^ 1];
-  const float sigma = block_scalar([&] { return static_cast<float>(eta * omega); });
+// The row pass likewise: sum dv^2 is added to a0, sum dv (A du) to a1.
+template <bool LIVE>
+__device__ __forceinline__ bool dual_pass(const MixedBuffers& b, int cur, bool add, float sigma,
+                                          unsigned char* dsmem, bool longs, float& a0, float& a1) {
+  const float* v = b.v[cur];
+  float* vn = b.v[cur ^ 1];
+  const float* au = b.au[cur];
+  float* aun = b.au[cur ^ 1];
   const float inv_sigma = 1.0f / sigma;
-  float a0 = 0.0f, a1 = 0.0f;  // sum dv^2, sum dv (A du)
   // Operands of row i: v, gu, gl, yhat, A u and (when the last step is still to be added)
   // v_sum.
   auto load = [&](int i, float* o) {
@@ -174,15 +127,82 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
     a0 = fmaf(d, d, a0);
     a1 = fmaf(d, adu, a1);
   };
-  if (!run_chunks<6>(b.csr_k, b.du, dsmem, b.piece_dual, load,
-                                                  epi) &&
-      threadIdx.x == 0) {
+  if (LIVE) return run_whole_chunks<6>(b.csr_k, b.du, dsmem, load, epi);
+  if (longs) {
+    run_chunk_long_rows<6>(b.csr_k, b.piece_dual, load, epi);
+    return true;
+  }
+  return run_chunks<6>(b.csr_k, b.du, dsmem, b.piece_dual, load, epi);
+}
+
+__global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
+  extern __shared__ __align__(16) unsigned char dsmem[];
+  __shared__ double scratch[kChunkScratch];
+  grid_dependency_wait();  // the previous kernel's results (launch_after)
+  Ctl* ctl = b.ctl;
+  // Every control field the pass reads, loaded together before the first test.
+  const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
+  const bool add = ctl->pending_add != 0;
+  const long long iteration = ctl->iteration, limit = ctl->iteration_limit;
+  const double omega = ctl->omega, eta = ctl->eta;
+  if (done != kRunning || eval_now != 0) return;
+  if (iteration >= limit) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->done = kIterationLimit;
+    return;
+  }
+  // The step's FP32 scalar, formed once per block: GB300 runs FP64 at 1/64 of the FP32 rate,
+  // so an FP64 division in each of 1,024 threads would hold the FP64 pipe for thousands of
+  // cycles per SM at the start of every launch.
+  const float tau = block_scalar([&] { return static_cast<float>(eta / omega); });
+  float mvf = 0.0f;
+  if (!primal_pass<false>(b, cur, add, tau, dsmem, false, mvf) && threadIdx.x == 0) {
+    raise_error(ctl);
+  }
+  double mv[1] = {static_cast<double>(mvf)};
+  if (b.csc_k.nlong == 0) {
+    // No long column to finish: each block publishes its partial, and the row pass's last
+    // block sums them in block order (primal_movement) when it takes the step decision. No
+    // block of this pass waits for another.
+    double out[1];
+    block_sum<1>(mv, scratch, out);
+    if (threadIdx.x == 0) b.part_primal[blockIdx.x] = out[0];
+    return;
+  }
+  if (!arrive_last<1>(mv, scratch, b.part_primal, &ctl->ticket[kTicketPrimal])) return;
+  mvf = 0.0f;
+  primal_pass<false>(b, cur, add, tau, dsmem, true, mvf);
+  mv[0] = static_cast<double>(mvf);
+  double longs[1], total[1];
+  block_sum<1>(mv, scratch, longs);
+  sum_partials<1>(b.part_primal, gridDim.x, scratch, total);
+  if (threadIdx.x == 0) {
+    ctl->mv_primal = 0.5 * omega * (total[0] + longs[0]);
+    ctl->ticket[kTicketPrimal] = 0;
+  }
+}
+
+__global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
+  extern __shared__ __align__(16) unsigned char dsmem[];
+  __shared__ double scratch[kChunkScratch];
+  grid_dependency_wait();  // the previous kernel's results (launch_after)
+  Ctl* ctl = b.ctl;
+  const int done = ctl->done, eval_now = ctl->eval_now, cur = ctl->cur;
+  const bool add = ctl->pending_add != 0;
+  const double omega = ctl->omega, eta = ctl->eta;
+  if (done != kRunning || eval_now != 0) return;
+  // The step-size factors of this step, loaded now for the decision the last block takes.
+  const double2 factors = threadIdx.x == 0
+                              ? step_factors(ctl->iteration, b.step_factors, b.step_factors_n)
+                              : make_double2(0.0, 0.0);
+  const float sigma = block_scalar([&] { return static_cast<float>(eta * omega); });
+  float a0 = 0.0f, a1 = 0.0f;  // sum dv^2, sum dv (A du)
+  if (!dual_pass<false>(b, cur, add, sigma, dsmem, false, a0, a1) && threadIdx.x == 0) {
     raise_error(ctl);
   }
   double acc2[2] = {static_cast<double>(a0), static_cast<double>(a1)};
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
   a0 = a1 = 0.0f;
-  run_chunk_long_rows<6>(b.csr_k, b.piece_dual, load, epi);
+  dual_pass<false>(b, cur, add, sigma, dsmem, true, a0, a1);
   acc2[0] = a0;
   acc2[1] = a1;
   double longs[2], total[2];
@@ -196,6 +216,95 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
       const double movement = mv_primal + (0.5 * (total[0] + longs[0])) / omega;
       step_decision(ctl, movement, fabs(total[1] + longs[1]), factors);
     }
+  }
+}
+
+// Up to `attempts` steps by one cooperative grid whose blocks meet between the passes, each taking the
+// decision from the same partials (as k_pdhg_steps): the passes above, chunk for chunk and warp for
+// warp, without the launches between them. Only for layouts whose windows hold the whole vectors
+// (mixed_steps_fit): with every layout's form in one kernel its registers spilled, and a step of the
+// 1M x 2M LP took 237 us, 184 us in launches. 4 x 3,000 x 6,000: 22.6 us a step, 26.9 in launches.
+__global__ void __launch_bounds__(kChunkThreads, 1) k_steps_f(MixedBuffers b, int attempts) {
+  extern __shared__ __align__(16) unsigned char dsmem[];
+  __shared__ double scratch[3 * (kChunkThreads / 32)];
+  __shared__ Ctl s_ctl;
+  __shared__ StepPrep s_prep;
+  __shared__ double s_sums[3];
+  __shared__ float s_tau, s_sigma;
+  constexpr int kWords = static_cast<int>(sizeof(Ctl) / sizeof(unsigned long long));
+  const int t = static_cast<int>(threadIdx.x), T = static_cast<int>(blockDim.x);
+  const int block = static_cast<int>(blockIdx.x), G = static_cast<int>(gridDim.x);
+  unsigned long long* const words = reinterpret_cast<unsigned long long*>(&s_ctl);
+  for (int k = t; k < kWords; k += T) {
+    words[k] = reinterpret_cast<const volatile unsigned long long*>(b.ctl)[k];
+  }
+  GridMeet grid;
+  grid.start(b.arrivals);
+  const auto meet = [&] {
+    if (grid.meet(&b.ctl->error)) return true;
+    if (t == 0) raise_error(b.ctl);  // the kernels that follow do nothing
+    return false;
+  };
+  __syncthreads();
+  if (t == 0) {
+    if (s_ctl.done == kRunning && s_ctl.eval_now == 0 &&
+        s_ctl.iteration >= s_ctl.iteration_limit) {
+      s_ctl.done = kIterationLimit;
+    }
+    s_tau = static_cast<float>(s_ctl.eta / s_ctl.omega);
+    s_sigma = static_cast<float>(s_ctl.eta * s_ctl.omega);
+  }
+  __syncthreads();
+  for (int a = 0; a < attempts; ++a) {
+    if (s_ctl.done != kRunning || s_ctl.eval_now != 0) break;
+    const int cur = s_ctl.cur;
+    const bool add = s_ctl.pending_add != 0;
+    if (t == T - 1) {
+      s_prep.set(&s_ctl, step_factors(s_ctl.iteration, b.step_factors, b.step_factors_n));
+    }
+    float mvf = 0.0f, a0 = 0.0f, a1 = 0.0f;
+    bool ok = true;
+    if (block < b.grid_step_primal) {
+      ok = primal_pass<true>(b, cur, add, s_tau, dsmem, false, mvf);
+    }
+    if (!ok && t == 0) b.ctl->error = 1;  // the blocks still meet: a wait that gave up ends the solve
+    if (!meet()) return;
+    if (block < b.grid_step_dual) {
+      ok = dual_pass<true>(b, cur, add, s_sigma, dsmem, false, a0, a1);
+    }
+    if (!ok && t == 0) b.ctl->error = 1;
+    double sums[3] = {static_cast<double>(mvf), static_cast<double>(a0), static_cast<double>(a1)};
+    double part[3];
+    block_sum<3>(sums, scratch, part);
+    if (t == 0) {
+      for (int q = 0; q < 3; ++q) b.part_steps[3 * block + q] = part[q];
+    }
+    if (!meet()) return;
+    if (t < 96) {
+      const int q = t >> 5;
+      const double sum = table_sum(G, [&](int k) { return __ldcg(b.part_steps + 3 * k + q); });
+      if ((t & 31) == 0) {
+        const double omega = s_ctl.omega;
+        s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? (0.5 * sum) / omega : sum);
+      }
+    }
+    __syncthreads();
+    if (t == 0) {
+      s_ctl.mv_primal = s_sums[0];
+      step_decision(&s_ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), s_prep);
+      if (s_ctl.eval_now == 0 && s_ctl.iteration >= s_ctl.iteration_limit) {
+        s_ctl.done = kIterationLimit;
+      }
+      s_tau = static_cast<float>(s_ctl.eta / s_ctl.omega);
+      s_sigma = static_cast<float>(s_ctl.eta * s_ctl.omega);
+    }
+    __syncthreads();
+  }
+  if (block == 0) {
+    s_ctl.error = *reinterpret_cast<volatile int*>(&b.ctl->error);
+    if (s_ctl.error != 0) s_ctl.done = kFault;
+    __syncthreads();
+    for (int k = t; k < kWords; k += T) reinterpret_cast<unsigned long long*>(b.ctl)[k] = words[k];
   }
 }
 
@@ -532,6 +641,36 @@ __global__ void k_to_float(const double* src, float* dst, long long count) {
   }
 }
 
+// Sum of squares of the scaled cost and of the rows' finite sides (the lower one where both are), for
+// the inner loop's relative residuals: per block, then by one block.
+constexpr int kNormBlocks = 304;
+__global__ void __launch_bounds__(kTileThreads) k_scaled_norms(int m, int n, const double* cs,
+                                                               const double* rl, const double* ru,
+                                                               double* part) {
+  __shared__ double scratch[2 * (kTileThreads / 32)];
+  double acc[2] = {0.0, 0.0}, out[2];
+  for (int j = grid_stride_begin(); j < n; j += gridDim.x * blockDim.x) {
+    acc[0] = fma(cs[j], cs[j], acc[0]);
+  }
+  for (int i = grid_stride_begin(); i < m; i += gridDim.x * blockDim.x) {
+    const double b = !isinf(rl[i]) ? rl[i] : (!isinf(ru[i]) ? ru[i] : 0.0);
+    acc[1] = fma(b, b, acc[1]);
+  }
+  block_sum<2>(acc, scratch, out);
+  if (threadIdx.x < 2) part[2 * blockIdx.x + threadIdx.x] = out[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(kTileThreads) k_scaled_norms_final(double* part) {
+  __shared__ double scratch[2 * (kTileThreads / 32)];
+  double acc[2] = {0.0, 0.0}, out[2];
+  for (int b = threadIdx.x; b < kNormBlocks; b += kTileThreads) {
+    acc[0] += part[2 * b];
+    acc[1] += part[2 * b + 1];
+  }
+  block_sum<2>(acc, scratch, out);
+  if (threadIdx.x < 2) part[2 * kNormBlocks + threadIdx.x] = out[threadIdx.x];
+}
+
 __global__ void k_fill_float(float* v, int count, float value) {
   for (int k = grid_stride_begin(); k < count; k += gridDim.x * blockDim.x) v[k] = value;
 }
@@ -654,6 +793,8 @@ bool configure_mixed_kernels() {
                            max_dynamic_smem(reinterpret_cast<const void*>(k_primal_f))),
       cudaFuncSetAttribute(k_dual_f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_dual_f))),
+      cudaFuncSetAttribute(k_steps_f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           max_dynamic_smem(reinterpret_cast<const void*>(k_steps_f))),
       cudaFuncSetAttribute(k_evalf_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF),
       cudaFuncSetAttribute(k_evalf_rows1, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF)};
   for (cudaError_t e : errs) {
@@ -715,6 +856,18 @@ void launch_mixed_step(const MixedBuffers& b, cudaStream_t s) {
   launch_mixed_dual(b, s);
 }
 
+bool mixed_steps_fit(const MixedBuffers& b) {
+  const auto whole = [](const ChunkSet& c) { return c.narrow && c.outer == nullptr && c.npieces == 0; };
+  return configure_mixed_kernels() && whole(b.csc_k) && whole(b.csr_k) &&
+         grid_fits(k_steps_f, std::max(b.grid_step_primal, b.grid_step_dual), kChunkThreads,
+                   std::max(b.smem_primal, b.smem_dual));
+}
+
+void launch_mixed_steps(const MixedBuffers& b, int attempts, cudaStream_t s) {
+  launch_grid(k_steps_f, std::max(b.grid_step_primal, b.grid_step_dual), kChunkThreads,
+              std::max(b.smem_primal, b.smem_dual), s, b, attempts);
+}
+
 void launch_mixed_evaluation(const MixedBuffers& b, cudaStream_t s) {
   k_evalf_rows0<<<b.grid_dual, kTileThreads, 0, s>>>(b);
   k_evalf_cols<<<b.grid_primal, kWideBlockThreads, kSmemF, s>>>(b);
@@ -769,6 +922,14 @@ void launch_sort_outer_values(const int2* rounds, int nrounds, const int* optr,
 void launch_to_float(const double* src, float* dst, long long count, cudaStream_t s) {
   if (count <= 0) return;
   k_to_float<<<egrid(count), 256, 0, s>>>(src, dst, count);
+}
+
+int scaled_norms_size() { return 2 * kNormBlocks + 2; }
+
+void launch_scaled_norms(int m, int n, const double* cs, const double* rl, const double* ru,
+                         double* part, cudaStream_t s) {
+  k_scaled_norms<<<kNormBlocks, kTileThreads, 0, s>>>(m, n, cs, rl, ru, part);
+  k_scaled_norms_final<<<1, kTileThreads, 0, s>>>(part);
 }
 
 void launch_fill_float(float* v, int count, float value, cudaStream_t s) {

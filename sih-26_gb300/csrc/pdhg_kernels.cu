@@ -85,19 +85,6 @@ __device__ bool fp64_stop_test(const Ctl* c, const Residuals& r) {
                                  (c->stop_at_request || meets_project_standard(r));
 }
 
-// The sum of get(0) .. get(n - 1) over a warp, in every lane: up to five per lane are read at once
-// and added as a tree, so 152 of them cost one latency and eight dependent additions.
-template <typename Get>
-__device__ __forceinline__ double table_sum(int n, Get get) {
-  const int lane = static_cast<int>(threadIdx.x) & 31;
-  double v[5];
-#pragma unroll
-  for (int u = 0; u < 5; ++u) v[u] = lane + 32 * u < n ? get(lane + 32 * u) : 0.0;
-  double sum = ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
-  for (int k = lane + 160; k < n; k += 32) sum += get(k);
-  return warp_sum(sum);
-}
-
 // ---- k_primal ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
   extern __shared__ __align__(128) unsigned char dsmem[];
@@ -450,6 +437,11 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
   }
   GridMeet grid;
   grid.start(b.arrivals);
+  const auto meet = [&] {
+    if (grid.meet(&b.ctl->error)) return true;
+    if (t == 0) raise_error(b.ctl);  // the kernels that follow do nothing
+    return false;
+  };
   __syncthreads();
   if (t == 0) {
     if (s_ctl.done == kRunning && s_ctl.eval_now == 0 &&
@@ -509,7 +501,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
     {
       SliceStart<kPairPiece> rows;
       if (block < b.csr.grid) start_slices(b.csr, rows);
-      if (!grid.meet(&b.ctl->error)) return;
+      if (!meet()) return;
       const double2* xd = b.xd;
       double* yn = b.y[cur ^ 1];
       const double sigma = s_sigma, inv_sigma = s_prep.inv_sigma;
@@ -555,7 +547,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
       for (int q = 0; q < 3; ++q) b.part_steps[3 * block + q] = part[q];
     }
     if (block < b.csc.grid) start_slices(b.csc, cols);
-    if (!grid.meet(&b.ctl->error)) return;
+    if (!meet()) return;
     // A warp per sum: the primal movement, the dual movement over omega, the interaction.
     if (t < 96) {
       const int q = t >> 5;

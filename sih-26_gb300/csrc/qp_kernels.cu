@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(qp_threads<G>()) k_qp_row(QpDev d, QpCtl* ctl,
 // An iteration over uniform rows: 8.9 us at 20,000 x 40,003 (14 us with launches), 14.2 us at 60,000.
 __global__ void __launch_bounds__(kQpSliceThreads, 1) k_qp_steps(QpDev d, QpCtl* ctl, int k0,
                                                                  int count) {
-  if (ctl->done != 0) return;
+  if (ctl->done != 0 || ctl->error != 0) return;
   const long long left = ctl->limit - (ctl->base + k0);
   const int iterations = left < count ? static_cast<int>(left) : count;
   if (iterations <= 0) return;

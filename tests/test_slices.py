@@ -208,3 +208,24 @@ def test_pdhg_steps_in_one_launch_match_the_oracle(oracle, lengths, n):
     ref = oracle.solve(lp, tolerance=1e-13, iteration_limit=40)
     assert np.abs(x - ref.col_value).max() <= 1e-9 * max(1.0, np.abs(ref.col_value).max())
     assert np.abs(y - ref.row_dual).max() <= 1e-9 * max(1.0, np.abs(ref.row_dual).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(1, 2), (33, 70), (900, 1500), (5000, 9000)])
+def test_mixed_steps_in_one_launch(monkeypatch, m, n):
+    """The mixed method's steps in one cooperative launch (windows that hold the whole vectors) and over
+    launches (a window capacity of half the longer vector): limits are exact inside and at the end
+    of a period, and objectives at a relative KKT of 1e-6 agree to 1e-4, a hundred times the KKT."""
+    lp = lp_with_rows(np.random.default_rng(n).integers(1, min(n, 12) + 1, size=m), n, seed=n)
+    runs = []
+    for cap in (None, str(max(4, max(m, n) // 2))):
+        if cap is not None:
+            monkeypatch.setenv("SANKHYA_GB300_WINDOW_CAP", cap)
+        with capi.PdhgEngine(0) as eng:
+            eng.load(lp)
+            for limit in (1, 41, 85):
+                r = eng.solve(tolerance=1e-13, precision="mixed", iteration_limit=limit)
+                assert r.iterations == limit or r.converged
+            runs.append(eng.solve(tolerance=1e-6, precision="mixed", iteration_limit=200000))
+    assert {r.status_name for r in runs} <= {"optimal", "feasible"}
+    assert abs(runs[0].objective - runs[1].objective) <= 1e-4 * max(1.0, abs(runs[1].objective))
