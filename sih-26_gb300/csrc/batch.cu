@@ -375,7 +375,7 @@ void BatchEngine::solve(const sankhya_gb300_params& p, sankhya_gb300_batch_item*
   // a sample of the batch before the solve (not part of the solve's device time).
   const int scale_grid = std::max(1, std::min(b.nmatrices, num_sms_ * 8));
   SGB_CUDA(cudaEventRecord(timing_[0], s));
-  launch_batch_scaling(b, scale_grid, s);
+  launch_batch_scaling(b, scale_grid, b.nmatrices <= num_sms_ ? kScaleMaxThreads : kBatchThreads, s);
   SGB_CUDA(cudaGetLastError());
   SGB_CUDA(cudaEventRecord(timing_[1], s));
   SGB_CUDA(cudaEventSynchronize(timing_[1]));

@@ -26,7 +26,8 @@
 
 namespace sgb {
 
-constexpr int kBatchThreads = 256;     // scaling launches
+constexpr int kBatchThreads = 256;     // scaling launches of many matrices,
+constexpr int kScaleMaxThreads = 1024; // of no more than the SMs
 constexpr int kBatchMaxThreads = 512;  // the largest block a batched solve runs with
 constexpr int kAdjThreads = 512;       // adjoint and polish launches, at most
 constexpr int kAdjVectors = 8;         // compact per-LP vectors of the square solves
@@ -138,7 +139,7 @@ struct AdjointBuffers {
   int lu_size;
 };
 
-void launch_batch_scaling(const BatchBuffers& b, int grid, cudaStream_t s);
+void launch_batch_scaling(const BatchBuffers& b, int grid, int threads, cudaStream_t s);
 // The adjoint and polish launches run blocks of a.threads threads with a.smem_bytes of dynamic
 // shared memory; adjoint_max_smem is the most they can have, adjoint_blocks_per_sm their
 // occupancy.
