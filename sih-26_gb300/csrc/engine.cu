@@ -692,7 +692,9 @@ void Engine::load(const sankhya_gb300_lp& lp) {
                                  &xu0_, &xu1_, &reduced_, &best_x_, &power_v_}) {
     a->allocate(static_cast<size_t>(n) + kPad);
   }
-  xd_.allocate(static_cast<size_t>(n) + kPad);
+  dx_.allocate(static_cast<size_t>(n) + kPad);
+  ax0_.allocate(static_cast<size_t>(m) + kPad);
+  ax1_.allocate(static_cast<size_t>(m) + kPad);
   for (DeviceArray<double>* a : {&rls_, &rus_, &dr_, &row_factor_[0], &row_factor_[1], &y0_, &y1_, &y_sum_, &y_rst_,
                                  &yu0_, &yu1_, &best_y_, &power_av_}) {
     a->allocate(static_cast<size_t>(m) + kPad);
@@ -730,12 +732,9 @@ void Engine::load(const sankhya_gb300_lp& lp) {
                                  sl_csr_.most_slices);
   resident_ = resident > 0 && resident_fits(step_, resident_smem_);
   // Larger LPs run a period's steps in one cooperative launch (us a step, launches first: uniform
-  // 5,000 x 10,001 18.4 and 14.5, 60,000 x 120,001 32.0 and 28.8; blocks 320,000 x 640,000 90.5 and
-  // 88.0; Zipf rows with 200,000 entries 48.0 and 40.5). Not large ones with rows of several pieces
-  // (Zipf, 2 million entries: 68 and 75), whose blocks end far apart.
-  constexpr int kLongRowNnz = 1 << 20;
-  const bool pieces = sl_csc_.view.nlong + sl_csr_.view.nlong > 0;
-  steps_ = !resident_ && cap < 0 && (!pieces || nnz_ <= kLongRowNnz) && pdhg_steps_fit(step_);
+  // 5,000 x 10,001 18.3 and 13.8, 60,000 x 120,001 30.8 and 26.9; blocks 500,000 x 1M 120.8 and 112.9;
+  // Zipf rows with 200,000 entries 42.1 and 31.1, with 2 million 58.4 and 56.8).
+  steps_ = !resident_ && cap < 0 && pdhg_steps_fit(step_);
   loaded_ = true;
 }
 
@@ -751,7 +750,7 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
                          int extent, int pass, int window_cap, int resident) {
   constexpr int kFullWindow = 32 * 1024;
   cudaStream_t s = stream_;
-  const int elem = static_cast<int>(pass == 0 ? sizeof(double) : sizeof(double2));
+  const int elem = static_cast<int>(sizeof(double));
   int wmax = std::min(fp64_window_capacity(pass), kFullWindow / elem);
   if (window_cap >= 0) {
     wmax = std::min(wmax, window_cap);
@@ -759,7 +758,7 @@ void Engine::plan_sliced(SliceDev& D, const std::vector<int>& lptr, const int* l
     wmax = 0;
   }
   const SlicePlan P =
-      plan_slices(lptr, lidx, lines, extent, wmax, 0.0, num_sms_, pass == 0 ? 1 : 2, resident);
+      plan_slices(lptr, lidx, lines, extent, wmax, 0.0, num_sms_, 1, resident);
   D.meta.upload(P.meta.data(), P.meta.size(), s);
   D.base.upload(P.base.data(), P.base.size(), s);
   D.items.upload(P.items.data(), P.items.size(), s);
@@ -913,7 +912,9 @@ void Engine::fill_buffers() {
   b.y[1] = y1_.ptr;
   b.x_sum = x_sum_.ptr;
   b.y_sum = y_sum_.ptr;
-  b.xd = xd_.ptr;
+  b.dx = dx_.ptr;
+  b.ax[0] = ax0_.ptr;
+  b.ax[1] = ax1_.ptr;
   b.c = cs_.ptr;
   b.l = ls_.ptr;
   b.u = us_.ptr;
@@ -939,6 +940,8 @@ void Engine::fill_buffers() {
   e.y[0] = y0_.ptr;
   e.y[1] = y1_.ptr;
   e.x_sum = x_sum_.ptr;
+  e.ax[0] = ax0_.ptr;
+  e.ax[1] = ax1_.ptr;
   e.y_sum = y_sum_.ptr;
   e.x_rst = x_rst_.ptr;
   e.y_rst = y_rst_.ptr;
@@ -1178,6 +1181,7 @@ void Engine::spmv_noalloc(int op, int scaled, const double* in, double* out,
 void Engine::init_iterates(const sankhya_gb300_params& p) {
   cudaStream_t s = stream_;
   launch_project_start(n_, ls_.ptr, us_.ptr, x0_.ptr, s);
+  if (!resident_) launch_spmv(step_.csr, x0_.ptr, ax0_.ptr, chunk_spmv_.ptr, tickets_.ptr + 1, s);
   launch_fill(y0_.ptr, m_, 0.0, s);
   launch_fill(x_sum_.ptr, n_, 0.0, s);
   launch_fill(y_sum_.ptr, m_, 0.0, s);

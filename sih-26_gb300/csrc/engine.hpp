@@ -193,7 +193,8 @@ class Engine {
   // Iterates.
   DeviceArray<double> x0_, x1_, y0_, y1_, x_sum_, y_sum_, x_rst_, y_rst_;
   DeviceArray<double> xu0_, xu1_, yu0_, yu1_, reduced_, best_x_, best_y_;
-  DeviceArray<double2> xd_;  // (2x' - x, x' - x) per column
+  DeviceArray<double> dx_;         // x' - x per column
+  DeviceArray<double> ax0_, ax1_;  // scaled A x per row, with x0_ and x1_
   // Reductions.
   DeviceArray<double> part_primal_, part_dual_, part_rows0_, part_cols_, part_rows1_;
   DeviceArray<double> chunk_primal_, chunk_dual_, chunk_cols_, chunk_rows_, chunk_spmv_;

@@ -101,9 +101,12 @@ struct StepBuffers {
   double* y[2];
   double* x_sum;
   double* y_sum;
-  // (2 x' - x, x' - x) of the step, written by k_primal and gathered by k_dual as ONE
-  // 16-byte element per entry: a scattered gather costs a cache sector whatever it reads.
-  double2* xd;
+  // x' - x per column, written by k_primal and gathered by k_dual, which forms A (2 x' - x) as
+  // A x + 2 A (x' - x) with A x carried per row (double-buffered with x): half the gathered bytes and
+  // half the products of gathering both. A carried sum's rounding cannot build up: every evaluation,
+  // at most 40 accepted steps apart, stores A x afresh.
+  double* dx;
+  double* ax[2];
   const double *c, *l, *u, *rl, *ru;  // scaled problem
   double* part_primal;   // [csc.grid + csc.nlong]
   double* part_dual;     // [(csr.grid + csr.nlong) * 2]
@@ -124,6 +127,7 @@ struct EvalBuffers {
   double* x_sum;
   double* y_sum;
   double *x_rst, *y_rst;
+  double* ax[2];                  // the steps' carried scaled A x (StepBuffers)
   const double *dr, *dc;          // row / column scale (Dr, Dc)
   const double* cost;             // minimise-space unscaled cost
   const double* col_cost;         // original-sense cost (for the model objective)

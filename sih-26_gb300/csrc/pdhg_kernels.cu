@@ -4,13 +4,15 @@
 // rows of slices.cuh (the FP32 method's step kernels run on the warp chunks of chunks.cuh
 // instead):
 //   k_primal  one pass over the CSC copy of Ahat: A^T y gathered per column, fused with the
-//             projected primal update x' = proj(x - tau (c + A^T y)), xbar = 2x' - x and
-//             dx = x' - x (written once per column so the row pass needs one FMA per entry
-//             and product), the primal half of the movement, and the deferred x_sum update.
-//   k_dual    one pass over the CSR copy: A xbar and A dx from ONE read of each row, fused
-//             with the Moreau dual update, the dual movement and the interaction dy^T A dx;
-//             its last block sums every block's partials in a fixed order and takes the
-//             step-size decision on the device.
+//             projected primal update x' = proj(x - tau (c + A^T y)), dx = x' - x (written
+//             once per column for the row pass), the primal half of the movement, and the
+//             deferred x_sum update.
+//   k_dual    one pass over the CSR copy: A dx gathered per row, A (2x' - x) = A x + 2 A dx
+//             with A x carried, fused with the Moreau dual update, the dual movement and the
+//             interaction dy^T A dx; its last block sums every block's partials in a fixed
+//             order and takes the step-size decision on the device.
+// Small LPs run a period's steps in one resident cluster kernel (k_pdhg_resident), larger ones
+// in one cooperative launch (k_pdhg_steps), with the same arithmetic per item.
 // The evaluation tick (src/pdhg/pdhg.cpp:341-483, src/pdhg/pdhg_evaluate.cpp) is three
 // fused passes over the UNSCALED values plus one vector pass; it runs only when the step
 // decision asks for it and otherwise returns at once.
@@ -35,8 +37,9 @@ namespace {
 long long g_launches = 0;
 
 constexpr int kScratch = 16 * (kSliceThreads / 32);
-// Entry rows per piece of the passes that gather a pair per entry (row pass of the 500,000 x 1M
-// block-angular LP: 86.5 us with 8, 86.6 with 6, 90.7 with 4; Zipf rows 60.3, 62.8, 63.8 us).
+// Entry rows per piece of the passes that gather a pair per entry (a row pass that gathered
+// (2x' - x, x' - x), 500,000 x 1M block-angular LP: 86.5 us with 8, 86.6 with 6, 90.7 with 4; Zipf
+// rows 60.3, 62.8, 63.8 us).
 constexpr int kPairPiece = kPiece;
 
 // Per-device state: whether the kernels' shared-memory limits are set on the device, and
@@ -132,8 +135,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
     const double xnj = clamp_box(__dsub_rn(xj, __dmul_rn(tau, gradient)), o[2], o[3]);
     xn[j] = xnj;
     const double d = xnj - xj;
-    // 2 x' is exact, so the FMA rounds once, as the reference's 2.0 * x' - x does.
-    b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
+    b.dx[j] = d;
     mv[0] = fma(d, d, mv[0]);
   };
   auto finish = [&](int l, int j, const double* s, const double* o) {
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
 __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
   extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
-  SliceStart<kPairPiece> start;
+  SliceStart<kPiece> start;
   start_slices(b.csr, start);
   grid_dependency_wait();  // the previous kernels' results (launch_after)
   Ctl* ctl = b.ctl;
@@ -173,37 +175,38 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
                               : make_double2(0.0, 0.0);
   const double* __restrict__ y = b.y[cur];
   double* __restrict__ yn = b.y[cur ^ 1];
-  const double2* __restrict__ xd = b.xd;
+  const double* __restrict__ dx = b.dx;
+  const double* __restrict__ ax = b.ax[cur];
+  double* __restrict__ axn = b.ax[cur ^ 1];
   __shared__ double s_inv_sigma;
   const double sigma = eta * omega;
   if (threadIdx.x == 0) s_inv_sigma = 1.0 / sigma;
   __syncthreads();
   const double inv_sigma = s_inv_sigma;
   double acc2[2] = {0.0, 0.0};  // sum dy^2, sum dy (A dx)
-  auto fetch = [&](int j) { return __ldg(xd + j); };
-  auto mac = [](double v, double2 p, double* acc) {
-    acc[0] = fma(v, p.x, acc[0]);
-    acc[1] = fma(v, p.y, acc[1]);
-  };
-  // Operands of row i: y, rl, ru and (when the last step is still to be added) y_sum.
+  auto fetch = [&](int j) { return __ldg(dx + j); };
+  auto mac = [](double v, double g, double* acc) { acc[0] = fma(v, g, acc[0]); };
+  // Operands of row i: y, rl, ru, (when the last step is still to be added) y_sum, and A x.
   auto load = [&](int i, double* o) {
     o[0] = y[i];
     o[1] = b.rl[i];
     o[2] = b.ru[i];
     o[3] = add ? b.y_sum[i] : 0.0;
+    o[4] = ax[i];
   };
   auto epi = [&](int i, const double* s, const double* o) {
     const double yi = o[0];
     if (add) b.y_sum[i] = o[3] + yi;
     // Unfused, as the reference rounds it (src/pdhg/pdhg.cpp:244-245): a fused
     // v - sigma * (v / sigma) would leave the division's rounding error on a free row.
-    const double v = __dadd_rn(yi, __dmul_rn(sigma, s[0]));
+    axn[i] = o[4] + s[0];
+    const double v = __dadd_rn(yi, __dmul_rn(sigma, fma(2.0, s[0], o[4])));
     const double p = row_projection(v, sigma, inv_sigma, o[1], o[2]);
     const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
     yn[i] = yni;
     const double d = yni - yi;
     acc2[0] = fma(d, d, acc2[0]);
-    acc2[1] = fma(d, s[1], acc2[1]);
+    acc2[1] = fma(d, s[0], acc2[1]);
   };
   auto finish = [&](int l, int i, const double* s, const double* o) {
     const double sums[2] = {acc2[0], acc2[1]};
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
       acc2[q] = sums[q];
     }
   };
-  if (!run_slices<true, 2, 4>(b.csr, start, xd, fetch, dsmem, b.chunk_dual, mac, load, epi,
+  if (!run_slices<true, 1, 5>(b.csr, start, dx, fetch, dsmem, b.chunk_dual, mac, load, epi,
                               finish) &&
       threadIdx.x == 0) {
     raise_error(ctl);
@@ -483,7 +486,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
         const double xnj = clamp_box(__dsub_rn(xj, __dmul_rn(tau, gradient)), o[2], o[3]);
         xn[j] = xnj;
         const double d = xnj - xj;
-        b.xd[j] = make_double2(fma(2.0, xnj, -xj), d);
+        b.dx[j] = d;
         sums[0] = fma(d, d, sums[0]);
       };
       auto finish = [&](int l, int j, const double* s, const double* o) {
@@ -499,33 +502,34 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
       }
     }
     {
-      SliceStart<kPairPiece> rows;
+      SliceStart<kPiece> rows;
       if (block < b.csr.grid) start_slices(b.csr, rows);
       if (!meet()) return;
-      const double2* xd = b.xd;
+      const double* dx = b.dx;
+      const double* ax = b.ax[cur];
+      double* axn = b.ax[cur ^ 1];
       double* yn = b.y[cur ^ 1];
       const double sigma = s_sigma, inv_sigma = s_prep.inv_sigma;
-      auto fetch = [&](int j) { return ld_live(xd + j); };
-      auto mac = [](double v, double2 p, double* acc) {
-        acc[0] = fma(v, p.x, acc[0]);
-        acc[1] = fma(v, p.y, acc[1]);
-      };
+      auto fetch = [&](int j) { return ld_live(dx + j); };
+      auto mac = [](double v, double g, double* acc) { acc[0] = fma(v, g, acc[0]); };
       auto load = [&](int i, double* o) {
         o[0] = y[i];
         o[1] = b.rl[i];
         o[2] = b.ru[i];
         o[3] = add ? b.y_sum[i] : 0.0;
+        o[4] = ax[i];
       };
       auto epi = [&](int i, const double* s, const double* o) {
         const double yi = o[0];
         if (add) b.y_sum[i] = o[3] + yi;
-        const double v = __dadd_rn(yi, __dmul_rn(sigma, s[0]));
+        axn[i] = o[4] + s[0];
+        const double v = __dadd_rn(yi, __dmul_rn(sigma, fma(2.0, s[0], o[4])));
         const double p = row_projection(v, sigma, inv_sigma, o[1], o[2]);
         const double yni = __dsub_rn(v, __dmul_rn(sigma, p));
         yn[i] = yni;
         const double d = yni - yi;
         sums[1] = fma(d, d, sums[1]);
-        sums[2] = fma(d, s[1], sums[2]);
+        sums[2] = fma(d, s[0], sums[2]);
       };
       auto finish = [&](int l, int i, const double* s, const double* o) {
         const double keep[2] = {sums[1], sums[2]};
@@ -537,7 +541,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
         }
       };
       if (block < b.csr.grid) {
-        run_slices<false, 2, 4>(b.csr, rows, xd, fetch, nullptr, b.chunk_dual, mac, load, epi,
+        run_slices<false, 1, 5>(b.csr, rows, dx, fetch, nullptr, b.chunk_dual, mac, load, epi,
                                 finish);
       }
     }
@@ -748,6 +752,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_eval_rows1(EvalBuffers e) 
   const bool avg = !fin && c->averaged > 0;
   const double* __restrict__ xu0 = e.xu[0];
   const double* __restrict__ xu1 = e.xu[1];
+  double* __restrict__ ax = e.ax[c->cur];
   double acc[2] = {0.0, 0.0};
   double cmax[2] = {0.0, 0.0};
   auto fetch = [&](int j) { return make_double2(xu0[j], avg ? xu1[j] : 0.0); };
@@ -757,6 +762,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_eval_rows1(EvalBuffers e) 
   };
   auto load = [](int, double*) {};
   auto epi = [&](int i, const double* s, const double*) {
+    if (!fin) ax[i] = e.dr[i] * s[0];  // the scaled A x of the current iterate, afresh
     const double rl = e.rl[i], ru = e.ru[i];
     const int nc = avg ? 2 : 1;
     for (int q = 0; q < nc; ++q) {
@@ -1435,7 +1441,7 @@ int fp64_window_capacity(int pass) {
              ? window_capacity(reinterpret_cast<const void*>(k_primal), kSliceBarBytes,
                                sizeof(double))
              : window_capacity(reinterpret_cast<const void*>(k_dual), kSliceBarBytes,
-                               sizeof(double2));
+                               sizeof(double));
 }
 
 void launch_primal_pass(const StepBuffers& b, cudaStream_t s) {
@@ -1444,7 +1450,7 @@ void launch_primal_pass(const StepBuffers& b, cudaStream_t s) {
 }
 
 void launch_dual_pass(const StepBuffers& b, cudaStream_t s) {
-  launch_after(k_dual, b.csr.grid, b.csr.threads, slice_smem<double2>(b.csr.wmax), s, b);
+  launch_after(k_dual, b.csr.grid, b.csr.threads, slice_smem<double>(b.csr.wmax), s, b);
   ++g_launches;
 }
 
