@@ -225,9 +225,7 @@ SGB_API int sankhya_gb300_pdhg_spmv(sankhya_gb300_pdhg* engine, int32_t op, int3
  * per device index and kept for the life of the process: after cudaDeviceReset (or anything
  * else that destroys the device's primary context) the kept address is stale, so a process
  * that resets a device must not call this entry point on it again. The call does not wait
- * for the product, so it cannot report a failure of the product itself: if a bounded wait in
- * the product gives up (a copy that never lands), the rows it could not finish are set to
- * NaN instead of being left with a result that looks valid. */
+ * for the product, so a failed device shows at the caller's next synchronisation. */
 #define SANKHYA_GB300_NOALLOC_MAX_CHUNKS 16384
 SGB_API int sankhya_gb300_pdhg_spmv_noalloc(sankhya_gb300_pdhg* engine, int32_t op,
                                             int32_t scaled, const double* device_in,
@@ -318,13 +316,16 @@ SGB_API int sankhya_gb300_batch_ray(sankhya_gb300_batch* batch, int32_t index, d
  * dl_dx[k] (cols), dl_dy[k] (rows) and dl_df[k], returns dL/dc, dL/d(row_lower),
  * dL/d(row_upper), dL/d(col_lower), dL/d(col_upper) by implicit differentiation of the
  * optimum: at the active set the PDHG fixed point reduces to two square linear systems with
- * the basis matrix A_RB, solved on the device on a compact copy of A_RB by preconditioned
- * conjugate gradients on its normal equations, with refinement passes. An equality row's
+ * the basis matrix A_RB, solved on the device on a compact copy of A_RB: bases of up to 1024
+ * columns by FP32 LU factors and FP64 refinement, with 4 n^2 bytes of device memory per LP in
+ * flight (n the batch's widest basis); larger ones, and those that FP32 factors cannot solve, by
+ * preconditioned conjugate gradients on the normal equations, with refinement passes. info's
+ * iterations are the refinement steps or the conjugate-gradient iterations. An equality row's
  * dL/db is dl_drl + dl_dru (only the side its multiplier's sign names is nonzero). Any
  * upstream pointer may be NULL (zero); any output pointer may be NULL. Minimisation and
  * maximisation LPs alike (the sense is folded as src/pdhg/pdhg.cpp:95-111 folds it). */
 typedef struct sankhya_gb300_adjoint_info {
-  int32_t status;      /* 0 ok, 1 degenerate optimum (|B| != |R|), 2 CG not converged */
+  int32_t status;      /* 0 ok, 1 degenerate optimum (|B| != |R|), 2 a solve not converged */
   int32_t basic_cols;  /* |B| */
   int32_t active_rows; /* |R| */
   int32_t iterations[2];
@@ -337,7 +338,7 @@ typedef struct sankhya_gb300_adjoint_info {
  * re-solved from the basis matrix A_RB (the adjoint's square solves, started from the
  * reported point); the polished point replaces the reported one when it is primal and dual
  * feasible within 1e-9, and items (may be NULL) receive the new status, objective and
- * residuals. info[k].status: 0 polished, 1 degenerate optimum, 2 CG not converged, 4 LP not
+ * residuals. info[k].status: 0 polished, 1 degenerate optimum, 2 a solve not converged, 4 LP not
  * converged, 5 polished point rejected. */
 SGB_API int sankhya_gb300_batch_polish(sankhya_gb300_batch* batch,
                                        sankhya_gb300_batch_item* items,
@@ -383,7 +384,8 @@ typedef struct sankhya_gb300_qp_params {
   double time_limit;        /* seconds; <= 0 is a zero budget, >= 1e300 means none */
   int64_t random_seed;      /* random_seed (both power-iteration starts) */
   int32_t periods_per_poll; /* 50-iteration check periods per CUDA-graph launch; 0 = auto */
-  int32_t column_lanes;     /* threads per column in the column pass: 1..32, 0 = auto */
+  int32_t column_lanes;     /* threads per column in the column pass: 1..32, 0 = auto (a mean of
+                               up to 64 entries: 1, on layouts of its own) */
   int32_t row_lanes;        /* threads per row in the row pass: 1..32, 0 = auto */
   int32_t staging;          /* 1: one-lane passes stage each warp's matrix slice in shared
                                memory (the same sums; measured slower on GB300, so 0 is the
