@@ -27,7 +27,7 @@ constexpr int kScratch = 16 * (kWideBlockThreads / 32);
 constexpr int kChunkScratch = 2 * (kChunkThreads / 32);
 // The FP32 evaluation tile blocks run 16 consumer warps (the FP32 layouts' lanes are chosen
 // for them).
-using EvalPipeF = TilePipe<float, 2, 0, kWideThreads>;
+using EvalPipeF = TilePipe<float, 2, kWideThreads>;
 constexpr int kSmemF = EvalPipeF::bytes();
 
 // A value formed by thread 0 and handed to every thread of the block (all threads call it).
