@@ -213,8 +213,10 @@ SGB_API int sankhya_gb300_pdhg_spmv(sankhya_gb300_pdhg* engine, int32_t op, int3
  * that hold their vectors in device memory and may not allocate: a device allocation
  * synchronises the whole GPU and fails when a caching allocator has already reserved the
  * memory. `device_in` (cols entries for op 0, rows for op 1) and `device_out` are device
- * pointers; the work is enqueued on `stream` (a cudaStream_t; NULL = the engine's stream)
- * and the call returns without waiting for it. Its only scratch is a fixed device array of
+ * pointers; the work is enqueued on `stream` (a cudaStream_t; NULL = the legacy default stream,
+ * CUDA's own meaning of NULL, or the engine's stream while the legacy one may not be used
+ * because a blocking stream is being captured) and the call returns without waiting for it. The
+ * engine's later calls come after a product enqueued with NULL. Its only scratch is a fixed device array of
  * SANKHYA_GB300_NOALLOC_MAX_CHUNKS partial sums (one per 2048 entries of each row longer than
  * 2048) plus a counter, 128 KiB that every GPU which loads this library keeps until the
  * process exits; a matrix that needs more slots is refused with

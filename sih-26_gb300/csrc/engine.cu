@@ -1169,13 +1169,33 @@ void Engine::spmv_noalloc(int op, int scaled, const double* in, double* out,
                a.nchunks, kCap, kCap, kNoAllocMaxChunks)};
   }
   SGB_CUDA(cudaSetDevice(device_));
-  cudaStream_t s = stream != nullptr ? stream : stream_;
+  // NULL is CUDA's own: the legacy default stream, on which a caller who names no stream has filled
+  // the vectors and reads the result, and which orders such products of several engines among
+  // themselves (they share the scratch). It cannot be used while a blocking stream is captured;
+  // then the engine's stream carries the product.
+  bool on_default = stream == nullptr;
+  if (on_default) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaError_t err = cudaStreamIsCapturing(cudaStreamLegacy, &status);
+    if (err == cudaErrorStreamCaptureImplicit) {
+      cudaGetLastError();
+      on_default = false;
+    } else {
+      SGB_CUDA(err);
+    }
+  }
+  cudaStream_t s = stream != nullptr ? stream : (on_default ? cudaStreamLegacy : stream_);
   double* chunks = nullptr;
   unsigned int* ticket = nullptr;
   SGB_CUDA(noalloc_scratch(device_, s, &chunks, &ticket));
   if (!scaled) a.val = op == 0 ? sl_csr_.raw.ptr : sl_csc_.raw.ptr;
   launch_spmv(a, in, out, chunks, ticket, s);
   SGB_CUDA(cudaGetLastError());
+  if (on_default) {
+    // The engine's own later work (a preconditioning rewrites the scaled values) comes after it.
+    SGB_CUDA(cudaEventRecord(done_event_[0], s));
+    SGB_CUDA(cudaStreamWaitEvent(stream_, done_event_[0], 0));
+  }
 }
 
 void Engine::init_iterates(const sankhya_gb300_params& p) {

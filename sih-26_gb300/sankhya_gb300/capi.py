@@ -360,8 +360,8 @@ class PdhgEngine:
     def spmv_device(self, op: int, device_in: int, device_out: int, scaled: bool = False,
                     stream: Optional[int] = None):
         """The product on caller-owned device buffers (raw device addresses), enqueued on
-        `stream` (a cudaStream_t handle; None = the engine's stream); allocates nothing and
-        does not wait for the work."""
+        `stream` (a cudaStream_t handle; None or 0 = the legacy default stream, torch's default
+        stream); allocates nothing and does not wait for the work."""
         _check(self._lib.sankhya_gb300_pdhg_spmv_noalloc(
             self._h, op, int(scaled), ctypes.c_void_p(device_in), ctypes.c_void_p(device_out),
             ctypes.c_void_p(stream) if stream else None))
