@@ -1605,22 +1605,36 @@ void launch_step_factors(double2* table, long long n, cudaStream_t s) {
   k_step_factors<<<std::max(1, device_sms()) * 8, 256, 0, s>>>(table, n);
 }
 
-void launch_spmv(const SliceSet& a, const double* x, double* y, double* chunk,
+namespace {
+
+// A product combines its rows of several pieces in its last block. Their counters are the step
+// kernels', which may run beside a product on another stream: it leaves them alone.
+SliceSet without_tickets(SliceSet a) {
+  a.tickets = nullptr;
+  return a;
+}
+
+}  // namespace
+
+void launch_spmv(const SliceSet& layout, const double* x, double* y, double* chunk,
                  unsigned int* ticket, cudaStream_t s) {
+  const SliceSet a = without_tickets(layout);
   if (a.nrows == 0) return;
   ++g_launches;
   k_spmv<false, false><<<a.grid, a.threads, 0, s>>>(a, x, y, chunk, ticket, nullptr, nullptr,
                                                     nullptr);
 }
 
-void launch_spmv_scaled(const SliceSet& a, const double* x, double* y, double* chunk,
+void launch_spmv_scaled(const SliceSet& layout, const double* x, double* y, double* chunk,
                         unsigned int* ticket, const double* by, cudaStream_t s) {
+  const SliceSet a = without_tickets(layout);
   ++g_launches;
   k_spmv<true, false><<<a.grid, a.threads, 0, s>>>(a, x, y, chunk, ticket, by, nullptr, nullptr);
 }
 
-void launch_spmv_norm(const SliceSet& a, const double* x, double* y, double* chunk,
+void launch_spmv_norm(const SliceSet& layout, const double* x, double* y, double* chunk,
                       unsigned int* ticket, double* part, double* norm, cudaStream_t s) {
+  const SliceSet a = without_tickets(layout);
   ++g_launches;
   k_spmv<false, true><<<a.grid, a.threads, 0, s>>>(a, x, y, chunk, ticket, nullptr, part, norm);
 }

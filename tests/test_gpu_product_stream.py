@@ -139,3 +139,33 @@ def test_without_a_stream_while_a_blocking_stream_is_captured():
             rt.cudaStreamDestroy(stream)
         torch.cuda.synchronize()
         assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_products_beside_solves(precision):
+    torch = pytest.importorskip("torch")
+    lp = skewed(13)
+    rng = np.random.default_rng(3)
+    x, y = rng.standard_normal(lp.cols), rng.standard_normal(lp.rows)
+    with capi.PdhgEngine(0) as eng:
+        eng.load(lp)
+        want = eng.spmv(0, x), eng.spmv(1, y)
+        eng.solve(tolerance=1e-12, iteration_limit=120, precision=precision)
+        points = eng.solution()
+        side = torch.cuda.Stream()
+        xd, yd = torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda()
+        outs = [(torch.zeros(lp.rows, dtype=torch.float64, device="cuda"),
+                 torch.zeros(lp.cols, dtype=torch.float64, device="cuda")) for _ in range(200)]
+        torch.cuda.synchronize()
+        for solve in range(4):
+            for ax, aty in outs[50 * solve:50 * solve + 50]:
+                eng.spmv_device(0, xd.data_ptr(), ax.data_ptr(), stream=side.cuda_stream)
+                eng.spmv_device(1, yd.data_ptr(), aty.data_ptr(), stream=side.cuda_stream)
+            eng.solve(tolerance=1e-12, iteration_limit=120, precision=precision)
+            for got, ref in zip(eng.solution(), points):
+                assert np.array_equal(got, ref), solve
+        side.synchronize()
+        for ax, aty in outs:
+            assert np.array_equal(ax.cpu().numpy(), want[0])
+            assert np.array_equal(aty.cpu().numpy(), want[1])
