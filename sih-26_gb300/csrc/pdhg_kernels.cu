@@ -398,7 +398,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_pdhg_resident(StepBuffe
       if (s_ctl.eval_now == 0 && s_ctl.iteration >= s_ctl.iteration_limit) {
         s_ctl.done = kIterationLimit;
       }
-      s_tau = s_ctl.eta * s_prep.inv_omega;
+      // eta / omega, rounded as the launch's first step has it: where a period is cut must not show.
+      s_tau = divide(s_ctl.eta, s_ctl.omega, s_prep.inv_omega);
       s_sigma = s_ctl.eta * s_ctl.omega;
     }
     __syncthreads();
@@ -574,7 +575,8 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
       if (s_ctl.eval_now == 0 && s_ctl.iteration >= s_ctl.iteration_limit) {
         s_ctl.done = kIterationLimit;
       }
-      s_tau = s_ctl.eta * s_prep.inv_omega;
+      // eta / omega, rounded as the launch's first step has it: where a period is cut must not show.
+      s_tau = divide(s_ctl.eta, s_ctl.omega, s_prep.inv_omega);
       s_sigma = s_ctl.eta * s_ctl.omega;
     }
     __syncthreads();
