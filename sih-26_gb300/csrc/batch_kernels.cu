@@ -1775,10 +1775,21 @@ __device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjVie
         float* const row = A + static_cast<size_t>(p) * n;
         if (p >= nb) {
           row[p] = 1.0f;
+          mem.row_most[p] = mem.col_most[p] = lu_exponent(1.0f);
           continue;
         }
         size_t e = static_cast<size_t>(r.base[p >> 5]) * 32 + (p & 31);
-        for (int q = 0; q < r.len[p]; ++q, e += 32) row[r.idx[e]] = static_cast<float>(r.val[e]);
+        float most = 0.0f;
+        for (int q = 0; q < r.len[p]; ++q, e += 32) {
+          const float v = static_cast<float>(r.val[e]);
+          row[r.idx[e]] = v;
+          most = fmaxf(most, fabsf(v));
+        }
+        mem.row_most[p] = lu_exponent(most);
+        e = static_cast<size_t>(c.base[p >> 5]) * 32 + (p & 31);
+        most = 0.0f;
+        for (int q = 0; q < c.len[p]; ++q, e += 32) most = fmaxf(most, fabsf(static_cast<float>(c.val[e])));
+        mem.col_most[p] = lu_exponent(most);
       }
       __syncthreads();
       const bool ok = lu_factor(A, n, mem);

@@ -9,7 +9,9 @@
 //
 // Right-looking in panels of kLuPanel columns:
 //   panel    a thread holds two rows of the panel in registers; per column a pivot by integer maxima
-//            of the magnitudes' bits, its row passed through shared memory, one rank-1 update
+//            of the magnitudes' bits, its row passed through shared memory, one rank-1 update; a
+//            pivot that is tiny beside what its row and its column held at the start is rounding
+//            (kLuPivotShare)
 //   U block  a thread per column solves with the panel's unit lower triangle, kLuCols at a time
 //   update   128 x 256 tiles, 8 x 8 a thread, L and U of the panel in shared memory
 // Rows stay in place: piv[k] is the row of the k-th pivot, act the rows without one.
@@ -26,32 +28,50 @@ constexpr int kLuMost = 2 * kLuThreads;  // two panel rows a thread
 constexpr int kLuPanel = 32;
 constexpr int kLuCols = 512;
 constexpr int kLuRow = kLuPanel + 4;  // floats of a row of the panel's triangle
+// The factorisation is refused where the largest entry left in a column is about 2^-16 of the largest
+// that the column, and of the largest that its row, held at the start, or less: 256 roundings of FP32.
+// A basis that is singular to FP32 leaves such pivots. Refinement would still converge where the
+// right-hand side lies in its range, to a solution with an arbitrary part from its null space, where
+// the conjugate gradients find the nearest. Both shares are asked for, so that rows or columns of
+// very different scale do not count as singular.
+constexpr int kLuPivotShare = 16;  // its exponent, negated
 
 __host__ __device__ inline int lu_size(int nb) { return (nb + kLuPanel - 1) / kLuPanel * kLuPanel; }
 
 // Dynamic shared memory of a factorisation of n = lu_size() columns.
 __host__ __device__ inline int lu_smem(int n) {
-  return 4 * (2 * n + kLuPanel * kLuRow + kLuPanel * n + kLuPanel * (n < kLuCols ? n : kLuCols));
+  return 4 * (2 * n + n / 2 + kLuPanel * kLuRow + kLuPanel * n + kLuPanel * (n < kLuCols ? n : kLuCols));
+}
+
+// The exponent field of v's size.
+__device__ __forceinline__ unsigned char lu_exponent(float v) {
+  return static_cast<unsigned char>(__float_as_uint(fabsf(v)) >> 23);
 }
 
 struct LuMem {
   int *piv, *act;
+  unsigned char *row_most, *col_most;  // exponents of the largest magnitudes by row, by column
   float *l11, *lt, *ut;
   __device__ __forceinline__ LuMem(unsigned char* smem, int n)
       : piv(reinterpret_cast<int*>(smem)),
         act(piv + n),
-        l11(reinterpret_cast<float*>(act + n)),
+        row_most(reinterpret_cast<unsigned char*>(act + n)),
+        col_most(row_most + n),
+        l11(reinterpret_cast<float*>(col_most + n)),
         lt(l11 + kLuPanel * kLuRow),
         ut(lt + kLuPanel * n) {}
 };
 
-// Factors the n x n matrix at A (rows of n floats) in place; m.piv receives the pivot rows. All
-// threads call it; false, in all, where a column has no usable pivot.
+// Factors the n x n matrix at A (rows of n floats) in place; m.piv receives the pivot rows, m.row_most
+// and m.col_most hold the exponents of the matrix's largest magnitudes. All threads call it; false,
+// in all, where a column has no usable pivot.
 static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
   __shared__ unsigned s_max[2][kLuThreads / 32];
   __shared__ int s_who[2][kLuThreads / 32];
   __shared__ __align__(16) float s_row[2][kLuPanel];
   __shared__ int s_count[2][kLuThreads / 32];
+  __shared__ int s_weak;
+  if (threadIdx.x == 0) s_weak = 0;
   const int t = static_cast<int>(threadIdx.x), lane = t & 31, warp = t >> 5;
   constexpr int W = kLuThreads / 32;
   const int ldu = n < kLuCols ? n : kLuCols;
@@ -105,7 +125,10 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
           if (j >= c) s_row[c & 1][j] = x;
           else m.l11[c * kLuRow + j] = x;
         }
-        m.piv[k0 + c] = second ? row[1] : row[0];
+        const int at = second ? row[1] : row[0];
+        m.piv[k0 + c] = at;
+        const int least = min(m.row_most[at], m.col_most[k0 + c]) - kLuPivotShare;
+        if (static_cast<int>(top >> 23) <= least) s_weak = 1;
         if (second) live[1] = false;
         else live[0] = false;
       }
@@ -120,6 +143,7 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
         for (int j = c + 1; j < kLuPanel; ++j) v[q][j] = fmaf(-l, s_row[c & 1][j], v[q][j]);
       }
     }
+    if (s_weak != 0) return false;
     // The panel goes back; the rows without a pivot close ranks, their multipliers in m.lt.
     unsigned stay[2];
 #pragma unroll
