@@ -166,8 +166,9 @@ SGB_API int sankhya_gb300_device_available(char* description, int32_t capacity);
 SGB_API int sankhya_gb300_device_free_memory(size_t* free_bytes, size_t* total_bytes);
 SGB_API int sankhya_gb300_device_compute_capability(int32_t* major, int32_t* minor);
 
-/* Device bytes the engine allocates for an LP of this size (replaces
- * estimate_pdhg_gpu_memory, src/gpu/gpu_memory.hpp:35-44). Pure arithmetic. */
+/* Device bytes the engine allocates at most for an LP of this size (replaces
+ * estimate_pdhg_gpu_memory, src/gpu/gpu_memory.hpp:35-44). Pure arithmetic: the layouts depend on
+ * the pattern too, so the figure bounds them, at 1.4 to 2.1 times what common patterns take. */
 SGB_API size_t sankhya_gb300_estimate_memory(int32_t rows, int32_t cols, int64_t nonzeros,
                                              int32_t precision);
 

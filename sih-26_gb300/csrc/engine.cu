@@ -278,22 +278,65 @@ std::string format(const char* fmt, ...) {
 
 }  // namespace
 
+// An upper bound, array by array, of what load() allocates and, for the mixed method, what
+// allocate_mixed() adds. Terms that depend on the pattern are bounded by what the layouts' rules leave
+// possible: a group of 128 lines stores at most 31 places more per entry of its longest short line
+// (64 at most, and no more than the group holds), and cut_chunks ends a chunk of fewer than 31 lines
+// only where the next line would overfill it or is long, so 3 / 256 of the entries bound those. (A
+// split layout also ends a chunk where the window changes; that is not bounded, but its windows hold
+// for runs of chunks by plan_windows' rule and few chunks are as short as the bound has them.)
 size_t estimate_memory(long long rows, long long cols, long long nnz, int precision) {
-  const size_t m = static_cast<size_t>(rows < 0 ? 0 : rows);
-  const size_t n = static_cast<size_t>(cols < 0 ? 0 : cols);
-  const size_t z = static_cast<size_t>(nnz < 0 ? 0 : nnz);
+  const long long z = std::max(nnz, 0LL);
+  const bool mixed = precision == SANKHYA_GB300_MIXED;
   size_t bytes = 0;
-  bytes += (m + 1 + n + 1) * sizeof(int) + 2 * z * sizeof(int);  // CSR + CSC pattern
-  bytes += (m + n) * sizeof(int2);                                // tiles (upper bound)
-  // The sliced layouts: indices, unscaled and scaled values (an eighth for the slices' padding;
-  // a padded slice has at most 31 empty places per entry of its longest row, and the rows are
-  // dealt by length), and the scaled values in the compressed order.
-  bytes += 2 * (z + z / 8) * (sizeof(int) + 2 * sizeof(double)) + 2 * z * sizeof(double);
-  bytes += 4 * (m + n);  // slice records
-  bytes += 20 * n * sizeof(double);     // column vectors (see Engine members)
-  bytes += 16 * m * sizeof(double);     // row vectors
-  if (precision == SANKHYA_GB300_MIXED) {
-    bytes += 2 * z * sizeof(float) + (10 * n + 8 * m) * sizeof(float);
+  // `count` arrays of `n` elements; the driver hands out large allocations in units of 2 MB.
+  const auto add = [&](int count, long long n, size_t size) {
+    constexpr size_t kUnit = 2u << 20;
+    size_t each = (static_cast<size_t>(std::max(n, 0LL)) + kPad) * size;
+    each = each < kUnit / 2 ? (each + 511) & ~size_t{511} : (each + kUnit - 1) / kUnit * kUnit;
+    bytes += static_cast<size_t>(count) * each;
+  };
+  for (const long long lines : {std::max(rows, 0LL), std::max(cols, 0LL)}) {
+    // The compressed pattern and values, and the FP32 evaluation's tiles.
+    add(1, lines + 1, sizeof(int));
+    add(1, z, sizeof(int));
+    add(1, z, sizeof(double));
+    add(1, lines + z / kCap, sizeof(Tile));
+    // The slices: indices, unscaled and scaled values, records; pieces of long lines.
+    const long long groups = (lines + kGroupRows - 1) / kGroupRows;
+    const long long places = z + 31 * std::min<long long>(kSliceLong * groups, z);
+    add(1, places, sizeof(int));
+    add(2, places, sizeof(double));
+    add(1, groups * kGroupRows, sizeof(unsigned short));
+    add(1, groups * kGroupSlices + 1, sizeof(unsigned int));
+    add(1, groups + 1024, sizeof(SliceSeg));
+    add(1, z / kSliceLong, sizeof(SliceItem));
+    add(3, z / kCap, sizeof(LongRow));
+    add(10, 2 * (z / kCap), sizeof(double));  // partials
+    add(1, 2 * (groups + z / kSliceLong), sizeof(double));  // the magnitudes' range
+    // The FP32 step passes' chunks, and the two parts of a split layout.
+    const long long chunks = lines / kChunkRows + 3 * z / kChunkCapF + 2;
+    add(1, chunks, sizeof(Tile));
+    add(1, chunks, sizeof(ChunkSeg));
+    add(2, chunks, sizeof(int));
+    add(2, lines + 1, sizeof(int));
+    add(2, z, sizeof(int));
+    add(1, z / kChunkCapF, sizeof(double));
+    if (!mixed) continue;
+    add(2, z, sizeof(float));
+    add(2, chunks * kChunkCapF, sizeof(float));
+    // The outer part, at most half of the entries: by column, and its sums.
+    add(3, z / 2, sizeof(float));
+    add(1, z / 2, sizeof(unsigned short));
+    add(1, lines, sizeof(float));
+  }
+  add(21, cols, sizeof(double));  // column vectors (see Engine's members), row vectors
+  add(18, rows, sizeof(double));
+  if (mixed) {
+    add(12, cols, sizeof(float));
+    add(12, rows, sizeof(float));
+    add(2, cols, sizeof(double));
+    add(2, rows, sizeof(double));
   }
   // Fixed: the kernels' device code (a 5.8 MB fatbin, loaded at the first launch, after a
   // caller's memory check), the partial-sum buffers and the control block; and the 16 MB
