@@ -5,11 +5,13 @@
 // entries. Each warp of a block works through its own chunks, one at a time, with no
 // barrier between warps:
 //   1. its lanes load the chunk's indices and values straight from global memory, and the per-row
-//      operands of the epilogue, lane l taking row r0 + l. A chunk's entries are PACKED for this:
-//      kChunkCapF places a chunk, lane l's eight (entries l, l + 32, ...) in runs of 16 bytes a lane,
-//      so three or four loads bring what took sixteen of 4 bytes. Where the windows hold all entries
-//      the packed indices are 16 bits from the window's start, and the next chunk's entries are in
-//      flight while this one is summed (with 32-bit indices the registers for that would spill);
+//      operands of the epilogue, lane l taking row r0 + l. Where the windows hold all entries they
+//      are PACKED for this: kChunkCapF places a chunk, lane l's eight (entries l, l + 32, ...) in
+//      runs of 16 bytes a lane, indices as 16 bits from the window's start, so three loads bring
+//      what takes sixteen of 4 bytes, and the next chunk's entries are on their way from when this
+//      one's are staged (asked for earlier they take registers that spill: 54.4 ms against 51.7 for
+//      400 iterations of the block-angular LP of 1M x 2M with nine entries a column). Elsewhere the
+//      loads are the sixteen, less those past the chunk's end;
 //   2. they gather the vector entry of each nonzero -- from the block's staged WINDOW of the
 //      vector in shared memory, or from L2 when the window does not hold it -- and stage the
 //      products in the warp's shared buffer;
@@ -72,9 +74,9 @@ struct ChunkSet {
   const int* ptr;        // rows + 1 (main part)
   const int* idx;        // nnz (+ kPad): the pieces' entries
   const float* val;      // nnz (+ kPad)
-  const float* pval;     // packed values, kChunkCapF per chunk
-  const void* pidx;      // packed indices: uint16 from the window's start, or int
-  int narrow;            // the packed indices are 16 bits
+  int narrow;            // the windows hold every entry of the chunks of whole rows, so these are packed:
+  const float* pval;     // values, kChunkCapF per chunk,
+  const unsigned short* pidx;  // indices from the window's start
   const Tile* chunks;
   const ChunkSeg* segs;
   const int* seg_start;  // per block: its segments [seg_start[b], seg_start[b + 1])
@@ -142,50 +144,68 @@ __device__ __forceinline__ int chunk_lanes(int R) {
   return 32 >> p;
 }
 
-// A lane's eight packed entries of a chunk.
+// A lane's eight entries of a chunk: packed, or (index -1 past the chunk's end) as the layout has them.
+// With 32-bit indices packing does not pay: most chunks of real LPs' columns, two to five entries each,
+// are half empty (400 iterations of a block-angular LP of 1M x 2M at two, three and five entries a
+// column: 44.2, 44.2 and 46.7 ms, packed 49.4, 48.6 and 49.8).
 template <bool NARROW>
-struct PackedEntries {
+struct ChunkEntries {
   static constexpr int kEach = kChunkCapF / 32;
-  static_assert(kEach == 8, "two float4 and one or two uint4 a lane");
+  static_assert(kEach == 8, "two float4 and a uint4 a lane");
+  float a[kEach];
+  int c[kEach];
+  __device__ __forceinline__ void load(const ChunkSet& cs, int, const Tile& ch) {
+    const int lane = static_cast<int>(threadIdx.x) & 31, n = ch.k1 - ch.k0;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      const int k = lane + 32 * j;
+      c[j] = k < n ? ld_stream(cs.idx + ch.k0 + k) : -1;
+      a[j] = k < n ? ld_stream(cs.val + ch.k0 + k) : 0.0f;
+    }
+  }
+  __device__ __forceinline__ void unpack(float (&va)[kEach], int (&vc)[kEach]) const {
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+      va[j] = a[j];
+      vc[j] = c[j];
+    }
+  }
+};
+
+template <>
+struct ChunkEntries<true> {
+  static constexpr int kEach = kChunkCapF / 32;
   float4 a0, a1;
-  uint4 x0, x1;
-  __device__ __forceinline__ void load(const ChunkSet& cs, int chunk) {
+  uint4 x0;
+  __device__ __forceinline__ void load(const ChunkSet& cs, int chunk, const Tile&) {
     const int lane = static_cast<int>(threadIdx.x) & 31;
     const float4* v = reinterpret_cast<const float4*>(cs.pval) + static_cast<size_t>(chunk) * 64 + lane;
     a0 = ld_stream(v);
     a1 = ld_stream(v + 32);
-    const uint4* x = reinterpret_cast<const uint4*>(cs.pidx) +
-                     static_cast<size_t>(chunk) * (NARROW ? 32 : 64) + lane;
-    x0 = ld_stream(x);
-    if (!NARROW) x1 = ld_stream(x + 32);
+    x0 = ld_stream(reinterpret_cast<const uint4*>(cs.pidx) + static_cast<size_t>(chunk) * 32 + lane);
   }
   __device__ __forceinline__ void unpack(float (&a)[kEach], int (&c)[kEach]) const {
     a[0] = a0.x, a[1] = a0.y, a[2] = a0.z, a[3] = a0.w;
     a[4] = a1.x, a[5] = a1.y, a[6] = a1.z, a[7] = a1.w;
-    if (NARROW) {
-      const unsigned w[4] = {x0.x, x0.y, x0.z, x0.w};
+    const unsigned w[4] = {x0.x, x0.y, x0.z, x0.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        c[2 * j] = static_cast<int>(w[j] & 0xffffu);
-        c[2 * j + 1] = static_cast<int>(w[j] >> 16);
-      }
-    } else {
-      c[0] = static_cast<int>(x0.x), c[1] = static_cast<int>(x0.y);
-      c[2] = static_cast<int>(x0.z), c[3] = static_cast<int>(x0.w);
-      c[4] = static_cast<int>(x1.x), c[5] = static_cast<int>(x1.y);
-      c[6] = static_cast<int>(x1.z), c[7] = static_cast<int>(x1.w);
+    for (int j = 0; j < 4; ++j) {
+      c[2 * j] = static_cast<int>(w[j] & 0xffffu);
+      c[2 * j + 1] = static_cast<int>(w[j] >> 16);
     }
   }
 };
 
 // One chunk of whole rows: gather, stage, sum, epilogue (all lanes of the warp call it).
-//   gather(c) -> float        the vector element of packed index c
+//   gather(c) -> float        the vector element of the entries' index c
+//   ahead()                   once the entries are staged: their registers are free
 //   load(row, ops)            the row's NR epilogue operands (lane-per-row, at chunk start)
 //   epi(row, sums, ops)       once per row, on the row's first lane
-template <int NR, bool NARROW, bool OUTER, typename Gather, typename Load, typename Epi>
+template <int NR, bool NARROW, bool OUTER, typename Gather, typename Ahead, typename Load,
+          typename Epi>
 __device__ __forceinline__ void chunk_step(const int* __restrict__ ptr, const Tile& ch,
-                                           const PackedEntries<NARROW>& e, float* buf,
-                                           const float* outer, Gather gather,
+                                           const ChunkEntries<NARROW>& e, float* buf,
+                                           const float* outer, Gather gather, Ahead ahead,
                                            Load load, Epi epi) {
   constexpr int J = kChunkCapF / 32;
   const int lane = static_cast<int>(threadIdx.x) & 31;
@@ -204,8 +224,11 @@ __device__ __forceinline__ void chunk_step(const int* __restrict__ ptr, const Ti
     e.unpack(a, c);
     // Past the chunk's end the entry is a zero that no row reads.
 #pragma unroll
-    for (int j = 0; j < J; ++j) buf[lane + 32 * j] = __fmul_rn(a[j], gather(c[j]));
+    for (int j = 0; j < J; ++j) {
+      buf[lane + 32 * j] = NARROW || c[j] >= 0 ? __fmul_rn(a[j], gather(c[j])) : 0.0f;
+    }
   }
+  ahead();
   __syncwarp();
   const int L = chunk_lanes(R);
   const int g = lane / L, sub = lane & (L - 1);
@@ -339,9 +362,9 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
     const ChunkSeg sg = cs.segs[s];
     // The warp's first chunk of the segment is on its way while the window is.
     Tile ch{0, 0, 0, 0};
-    PackedEntries<NARROW> e;
+    ChunkEntries<NARROW> e;
     if (sg.c0 + warp < sg.c1) {
-      if (NARROW) e.load(cs, sg.c0 + warp);
+      if (NARROW) e.load(cs, sg.c0 + warp, ch);
       ch = cs.chunks[sg.c0 + warp];
     }
     if (sg.len > 0) {
@@ -362,7 +385,7 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
       phase ^= 1u;
     }
     const int lo = sg.lo, len = sg.len;
-    // Of column c, and of packed index c.
+    // Of column c, and of an entry's index c.
     auto gather_column = [&](int c) {
       const unsigned o = static_cast<unsigned>(c - lo);
       return o < static_cast<unsigned>(len) ? win[o] : element<LIVE>(vec + c);
@@ -371,19 +394,18 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
     for (int c = sg.c0 + warp; c < sg.c1; c += W) {
       if (s_abort) break;
       Tile next{0, 0, 0, 0};
-      PackedEntries<NARROW> ahead;
-      if (!NARROW) e.load(cs, c);
-      if (c + W < sg.c1) {
-        if (NARROW) ahead.load(cs, c + W);
-        next = cs.chunks[c + W];
-      }
+      if (!NARROW && ch.r1 >= 0) e.load(cs, c, ch);
+      if (c + W < sg.c1) next = cs.chunks[c + W];
+      const auto ahead = [&] {
+        if (NARROW && c + W < sg.c1) e.load(cs, c + W, next);
+      };
       if (!LIVE && ch.r1 < 0) {
         chunk_piece(cs, ch, piece_part, gather_column);
+        ahead();
       } else {
-        chunk_step<NR, NARROW, OUTER>(cs.ptr, ch, e, buf, cs.outer, gather, load, epi);
+        chunk_step<NR, NARROW, OUTER>(cs.ptr, ch, e, buf, cs.outer, gather, ahead, load, epi);
       }
       ch = next;
-      if (NARROW) e = ahead;
     }
   }
   __syncthreads();
@@ -399,19 +421,13 @@ __device__ __forceinline__ bool run_chunks_impl(const ChunkSet& cs, const float*
 }
 
 // Visit this block's chunks (kernel launched with a multiple of 32 threads, every thread
-// calls it). Returns false -- in every thread -- if a wait gave up.
-template <int NR, typename Load, typename Epi>
+// calls it): NARROW as cs.narrow says, OUTER where cs.outer is not null, a kernel per form. Returns false
+// -- in every thread -- if a wait gave up.
+template <bool NARROW, bool OUTER, int NR, typename Load, typename Epi>
 __device__ __forceinline__ bool run_chunks(const ChunkSet& cs, const float* vec,
                                            unsigned char* dsmem, double* piece_part, Load load,
                                            Epi epi) {
-  if (cs.narrow) {
-    return cs.outer != nullptr
-               ? run_chunks_impl<false, true, true, NR>(cs, vec, dsmem, piece_part, load, epi)
-               : run_chunks_impl<false, true, false, NR>(cs, vec, dsmem, piece_part, load, epi);
-  }
-  return cs.outer != nullptr
-             ? run_chunks_impl<false, false, true, NR>(cs, vec, dsmem, piece_part, load, epi)
-             : run_chunks_impl<false, false, false, NR>(cs, vec, dsmem, piece_part, load, epi);
+  return run_chunks_impl<false, NARROW, OUTER, NR>(cs, vec, dsmem, piece_part, load, epi);
 }
 
 // The same in a kernel that writes the vector itself, for layouts of narrow indices without pieces or

@@ -324,7 +324,8 @@ size_t estimate_memory(long long rows, long long cols, long long nnz, int precis
     add(1, z / kChunkCapF, sizeof(double));
     if (!mixed) continue;
     add(2, z, sizeof(float));
-    add(2, chunks * kChunkCapF, sizeof(float));
+    add(1, chunks * kChunkCapF, sizeof(float));
+    add(1, chunks * kChunkCapF, sizeof(unsigned short));
     // The outer part, at most half of the entries: by column, and its sums.
     add(3, z / 2, sizeof(float));
     add(1, z / 2, sizeof(unsigned short));
@@ -428,13 +429,9 @@ void Engine::allocate_mixed() {
   for (DeviceArray<double>* a : {&anchor_x_, &aty64_}) a->allocate(n);
   for (DeviceArray<double>* a : {&anchor_y_, &ax64_}) a->allocate(m);
   for (ChunkDev* D : {&ck_csc_f_, &ck_csr_f_}) {
-    const size_t places = static_cast<size_t>(D->nchunks) * kChunkCapF;
+    const size_t places = D->narrow ? static_cast<size_t>(D->nchunks) * kChunkCapF : 0;
     D->pval.allocate(places);
-    if (D->narrow) {
-      D->pidx16.allocate(places);
-    } else {
-      D->pidx32.allocate(places);
-    }
+    D->pidx.allocate(places);
     if (!D->split) continue;
     D->fval.allocate_padded(static_cast<size_t>(D->nmain), kPad, s);
     D->foval.allocate_padded(static_cast<size_t>(D->nouter), kPad, s);
@@ -449,10 +446,8 @@ void Engine::allocate_mixed() {
   part_steps_f_.allocate(3 * static_cast<size_t>(std::max(ck_csc_f_.grid, ck_csr_f_.grid)));
   fill_mixed_buffers();
   steps_f_ = mixed_steps_fit(mixed_);
-  launch_pack_indices(mixed_.csc_k, ck_csc_f_.nchunks, ck_csc_f_.lo.ptr,
-                      const_cast<void*>(mixed_.csc_k.pidx), s);
-  launch_pack_indices(mixed_.csr_k, ck_csr_f_.nchunks, ck_csr_f_.lo.ptr,
-                      const_cast<void*>(mixed_.csr_k.pidx), s);
+  launch_pack_indices(mixed_.csc_k, ck_csc_f_.nchunks, ck_csc_f_.lo.ptr, ck_csc_f_.pidx.ptr, s);
+  launch_pack_indices(mixed_.csr_k, ck_csr_f_.nchunks, ck_csr_f_.lo.ptr, ck_csr_f_.pidx.ptr, s);
   mixed_ready_ = true;
 }
 
@@ -904,8 +899,7 @@ void Engine::plan_layout(ChunkDev& D, const std::vector<int>& lptr, const int* l
   D.opos.release();
   D.fosorted.release();
   D.pval.release();
-  D.pidx16.release();
-  D.pidx32.release();
+  D.pidx.release();
 }
 
 ChunkSet Engine::chunk_set(const ChunkDev& D, const int* full_ptr, const int* full_idx,
@@ -921,7 +915,7 @@ ChunkSet Engine::chunk_set(const ChunkDev& D, const int* full_ptr, const int* fu
   c.wmax = D.wmax;
   c.narrow = D.narrow ? 1 : 0;
   c.pval = D.pval.ptr;
-  c.pidx = D.narrow ? static_cast<const void*>(D.pidx16.ptr) : static_cast<const void*>(D.pidx32.ptr);
+  c.pidx = D.pidx.ptr;
   if (D.split) {
     c.ptr = D.ptr.ptr;
     c.idx = D.idx.ptr;

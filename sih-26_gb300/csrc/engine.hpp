@@ -157,10 +157,11 @@ class Engine {
     DeviceArray<unsigned short> opos;  // their places in the order of the rows
     DeviceArray<float> fosorted;
     DeviceArray<double> pieces;  // piece partials
-    // Packed entries, allocated and filled when the mixed method first runs; the values each solve.
+    // Packed entries of a narrow layout, allocated and filled when the mixed method first runs; the
+    // values each solve.
     DeviceArray<float> pval;
-    DeviceArray<unsigned short> pidx16;
-    DeviceArray<int> pidx32, lo;
+    DeviceArray<unsigned short> pidx;
+    DeviceArray<int> lo;
     bool narrow = false;
     int nchunks = 0;
     int nlong = 0, npieces = 0, wmax = 0, grid = 1, smem = 0, nrows = 0;

@@ -340,7 +340,9 @@ ChunkPlan plan_chunks(const std::vector<int>& ptr, const int* idx, int lines, in
                  "staged %.4f, %zu chunks, %zu windows, %zu segments, %zu outer entries, "
                  "%zu outer rounds, %d pieces\n",
                  lines, nnz, cap, p.wmax, p.coverage,
-                 p.split ? "split" : (p.wmax > 0 ? "windowed" : "unstaged"), p.staged,
+                 p.split ? (p.narrow ? "split, packed" : "split")
+                         : (p.wmax == 0 ? "unstaged" : (p.narrow ? "windowed, packed" : "windowed")),
+                 p.staged,
                  p.chunks.size(), windows.size(), p.segs.size(), p.oidx.size(),
                  p.orounds.size(), p.npieces);
   }

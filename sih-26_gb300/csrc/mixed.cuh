@@ -103,9 +103,10 @@ void launch_round_build(const RoundBuffers& r, cudaStream_t s);
 // xbar += u_best / dp (clamped to the box), ybar += v_best / dd; best_x = xbar Dc,
 // best_y = ybar Dr for the exact evaluation.
 void launch_round_update(const RoundBuffers& r, cudaStream_t s);
-// The packed entries of a layout's `count` chunks (chunks.cuh): the indices (lo: the chunks' windows'
-// starts, read where cs.narrow), once per load, and the values, once per solve.
-void launch_pack_indices(const ChunkSet& cs, int count, const int* lo, void* out, cudaStream_t s);
+// The packed entries of a narrow layout's `count` chunks (chunks.cuh; nothing for others): the indices
+// (lo: the chunks' windows' starts), once per load, and the values, once per solve.
+void launch_pack_indices(const ChunkSet& cs, int count, const int* lo, unsigned short* out,
+                         cudaStream_t s);
 void launch_pack_values(const ChunkSet& cs, int count, float* out, cudaStream_t s);
 // A split layout's outer entries by column within each round (chunks.cuh): columns and places once per
 // load, values once per solve.

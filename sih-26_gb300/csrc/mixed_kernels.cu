@@ -50,8 +50,9 @@ __device__ __forceinline__ int grid_stride_begin() {
 
 // ---- Inner step ----------------------------------------------------------------------------
 // The column pass of the block's chunks (or, longs, of the long columns): the squared movement is
-// added to mvf. False where a wait gave up. LIVE: one pass of many in the kernel (k_steps_f).
-template <bool LIVE>
+// added to mvf. False where a wait gave up. LIVE: one pass of many in the kernel (k_steps_f). NARROW,
+// OUTER: the layout's form (run_chunks).
+template <bool LIVE, bool NARROW, bool OUTER>
 __device__ __forceinline__ bool primal_pass(const MixedBuffers& b, int cur, bool add, float tau,
                                             unsigned char* dsmem, bool longs, float& mvf) {
   const float* u = b.u[cur];
@@ -79,11 +80,11 @@ __device__ __forceinline__ bool primal_pass(const MixedBuffers& b, int cur, bool
     run_chunk_long_rows<5>(b.csc_k, b.piece_primal, load, epi);
     return true;
   }
-  return run_chunks<5>(b.csc_k, b.v[cur], dsmem, b.piece_primal, load, epi);
+  return run_chunks<NARROW, OUTER, 5>(b.csc_k, b.v[cur], dsmem, b.piece_primal, load, epi);
 }
 
 // The row pass likewise: sum dv^2 is added to a0, sum dv (A du) to a1.
-template <bool LIVE>
+template <bool LIVE, bool NARROW, bool OUTER>
 __device__ __forceinline__ bool dual_pass(const MixedBuffers& b, int cur, bool add, float sigma,
                                           unsigned char* dsmem, bool longs, float& a0, float& a1) {
   const float* v = b.v[cur];
@@ -132,9 +133,10 @@ __device__ __forceinline__ bool dual_pass(const MixedBuffers& b, int cur, bool a
     run_chunk_long_rows<6>(b.csr_k, b.piece_dual, load, epi);
     return true;
   }
-  return run_chunks<6>(b.csr_k, b.du, dsmem, b.piece_dual, load, epi);
+  return run_chunks<NARROW, OUTER, 6>(b.csr_k, b.du, dsmem, b.piece_dual, load, epi);
 }
 
+template <bool NARROW, bool OUTER>
 __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
   extern __shared__ __align__(16) unsigned char dsmem[];
   __shared__ double scratch[kChunkScratch];
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
   // cycles per SM at the start of every launch.
   const float tau = block_scalar([&] { return static_cast<float>(eta / omega); });
   float mvf = 0.0f;
-  if (!primal_pass<false>(b, cur, add, tau, dsmem, false, mvf) && threadIdx.x == 0) {
+  if (!primal_pass<false, NARROW, OUTER>(b, cur, add, tau, dsmem, false, mvf) && threadIdx.x == 0) {
     raise_error(ctl);
   }
   double mv[1] = {static_cast<double>(mvf)};
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
   }
   if (!arrive_last<1>(mv, scratch, b.part_primal, &ctl->ticket[kTicketPrimal])) return;
   mvf = 0.0f;
-  primal_pass<false>(b, cur, add, tau, dsmem, true, mvf);
+  primal_pass<false, NARROW, OUTER>(b, cur, add, tau, dsmem, true, mvf);
   mv[0] = static_cast<double>(mvf);
   double longs[1], total[1];
   block_sum<1>(mv, scratch, longs);
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
   }
 }
 
+template <bool NARROW, bool OUTER>
 __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
   extern __shared__ __align__(16) unsigned char dsmem[];
   __shared__ double scratch[kChunkScratch];
@@ -196,13 +199,13 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
                               : make_double2(0.0, 0.0);
   const float sigma = block_scalar([&] { return static_cast<float>(eta * omega); });
   float a0 = 0.0f, a1 = 0.0f;  // sum dv^2, sum dv (A du)
-  if (!dual_pass<false>(b, cur, add, sigma, dsmem, false, a0, a1) && threadIdx.x == 0) {
+  if (!dual_pass<false, NARROW, OUTER>(b, cur, add, sigma, dsmem, false, a0, a1) && threadIdx.x == 0) {
     raise_error(ctl);
   }
   double acc2[2] = {static_cast<double>(a0), static_cast<double>(a1)};
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
   a0 = a1 = 0.0f;
-  dual_pass<false>(b, cur, add, sigma, dsmem, true, a0, a1);
+  dual_pass<false, NARROW, OUTER>(b, cur, add, sigma, dsmem, true, a0, a1);
   acc2[0] = a0;
   acc2[1] = a1;
   double longs[2], total[2];
@@ -265,12 +268,12 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_steps_f(MixedBuffers b, in
     float mvf = 0.0f, a0 = 0.0f, a1 = 0.0f;
     bool ok = true;
     if (block < b.grid_step_primal) {
-      ok = primal_pass<true>(b, cur, add, s_tau, dsmem, false, mvf);
+      ok = primal_pass<true, true, false>(b, cur, add, s_tau, dsmem, false, mvf);
     }
     if (!ok && t == 0) b.ctl->error = 1;  // the blocks still meet: a wait that gave up ends the solve
     if (!meet()) return;
     if (block < b.grid_step_dual) {
-      ok = dual_pass<true>(b, cur, add, s_sigma, dsmem, false, a0, a1);
+      ok = dual_pass<true, true, false>(b, cur, add, s_sigma, dsmem, false, a0, a1);
     }
     if (!ok && t == 0) b.ctl->error = 1;
     double sums[3] = {static_cast<double>(mvf), static_cast<double>(a0), static_cast<double>(a1)};
@@ -675,27 +678,25 @@ __global__ void k_fill_float(float* v, int count, float value) {
   for (int k = grid_stride_begin(); k < count; k += gridDim.x * blockDim.x) v[k] = value;
 }
 
-// The packed entries of a chunk layout (chunks.cuh), a warp per chunk: the indices (narrow ones from
-// their window's start, lo[chunk]) and the values. Lane l's entry j of chunk c is at
-// packed_place(c, l, j): values and 32-bit indices in two runs of four a lane, narrow ones in one of
-// eight.
+// The packed entries of a narrow chunk layout (chunks.cuh), a warp per chunk: the indices from their
+// window's start, lo[chunk], and the values. Lane l's entry j of chunk c is at packed_place(c, l, j) of
+// the values, which lie in two runs of four a lane, and in one run of eight of the indices.
 __device__ __forceinline__ size_t packed_place(int c, int lane, int j) {
   return static_cast<size_t>(c) * kChunkCapF + (j >> 2) * 128 + lane * 4 + (j & 3);
 }
 
-template <typename I>
-__global__ void k_pack_indices(const Tile* chunks, int count, const int* lo, const int* idx, I* out) {
+__global__ void k_pack_indices(const Tile* chunks, int count, const int* lo, const int* idx,
+                               unsigned short* out) {
   const int c = static_cast<int>(blockIdx.x) * 8 + static_cast<int>(threadIdx.x >> 5);
   if (c >= count) return;
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const Tile ch = chunks[c];
   const int n = ch.r1 < 0 ? 0 : ch.k1 - ch.k0;
-  const int from = sizeof(I) == 2 ? lo[c] : 0;
+  const int from = lo[c];
   for (int j = 0; j < kChunkCapF / 32; ++j) {
     const int k = lane + 32 * j;
-    const I at = k < n ? static_cast<I>(idx[ch.k0 + k] - from) : I(0);
-    out[sizeof(I) == 2 ? static_cast<size_t>(c) * kChunkCapF + lane * 8 + j
-                       : packed_place(c, lane, j)] = at;
+    out[static_cast<size_t>(c) * kChunkCapF + lane * 8 + j] =
+        static_cast<unsigned short>(k < n ? idx[ch.k0 + k] - from : 0);
   }
 }
 
@@ -769,6 +770,13 @@ int egrid(long long count) {
 
 // Per-device state: whether the kernels' shared-memory limits are set on the device, and
 // the evaluation kernels' occupancy there.
+// The step passes' kernels by the form of their layout: [narrow][split].
+using StepKernel = void (*)(MixedBuffers);
+constexpr StepKernel kPrimalForms[2][2] = {{k_primal_f<false, false>, k_primal_f<false, true>},
+                                           {k_primal_f<true, false>, k_primal_f<true, true>}};
+constexpr StepKernel kDualForms[2][2] = {{k_dual_f<false, false>, k_dual_f<false, true>},
+                                         {k_dual_f<true, false>, k_dual_f<true, true>}};
+
 constexpr int kMaxDevices = 64;
 struct MixedConfig {
   bool configured;
@@ -788,11 +796,17 @@ bool configure_mixed_kernels() {
   std::lock_guard<std::mutex> lock(g_mixed_mutex);
   MixedConfig& c = g_mixed[dev];
   if (c.configured) return true;
+  for (const auto& forms : {kPrimalForms, kDualForms}) {
+    for (int form = 0; form < 4; ++form) {
+      const void* f = reinterpret_cast<const void*>(forms[form >> 1][form & 1]);
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               max_dynamic_smem(f)) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+    }
+  }
   const cudaError_t errs[] = {
-      cudaFuncSetAttribute(k_primal_f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           max_dynamic_smem(reinterpret_cast<const void*>(k_primal_f))),
-      cudaFuncSetAttribute(k_dual_f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           max_dynamic_smem(reinterpret_cast<const void*>(k_dual_f))),
       cudaFuncSetAttribute(k_steps_f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_steps_f))),
       cudaFuncSetAttribute(k_evalf_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemF),
@@ -828,10 +842,13 @@ int mixed_blocks_per_sm() {
 // kWindowBytesMax, in gathered floats (a multiple of 1024).
 int mixed_window_capacity(int pass) {
   configure_mixed_kernels();
-  const void* k = pass == 0 ? reinterpret_cast<const void*>(k_primal_f)
-                            : reinterpret_cast<const void*>(k_dual_f);
-  const int budget =
-      std::min(max_dynamic_smem(k) - chunk_smem(kChunkThreads / 32, 0), kWindowBytesMax);
+  // One capacity for all forms: the layout that it shapes decides the form.
+  int most = kWindowBytesMax + chunk_smem(kChunkThreads / 32, 0);
+  for (int form = 0; form < 4; ++form) {
+    const StepKernel k = (pass == 0 ? kPrimalForms : kDualForms)[form >> 1][form & 1];
+    most = std::min(most, max_dynamic_smem(reinterpret_cast<const void*>(k)));
+  }
+  const int budget = most - chunk_smem(kChunkThreads / 32, 0);
   return budget > 0 ? (budget / static_cast<int>(sizeof(float))) & ~1023 : 0;
 }
 
@@ -844,11 +861,13 @@ int mixed_step_smem(int pass, int wmax) {
 // each occupies a whole SM, and its blocks are placed as the previous kernel's leave, so the
 // launch and the SM's reconfiguration overlap that kernel's last blocks.
 void launch_mixed_primal(const MixedBuffers& b, cudaStream_t s) {
-  launch_after(k_primal_f, b.grid_step_primal, kChunkThreads, b.smem_primal, s, b);
+  launch_after(kPrimalForms[b.csc_k.narrow != 0][b.csc_k.outer != nullptr], b.grid_step_primal,
+               kChunkThreads, b.smem_primal, s, b);
 }
 
 void launch_mixed_dual(const MixedBuffers& b, cudaStream_t s) {
-  launch_after(k_dual_f, b.grid_step_dual, kChunkThreads, b.smem_dual, s, b);
+  launch_after(kDualForms[b.csr_k.narrow != 0][b.csr_k.outer != nullptr], b.grid_step_dual,
+               kChunkThreads, b.smem_dual, s, b);
 }
 
 void launch_mixed_step(const MixedBuffers& b, cudaStream_t s) {
@@ -887,19 +906,14 @@ void launch_round_update(const RoundBuffers& r, cudaStream_t s) {
   k_round_update<<<egrid(r.m > r.n ? r.m : r.n), 256, 0, s>>>(r);
 }
 
-void launch_pack_indices(const ChunkSet& cs, int count, const int* lo, void* out, cudaStream_t s) {
-  if (count <= 0) return;
-  if (cs.narrow) {
-    k_pack_indices<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, lo, cs.idx,
-                                                   static_cast<unsigned short*>(out));
-  } else {
-    k_pack_indices<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, lo, cs.idx,
-                                                   static_cast<int*>(out));
-  }
+void launch_pack_indices(const ChunkSet& cs, int count, const int* lo, unsigned short* out,
+                         cudaStream_t s) {
+  if (count <= 0 || !cs.narrow) return;
+  k_pack_indices<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, lo, cs.idx, out);
 }
 
 void launch_pack_values(const ChunkSet& cs, int count, float* out, cudaStream_t s) {
-  if (count <= 0) return;
+  if (count <= 0 || !cs.narrow) return;
   k_pack_values<<<(count + 7) / 8, 256, 0, s>>>(cs.chunks, count, cs.val, out);
 }
 
