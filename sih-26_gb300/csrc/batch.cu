@@ -119,18 +119,8 @@ void BatchEngine::load(int count, const sankhya_gb300_lp* lps) {
         rval[base + slot] = lp.values[k];
       }
     }
-    // Slice padding of a compact basis matrix in either orientation (ensure_adjoint_buffers).
-    const auto padding = [](const int* p, int lines) {
-      long long longest = 0, past = 0;
-      for (int q = 0; q < lines; ++q) {
-        const long long len = p[q + 1] - p[q];
-        longest = std::max(longest, len);
-        past += len > kSortLength;
-      }
-      return 32 * longest * (2 + (past + 31) / 32);
-    };
-    mats_.back().line_padding =
-        std::max(padding(r.data(), m), padding(lp.col_starts, n));
+    mats_.back().basis_places = std::max(basis_places(r.data(), m, std::min(m, n)),
+                                         basis_places(lp.col_starts, n, std::min(m, n)));
     rptr.insert(rptr.end(), r.begin(), r.end());
     nz += nnz;
     cp += n + 1;
@@ -677,9 +667,6 @@ void BatchEngine::ensure_adjoint_buffers() {
   a_krl_.allocate(M);
   a_kcb_.allocate(M + static_cast<size_t>(count_));
   a_krb_.allocate(M + static_cast<size_t>(count_));
-  // Each LP's compact basis matrix holds at most its matrix's entries, and its slices' padding:
-  // lines come longest first, so a slice is no wider than the lines of the slice before it, which
-  // leaves the first slice (and those of lines past the sort's range) to be covered.
   std::vector<long long> knz(static_cast<size_t>(count_));
   long long nz = 0;
   const size_t room = static_cast<size_t>(adjoint_max_smem());
@@ -689,7 +676,7 @@ void BatchEngine::ensure_adjoint_buffers() {
     const BatchInstance& I = inst_[static_cast<size_t>(k)];
     const BatchMatrix& M = mats_[static_cast<size_t>(I.matrix)];
     knz[static_cast<size_t>(k)] = nz;
-    nz += M.nnz + M.line_padding;
+    nz += M.basis_places;
     // Shared memory that holds the LP's solves whatever its basis, and with a basis of half
     // its entries (solve_basis: six vectors, both matrices, the slices' records).
     const size_t d = static_cast<size_t>(std::min(I.m, I.n));

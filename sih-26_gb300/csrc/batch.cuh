@@ -22,6 +22,8 @@
 // the row box along d must be positive); see batch_farkas in batch_kernels.cu.
 #pragma once
 
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace sgb {
@@ -35,6 +37,24 @@ constexpr int kAdjVectors = 8;         // compact per-LP vectors of the square s
 // Lines of a basis matrix longer than this are ordered among the longest in index order.
 constexpr int kSortLength = 1023;
 
+// The most places that the slices of a basis matrix take (build_basis), for a matrix with these lines:
+// at most `basic` of them, none longer than `basic`. They come longest first, so a slice is no wider
+// than the lines of the slice before it, which leaves the first slice (and those of lines past the
+// sort's range) to be covered beside the entries; and no slice is wider than the longest line.
+inline long long basis_places(const int* starts, int lines, int basic) {
+  long long longest = 0, past = 0;
+  for (int q = 0; q < lines; ++q) {
+    const int len = std::min(starts[q + 1] - starts[q], basic);
+    longest = std::max<long long>(longest, len);
+    past += len > kSortLength;
+  }
+  const long long nnz = lines > 0 ? starts[lines] - starts[0] : 0;
+  const long long entries = std::min(nnz, longest * basic);
+  past = std::min<long long>(past, basic);
+  return std::min(entries + 32 * longest * (2 + (past + 31) / 32),
+                  32 * longest * ((basic + 31) / 32));
+}
+
 // A distinct constraint matrix. Offsets index the packed arrays of BatchBuffers.
 struct BatchMatrix {
   int m, n;
@@ -46,7 +66,7 @@ struct BatchMatrix {
   long long nnz;
   double spectral_norm;  // written by the scaling launch
   double scaled_min_abs, scaled_max_abs;
-  long long line_padding;  // most padding the slices of a compact basis matrix can need
+  long long basis_places;  // of a basis matrix's slices in either orientation, at most
 };
 
 // One LP of the batch.
