@@ -319,11 +319,12 @@ SGB_API int sankhya_gb300_batch_ray(sankhya_gb300_batch* batch, int32_t index, d
  * dl_dx[k] (cols), dl_dy[k] (rows) and dl_df[k], returns dL/dc, dL/d(row_lower),
  * dL/d(row_upper), dL/d(col_lower), dL/d(col_upper) by implicit differentiation of the
  * optimum: at the active set the PDHG fixed point reduces to two square linear systems with
- * the basis matrix A_RB, solved on the device on a compact copy of A_RB: bases of up to 1024
- * columns by FP32 LU factors and FP64 refinement, with 4 n^2 bytes of device memory per LP in
- * flight (n the batch's widest basis); larger ones, and those that FP32 factors cannot solve, by
- * preconditioned conjugate gradients on the normal equations, with refinement passes. info's
- * iterations are the refinement steps or the conjugate-gradient iterations. An equality row's
+ * the basis matrix A_RB, solved on the device on a compact copy of A_RB: LPs of min(rows, cols) up
+ * to 1024 by FP32 LU factors and FP64 refinement, with 4 n^2 bytes of device memory per LP in
+ * flight (n the largest such min of the batch; fewer LPs are in flight where memory is short; held
+ * until a batch without such LPs is loaded or the engine is destroyed); larger ones, and bases that
+ * FP32 factors cannot solve, by preconditioned conjugate gradients on the normal equations, with
+ * refinement passes. An LP's gradients do not depend on the rest of its batch. info's iterations are the refinement steps or the conjugate-gradient iterations. An equality row's
  * dL/db is dl_drl + dl_dru (only the side its multiplier's sign names is nonzero). Any
  * upstream pointer may be NULL (zero); any output pointer may be NULL. Minimisation and
  * maximisation LPs alike (the sense is folded as src/pdhg/pdhg.cpp:95-111 folds it). */

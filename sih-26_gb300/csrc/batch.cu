@@ -670,31 +670,29 @@ void BatchEngine::ensure_adjoint_buffers() {
   std::vector<long long> knz(static_cast<size_t>(count_));
   long long nz = 0;
   const size_t room = static_cast<size_t>(adjoint_max_smem());
-  size_t need = 0, likely = 0;
-  int widest = 1;
+  size_t need = 0;
+  a_lu_size_ = 0;
   for (int k = 0; k < count_; ++k) {
     const BatchInstance& I = inst_[static_cast<size_t>(k)];
     const BatchMatrix& M = mats_[static_cast<size_t>(I.matrix)];
     knz[static_cast<size_t>(k)] = nz;
     nz += M.basis_places;
-    // Shared memory that holds the LP's solves whatever its basis, and with a basis of half
-    // its entries (solve_basis: six vectors, both matrices, the slices' records).
+    // Shared memory that holds the LP's solves whatever its basis (solve_basis: six vectors, both
+    // matrices, the slices' records).
     const size_t d = static_cast<size_t>(std::min(I.m, I.n));
-    widest = std::max(widest, std::min(I.m, I.n));
     const size_t z = static_cast<size_t>(M.nnz);
     need = std::max(need, 64 * d + 20 * (z + 64 * 16) + 256);
-    likely = std::max(likely, 64 * d + 11 * z);
+    // Bases that a block factors densely (dense_lu.cuh) are solved so, whatever the rest of the batch.
+    const int size = lu_size(std::min(I.m, I.n));
+    if (size <= kLuMost && static_cast<size_t>(lu_smem(size)) <= room) {
+      a_lu_size_ = std::max(a_lu_size_, size);
+    }
   }
-  // One block of 256 threads holds the FP64 pipe busy from shared memory; gathers from global
-  // memory want more warps in flight.
   a_smem_ = static_cast<int>(std::min(room, need)) & ~15;
-  a_threads_ = likely <= room ? 256 : kAdjThreads;
-  // Bases that a block factors densely (dense_lu.cuh) are solved so, all of the batch's or none.
-  a_lu_size_ = 0;
-  if (widest <= kLuMost && static_cast<size_t>(lu_smem(lu_size(widest))) <= room) {
-    a_lu_size_ = lu_size(widest);
+  if (a_lu_size_ > 0) {
     a_smem_ = std::max(a_smem_, (lu_smem(a_lu_size_) + 15) & ~15);
-    a_threads_ = kLuThreads;
+  } else {
+    a_lu_.release();
   }
   const size_t Z = static_cast<size_t>(std::max(nz, 1LL));
   a_kci_.allocate(Z);
@@ -711,25 +709,29 @@ void BatchEngine::ensure_adjoint_buffers() {
   adjoint_ready_ = true;
 }
 
-// The blocks of an adjoint or polish launch; with them the LU workspaces, one per block. Without the
-// memory for those the solves run by conjugate gradients.
+// The blocks of an adjoint or polish launch; with them the LU workspaces, one per block, as many as
+// there is memory for. Without the memory for one the solves run by conjugate gradients.
 int BatchEngine::adjoint_grid(AdjointBuffers* a) {
-  const int grid = std::max(
-      1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(a->threads, a->smem_bytes)));
+  int grid =
+      std::max(1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(kAdjThreads, a->smem_bytes)));
   a->lu = nullptr;
   a->lu_size = a_lu_size_;
-  if (a_lu_size_ > 0) {
-    const size_t each = static_cast<size_t>(a_lu_size_) * a_lu_size_;
-    size_t free_bytes = 0, total = 0;
-    const bool room = a_lu_.capacity >= each * grid ||
-                      (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess &&
-                       each * grid * sizeof(float) < free_bytes / 2);
-    if (room) {
-      a_lu_.allocate(each * grid);
-      a->lu = a_lu_.ptr;
-    }
+  if (a_lu_size_ == 0) return grid;
+  const size_t each = static_cast<size_t>(a_lu_size_) * a_lu_size_;
+  size_t free_bytes = 0, total = 0;
+  SGB_CUDA(cudaMemGetInfo(&free_bytes, &total));
+  const int blocks =
+      lu_workspaces(grid, each * sizeof(float), free_bytes + a_lu_.capacity * sizeof(float));
+  try {
+    a_lu_.allocate(each * blocks);
+  } catch (const EngineError& error) {
+    if (error.code != SANKHYA_GB300_ERROR_MEMORY) throw;
+    cudaGetLastError();
+    a_lu_.release();
+    return grid;
   }
-  return grid;
+  a->lu = a_lu_.ptr;
+  return blocks;
 }
 
 AdjointBuffers BatchEngine::adjoint_buffers() {
@@ -762,8 +764,8 @@ AdjointBuffers BatchEngine::adjoint_buffers() {
   a.outcome = a_out_.ptr;
   a.max_iterations = 20000;
   a.cg_tolerance = 1e-13;
-  a.threads = a_threads_;
   a.smem_bytes = a_smem_;
+  a.smem_most = adjoint_max_smem();
   return a;
 }
 

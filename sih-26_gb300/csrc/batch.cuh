@@ -31,7 +31,7 @@ namespace sgb {
 constexpr int kBatchThreads = 256;     // scaling launches of many matrices,
 constexpr int kScaleMaxThreads = 1024; // of no more than the SMs
 constexpr int kBatchMaxThreads = 512;  // the largest block a batched solve runs with
-constexpr int kAdjThreads = 512;       // adjoint and polish launches, at most
+constexpr int kAdjThreads = 512;       // adjoint and polish launches
 constexpr int kAdjVectors = 8;         // compact per-LP vectors of the square solves
 
 // Lines of a basis matrix longer than this are ordered among the longest in index order.
@@ -154,13 +154,13 @@ struct AdjointBuffers {
   int max_iterations;                              // per conjugate-gradient run
   double cg_tolerance;
   int* tmp;                                        // m per LP
-  int threads, smem_bytes;                         // of the launches
+  int smem_bytes, smem_most;                       // of the launches; of any launch
   float* lu;                                       // lu_size^2 per block, or null (dense_lu.cuh)
-  int lu_size;
+  int lu_size;                                     // LPs of min(m, n) up to it are factored
 };
 
 void launch_batch_scaling(const BatchBuffers& b, int grid, int threads, cudaStream_t s);
-// The adjoint and polish launches run blocks of a.threads threads with a.smem_bytes of dynamic
+// The adjoint and polish launches run blocks of kAdjThreads threads with a.smem_bytes of dynamic
 // shared memory; adjoint_max_smem is the most they can have, adjoint_blocks_per_sm their
 // occupancy.
 void launch_batch_adjoint(const BatchBuffers& b, const AdjointBuffers& a, int grid,

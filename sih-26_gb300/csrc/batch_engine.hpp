@@ -77,7 +77,7 @@ class BatchEngine {
   DeviceArray<BatchInstance> d_inst_;
   DeviceArray<int> d_order_;
   DeviceArray<float> a_lu_;  // the adjoint's and the polish's LU workspaces
-  int a_lu_size_ = 0;        // columns each holds; 0: none
+  int a_lu_size_ = 0;        // columns each holds; 0: no LP of the batch is factored
   DeviceArray<double2> step_factors_;  // for iteration counts below kBatchStepFactors (1 MB)
   DeviceArray<unsigned int> d_queue_;
   DeviceArray<int> csc_ptr_, csc_idx_, csr_ptr_, csr_idx_;
@@ -108,7 +108,7 @@ class BatchEngine {
   DeviceArray<unsigned int> a_kcb_, a_krb_;
   DeviceArray<double> a_kcv_, a_krv_;
   DeviceArray<long long> a_knz_;
-  int a_smem_ = 0, a_threads_ = 256;
+  int a_smem_ = 0;
   DeviceArray<signed char> a_cs_, a_rs_;
   DeviceArray<AdjointOutcome> a_out_;
   long long total_n_ = 0, total_m_ = 0, mat_n_ = 0, mat_m_ = 0;

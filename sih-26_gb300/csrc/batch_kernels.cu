@@ -25,6 +25,7 @@ namespace sgb {
 namespace {
 
 constexpr int kBScratch = 16 * (kBatchMaxThreads / 32);
+static_assert(kAdjThreads == kLuThreads, "the factorisation's block");
 // A dual change d is accepted as a Farkas certificate when its value (see batch_farkas) is
 // above this share of the magnitude of the terms that make it up, at two evaluations in a
 // row. For a feasible LP the value is <= 0 in exact arithmetic.
@@ -1587,7 +1588,10 @@ __device__ __forceinline__ void quick_sum(double (&v)[NV], double* scratch) {
   static_assert(NV == 1 || NV == 2, "the warps' totals of one warp's lanes");
   __shared__ double s_total[NV];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  warp_sums<NV>(v);
+  long long bits = 0;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) bits |= __double_as_longlong(v[q]);
+  if (__any_sync(0xffffffffu, bits != 0)) warp_sums<NV>(v);
   if ((lane & (32 / NV - 1)) == 0) scratch[warp_sums_index<NV>(lane) * nw + warp] = v[0];
   __syncthreads();
   if (warp == 0) {
@@ -1611,13 +1615,14 @@ constexpr int kSqVectors = 6;
 // Bound by the FP64 pipe: per line and iteration the two products' entries and eight vector
 // operations. So no thread repeats a division: the reciprocals of the preconditioner are formed
 // once, and the two step scalars by one thread each while the other warps are in the products
-// (512 threads each forming the three scalars took as long as the products).
+// (512 threads each forming the three scalars took as long as the products). The first T threads work;
+// a line's place among them, and so every sum's order, is the LP's own.
 template <typename I>
 __device__ __forceinline__ int pcg_sf(const Lines<I>& S, const Lines<I>& F, int nb,
                                       const SqVectors& x, double* scratch, int max_it,
-                                      double tol) {
+                                      double tol, int T) {
   __shared__ double s_alpha, s_inv;
-  const int T = blockDim.x, th = threadIdx.x;
+  const int th = threadIdx.x < T ? threadIdx.x : nb;  // past every line
   double a0[2] = {0.0, 0.0};
   for (int k = th; k < nb; k += T) {
     const double rk = x.r[k], wk = rk * x.dinv[k];
@@ -1639,8 +1644,8 @@ __device__ __forceinline__ int pcg_sf(const Lines<I>& S, const Lines<I>& F, int 
     }
     quick_sum<1>(a1, scratch);  // also publishes t
     if (!(a1[0] > 0.0)) break;
-    if (th == T - 1) s_alpha = rw / a1[0];
-    if (th == T - 33) s_inv = 1.0 / rw;
+    if (threadIdx.x == T - 1) s_alpha = rw / a1[0];
+    if (threadIdx.x == T - 33) s_inv = 1.0 / rw;
     for (int k = th; k < nb; k += T) x.q[k] = line_dot(S, k, x.t);
     __syncthreads();
     const double alpha = s_alpha, inv = s_inv;
@@ -1674,8 +1679,8 @@ template <typename I>
 __device__ __forceinline__ int solve_square(const Lines<I>& S, const Lines<I>& F, int nb,
                                             const double* h, double* u, const SqVectors& x,
                                             double* scratch, int max_it, double tol,
-                                            double* rel) {
-  const int T = blockDim.x, th = threadIdx.x;
+                                            double* rel, int T) {
+  const int th = threadIdx.x < T ? threadIdx.x : nb;
   double a0[1] = {0.0};
   for (int k = th; k < nb; k += T) {
     double d = 0.0;
@@ -1702,7 +1707,7 @@ __device__ __forceinline__ int solve_square(const Lines<I>& S, const Lines<I>& F
     // a solve started next to the answer (a polish from the PDHG point, or from a neighbour's
     // vertex, sankhya_gb300_batch_set_point) must still solve its small correction to full
     // accuracy, or two neighbouring solves carry different errors of the correction's size.
-    its += pcg_sf(S, F, nb, x, scratch, max_it, fmin(tol * hnorm / rnorm, kPassReduction));
+    its += pcg_sf(S, F, nb, x, scratch, max_it, fmin(tol * hnorm / rnorm, kPassReduction), T);
     __syncthreads();  // z is complete
     for (int k = th; k < nb; k += T) u[k] += line_dot(F, k, x.z);
     __syncthreads();
@@ -1712,9 +1717,21 @@ __device__ __forceinline__ int solve_square(const Lines<I>& S, const Lines<I>& F
 
 // The LP's basis in this block: its factors (dense_lu.cuh) and its copies in shared memory.
 struct BasisState {
+  bool dense;    // the launch has workspaces and the LP is one of those that are factored
+  int threads;   // of the iterations
   int factored;  // 0 not yet, 1 the factors are in the block's workspace, -1 not to be had
   bool copied;   // the matrices are in shared memory (the factors' pivots are not)
 };
+
+// One half of the block holds the FP64 pipe busy from shared memory (1,100 x 2,200, 64 LPs: 52.1 ms, 56.3
+// with all of it); gathers from global memory want more warps in flight. By the LP's size alone, with
+// a basis of half its entries (six vectors, both matrices), so that its sums do not depend on the batch.
+__device__ __forceinline__ BasisState basis_state(const AdjointBuffers& a, const BatchInstance& I,
+                                                  const BatchMatrix& M) {
+  const long long d = min(I.m, I.n), likely = 64 * d + 11 * M.nnz;
+  return BasisState{a.lu != nullptr && d <= a.lu_size, likely <= a.smem_most ? kAdjThreads / 2 : kAdjThreads,
+                    0, false};
+}
 
 // S u = h (F = S') by refinement with the block's LU factors; u as for solve_square. Returns the
 // refinement steps, or -1 - steps where they did not reach tol, with u as it was. The residual, formed
@@ -1775,7 +1792,7 @@ __device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjVie
         float* const row = A + static_cast<size_t>(p) * n;
         if (p >= nb) {
           row[p] = 1.0f;
-          mem.row_most[p] = mem.col_most[p] = lu_exponent(1.0f);
+          mem.row_most(n)[p] = mem.col_most(n)[p] = lu_exponent(1.0f);
           continue;
         }
         size_t e = static_cast<size_t>(r.base[p >> 5]) * 32 + (p & 31);
@@ -1785,11 +1802,11 @@ __device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjVie
           row[r.idx[e]] = v;
           most = fmaxf(most, fabsf(v));
         }
-        mem.row_most[p] = lu_exponent(most);
+        mem.row_most(n)[p] = lu_exponent(most);
         e = static_cast<size_t>(c.base[p >> 5]) * 32 + (p & 31);
         most = 0.0f;
         for (int q = 0; q < c.len[p]; ++q, e += 32) most = fmaxf(most, fabsf(static_cast<float>(c.val[e])));
-        mem.col_most[p] = lu_exponent(most);
+        mem.col_most(n)[p] = lu_exponent(most);
       }
       __syncthreads();
       const bool ok = lu_factor(A, n, mem);
@@ -1828,14 +1845,15 @@ __device__ __noinline__ int solve_factored(const AdjointBuffers& a, const AdjVie
   return -1 - steps;
 }
 
-// The solve of the LP's basis: with LU factors where the launch has a workspace for them
-// (AdjointBuffers::lu) and the basis is not too ill-conditioned for FP32 factors, else by conjugate
+// The solve of the LP's basis: with LU factors where the launch has workspaces for them
+// (AdjointBuffers::lu), the LP's size is in their range (the LP's, so that its solves are the same in
+// every batch) and the basis is not too ill-conditioned for FP32 factors, else by conjugate
 // gradients with the storage this LP gets (see above). `rows` solves with A_RB (S = rows), otherwise
 // with its transpose. Returns the refinement steps or iterations.
 __device__ int solve_basis(const AdjointBuffers& a, const AdjView& w, unsigned char* smem, int nb,
                            BasisState* state, bool rows, const double* h, double* u, double* scratch,
                            double* rel) {
-  if (a.lu != nullptr && state->factored >= 0 && !state->copied && nb <= a.lu_size) {
+  if (state->dense && state->factored >= 0 && !state->copied) {
     const int steps = solve_factored(a, w, smem, nb, state, rows, h, u, scratch, rel);
     if (steps >= 0) return steps;
   }
@@ -1882,24 +1900,24 @@ __device__ int solve_basis(const AdjointBuffers& a, const AdjView& w, unsigned c
     }
     const Lines<unsigned short> r{rl, rb, ri, rv}, c{cl, cb, ci, cv};
     return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
-                        a.cg_tolerance, rel);
+                        a.cg_tolerance, rel, state->threads);
   }
   const Lines<int> r{w.krl, w.krb, w.kri, w.krv}, c{w.kcl, w.kcb, w.kci, w.kcv};
   if (vec <= room) {
     double* const d = reinterpret_cast<double*>(smem);
     const SqVectors x{d, d + nb, d + 2 * nb, d + 3 * nb, d + 4 * nb, d + 5 * nb};
     return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
-                        a.cg_tolerance, rel);
+                        a.cg_tolerance, rel, state->threads);
   }
   if (2 * static_cast<size_t>(nb) * sizeof(double) <= room) {
     double* const d = reinterpret_cast<double*>(smem);
     const SqVectors x{d, d + nb, w.kw[4], w.kw[5], w.kw[6], w.kw[7]};
     return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
-                        a.cg_tolerance, rel);
+                        a.cg_tolerance, rel, state->threads);
   }
   const SqVectors x{w.kw[2], w.kw[3], w.kw[4], w.kw[5], w.kw[6], w.kw[7]};
   return solve_square(rows ? r : c, rows ? c : r, nb, h, u, x, scratch, a.max_iterations,
-                      a.cg_tolerance, rel);
+                      a.cg_tolerance, rel, state->threads);
 }
 
 __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b,
@@ -1919,7 +1937,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_adjoint(BatchBuffers b
     if (t == 0) {
       s_view = make_view(b, I, M);
       s_adj = make_adj_view(a, I, li);
-      s_basis = BasisState{0, false};
+      s_basis = basis_state(a, I, M);
     }
     __syncthreads();
     const LpView& v = s_view;
@@ -2019,7 +2037,7 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_batch_polish(BatchBuffers b,
     if (t == 0) {
       s_view = make_view(b, I, M);
       s_adj = make_adj_view(a, I, li);
-      s_basis = BasisState{0, false};
+      s_basis = basis_state(a, I, M);
     }
     __syncthreads();
     const LpView& v = s_view;
@@ -2165,14 +2183,14 @@ void launch_batch_adjoint(const BatchBuffers& b, const AdjointBuffers& a, int gr
   // A failure here stays the last error, which the caller's launch check reports.
   cudaFuncSetAttribute(k_batch_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        a.smem_bytes);
-  k_batch_adjoint<<<grid, a.threads, a.smem_bytes, s>>>(b, a);
+  k_batch_adjoint<<<grid, kAdjThreads, a.smem_bytes, s>>>(b, a);
 }
 
 void launch_batch_polish(const BatchBuffers& b, const AdjointBuffers& a, int grid,
                          cudaStream_t s) {
   // A failure here stays the last error, which the caller's launch check reports.
   cudaFuncSetAttribute(k_batch_polish, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_bytes);
-  k_batch_polish<<<grid, a.threads, a.smem_bytes, s>>>(b, a);
+  k_batch_polish<<<grid, kAdjThreads, a.smem_bytes, s>>>(b, a);
 }
 
 int adjoint_max_smem() {

@@ -19,6 +19,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sgb {
@@ -43,6 +45,14 @@ __host__ __device__ inline int lu_smem(int n) {
   return 4 * (2 * n + n / 2 + kLuPanel * kLuRow + kLuPanel * n + kLuPanel * (n < kLuCols ? n : kLuCols));
 }
 
+// The workspaces, of `each` bytes and one a block, of a launch that would have `blocks` blocks: with
+// less than twice their memory free the launch has fewer blocks, so that which solves an LP gets, and
+// their bits, do not depend on what else is on the device.
+inline int lu_workspaces(int blocks, size_t each, size_t free_bytes) {
+  const size_t fit = free_bytes / 2 / each;
+  return static_cast<int>(std::max<size_t>(1, std::min<size_t>(fit, static_cast<size_t>(blocks))));
+}
+
 // The exponent field of v's size.
 __device__ __forceinline__ unsigned char lu_exponent(float v) {
   return static_cast<unsigned char>(__float_as_uint(fabsf(v)) >> 23);
@@ -50,16 +60,18 @@ __device__ __forceinline__ unsigned char lu_exponent(float v) {
 
 struct LuMem {
   int *piv, *act;
-  unsigned char *row_most, *col_most;  // exponents of the largest magnitudes by row, by column
   float *l11, *lt, *ut;
   __device__ __forceinline__ LuMem(unsigned char* smem, int n)
       : piv(reinterpret_cast<int*>(smem)),
         act(piv + n),
-        row_most(reinterpret_cast<unsigned char*>(act + n)),
-        col_most(row_most + n),
-        l11(reinterpret_cast<float*>(col_most + n)),
+        l11(reinterpret_cast<float*>(act + n + n / 2)),
         lt(l11 + kLuPanel * kLuRow),
         ut(lt + kLuPanel * n) {}
+  // Exponents of the matrix's largest magnitudes by row and by column, between act and l11.
+  __device__ __forceinline__ unsigned char* row_most(int n) const {
+    return reinterpret_cast<unsigned char*>(act + n);
+  }
+  __device__ __forceinline__ unsigned char* col_most(int n) const { return row_most(n) + n; }
 };
 
 // Factors the n x n matrix at A (rows of n floats) in place; m.piv receives the pivot rows, m.row_most
@@ -70,6 +82,7 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
   __shared__ int s_who[2][kLuThreads / 32];
   __shared__ __align__(16) float s_row[2][kLuPanel];
   __shared__ int s_count[2][kLuThreads / 32];
+  __shared__ unsigned s_top[kLuPanel];
   __shared__ int s_weak;
   if (threadIdx.x == 0) s_weak = 0;
   const int t = static_cast<int>(threadIdx.x), lane = t & 31, warp = t >> 5;
@@ -125,10 +138,8 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
           if (j >= c) s_row[c & 1][j] = x;
           else m.l11[c * kLuRow + j] = x;
         }
-        const int at = second ? row[1] : row[0];
-        m.piv[k0 + c] = at;
-        const int least = min(m.row_most[at], m.col_most[k0 + c]) - kLuPivotShare;
-        if (static_cast<int>(top >> 23) <= least) s_weak = 1;
+        m.piv[k0 + c] = second ? row[1] : row[0];
+        s_top[c] = top;
         if (second) live[1] = false;
         else live[0] = false;
       }
@@ -143,7 +154,10 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
         for (int j = c + 1; j < kLuPanel; ++j) v[q][j] = fmaf(-l, s_row[c & 1][j], v[q][j]);
       }
     }
-    if (s_weak != 0) return false;
+    if (t < kLuPanel) {
+      const int least = min(m.row_most(n)[m.piv[k0 + t]], m.col_most(n)[k0 + t]) - kLuPivotShare;
+      if (static_cast<int>(s_top[t] >> 23) <= least) s_weak = 1;
+    }
     // The panel goes back; the rows without a pivot close ranks, their multipliers in m.lt.
     unsigned stay[2];
 #pragma unroll
@@ -159,6 +173,7 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
       if (lane == 0) s_count[q][warp] = __popc(stay[q]);
     }
     __syncthreads();
+    if (s_weak != 0) return false;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       if (!live[q]) continue;

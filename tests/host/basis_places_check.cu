@@ -2,7 +2,8 @@
 // against the places that the batch's rules give: random matrices, even, skewed, tall and wide, with
 // lines past the sort's range, and random bases of each, dealt longest first (lines past the range in
 // index order) to slices as wide as their longest line. And the bound of a wide LP with a dense row
-// stays with the basis, not with the row. Prints OK and exits 0, or the first failure.
+// stays with the basis, not with the row. The workspaces of the dense factors: as many as blocks where
+// half of the free memory holds them, else fewer, never none. Prints OK and exits 0, or the first failure.
 #include <algorithm>
 #include <cstdio>
 #include <numeric>
@@ -10,6 +11,7 @@
 #include <vector>
 
 #include "batch.cuh"
+#include "dense_lu.cuh"
 
 using namespace sgb;
 
@@ -99,6 +101,11 @@ int main() {
   one[0] = 0;
   if (basis_places(wide.data(), 10, 10) > 32 * 10 || basis_places(one.data(), 100, 100) > 32 * 100 * 4) {
     std::printf("FAIL wide: %lld %lld\n", basis_places(wide.data(), 10, 10), basis_places(one.data(), 100, 100));
+    return 1;
+  }
+  if (lu_workspaces(152, 4 << 20, size_t{200} << 30) != 152 || lu_workspaces(152, 4 << 20, 80 << 20) != 10 ||
+      lu_workspaces(152, 4 << 20, 1 << 20) != 1 || lu_workspaces(1, 4096, 0) != 1) {
+    std::printf("FAIL workspaces\n");
     return 1;
   }
   std::printf("OK\n");
