@@ -245,12 +245,22 @@ __host__ __device__ __forceinline__ double clamp_box_or_nan(double v, double lo,
 // FMA, q + r (1/sigma) rounded once, which is the correctly rounded quotient for operands and
 // results in the normal range (tests/host/qp_division_check.c holds it to IEEE division). Three FP64
 // instructions where a division takes a dozen. An exact first product (r = 0) or a residual that is
-// not a number keeps the product.
-__device__ __forceinline__ double divide(double v, double sigma, double inv) {
+// not finite (an infinite v, or a quotient past the largest number) keeps the product.
+__host__ __device__ __forceinline__ double divide(double v, double sigma, double inv) {
+#ifdef __CUDA_ARCH__
   const double q = __dmul_rn(v, inv);
+#else
+  const double q = v * inv;
+#endif
   const double r = fma(-q, sigma, v);
+#ifdef __CUDA_ARCH__
   const long long size = __double_as_longlong(r) & 0x7fffffffffffffffLL;
-  return size == 0 || size > 0x7ff0000000000000LL ? q : fma(r, inv, q);
+#else
+  long long size;
+  memcpy(&size, &r, sizeof(size));
+  size &= 0x7fffffffffffffffLL;
+#endif
+  return size == 0 || size >= 0x7ff0000000000000LL ? q : fma(r, inv, q);
 }
 
 __device__ __forceinline__ float clamp_box(float v, float lo, float hi) {
