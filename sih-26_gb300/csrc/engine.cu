@@ -49,6 +49,7 @@ Trace::~Trace() {}
 
 void cuda_check(cudaError_t err, const char* what, const char* file, int line) {
   if (err == cudaSuccess) return;
+  cudaGetLastError();  // reported here; the next launch check must not report it again
   char buf[512];
   std::snprintf(buf, sizeof(buf), "CUDA error %s (%s) in %s at %s:%d", cudaGetErrorName(err),
                 cudaGetErrorString(err), what, file, line);

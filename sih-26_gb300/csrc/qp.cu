@@ -63,7 +63,6 @@ QpEngine::QpEngine(int device) : device_(device) {
   norms_.allocate(2 * (kQpPowerSteps + 1));
   product_ticket_.allocate(1);
   SGB_CUDA(cudaMemset(product_ticket_.ptr, 0, sizeof(unsigned int)));
-  dot_out_.allocate(1);
 }
 
 QpEngine::~QpEngine() {
@@ -221,6 +220,10 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
       rows_sliced == rows_sliced_) {
     return;
   }
+  // Until the new layout stands there is none: what throws on the way (memory, a launch) must not leave
+  // the old one's name, or its graph, on arrays that are already replaced.
+  destroy_graph();
+  col_lanes_ = row_lanes_ = 0;
   cudaStream_t s = stream_;
   std::vector<QpChunk> cc, rc;
   const int chunk = nnz_a_ > kQpShortChunkNnz ? kQpMidChunk : kQpShortChunk;
@@ -250,11 +253,9 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
     row_short_blocks_ = row_slices_.view.blocks;
   }
   obj_part_.allocate_padded(static_cast<size_t>(col_short_blocks_), 1, s);
-  col_lanes_ = col_lanes;
-  row_lanes_ = row_lanes;
-  cols_sliced_ = cols_sliced;
-  rows_sliced_ = rows_sliced;
-  const QpDev d = dev();
+  QpDev d = dev();
+  d.col_lanes = col_lanes;
+  d.row_lanes = row_lanes;
   // The smallest QPs iterate in one block (slices.cuh). The line is kQpResidentItems, not what a
   // block or a cluster holds: kernel_launches is read as at least two per iteration from 200 x 400
   // on (tests/test_gpu_qp.py).
@@ -282,7 +283,10 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
   product_part_.allocate(2 * (static_cast<size_t>(qp_product_blocks(d)) +
                               std::max(nlong_cols_, nlong_rows_)));
   SGB_CUDA(cudaStreamSynchronize(s));
-  destroy_graph();
+  col_lanes_ = col_lanes;
+  row_lanes_ = row_lanes;
+  cols_sliced_ = cols_sliced;
+  rows_sliced_ = rows_sliced;
 }
 
 QpDev QpEngine::dev() const {

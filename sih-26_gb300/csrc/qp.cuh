@@ -17,9 +17,9 @@
 // pass on A x, the column pass on the gradient at x) plus one single-block kernel that takes
 // the decision on the device. A row or column is summed by a group of G lanes (G = 1..32,
 // from the mean entries per item); one longer than 64 G entries is cut into chunks of
-// kQpChunk entries, each summed by a warp, and the last chunk to finish (a ticket per item)
-// adds the chunks' sums in chunk order and runs the item's epilogue. Every sum is taken in a
-// fixed order, so a solve is reproducible bit for bit.
+// at most 512 or 1,024 entries (qp_layout.hpp), each summed by a warp, and the last chunk to
+// finish (a ticket per item) adds the chunks' sums in chunk order and runs the item's epilogue.
+// Every sum is taken in a fixed order, so a solve is reproducible bit for bit.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -50,8 +50,7 @@ class QpEngine {
   DeviceArray<int> a_cs_, a_ri_, a_rs_, a_ci_, q_rs_, q_ci_;
   DeviceArray<double> a_cv_, a_rv_, q_v_, cost_, col_lower_, col_upper_, row_lower_,
       row_upper_;
-  DeviceArray<double> x0_, x1_, xbar_, y_, col_dual_, row_dual_, vec_n_, vec_m_, dot_part_,
-      dot_out_;
+  DeviceArray<double> x0_, x1_, xbar_, y_, col_dual_, row_dual_, vec_n_, vec_m_, dot_part_;
 
   // Layout for the current lanes.
   int col_lanes_ = 0, row_lanes_ = 0;
