@@ -1472,9 +1472,10 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   launches_ = launches_setup + (kernel_launch_count() - count_after_capture) +
               graphs_launched_ * graph_launches_;
   r->kernel_launches = launches_;
-  // A resident step gathers every entry from shared memory.
-  r->staged_fraction[0] = resident_ ? 1.0 : sl_csc_.staged;
-  r->staged_fraction[1] = resident_ ? 1.0 : sl_csr_.staged;
+  // A resident step gathers every entry from shared memory, one of a cooperative launch none,
+  // whatever windows the layouts have for the passes by themselves.
+  r->staged_fraction[0] = resident_ ? 1.0 : (steps_ ? 0.0 : sl_csc_.staged);
+  r->staged_fraction[1] = resident_ ? 1.0 : (steps_ ? 0.0 : sl_csr_.staged);
   if (c.error) {
     throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "a tile copy did not complete in time"};
   }
