@@ -133,6 +133,14 @@ inline bool cluster_fits(Kernel kernel, int blocks, int threads, int smem) {
 }
 
 // ---- A grid whose blocks meet --------------------------------------------------------------
+// What a control block's error word holds when a bounded wait gave up, and what the host says then.
+constexpr int kCopyFault = 1;  // for a window or tile copy
+constexpr int kMeetFault = 2;  // for the other blocks of the grid
+inline const char* fault_message(int error) {
+  return error == kMeetFault ? "the blocks of a step kernel did not meet in time"
+                             : "a tile copy did not complete in time";
+}
+
 // A cooperative launch: all blocks run at once, so they may wait for one another. `counter` counts
 // arrivals over launches of the same grid (a multiple of gridDim.x between launches, 64 bits, so it
 // never wraps) and is zeroed with the control block it lives in.
@@ -149,7 +157,8 @@ struct GridMeet {
   }
   // All threads of all blocks meet: what each wrote before is visible to the others after (through
   // ld_live, never through the read-only path). Returns false, in every thread of the block, if
-  // the others did not arrive within kMeetPolls polls (about a second) or `error` was raised.
+  // the others did not arrive within kMeetPolls polls (half a second or more); *error is kMeetFault then.
+  // A block that gave up must not meet again, so the others give up at their next meeting.
   __device__ __forceinline__ bool meet(int* error) {
     constexpr int kMeetPolls = 1 << 21;
     __shared__ int s_met;
@@ -163,7 +172,7 @@ struct GridMeet {
         asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(counter) : "memory");
       } while (now < target && ++polls < kMeetPolls);
       s_met = now >= target;
-      if (now < target) *reinterpret_cast<volatile int*>(error) = 1;
+      if (now < target) *reinterpret_cast<volatile int*>(error) = kMeetFault;
     }
     __syncthreads();
     return s_met != 0;

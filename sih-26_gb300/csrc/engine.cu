@@ -1477,7 +1477,7 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   r->staged_fraction[0] = resident_ ? 1.0 : (steps_ ? 0.0 : sl_csc_.staged);
   r->staged_fraction[1] = resident_ ? 1.0 : (steps_ ? 0.0 : sl_csr_.staged);
   if (c.error) {
-    throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "a tile copy did not complete in time"};
+    throw EngineError{SANKHYA_GB300_ERROR_DEVICE, fault_message(c.error)};
   }
   r->iterations = c.iteration;
   r->attempts = c.attempts;
@@ -1636,7 +1636,7 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
     SGB_CUDA(cudaMemcpyAsync(&c, ctl_mixed_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     SGB_CUDA(cudaStreamSynchronize(s));
     if (c.error) {
-      throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "a tile copy did not complete in time"};
+      throw EngineError{SANKHYA_GB300_ERROR_DEVICE, fault_message(c.error)};
     }
     // A restart moves the anchor to the current iterate (the restart point); otherwise to
     // the better of the last evaluated candidates.

@@ -75,7 +75,7 @@ struct Ctl {
   int do_restart;
   int final_mode;   // the evaluation kernels evaluate (best_x, best_y) only
   int stop_rule;    // 0: the reference's stopping test; 1: relative KKT only
-  int error;        // a bounded wait gave up (nonzero: the host stops with an error)
+  int error;        // a bounded wait gave up (kCopyFault, kMeetFault: the host stops with an error)
   int inner_mode;   // the mixed method's inner loop: a restart ends the round
   double movement, interaction;  // of the last attempted step
   double mv_primal;              // primal half of the movement, from k_primal's last block

@@ -40,7 +40,7 @@ __device__ __forceinline__ float block_scalar(F f) {
 }
 
 __device__ __forceinline__ void raise_error(Ctl* c) {
-  c->error = 1;
+  c->error = kCopyFault;
   c->done = kFault;
 }
 
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_steps_f(MixedBuffers b, in
   grid.start(b.arrivals);
   const auto meet = [&] {
     if (grid.meet(&b.ctl->error)) return true;
-    if (t == 0) raise_error(b.ctl);  // the kernels that follow do nothing
+    if (t == 0) b.ctl->done = kFault;  // the kernels that follow do nothing
     return false;
   };
   __syncthreads();
@@ -270,12 +270,12 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_steps_f(MixedBuffers b, in
     if (block < b.grid_step_primal) {
       ok = primal_pass<true, true, false>(b, cur, add, s_tau, dsmem, false, mvf);
     }
-    if (!ok && t == 0) b.ctl->error = 1;  // the blocks still meet: a wait that gave up ends the solve
+    if (!ok && t == 0) b.ctl->error = kCopyFault;  // the blocks still meet: a wait that gave up ends the solve
     if (!meet()) return;
     if (block < b.grid_step_dual) {
       ok = dual_pass<true, true, false>(b, cur, add, s_sigma, dsmem, false, a0, a1);
     }
-    if (!ok && t == 0) b.ctl->error = 1;
+    if (!ok && t == 0) b.ctl->error = kCopyFault;
     double sums[3] = {static_cast<double>(mvf), static_cast<double>(a0), static_cast<double>(a1)};
     double part[3];
     block_sum<3>(sums, scratch, part);

@@ -77,7 +77,7 @@ int device_sms() {
 }
 
 __device__ __forceinline__ void raise_error(Ctl* c) {
-  c->error = 1;
+  c->error = kCopyFault;
   c->done = kFault;
 }
 
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
   grid.start(b.arrivals);
   const auto meet = [&] {
     if (grid.meet(&b.ctl->error)) return true;
-    if (t == 0) raise_error(b.ctl);  // the kernels that follow do nothing
+    if (t == 0) b.ctl->done = kFault;  // the kernels that follow do nothing
     return false;
   };
   __syncthreads();

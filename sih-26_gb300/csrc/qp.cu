@@ -546,7 +546,7 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
       }
     }
     if (now.error != 0) {
-      throw EngineError{SANKHYA_GB300_ERROR_DEVICE, "the blocks of a step kernel did not meet"};
+      throw EngineError{SANKHYA_GB300_ERROR_DEVICE, fault_message(now.error)};
     }
     base = now.base;
     if (now.done) {
