@@ -712,16 +712,18 @@ void BatchEngine::ensure_adjoint_buffers() {
 // The blocks of an adjoint or polish launch; with them the LU workspaces, one per block, as many as
 // there is memory for. Without the memory for one the solves run by conjugate gradients.
 int BatchEngine::adjoint_grid(AdjointBuffers* a) {
-  int grid =
+  const int grid =
       std::max(1, std::min(count_, num_sms_ * adjoint_blocks_per_sm(kAdjThreads, a->smem_bytes)));
   a->lu = nullptr;
   a->lu_size = a_lu_size_;
   if (a_lu_size_ == 0) return grid;
   const size_t each = static_cast<size_t>(a_lu_size_) * a_lu_size_;
-  size_t free_bytes = 0, total = 0;
-  SGB_CUDA(cudaMemGetInfo(&free_bytes, &total));
-  const int blocks =
-      lu_workspaces(grid, each * sizeof(float), free_bytes + a_lu_.capacity * sizeof(float));
+  int blocks = grid;
+  if (a_lu_.capacity < each * grid) {  // the question takes 30 us
+    size_t free_bytes = 0, total = 0;
+    SGB_CUDA(cudaMemGetInfo(&free_bytes, &total));
+    blocks = lu_workspaces(grid, each * sizeof(float), free_bytes + a_lu_.capacity * sizeof(float));
+  }
   try {
     a_lu_.allocate(each * blocks);
   } catch (const EngineError& error) {

@@ -82,7 +82,6 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
   __shared__ int s_who[2][kLuThreads / 32];
   __shared__ __align__(16) float s_row[2][kLuPanel];
   __shared__ int s_count[2][kLuThreads / 32];
-  __shared__ unsigned s_top[kLuPanel];
   __shared__ int s_weak;
   if (threadIdx.x == 0) s_weak = 0;
   const int t = static_cast<int>(threadIdx.x), lane = t & 31, warp = t >> 5;
@@ -139,7 +138,6 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
           else m.l11[c * kLuRow + j] = x;
         }
         m.piv[k0 + c] = second ? row[1] : row[0];
-        s_top[c] = top;
         if (second) live[1] = false;
         else live[0] = false;
       }
@@ -153,10 +151,6 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
 #pragma unroll
         for (int j = c + 1; j < kLuPanel; ++j) v[q][j] = fmaf(-l, s_row[c & 1][j], v[q][j]);
       }
-    }
-    if (t < kLuPanel) {
-      const int least = min(m.row_most(n)[m.piv[k0 + t]], m.col_most(n)[k0 + t]) - kLuPivotShare;
-      if (static_cast<int>(s_top[t] >> 23) <= least) s_weak = 1;
     }
     // The panel goes back; the rows without a pivot close ranks, their multipliers in m.lt.
     unsigned stay[2];
@@ -173,7 +167,11 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
       if (lane == 0) s_count[q][warp] = __popc(stay[q]);
     }
     __syncthreads();
-    if (s_weak != 0) return false;
+    if (t < kLuPanel) {  // the panel's pivots, kLuPivotShare
+      const int at = m.piv[k0 + t];
+      const int least = min(m.row_most(n)[at], m.col_most(n)[k0 + t]) - kLuPivotShare;
+      if (lu_exponent(A[static_cast<size_t>(at) * n + k0 + t]) <= least) s_weak = 1;
+    }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       if (!live[q]) continue;
@@ -188,6 +186,7 @@ static __device__ __noinline__ bool lu_factor(float* A, int n, LuMem m) {
     }
     na -= kLuPanel;
     __syncthreads();
+    if (s_weak != 0) return false;
     for (int j0 = k0 + kLuPanel; j0 < n; j0 += kLuCols) {
       if (j0 + t < n) {
         float x[kLuPanel];
