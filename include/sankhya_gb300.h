@@ -18,7 +18,9 @@
  * Threads: an engine handle holds one LP (or one batch) and its device state, so calls on
  * one handle must not overlap; a caller that shares a handle between threads serialises
  * them, as the seam does for its one engine. Different handles are independent, except that
- * the kernel-launch count the results report is kept per process.
+ * the kernel-launch count the results report is kept per process, and that a solve whose
+ * periods are single cooperative launches starts each when every SM of the device has room for
+ * a block: beside a kernel that holds SMs for long (a batch in another thread) it waits for it.
  */
 #ifndef SANKHYA_GB300_H
 #define SANKHYA_GB300_H
@@ -236,8 +238,9 @@ SGB_API int sankhya_gb300_pdhg_spmv_noalloc(sankhya_gb300_pdhg* engine, int32_t 
 
 /* Measurement hook: time `reps` attempted PDHG steps on the state the last solve left,
  * each kernel bracketed by CUDA events on the engine's stream. ms[0] = mean duration of the
- * primal (column) pass, ms[1] = mean duration of the dual (row) pass, in milliseconds. The
- * solve's results are restored afterwards. */
+ * primal (column) pass, ms[1] = mean duration of the dual (row) pass, in milliseconds. These are
+ * the passes by themselves; a solve may run a whole period of them in one launch (FP64 solves, and
+ * mixed ones of small LPs). The solve's results are restored afterwards. */
 SGB_API int sankhya_gb300_pdhg_time_kernels(sankhya_gb300_pdhg* engine, int32_t reps,
                                             double* ms);
 
