@@ -18,9 +18,10 @@
  * Threads: an engine handle holds one LP (or one batch) and its device state, so calls on
  * one handle must not overlap; a caller that shares a handle between threads serialises
  * them, as the seam does for its one engine. Different handles are independent, except that
- * the kernel-launch count the results report is kept per process, and that a solve whose
- * periods are single cooperative launches starts each when every SM of the device has room for
- * a block: beside a kernel that holds SMs for long (a batch in another thread) it waits for it.
+ * the kernel-launch count the results report is kept per process. (A solve whose periods are
+ * single cooperative launches, which need every SM, asks when it starts whether other kernels hold
+ * some, and launches its passes one by one then, with the same results; where a long kernel, such
+ * as another thread's batch, starts while the solve runs, the solve waits for it.)
  */
 #ifndef SANKHYA_GB300_H
 #define SANKHYA_GB300_H

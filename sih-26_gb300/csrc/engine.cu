@@ -107,6 +107,7 @@ template struct DeviceArray<BatchOutcome>;
 template struct DeviceArray<AdjointOutcome>;
 template struct DeviceArray<signed char>;
 template struct DeviceArray<long long>;
+template struct DeviceArray<unsigned long long>;
 template struct DeviceArray<ChunkSeg>;
 template struct DeviceArray<QpChunk>;
 template struct DeviceArray<QpCtl>;
@@ -447,6 +448,7 @@ void Engine::allocate_mixed() {
   part_steps_f_.allocate(3 * static_cast<size_t>(std::max(ck_csc_f_.grid, ck_csr_f_.grid)));
   fill_mixed_buffers();
   steps_f_ = mixed_steps_fit(mixed_);
+  if (steps_f_) launch_load_mixed_passes(s);
   launch_pack_indices(mixed_.csc_k, ck_csc_f_.nchunks, ck_csc_f_.lo.ptr, ck_csc_f_.pidx.ptr, s);
   launch_pack_indices(mixed_.csr_k, ck_csr_f_.nchunks, ck_csr_f_.lo.ptr, ck_csr_f_.pidx.ptr, s);
   mixed_ready_ = true;
@@ -493,6 +495,8 @@ void Engine::fill_mixed_buffers() {
   b.arrivals = arrivals_.ptr + 1;
   b.csc_k = chunk_set(ck_csc_f_, csc_ptr_.ptr, csc_idx_.ptr, csc_f_.ptr);
   b.csr_k = chunk_set(ck_csr_f_, csr_ptr_.ptr, csr_idx_.ptr, csr_f_.ptr);
+  const auto whole = [](const ChunkSet& c) { return c.narrow && c.outer == nullptr && c.npieces == 0; };
+  b.whole = whole(b.csc_k) && whole(b.csr_k) ? 1 : 0;
   b.piece_primal = ck_csc_f_.pieces.ptr;
   b.piece_dual = ck_csr_f_.pieces.ptr;
   b.part_rows0 = part_rows0_.ptr;
@@ -510,6 +514,27 @@ void Engine::fill_mixed_buffers() {
   b.n = n_;
 }
 
+int Engine::enqueue_mixed_steps(int steps, int slot, bool together) {
+  int launches = 0;
+  if (together) {
+    // The kernel ends where an evaluation falls due, at most 40 accepted steps on.
+    for (int k = 0; k < steps; k += kResidentAttempts) {
+      launch_mixed_steps(mixed_, std::min(kResidentAttempts, steps - k), stream_);
+      launch_mixed_evaluation(mixed_, stream_);
+      launches += 5;
+    }
+  } else {
+    for (int k = 0; k < steps; ++k) {
+      launch_mixed_step(mixed_, stream_);
+      if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_mixed_evaluation(mixed_, stream_);
+    }
+    launches = graph_kernel_launches(steps);
+  }
+  cudaMemcpyAsync(snapshot_mixed_ + slot, ctl_mixed_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost,
+                  stream_);
+  return launches;
+}
+
 void Engine::build_mixed_graphs(int steps) {
   if (mgraph_steps_ == steps && mgraph_exec_[0] != nullptr) return;
   for (auto& g : mgraph_exec_) {
@@ -519,23 +544,7 @@ void Engine::build_mixed_graphs(int steps) {
   for (int slot = 0; slot < 2; ++slot) {
     cudaGraph_t graph = nullptr;
     SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    if (steps_f_) {
-      // The kernel ends where an evaluation falls due, at most 40 accepted steps on.
-      mgraph_launches_ = 0;
-      for (int k = 0; k < steps; k += kResidentAttempts) {
-        launch_mixed_steps(mixed_, std::min(kResidentAttempts, steps - k), stream_);
-        launch_mixed_evaluation(mixed_, stream_);
-        mgraph_launches_ += 5;
-      }
-    } else {
-      for (int k = 0; k < steps; ++k) {
-        launch_mixed_step(mixed_, stream_);
-        if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_mixed_evaluation(mixed_, stream_);
-      }
-      mgraph_launches_ = graph_kernel_launches(steps);
-    }
-    cudaMemcpyAsync(snapshot_mixed_ + slot, ctl_mixed_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost,
-                    stream_);
+    mgraph_launches_ = enqueue_mixed_steps(steps, slot, steps_f_);
     const cudaError_t end = cudaStreamEndCapture(stream_, &graph);
     SGB_CUDA(end);
     const cudaError_t inst = cudaGraphInstantiate(&mgraph_exec_[slot], graph, 0);
@@ -739,8 +748,8 @@ void Engine::load(const sankhya_gb300_lp& lp) {
     a->allocate(static_cast<size_t>(m) + kPad);
   }
   const int pgrid = std::max(grid_c, grid_r) + num_sms_ * 8;
-  part_primal_.allocate(static_cast<size_t>(grid_c) + sl_csc_.view.nlong);
-  part_dual_.allocate(2 * (static_cast<size_t>(grid_r) + sl_csr_.view.nlong));
+  part_primal_.allocate(static_cast<size_t>(grid_c));
+  part_dual_.allocate(2 * static_cast<size_t>(grid_r));
   part_rows0_.allocate(static_cast<size_t>(grid_r) * kEvalRowSlots);
   part_cols_.allocate(static_cast<size_t>(grid_c + 1) * kEvalColSlots);
   part_rows1_.allocate(static_cast<size_t>(grid_r) * kEvalRowSlots);
@@ -763,6 +772,7 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   part_steps_.allocate(step_parts);
   SGB_CUDA(cudaMemsetAsync(part_steps_.ptr, 0, step_parts * sizeof(double), s));
   arrivals_.allocate(2);  // FP64 and mixed
+  room_.allocate(2);
   tickets_.allocate(4);
   SGB_CUDA(cudaMemsetAsync(tickets_.ptr, 0, 4 * sizeof(unsigned int), s));
   SGB_CUDA(cudaStreamSynchronize(s));
@@ -774,6 +784,7 @@ void Engine::load(const sankhya_gb300_lp& lp) {
   // 5,000 x 10,001 18.3 and 13.8, 60,000 x 120,001 30.8 and 26.9; blocks 500,000 x 1M 120.8 and 112.9;
   // Zipf rows with 200,000 entries 42.1 and 31.1, with 2 million 58.4 and 56.8).
   steps_ = !resident_ && cap < 0 && pdhg_steps_fit(step_);
+  if (steps_) launch_load_passes(s);
   loaded_ = true;
 }
 
@@ -960,8 +971,6 @@ void Engine::fill_buffers() {
   b.ru = rus_.ptr;
   b.step_factors = step_factors_.ptr;
   b.step_factors_n = kStepFactorTable;
-  b.part_primal = part_primal_.ptr;
-  b.part_dual = part_dual_.ptr;
   b.chunk_primal = chunk_primal_.ptr;
   b.chunk_dual = chunk_dual_.ptr;
   b.part_steps = part_steps_.ptr;
@@ -1253,6 +1262,27 @@ void Engine::init_iterates(const sankhya_gb300_params& p) {
   (void)p;
 }
 
+void Engine::enqueue_steps(int steps, int slot, bool together) {
+  if (together) {
+    // Both kernels end where an evaluation falls due, at most 40 accepted steps on.
+    for (int k = 0; k < steps; k += kResidentAttempts) {
+      const int attempts = std::min(kResidentAttempts, steps - k);
+      if (resident_) {
+        launch_pdhg_resident(step_, attempts, resident_smem_, stream_);
+      } else {
+        launch_pdhg_steps(step_, attempts, stream_);
+      }
+      launch_evaluation(eval_, stream_);
+    }
+  } else {
+    for (int k = 0; k < steps; ++k) {
+      launch_pdhg_step(step_, stream_);
+      if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_evaluation(eval_, stream_);
+    }
+  }
+  cudaMemcpyAsync(snapshot_ + slot, ctl_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_);
+}
+
 void Engine::build_graphs(int steps) {
   if (graph_steps_ == steps && graph_exec_[0] != nullptr) return;
   destroy_graphs();
@@ -1260,25 +1290,8 @@ void Engine::build_graphs(int steps) {
     cudaGraph_t graph = nullptr;
     SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     const long long before = kernel_launch_count();
-    if (resident_ || steps_) {
-      // Both kernels end where an evaluation falls due, at most 40 accepted steps on.
-      for (int k = 0; k < steps; k += kResidentAttempts) {
-        const int attempts = std::min(kResidentAttempts, steps - k);
-        if (resident_) {
-          launch_pdhg_resident(step_, attempts, resident_smem_, stream_);
-        } else {
-          launch_pdhg_steps(step_, attempts, stream_);
-        }
-        launch_evaluation(eval_, stream_);
-      }
-    } else {
-      for (int k = 0; k < steps; ++k) {
-        launch_pdhg_step(step_, stream_);
-        if ((k + 1) % kEvalStride == 0 || k + 1 == steps) launch_evaluation(eval_, stream_);
-      }
-    }
+    enqueue_steps(steps, slot, resident_ || steps_);
     graph_launches_ = static_cast<int>(kernel_launch_count() - before);
-    cudaMemcpyAsync(snapshot_ + slot, ctl_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_);
     const cudaError_t end = cudaStreamEndCapture(stream_, &graph);
     SGB_CUDA(end);
     const cudaError_t inst = cudaGraphInstantiate(&graph_exec_[slot], graph, 0);
@@ -1288,15 +1301,14 @@ void Engine::build_graphs(int steps) {
   graph_steps_ = steps;
 }
 
-void Engine::run_graphs(const sankhya_gb300_params& p, double t0, cudaGraphExec_t* graphs,
-                        Ctl* snapshot, bool forward_log, long long iteration_offset,
-                        int* stop_status) {
+void Engine::run_steps(const sankhya_gb300_params& p, double t0,
+                       const std::function<void(int)>& enqueue, Ctl* snapshot, bool forward_log,
+                       long long iteration_offset, int* stop_status) {
   Trace trace("pdhg iterations");
   const bool has_time_limit = p.time_limit < 1e300;
   long long logged = 0;
   auto launch = [&](int slot) {
-    ++graphs_launched_;
-    SGB_CUDA(cudaGraphLaunch(graphs[slot], stream_));
+    enqueue(slot);
     SGB_CUDA(cudaEventRecord(done_event_[slot], stream_));
   };
   // The time limit is checked before any step, as the reference's loop does.
@@ -1352,11 +1364,18 @@ void Engine::setup(const sankhya_gb300_params& p, sankhya_gb300_result* r, doubl
   Trace trace("pdhg scaling");
   cudaStream_t s = stream_;
   SGB_CUDA(cudaMemsetAsync(arrivals_.ptr, 0, 2 * sizeof(unsigned long long), s));
+  const bool together = p.precision == SANKHYA_GB300_MIXED ? steps_f_ : steps_;
+  if (together) launch_room(room_.ptr, num_sms_, s);
   *norm = scale_and_norm(p.random_seed);
   double mm[2] = {0.0, 0.0};
   SGB_CUDA(cudaMemcpyAsync(mm, minmax_.ptr + 2 * scale_blocks(sl_csc_.view), 2 * sizeof(double),
                            cudaMemcpyDeviceToHost, s));
+  unsigned long long span[2] = {0, 0};
+  if (together) {
+    SGB_CUDA(cudaMemcpyAsync(span, room_.ptr, sizeof(span), cudaMemcpyDeviceToHost, s));
+  }
   SGB_CUDA(cudaStreamSynchronize(s));
+  crowded_ = together && crowded(span);
   r->scaled_max_abs = mm[0];
   r->scaled_min_abs = mm[1];
   r->spectral_norm = *norm;
@@ -1457,9 +1476,20 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   const long long launches_setup = kernel_launch_count() - launches_before;
   // Capture launches nothing. A resident step takes a fraction of the time, so by default a graph
   // holds one evaluation period of them, rejected steps included.
-  build_graphs(p.steps_per_poll > 0 ? p.steps_per_poll : (resident_ || steps_ ? kResidentAttempts : 32));
+  const int steps =
+      p.steps_per_poll > 0 ? p.steps_per_poll : (resident_ || steps_ ? kResidentAttempts : 32);
+  if (!crowded_) build_graphs(steps);
   const long long count_after_capture = kernel_launch_count();
-  run_graphs(p, t0, graph_exec_, snapshot_, true, 0, &stop_status);
+  const auto enqueue = [&](int slot) {
+    if (crowded_) {
+      enqueue_steps(steps, slot, false);
+      SGB_CUDA(cudaGetLastError());
+      return;
+    }
+    ++graphs_launched_;
+    SGB_CUDA(cudaGraphLaunch(graph_exec_[slot], stream_));
+  };
+  run_steps(p, t0, enqueue, snapshot_, true, 0, &stop_status);
   const double t_end_loop = now_seconds();
   final_evaluation();
   SGB_CUDA(cudaEventRecord(timing_[1], s));
@@ -1474,8 +1504,9 @@ void Engine::solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, 
   r->kernel_launches = launches_;
   // A resident step gathers every entry from shared memory, one of a cooperative launch none,
   // whatever windows the layouts have for the passes by themselves.
-  r->staged_fraction[0] = resident_ ? 1.0 : (steps_ ? 0.0 : sl_csc_.staged);
-  r->staged_fraction[1] = resident_ ? 1.0 : (steps_ ? 0.0 : sl_csr_.staged);
+  const bool together = steps_ && !crowded_;
+  r->staged_fraction[0] = resident_ ? 1.0 : (together ? 0.0 : sl_csc_.staged);
+  r->staged_fraction[1] = resident_ ? 1.0 : (together ? 0.0 : sl_csr_.staged);
   if (c.error) {
     throw EngineError{SANKHYA_GB300_ERROR_DEVICE, fault_message(c.error)};
   }
@@ -1518,7 +1549,17 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
   const long long launches_setup = kernel_launch_count() - launches_before;
 
   const int steps = p.steps_per_poll > 0 ? p.steps_per_poll : (steps_f_ ? kResidentAttempts : 32);
-  build_mixed_graphs(steps);
+  if (!crowded_) build_mixed_graphs(steps);
+  long long step_launches = 0;
+  const auto enqueue = [&](int slot) {
+    if (crowded_) {
+      step_launches += enqueue_mixed_steps(steps, slot, false);
+      SGB_CUDA(cudaGetLastError());
+      return;
+    }
+    SGB_CUDA(cudaGraphLaunch(mgraph_exec_[slot], stream_));
+    step_launches += mgraph_launches_;
+  };
   const long long limit = p.iteration_limit < 0 ? 1000000 : p.iteration_limit;
   const double inf = std::numeric_limits<double>::infinity();
   const int rgrid = std::min(num_sms_ * 4, std::max(1, (std::max(m_, n_) + 255) / 256));
@@ -1632,7 +1673,7 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
     extra_launches_ += 10;
     SGB_CUDA(cudaGetLastError());
     int round_stop = SANKHYA_GB300_ITERATION_LIMIT;
-    run_graphs(p, t0, mgraph_exec_, snapshot_mixed_, false, 0, &round_stop);
+    run_steps(p, t0, enqueue, snapshot_mixed_, false, 0, &round_stop);
     SGB_CUDA(cudaMemcpyAsync(&c, ctl_mixed_.ptr, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
     SGB_CUDA(cudaStreamSynchronize(s));
     if (c.error) {
@@ -1680,8 +1721,7 @@ void Engine::solve_mixed(const sankhya_gb300_params& p, sankhya_gb300_result* r,
   float device_ms = 0.0f;
   SGB_CUDA(cudaEventElapsedTime(&device_ms, timing_[0], timing_[1]));
   r->device_seconds = 1e-3 * device_ms;
-  launches_ = launches_setup + extra_launches_ +
-              graphs_launched_ * mgraph_launches_;
+  launches_ = launches_setup + extra_launches_ + step_launches;
   r->kernel_launches = launches_;
   r->staged_fraction[0] = ck_csc_f_.staged;
   r->staged_fraction[1] = ck_csr_f_.staged;

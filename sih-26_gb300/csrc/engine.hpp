@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -87,16 +88,20 @@ class Engine {
   void draw_power_start(long long seed);
   double norm_from_steps();
   void init_iterates(const sankhya_gb300_params& p);
+  // `steps` attempted steps with their evaluations on the stream, and the control block's copy to the
+  // snapshot slot. together: in cooperative launches (or the resident kernel), else pass by pass.
+  void enqueue_steps(int steps, int slot, bool together);
+  int enqueue_mixed_steps(int steps, int slot, bool together);  // its kernels
   void build_graphs(int steps);
   void build_mixed_graphs(int steps);
   void destroy_graphs();
   void fill_buffers();
   void fill_mixed_buffers();
   void allocate_mixed();
-  // Runs CUDA graphs of `graph_steps_` steps until the control block behind `snapshot` says
-  // done, the time limit passes or the interrupt flag is raised.
-  void run_graphs(const sankhya_gb300_params& p, double t0, cudaGraphExec_t* graphs,
-                  Ctl* snapshot, bool forward_log, long long iteration_offset, int* stop_status);
+  // Runs runs of steps, each enqueued by enqueue(slot), until the control block behind `snapshot`
+  // says done, the time limit passes or the interrupt flag is raised.
+  void run_steps(const sankhya_gb300_params& p, double t0, const std::function<void(int)>& enqueue,
+                 Ctl* snapshot, bool forward_log, long long iteration_offset, int* stop_status);
   void final_evaluation();
   void setup(const sankhya_gb300_params& p, sankhya_gb300_result* r, double* norm);
   void solve_fp64(const sankhya_gb300_params& p, sankhya_gb300_result* r, double t0);
@@ -208,9 +213,13 @@ class Engine {
   int graph_steps_ = 0;
   int graph_launches_ = 0;  // engine kernels per step graph
   bool steps_ = false;      // FP64 steps run in launch_pdhg_steps' kernel
+  // The current solve found other kernels on SMs (launch_room): its steps run pass by pass instead, with
+  // the same sums, and without a graph, whose instantiation would wait for those kernels.
+  bool crowded_ = false;
+  DeviceArray<unsigned long long> room_;
   DeviceArray<double> part_steps_, part_steps_f_, scaled_norms_;
   bool steps_f_ = false;    // the mixed method's steps run in launch_mixed_steps' kernel
-  int mgraph_launches_ = 0;
+  int mgraph_launches_ = 0;  // engine kernels per mixed step graph
   DeviceArray<unsigned long long> arrivals_;
   bool resident_ = false;   // FP64 steps run in the resident kernel,
   int resident_smem_ = 0;   // with this much shared memory a block

@@ -108,11 +108,9 @@ struct StepBuffers {
   double* dx;
   double* ax[2];
   const double *c, *l, *u, *rl, *ru;  // scaled problem
-  double* part_primal;   // [csc.grid + csc.nlong]
-  double* part_dual;     // [(csr.grid + csr.nlong) * 2]
   double* chunk_primal;  // [csc.nchunks]
   double* chunk_dual;    // [csr.nchunks * 2]
-  double* part_steps;    // [(the larger grid + 2 csc.nlong + csr.nlong) * 3] (k_pdhg_steps)
+  double* part_steps;    // [(the larger grid + 2 csc.nlong + csr.nlong) * 3] (step_totals)
   unsigned long long* arrivals;  // GridMeet's counter
   // The step-size factors by iteration count (decisions.cuh, step_factors).
   const double2* step_factors;
@@ -206,6 +204,13 @@ int resident_threads(const StepBuffers& b);
 // falls due; pdhg_steps_fit: whether the device runs its blocks at once.
 void launch_pdhg_steps(const StepBuffers& b, int attempts, cudaStream_t s);
 bool pdhg_steps_fit(const StepBuffers& b);
+// Launches the passes by themselves to no effect. A kernel's first launch waits for the device's other
+// kernels (its code is loaded then), which a solve beside them must not.
+void launch_load_passes(cudaStream_t s);
+// Asks whether every SM has room for a block of a cooperative grid, without waiting for one (k_room):
+// span receives what crowded(), on the host's copy, decides by.
+void launch_room(unsigned long long* span, int sms, cudaStream_t s);
+bool crowded(const unsigned long long* span);
 void launch_scaling(const ScalingBuffers& b, cudaStream_t s);
 // The sliced copy of a compressed layout's indices and values, and the values back.
 void launch_slice_fill(const SliceSet& S, const int* ptr, const int* idx, const double* val,

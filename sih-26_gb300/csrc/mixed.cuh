@@ -31,6 +31,7 @@ struct MixedBuffers {
   Ctl* ctl;                  // the inner loop's control block
   TileSet<float> csc, csr;   // scaled values in FP32 (evaluation tile layouts)
   ChunkSet csc_k, csr_k;  // the step passes' chunk layouts
+  int whole;              // both are packed over whole vectors, without pieces: k_steps_f may run them
   float* u[2];
   float* v[2];
   float* u_sum;
@@ -91,9 +92,10 @@ void launch_mixed_step(const MixedBuffers& b, cudaStream_t s);
 void launch_mixed_primal(const MixedBuffers& b, cudaStream_t s);
 void launch_mixed_dual(const MixedBuffers& b, cudaStream_t s);
 // Up to `attempts` attempted steps in one cooperative launch, which ends early where an evaluation
-// falls due; mixed_steps_fit: whether the layouts' windows hold the whole vectors and the device
-// runs its blocks at once.
+// falls due; mixed_steps_fit: whether the layouts' windows hold the whole vectors (MixedBuffers::whole)
+// and the device runs its blocks at once.
 void launch_mixed_steps(const MixedBuffers& b, int attempts, cudaStream_t s);
+void launch_load_mixed_passes(cudaStream_t s);  // as launch_load_passes (kernels.cuh)
 bool mixed_steps_fit(const MixedBuffers& b);
 void launch_mixed_evaluation(const MixedBuffers& b, cudaStream_t s);
 // Residual measures of the anchor (needs ax, aty computed): out[0..2].

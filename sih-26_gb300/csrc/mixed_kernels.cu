@@ -136,8 +136,23 @@ __device__ __forceinline__ bool dual_pass(const MixedBuffers& b, int cur, bool a
   return run_chunks<NARROW, OUTER, 6>(b.csr_k, b.du, dsmem, b.piece_dual, load, epi);
 }
 
+// The three sums of a step's decision in layouts that k_steps_f may run (MixedBuffers::whole), a warp each:
+// get(k, q) reads block k's partial of sum q.
+template <typename Get>
+__device__ __forceinline__ void whole_totals(const MixedBuffers& b, double omega, Get get,
+                                             double* s_sums) {
+  if (threadIdx.x >= 96) return;
+  const int q = static_cast<int>(threadIdx.x) >> 5;
+  const double sum = table_sum(max(b.grid_step_primal, b.grid_step_dual),
+                               [&](int k) { return get(k, q); });
+  if ((threadIdx.x & 31) == 0) {
+    s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? (0.5 * sum) / omega : sum);
+  }
+}
+
 template <bool NARROW, bool OUTER>
 __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
+  if (b.ctl == nullptr) return;  // launch_load_mixed_passes
   extern __shared__ __align__(16) unsigned char dsmem[];
   __shared__ double scratch[kChunkScratch];
   grid_dependency_wait();  // the previous kernel's results (launch_after)
@@ -185,6 +200,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_primal_f(MixedBuffers b) {
 
 template <bool NARROW, bool OUTER>
 __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
+  if (b.ctl == nullptr) return;  // launch_load_mixed_passes
   extern __shared__ __align__(16) unsigned char dsmem[];
   __shared__ double scratch[kChunkScratch];
   grid_dependency_wait();  // the previous kernel's results (launch_after)
@@ -204,6 +220,23 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_dual_f(MixedBuffers b) {
   }
   double acc2[2] = {static_cast<double>(a0), static_cast<double>(a1)};
   if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
+  if (NARROW && !OUTER && b.whole != 0) {
+    // A layout that k_steps_f may run: its sums, in its order.
+    __shared__ double s_sums[3];
+    whole_totals(b, omega, [&](int k, int q) {
+      return q == 0 ? (k < b.grid_step_primal ? __ldcg(b.part_primal + k) : 0.0)
+                    : (k < b.grid_step_dual ? __ldcg(b.part_dual + 2 * k + q - 1) : 0.0);
+    }, s_sums);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      ctl->ticket[kTicketDual] = 0;
+      if (ctl->done == kRunning) {
+        ctl->mv_primal = s_sums[0];
+        step_decision(ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), factors);
+      }
+    }
+    return;
+  }
   a0 = a1 = 0.0f;
   dual_pass<false, NARROW, OUTER>(b, cur, add, sigma, dsmem, true, a0, a1);
   acc2[0] = a0;
@@ -236,7 +269,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_steps_f(MixedBuffers b, in
   __shared__ float s_tau, s_sigma;
   constexpr int kWords = static_cast<int>(sizeof(Ctl) / sizeof(unsigned long long));
   const int t = static_cast<int>(threadIdx.x), T = static_cast<int>(blockDim.x);
-  const int block = static_cast<int>(blockIdx.x), G = static_cast<int>(gridDim.x);
+  const int block = static_cast<int>(blockIdx.x);
   unsigned long long* const words = reinterpret_cast<unsigned long long*>(&s_ctl);
   for (int k = t; k < kWords; k += T) {
     words[k] = reinterpret_cast<const volatile unsigned long long*>(b.ctl)[k];
@@ -283,14 +316,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_steps_f(MixedBuffers b, in
       for (int q = 0; q < 3; ++q) b.part_steps[3 * block + q] = part[q];
     }
     if (!meet()) return;
-    if (t < 96) {
-      const int q = t >> 5;
-      const double sum = table_sum(G, [&](int k) { return __ldcg(b.part_steps + 3 * k + q); });
-      if ((t & 31) == 0) {
-        const double omega = s_ctl.omega;
-        s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? (0.5 * sum) / omega : sum);
-      }
-    }
+    whole_totals(b, s_ctl.omega, [&](int k, int q) { return __ldcg(b.part_steps + 3 * k + q); }, s_sums);
     __syncthreads();
     if (t == 0) {
       s_ctl.mv_primal = s_sums[0];
@@ -876,10 +902,14 @@ void launch_mixed_step(const MixedBuffers& b, cudaStream_t s) {
 }
 
 bool mixed_steps_fit(const MixedBuffers& b) {
-  const auto whole = [](const ChunkSet& c) { return c.narrow && c.outer == nullptr && c.npieces == 0; };
-  return configure_mixed_kernels() && whole(b.csc_k) && whole(b.csr_k) &&
+  return configure_mixed_kernels() && b.whole != 0 &&
          grid_fits(k_steps_f, std::max(b.grid_step_primal, b.grid_step_dual), kChunkThreads,
                    std::max(b.smem_primal, b.smem_dual));
+}
+
+void launch_load_mixed_passes(cudaStream_t s) {
+  k_primal_f<true, false><<<1, 32, 0, s>>>(MixedBuffers{});
+  k_dual_f<true, false><<<1, 32, 0, s>>>(MixedBuffers{});
 }
 
 void launch_mixed_steps(const MixedBuffers& b, int attempts, cudaStream_t s) {

@@ -88,8 +88,27 @@ __device__ bool fp64_stop_test(const Ctl* c, const Residuals& r) {
                                  (c->stop_at_request || meets_project_standard(r));
 }
 
+// The three sums of a step's decision, a warp each (the block's first 96 threads): the primal movement,
+// the dual movement over omega, the interaction. From the blocks' partials, those of the long columns
+// (half: which of their two sets) and those of the long rows; entries that a column or a row does not
+// have, or a block past its layout's grid, stay zero. The order is the same whichever kernel adds.
+__device__ __forceinline__ void step_totals(const StepBuffers& b, int half, double omega,
+                                            double inv_omega, double* s_sums) {
+  if (threadIdx.x >= 96) return;
+  const int q = static_cast<int>(threadIdx.x) >> 5;
+  const int G = max(b.csc.grid, b.csr.grid), nc = b.csc.nlong;
+  const double sum = table_sum(G + nc + b.csr.nlong, [&](int k) {
+    const int skip = k < G ? 0 : (k < G + nc ? half * nc : nc);
+    return __ldcg(b.part_steps + 3 * (k + skip) + q);
+  });
+  if ((threadIdx.x & 31) == 0) {
+    s_sums[q] = q == 0 ? 0.5 * omega * sum : (q == 1 ? 0.5 * sum * inv_omega : sum);
+  }
+}
+
 // ---- k_primal ----------------------------------------------------------------------------
 __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
+  if (b.ctl == nullptr) return;  // launch_load_passes
   extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
   SliceStart<kPiece> start;
@@ -142,7 +161,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
     const double sum = mv[0];
     mv[0] = 0.0;
     epi(j, s, o);
-    b.part_primal[b.csc.grid + l] = mv[0];
+    b.part_steps[3 * (max(b.csc.grid, b.csr.grid) + l)] = mv[0];
     mv[0] = sum;
   };
   if (!run_slices<true, 1, 5>(b.csc, start, y, fetch, dsmem, b.chunk_primal, mac, load, epi,
@@ -150,15 +169,16 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_primal(StepBuffers b) {
       threadIdx.x == 0) {
     raise_error(ctl);
   }
-  // Each block publishes its partial, and k_dual's last block sums them in block order
-  // (primal_movement). No block of this pass waits for another.
+  // Each block publishes its partial, and k_dual's last block sums them (step_totals). No block of
+  // this pass waits for another.
   double out[1];
   block_sum<1>(mv, scratch, out);
-  if (threadIdx.x == 0) b.part_primal[blockIdx.x] = out[0];
+  if (threadIdx.x == 0) b.part_steps[3 * blockIdx.x] = out[0];
 }
 
 // ---- k_dual ------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
+  if (b.ctl == nullptr) return;  // launch_load_passes
   extern __shared__ __align__(128) unsigned char dsmem[];
   __shared__ double scratch[kScratch];
   SliceStart<kPiece> start;
@@ -169,20 +189,20 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
   const bool add = ctl->pending_add != 0;
   const double omega = ctl->omega, eta = ctl->eta;
   if (done != kRunning || eval_now != 0) return;
-  // The step-size factors of this step, loaded now for the decision the last block takes.
-  const double2 factors = threadIdx.x == 0
-                              ? step_factors(ctl->iteration, b.step_factors, b.step_factors_n)
-                              : make_double2(0.0, 0.0);
+  // What the last block's decision needs beside the sums, formed now.
+  __shared__ StepPrep s_prep;
+  __shared__ double s_sums[3];
+  if (threadIdx.x == blockDim.x - 1) {
+    s_prep.set(ctl, step_factors(ctl->iteration, b.step_factors, b.step_factors_n));
+  }
   const double* __restrict__ y = b.y[cur];
   double* __restrict__ yn = b.y[cur ^ 1];
   const double* __restrict__ dx = b.dx;
   const double* __restrict__ ax = b.ax[cur];
   double* __restrict__ axn = b.ax[cur ^ 1];
-  __shared__ double s_inv_sigma;
   const double sigma = eta * omega;
-  if (threadIdx.x == 0) s_inv_sigma = 1.0 / sigma;
   __syncthreads();
-  const double inv_sigma = s_inv_sigma;
+  const double inv_sigma = s_prep.inv_sigma;
   double acc2[2] = {0.0, 0.0};  // sum dy^2, sum dy (A dx)
   auto fetch = [&](int j) { return __ldg(dx + j); };
   auto mac = [](double v, double g, double* acc) { acc[0] = fma(v, g, acc[0]); };
@@ -212,8 +232,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
     const double sums[2] = {acc2[0], acc2[1]};
     acc2[0] = acc2[1] = 0.0;
     epi(i, s, o);
+    const int at = max(b.csc.grid, b.csr.grid) + 2 * b.csc.nlong + l;
     for (int q = 0; q < 2; ++q) {
-      b.part_dual[2 * (b.csr.grid + l) + q] = acc2[q];
+      b.part_steps[3 * at + 1 + q] = acc2[q];
       acc2[q] = sums[q];
     }
   };
@@ -222,16 +243,25 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_dual(StepBuffers b) {
       threadIdx.x == 0) {
     raise_error(ctl);
   }
-  if (!arrive_last<2>(acc2, scratch, b.part_dual, &ctl->ticket[kTicketDual])) return;
-  double total[2];
-  sum_partials<2>(b.part_dual, b.csr.grid + b.csr.nlong, scratch, total);
-  const double mv_primal = primal_movement(true, b.part_primal, b.csc.grid + b.csc.nlong, omega, ctl,
-                                           scratch);
+  double out[2];
+  block_sum<2>(acc2, scratch, out);
+  __shared__ int s_last;
+  if (threadIdx.x == 0) {
+    b.part_steps[3 * blockIdx.x + 1] = out[0];
+    b.part_steps[3 * blockIdx.x + 2] = out[1];
+    __threadfence();
+    s_last = atomicAdd(&ctl->ticket[kTicketDual], 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  step_totals(b, 0, omega, s_prep.inv_omega, s_sums);
+  __syncthreads();
   if (threadIdx.x == 0) {
     ctl->ticket[kTicketDual] = 0;
     if (ctl->done == kRunning) {
-      const double movement = mv_primal + (0.5 * total[0]) / omega;
-      step_decision(ctl, movement, fabs(total[1]), factors);
+      ctl->mv_primal = s_sums[0];
+      step_decision(ctl, s_sums[0] + s_sums[1], fabs(s_sums[2]), s_prep);
     }
   }
 }
@@ -434,7 +464,6 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
   constexpr int kWords = static_cast<int>(sizeof(Ctl) / sizeof(unsigned long long));
   const int t = static_cast<int>(threadIdx.x), T = static_cast<int>(blockDim.x);
   const int block = static_cast<int>(blockIdx.x), G = static_cast<int>(gridDim.x);
-  const int lane = t & 31;
   unsigned long long* const words = reinterpret_cast<unsigned long long*>(&s_ctl);
   for (int k = t; k < kWords; k += T) {
     words[k] = reinterpret_cast<const volatile unsigned long long*>(b.ctl)[k];
@@ -553,21 +582,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
     }
     if (block < b.csc.grid) start_slices(b.csc, cols);
     if (!meet()) return;
-    // A warp per sum: the primal movement, the dual movement over omega, the interaction.
-    if (t < 96) {
-      const int q = t >> 5;
-      // The blocks', the long columns' of this attempt (a block still at the last decision reads the
-      // other half) and the long rows'; entries that a column or a row does not have stay zero.
-      const int nc = b.csc.nlong;
-      const double sum = table_sum(G + nc + b.csr.nlong, [&](int k) {
-        const int skip = k < G ? 0 : (k < G + nc ? (a & 1) * nc : nc);
-        return __ldcg(b.part_steps + 3 * (k + skip) + q);
-      });
-      if (lane == 0) {
-        s_sums[q] = q == 0 ? 0.5 * s_ctl.omega * sum
-                           : (q == 1 ? 0.5 * sum * s_prep.inv_omega : sum);
-      }
-    }
+    // The long columns' partials of this attempt: a block still at the last decision reads the other
+    // half.
+    step_totals(b, a & 1, s_ctl.omega, s_prep.inv_omega, s_sums);
     __syncthreads();
     if (t == 0) {
       s_ctl.mv_primal = s_sums[0];
@@ -583,6 +600,27 @@ __global__ void __launch_bounds__(kSliceThreads, 1) k_pdhg_steps(StepBuffers b, 
   }
   if (block == 0) {
     for (int k = t; k < kWords; k += T) reinterpret_cast<unsigned long long*>(b.ctl)[k] = words[k];
+  }
+}
+
+// ---- Room for a cooperative grid -------------------------------------------------------------
+// A cooperative launch starts when every SM has room for its block: beside a kernel that holds SMs for
+// seconds (a batch in another thread) it would wait for that kernel's end, where launches of single
+// passes share what is free. So a solve asks first. A block here takes all of an SM's shared memory, so
+// that no other block is resident beside it, notes when it started and stays kRoomStay ns; it waits
+// for nobody. span[0] = ~(first start), span[1] = last start: where SMs are held, blocks start that
+// late or later.
+constexpr long long kRoomStay = 8000;
+__device__ __forceinline__ long long global_ns() {
+  long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+__global__ void k_room(unsigned long long* span) {
+  const long long start = global_ns();
+  atomicMax(span, ~static_cast<unsigned long long>(start));
+  atomicMax(span + 1, static_cast<unsigned long long>(start));
+  for (int polls = 0; polls < 100000 && global_ns() - start < kRoomStay; ++polls) {
   }
 }
 
@@ -1419,6 +1457,8 @@ bool configure_fp64_kernels() {
                            max_dynamic_smem(reinterpret_cast<const void*>(k_primal))),
       cudaFuncSetAttribute(k_dual, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_dual))),
+      cudaFuncSetAttribute(k_room, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           max_dynamic_smem(reinterpret_cast<const void*>(k_room))),
       cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            max_dynamic_smem(reinterpret_cast<const void*>(k_pdhg_resident))),
       cudaFuncSetAttribute(k_pdhg_resident, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
@@ -1447,12 +1487,13 @@ int fp64_window_capacity(int pass) {
 }
 
 void launch_primal_pass(const StepBuffers& b, cudaStream_t s) {
-  launch_after(k_primal, b.csc.grid, b.csc.threads, slice_smem<double>(b.csc.wmax), s, b);
+  // As many threads as k_pdhg_steps has, so that the warps' slices, and every sum, are the same.
+  launch_after(k_primal, b.csc.grid, kSliceThreads, slice_smem<double>(b.csc.wmax), s, b);
   ++g_launches;
 }
 
 void launch_dual_pass(const StepBuffers& b, cudaStream_t s) {
-  launch_after(k_dual, b.csr.grid, b.csr.threads, slice_smem<double>(b.csr.wmax), s, b);
+  launch_after(k_dual, b.csr.grid, kSliceThreads, slice_smem<double>(b.csr.wmax), s, b);
   ++g_launches;
 }
 
@@ -1481,6 +1522,23 @@ bool resident_fits(const StepBuffers& b, int smem) {
 void launch_pdhg_resident(const StepBuffers& b, int attempts, int smem, cudaStream_t s) {
   ++g_launches;
   launch_cluster(k_pdhg_resident, b.csc.grid, resident_threads(b), smem, s, b, attempts);
+}
+
+void launch_load_passes(cudaStream_t s) {
+  g_launches += 2;
+  k_primal<<<1, 32, 0, s>>>(StepBuffers{});
+  k_dual<<<1, 32, 0, s>>>(StepBuffers{});
+}
+
+void launch_room(unsigned long long* span, int sms, cudaStream_t s) {
+  configure_fp64_kernels();
+  ++g_launches;
+  cudaMemsetAsync(span, 0, 2 * sizeof(unsigned long long), s);
+  k_room<<<sms, 1, max_dynamic_smem(reinterpret_cast<const void*>(k_room)), s>>>(span);
+}
+
+bool crowded(const unsigned long long* span) {
+  return span[1] - ~span[0] >= static_cast<unsigned long long>(kRoomStay / 2);
 }
 
 bool pdhg_steps_fit(const StepBuffers& b) {

@@ -62,6 +62,8 @@ QpEngine::QpEngine(int device) : device_(device) {
   dot_part_.allocate(kQpDotBlocks);
   norms_.allocate(2 * (kQpPowerSteps + 1));
   product_ticket_.allocate(1);
+  room_.allocate(2);
+  for (auto& e : timing_) SGB_CUDA(cudaEventCreate(&e));
   SGB_CUDA(cudaMemset(product_ticket_.ptr, 0, sizeof(unsigned int)));
 }
 
@@ -70,6 +72,9 @@ QpEngine::~QpEngine() {
   destroy_graph();
   if (ctl_host_ != nullptr) cudaFreeHost(ctl_host_);
   if (hist_host_ != nullptr) cudaFreeHost(hist_host_);
+  for (cudaEvent_t e : timing_) {
+    if (e != nullptr) cudaEventDestroy(e);
+  }
   if (stream_ != nullptr) cudaStreamDestroy(stream_);
 }
 
@@ -272,6 +277,7 @@ void QpEngine::layout(int col_lanes, int row_lanes, bool cols_sliced, bool rows_
   steps_ = !resident_ && std::max(m_, n_) > kQpStepItems && cols_sliced &&
            (rows_sliced || m_ == 0) && qp_steps_fit(d);
   resident_smem_ = resident_ ? static_cast<int>(smem) : 0;
+  if (steps_) qp_launch_load_passes(s);
   if (cols_sliced) {
     qp_launch_slice_fill(d, true, col_slices_.idx1.ptr, col_slices_.val1.ptr,
                          col_slices_.idx2.ptr, col_slices_.val2.ptr, s);
@@ -402,17 +408,30 @@ void QpEngine::build_graph(int periods) {
   // A change of the layout has destroyed the graph.
   if (graph_ != nullptr && graph_periods_ == periods && graph_stage_ == stage_) return;
   destroy_graph();
-  const QpDev d = dev();
-  QpCtl* ctl = ctl_.ptr;
   const long long before = qp_kernel_launch_count();
   cudaGraph_t graph = nullptr;
   SGB_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+  enqueue(periods, resident_ || steps_);
+  const cudaError_t end = cudaStreamEndCapture(stream_, &graph);
+  SGB_CUDA(end);
+  const cudaError_t inst = cudaGraphInstantiate(&graph_, graph, 0);
+  cudaGraphDestroy(graph);
+  SGB_CUDA(inst);
+  graph_nodes_ = qp_kernel_launch_count() - before;
+  graph_periods_ = periods;
+  graph_stage_ = stage_;
+}
+
+void QpEngine::enqueue(int periods, bool together) {
+  const QpDev d = dev();
+  QpCtl* ctl = ctl_.ptr;
   for (int p = 0; p < periods; ++p) {
-    if (resident_) {
+    if (together && resident_) {
       qp_launch_resident(d, ctl, p * kQpCheckEvery, kQpCheckEvery, 0, resident_smem_, stream_);
+    } else if (together) {
+      qp_launch_steps(d, ctl, p * kQpCheckEvery, kQpCheckEvery, stream_);
     }
-    if (steps_) qp_launch_steps(d, ctl, p * kQpCheckEvery, kQpCheckEvery, stream_);
-    for (int it = 0; it < kQpCheckEvery && !resident_ && !steps_; ++it) {
+    for (int it = 0; it < kQpCheckEvery && !together; ++it) {
       const int k = p * kQpCheckEvery + it;
       qp_launch_column_pass(d, ctl, kQpStep, k, k & 1, stream_);
       if (m_ > 0) qp_launch_row_pass(d, ctl, kQpStep, k, 0, stream_);
@@ -424,14 +443,6 @@ void QpEngine::build_graph(int periods) {
     qp_launch_decide(d, ctl, last, p, stream_);
   }
   qp_launch_advance(ctl, periods * kQpCheckEvery, stream_);
-  const cudaError_t end = cudaStreamEndCapture(stream_, &graph);
-  SGB_CUDA(end);
-  const cudaError_t inst = cudaGraphInstantiate(&graph_, graph, 0);
-  cudaGraphDestroy(graph);
-  SGB_CUDA(inst);
-  graph_nodes_ = qp_kernel_launch_count() - before;
-  graph_periods_ = periods;
-  graph_stage_ = stage_;
 }
 
 void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* r) {
@@ -471,18 +482,12 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
   periods = std::min(periods, kQpMaxPeriods);
   const long long launches_before = qp_kernel_launch_count();
 
-  cudaEvent_t ev[4];
-  for (auto& e : ev) SGB_CUDA(cudaEventCreate(&e));
-  struct EventGuard {
-    cudaEvent_t* e;
-    ~EventGuard() {
-      for (int k = 0; k < 4; ++k) cudaEventDestroy(e[k]);
-    }
-  } guard{ev};
+  const auto& ev = timing_;
   SGB_CUDA(cudaEventRecord(ev[0], stream_));
 
   // Step sizes (src/qp/qp_condat_vu.cpp:195-208).
   const auto seed = static_cast<unsigned>(p.random_seed);
+  if (steps_) launch_room(room_.ptr, num_sms_, stream_);
   const double norm_a = spectral_norm(seed);
   const double norm_q = hessian_norm(seed);
   const double margin = 1.05;
@@ -510,7 +515,16 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
   SGB_CUDA(cudaMemcpyAsync(ctl_.ptr, &c, sizeof(QpCtl), cudaMemcpyHostToDevice, stream_));
   SGB_CUDA(cudaEventRecord(ev[1], stream_));
   const long long launches_setup = qp_kernel_launch_count() - launches_before;
-  build_graph(periods);
+  // Where other kernels hold SMs the steps run pass by pass, with the same sums, and without a graph, whose
+  // instantiation would wait for those kernels.
+  unsigned long long span[2] = {0, 0};
+  if (steps_) {
+    SGB_CUDA(cudaMemcpyAsync(span, room_.ptr, sizeof(span), cudaMemcpyDeviceToHost, stream_));
+    SGB_CUDA(cudaStreamSynchronize(stream_));
+  }
+  const bool alone = !steps_ || !crowded(span);
+  if (alone) build_graph(periods);
+  long long enqueued = 0;  // kernels outside the graph
 
   int status = SANKHYA_GB300_ITERATION_LIMIT;
   long long base = 0, graphs = 0;
@@ -527,7 +541,14 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
       r->ceiling = ceiling ? 1 : 0;
       break;
     }
-    SGB_CUDA(cudaGraphLaunch(graph_, stream_));
+    if (alone) {
+      SGB_CUDA(cudaGraphLaunch(graph_, stream_));
+    } else {
+      const long long before = qp_kernel_launch_count();
+      enqueue(periods, false);
+      SGB_CUDA(cudaGetLastError());
+      enqueued += qp_kernel_launch_count() - before;
+    }
     ++graphs;
     SGB_CUDA(cudaMemcpyAsync(ctl_host_, ctl_.ptr, sizeof(QpCtl), cudaMemcpyDeviceToHost,
                              stream_));
@@ -584,7 +605,7 @@ void QpEngine::solve(const sankhya_gb300_qp_params& p, sankhya_gb300_qp_result* 
   r->setup_seconds = 1e-3 * ms_setup;
   r->loop_seconds = 1e-3 * ms_loop;
   r->device_seconds = 1e-3 * ms_all;
-  r->kernel_launches = launches_setup + graphs * graph_nodes_ +
+  r->kernel_launches = launches_setup + (alone ? graphs * graph_nodes_ : enqueued) +
                        (qp_kernel_launch_count() - launches_report);
   const char* what = status == SANKHYA_GB300_OPTIMAL      ? "optimal"
                      : status == SANKHYA_GB300_TIME_LIMIT ? "time limit"

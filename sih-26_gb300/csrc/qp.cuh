@@ -139,6 +139,7 @@ long long qp_resident_smem(int m, int n, long long rows_q, long long rows_a, lon
 bool qp_resident_fits(long long smem);
 // Iterations k0 .. k0 + count - 1 of the graph (k0 even: x is in buffer 0) on sliced items in one
 // cooperative launch; qp_steps_fit: whether the device runs its blocks at once.
+void qp_launch_load_passes(cudaStream_t s);  // as launch_load_passes (kernels.cuh)
 void qp_launch_steps(const QpDev& d, QpCtl* ctl, int k0, int count, cudaStream_t s);
 bool qp_steps_fit(const QpDev& d);
 // The decision after the check whose last iteration is graph index k (period p).

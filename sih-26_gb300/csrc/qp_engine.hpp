@@ -32,6 +32,9 @@ class QpEngine {
   QpDev dev() const;
   double spectral_norm(unsigned seed);
   double hessian_norm(unsigned seed);
+  // The kernels of `periods` check periods on the stream. together: their steps in cooperative launches
+  // (or the resident kernel), else pass by pass.
+  void enqueue(int periods, bool together);
   void build_graph(int periods);
   void destroy_graph();
 
@@ -75,6 +78,8 @@ class QpEngine {
   DeviceArray<unsigned int> col_tickets_, row_tickets_;
   DeviceArray<double> long_col_obj_, obj_part_, product_part_, norms_;
   DeviceArray<unsigned int> product_ticket_;
+  DeviceArray<unsigned long long> room_;  // launch_room
+  cudaEvent_t timing_[4] = {};  // kept: making one may wait for the device's other kernels
 
   DeviceArray<QpCtl> ctl_;
   DeviceArray<QpHist> hist_;
