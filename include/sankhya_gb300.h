@@ -328,9 +328,10 @@ SGB_API int sankhya_gb300_batch_ray(sankhya_gb300_batch* batch, int32_t index, d
  * flight (n the largest such min of the batch; fewer LPs are in flight where memory is short; held
  * until a batch without such LPs is loaded or the engine is destroyed); larger ones, and bases that
  * FP32 factors cannot solve, by preconditioned conjugate gradients on the normal equations, with
- * refinement passes. An LP's gradients do not depend on the rest of its batch. info's iterations are the refinement steps or the conjugate-gradient iterations. An equality row's
- * dL/db is dl_drl + dl_dru (only the side its multiplier's sign names is nonzero). Any
- * upstream pointer may be NULL (zero); any output pointer may be NULL. Minimisation and
+ * refinement passes. An LP's gradients do not depend on the rest of its batch. info's iterations
+ * are the refinement steps or the conjugate-gradient iterations. An equality row's dL/db is
+ * dl_drl + dl_dru (only the side its multiplier's sign names is nonzero). Any upstream pointer may
+ * be NULL (zero); any output pointer may be NULL. Minimisation and
  * maximisation LPs alike (the sense is folded as src/pdhg/pdhg.cpp:95-111 folds it). */
 typedef struct sankhya_gb300_adjoint_info {
   int32_t status;      /* 0 ok, 1 degenerate optimum (|B| != |R|), 2 a solve not converged */

@@ -69,10 +69,14 @@ static bool check(const std::vector<int>& want, int n, int bases) {
     for (int k = 0; k < nb; ++k) in_r[r[k]] = in_c[c[k]] = 1;
     std::vector<int> lr, lc;
     for (int i = 0; i < m; ++i) {
-      if (in_r[i]) lr.push_back(static_cast<int>(std::count_if(rows[i].begin(), rows[i].end(), [&](int j) { return in_c[j]; })));
+      if (!in_r[i]) continue;
+      lr.push_back(static_cast<int>(
+          std::count_if(rows[i].begin(), rows[i].end(), [&](int j) { return in_c[j]; })));
     }
     for (int j = 0; j < n; ++j) {
-      if (in_c[j]) lc.push_back(static_cast<int>(std::count_if(cols[j].begin(), cols[j].end(), [&](int i) { return in_r[i]; })));
+      if (!in_c[j]) continue;
+      lc.push_back(static_cast<int>(
+          std::count_if(cols[j].begin(), cols[j].end(), [&](int i) { return in_r[i]; })));
     }
     if (slices_of(lr) > by_row || slices_of(lc) > by_col) {
       std::printf("FAIL %d x %d basis of %d: %lld > %lld or %lld > %lld\n", m, n, nb, slices_of(lr),
